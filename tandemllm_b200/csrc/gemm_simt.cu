@@ -3,7 +3,8 @@
 //
 //   C[m, n] = sum_k A[m, k] * W[n, k] (+ bias[n])            both operands row-major with k contiguous
 //
-// Each output element is accumulated over k = 0..K-1 in ascending order by one thread, so a row's result
+// Each output element is accumulated in an order that depends on k alone (ascending, by one thread; the kernels for
+// 16-byte pieces: four such chains, see there), so a row's result
 // does not depend on how many other rows the call has (the reference's row invariance,
 // engine/models/lfm2_moe/kernels.py:290-306). The same kernel runs the experts: a tile map built on the
 // device (moe_route.cu) names, per row tile, the expert whose weights it multiplies by and the rows of
@@ -237,8 +238,260 @@ __global__ void __launch_bounds__(256) gemm_tall_narrow_kernel(GemmParams p) {
   }
 }
 
+// ---- 32-bit operands whose rows are whole 16-byte pieces ----
+//
+// The kernels above fetch a number at a time, wait for a tile before they multiply it and were what a 32-bit prompt
+// consisted of. These take 16 bytes a load and keep four stages of 32 k-elements in flight (cp.async).
+//
+// CTA: BM rows by 64 outputs (gated: 32 gate rows and the 32 up rows of the same outputs), eight warps that all hold the whole
+// tile and take one of a stage's eight k-quads each; their sums meet in shared memory at the end. What bounds such a
+// kernel is the multiply-adds and what shared memory hands to the registers, 128 bytes a clock: a 16-byte load feeds 16
+// multiply-adds with 8 x 8 outputs a thread, as many as the SM does meanwhile, and a warp on a tile of its own is what
+// makes 8 x 8 possible with tiles small enough to fill the GPU. Measured at 150 rows: 14336 outputs of 2048 in 281 us
+// (31 TFLOP/s), the eleven plain products of a three-layer pass 364 -> 168 us each on average, the experts' gate/up of
+// 600 pairs 1135 -> 448 us. A thread's rows lie 4 and its columns 8 apart, so a quarter of a warp reads one row or eight neighbouring ones:
+// with 36 floats a row the eight meet no bank twice.
+//
+// An output is the sum of eight chains, chain q in ascending order over the quads q, q + 8, ..., added in order: which k
+// a chain has depends on k alone, whatever the tile's height, so a row still does not depend on the others, and eight
+// short chains lose less than one long one.
+constexpr int FK = 32, FPITCH = FK + 4, FSTAGES = 4, FN = 64, FWARPS = 8;
+
+template <int BM_>
+struct F32Tile {
+  static constexpr int TM = BM_ / 4;                                  // outputs a thread: TM x 8
+  static constexpr int STAGE = (BM_ + FN) * FPITCH;                   // floats
+  static constexpr int RED = FWARPS * BM_ * FN;                       // the warps' sums
+  static constexpr int SMEM = (FSTAGES * STAGE > RED ? FSTAGES * STAGE : RED) * 4;
+  static constexpr int LOADS = (BM_ + FN + 31) / 32;                  // 16-byte pieces a thread and stage
+};
+
+__device__ __forceinline__ void cp16(uint32_t dst, const float* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+// two multiply-adds on neighbouring numbers
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float both(unsigned long long v) {
+  return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+
+// `sub`: how many CTA tiles a tile of the plan is cut into (grouped)
+template <int BM_, bool GATED>
+__global__ void __launch_bounds__(256, 2) gemm_f32_kernel(GemmParams p, int sub) {
+  using T = F32Tile<BM_>;
+  constexpr int TM_ = T::TM;
+  extern __shared__ float4 f32_smem[];
+  float* tiles = reinterpret_cast<float*>(f32_smem);
+  int row0 = blockIdx.y * BM_, rows;
+  const float* W = (const float*)p.W;
+  if (p.tile_group) {
+    const int t = blockIdx.y / sub, off = (blockIdx.y - t * sub) * BM_;
+    if (t >= *p.n_tiles) return;
+    rows = min(BM_, p.tile_rows[t] - off);
+    if (rows <= 0) return;
+    row0 = p.tile_row0[t] + off;
+    W += (long long)p.tile_group[t] * p.w_group_stride;
+  } else {
+    rows = min(BM_, p.M - row0);
+  }
+  constexpr int OUTS = GATED ? FN / 2 : FN;          // outputs a CTA
+  const int col0 = blockIdx.x * OUTS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = lane >> 3, tx = lane & 7;
+
+  // what this thread loads: 16 bytes at k offset 4 (tid % 8) of rows tid / 8, + 32, ... of [A tile; W tile]
+  const int lk = (tid & 7) * 4;
+  const float* src[T::LOADS];
+  bool ok[T::LOADS];
+#pragma unroll
+  for (int i = 0; i < T::LOADS; ++i) {
+    const int r = (tid >> 3) + 32 * i;
+    src[i] = W;
+    ok[i] = false;
+    if (r < BM_) {
+      if (r < rows) {
+        const int m = row0 + r;
+        src[i] = (const float*)p.A + (p.a_gather ? (long long)(p.a_gather[m] / p.a_div) : (long long)m) * p.lda;
+        ok[i] = true;
+      }
+    } else if (r < BM_ + FN) {
+      const int j = r - BM_;
+      const int n = col0 + (GATED && j >= OUTS ? j - OUTS : j);
+      if (n < p.N) {
+        src[i] = W + (long long)(GATED && j >= OUTS ? n + p.N : n) * p.ldw;
+        ok[i] = true;
+      }
+    }
+  }
+  const int steps = (p.K + FK - 1) / FK;
+  const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)(((tid >> 3) * FPITCH + lk) * 4);
+  auto load = [&](int step) {
+    if (step < steps) {
+      const int k = step * FK + lk;
+      const uint32_t at = smem0 + (uint32_t)((step % FSTAGES) * T::STAGE * 4);
+#pragma unroll
+      for (int i = 0; i < T::LOADS; ++i)
+        if ((tid >> 3) + 32 * i < BM_ + FN) {
+          const bool in = ok[i] && k < p.K;          // (K is a multiple of 4)
+          cp16(at + (uint32_t)(32 * i * FPITCH * 4), in ? src[i] + k : W, in);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float acc[TM_][8];
+#pragma unroll
+  for (int i = 0; i < TM_; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+
+  for (int s = 0; s < FSTAGES - 1; ++s) load(s);
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
+    __syncthreads();                                  // the stage is here, and everybody is done with the one before
+    load(step + FSTAGES - 1);
+    const float* st = tiles + (step % FSTAGES) * T::STAGE + warp * 4;
+    const float* a_at = st + ty * FPITCH, * w_at = st + (BM_ + tx) * FPITCH;
+    float4 w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(w_at + j * 8 * FPITCH);
+#pragma unroll
+    for (int m = 0; m < TM_; ++m) {
+      const float4 a = *reinterpret_cast<const float4*>(a_at + m * 4 * FPITCH);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        acc[m][j] = fmaf(a.x, w[j].x, acc[m][j]);
+        acc[m][j] = fmaf(a.y, w[j].y, acc[m][j]);
+        acc[m][j] = fmaf(a.z, w[j].z, acc[m][j]);
+        acc[m][j] = fmaf(a.w, w[j].w, acc[m][j]);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  float* red = tiles;                                // [warps][8 TM][32]
+#pragma unroll
+  for (int m = 0; m < TM_; ++m)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[((warp * TM_ + m) * 8 + j) * 32 + lane] = acc[m][j];
+  __syncthreads();
+  auto sum = [&](int m, int j) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < FWARPS; ++w) v += red[((w * TM_ + m) * 8 + j) * 32 + lane];
+    return v;
+  };
+  float* C = (float*)p.C;
+  // a warp stores column block `warp` (gated: rows of either parity of the outputs' block warp % 4)
+#pragma unroll
+  for (int i = 0; i < (GATED ? TM_ / 2 : TM_); ++i) {
+    const int m = GATED ? 2 * i + (warp >> 2) : i;
+    const int j = GATED ? warp & 3 : warp;
+    const int lr = ty + 4 * m, n = col0 + tx + 8 * j;
+    const float v = sum(m, j), u = GATED ? sum(m, j + 4) : 0.f;
+    if (lr >= rows || n >= p.N) continue;
+    const long long r = row0 + lr;
+    if constexpr (GATED) {
+      const float rw = pair_weight(p.pair_weight, p.weight_index, r);
+      C[r * p.ldc + n] = gated(rw * v, rw * u, p.swiglu, p.ga0, p.ga1);
+    } else {
+      const float x = v + (p.bias ? p.bias[n] : 0.f);
+      C[r * p.ldc + n] = p.swiglu < 0 ? gate_activation(x, -p.swiglu) : x;
+    }
+  }
+}
+
+// Up to 8 rows: bound by the weights' bytes. A warp takes two outputs, each lane 16 bytes of either weight row, four k-steps in
+// flight. Four chains a lane and row (one a component), then the lanes. The head of one row (65536 x 2048, 537 MB):
+// 231 -> 78 us, 6.9 TB/s.
+template <int MAXM>
+__global__ void __launch_bounds__(256) gemm_f32_few_kernel(GemmParams p) {
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int n0 = 2 * warp;
+  if (n0 >= p.N) return;
+  const float* A = (const float*)p.A;
+  const float* w0 = (const float*)p.W + (long long)n0 * p.ldw;
+  const float* w1 = n0 + 1 < p.N ? w0 + p.ldw : w0;
+  unsigned long long acc[MAXM][2][2];
+#pragma unroll
+  for (int m = 0; m < MAXM; ++m) acc[m][0][0] = acc[m][0][1] = acc[m][1][0] = acc[m][1][1] = 0ull;
+  constexpr int U = 4;
+  for (int k0 = lane * 4; k0 < p.K; k0 += 128 * U) {
+    ulonglong2 a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + 128 * u;
+      a[u] = b[u] = make_ulonglong2(0ull, 0ull);
+      if (k < p.K) {
+        a[u] = *reinterpret_cast<const ulonglong2*>(w0 + k);
+        b[u] = *reinterpret_cast<const ulonglong2*>(w1 + k);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + 128 * u;
+      if (k >= p.K) break;
+#pragma unroll
+      for (int m = 0; m < MAXM; ++m) {
+        if (m >= p.M) break;
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(A + (long long)m * p.lda + k);
+        fma2(acc[m][0][0], x.x, a[u].x);
+        fma2(acc[m][0][1], x.y, a[u].y);
+        fma2(acc[m][1][0], x.x, b[u].x);
+        fma2(acc[m][1][1], x.y, b[u].y);
+      }
+    }
+  }
+  float* C = (float*)p.C;
+#pragma unroll
+  for (int m = 0; m < MAXM; ++m) {
+    if (m >= p.M) break;
+    const float v0 = warp_sum(both(acc[m][0][0]) + both(acc[m][0][1])), v1 = warp_sum(both(acc[m][1][0]) + both(acc[m][1][1]));
+    if (lane < 2 && n0 + lane < p.N)
+      C[(long long)m * p.ldc + n0 + lane] = (lane ? v1 : v0) + (p.bias ? p.bias[n0 + lane] : 0.f);
+  }
+}
+
+template <int BM_, bool GATED>
+static int launch_f32(const GemmParams& p, int max_tiles, cudaStream_t stream) {
+  const int sub = p.tile_group ? BM / BM_ : 1;       // (a plan's tiles hold at most BM rows)
+  auto kernel = gemm_f32_kernel<BM_, GATED>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BM_>::SMEM);
+  if (e != cudaSuccess) return (int)e;
+  const unsigned y = p.tile_group ? (unsigned)(max_tiles * sub) : (unsigned)ceil_div(p.M, BM_);
+  kernel<<<dim3(ceil_div(p.N, GATED ? FN / 2 : FN), y), 256, F32Tile<BM_>::SMEM, stream>>>(p, sub);
+  return 0;
+}
+
+// Whether the 16-byte kernels take these operands: rows that are whole pieces, a grid within its limit, and not one of the
+// narrow products (a router's), which have kernels of their own.
+static bool f32_pieces(const GemmParams& p, int max_tiles) {
+  if (p.K % 4 || p.lda % 4 || p.ldw % 4 || p.w_group_stride % 4 || ((uintptr_t)p.A & 15) || ((uintptr_t)p.W & 15)) return false;
+  if (p.tile_group) return (long long)max_tiles * (BM / 16) <= 65535;
+  return p.N > 64 && ceil_div(p.M, 16) <= 65535 && (p.M > 8 || p.N > 512 || p.K < 512);
+}
+
+static int launch_f32_any(const GemmParams& p, int max_tiles, cudaStream_t stream) {
+  if (!p.tile_group && p.M <= 8) {
+    const int blocks = ceil_div(p.N, 16);
+    if (p.M == 1) gemm_f32_few_kernel<1><<<blocks, 256, 0, stream>>>(p);
+    else if (p.M <= 4) gemm_f32_few_kernel<4><<<blocks, 256, 0, stream>>>(p);
+    else gemm_f32_few_kernel<8><<<blocks, 256, 0, stream>>>(p);
+    return 0;
+  }
+  // tiles of 16 rows for what fits one; grouped, where an expert has as few on average (max_tiles: the experts or more)
+  const bool low = p.tile_group ? p.M <= 10 * max_tiles : p.M <= 16;
+  if (p.swiglu > 0) return low ? launch_f32<16, true>(p, max_tiles, stream) : launch_f32<32, true>(p, max_tiles, stream);
+  return low ? launch_f32<16, false>(p, max_tiles, stream) : launch_f32<32, false>(p, max_tiles, stream);
+}
+
 template <typename TIn, typename TOut>
 static int launch(const GemmParams& p, int max_tiles, cudaStream_t stream) {
+  if constexpr (sizeof(TIn) == 4) {
+    if (f32_pieces(p, max_tiles)) return launch_f32_any(p, max_tiles, stream);
+  }
   if (!p.tile_group && !p.swiglu && p.N <= 64 && p.M > 64) {
     gemm_tall_narrow_kernel<TIn, TOut><<<ceil_div(p.M, 16), 256, 0, stream>>>(p);
     return 0;
@@ -275,10 +528,12 @@ extern "C" int tl_gemm_simt(const void* A, long long lda, const void* W, long lo
   GemmParams p = {};
   p.A = A; p.W = W; p.bias = bias; p.C = C; p.lda = lda; p.ldw = ldw; p.ldc = ldc;
   p.M = M; p.N = N; p.K = K; p.a_div = 1;
-  if (in_dtype == TL_FP32 && out_dtype == TL_FP32) launch<float, float>(p, 0, stream);
-  else if (in_dtype == TL_BF16 && out_dtype == TL_BF16) launch<bf16, bf16>(p, 0, stream);
-  else if (in_dtype == TL_BF16 && out_dtype == TL_FP32) launch<bf16, float>(p, 0, stream);
+  int e = 0;
+  if (in_dtype == TL_FP32 && out_dtype == TL_FP32) e = launch<float, float>(p, 0, stream);
+  else if (in_dtype == TL_BF16 && out_dtype == TL_BF16) e = launch<bf16, bf16>(p, 0, stream);
+  else if (in_dtype == TL_BF16 && out_dtype == TL_FP32) e = launch<bf16, float>(p, 0, stream);
   else TL_REQUIRE(false, "gemm: input dtype %d with output dtype %d is not implemented", in_dtype, out_dtype);
+  if (e) return e;
   TL_LAUNCH_CHECK();
   return 0;
 }
@@ -302,10 +557,12 @@ extern "C" int tl_gemm_simt_grouped(const void* A, long long lda, const int* a_g
   p.tile_group = tile_group; p.tile_row0 = tile_row0; p.tile_rows = tile_rows; p.n_tiles = n_tiles;
   p.a_gather = a_gather; p.a_div = a_div; p.swiglu = swiglu; p.pair_weight = row_weight; p.weight_index = weight_index;
   p.ga0 = tl_gate_constants[0]; p.ga1 = tl_gate_constants[1];
-  if (in_dtype == TL_FP32 && out_dtype == TL_FP32) launch<float, float>(p, max_tiles, stream);
-  else if (in_dtype == TL_BF16 && out_dtype == TL_BF16) launch<bf16, bf16>(p, max_tiles, stream);
-  else if (in_dtype == TL_BF16 && out_dtype == TL_FP32) launch<bf16, float>(p, max_tiles, stream);
+  int e = 0;
+  if (in_dtype == TL_FP32 && out_dtype == TL_FP32) e = launch<float, float>(p, max_tiles, stream);
+  else if (in_dtype == TL_BF16 && out_dtype == TL_BF16) e = launch<bf16, bf16>(p, max_tiles, stream);
+  else if (in_dtype == TL_BF16 && out_dtype == TL_FP32) e = launch<bf16, float>(p, max_tiles, stream);
   else TL_REQUIRE(false, "grouped gemm: input dtype %d with output dtype %d is not implemented", in_dtype, out_dtype);
+  if (e) return e;
   TL_LAUNCH_CHECK();
   return 0;
 }

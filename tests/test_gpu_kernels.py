@@ -406,6 +406,38 @@ def test_gemm_row_does_not_depend_on_the_other_rows():
     assert torch.equal(big[60:75], small)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 514, 4), (1, 70, 516), (3, 515, 132), (8, 1030, 520), (9, 65, 4), (16, 129, 36), (17, 66, 100),
+                                   (33, 130, 2048), (65, 192, 260), (600, 2048, 68), (64, 2049, 128)])
+def test_gemm_simt_in_16_byte_pieces(M, N, K):
+    """The 32-bit kernels for rows of whole 16-byte pieces, at the edges of their tiles (16 and 32 rows, 64 outputs, 32
+    k-elements, 4 stages), against 64-bit: chains of at most K / 4 products (and 8 sums of chains) are off by at most
+    K / 4 + 8 roundings of the sum of absolute values. And a row alone, or among fewer, has the same bits wherever both
+    calls take the tiled kernel (more than 8 rows)."""
+    o = ops()
+    x, w, b = rnd(M, K, seed=6), rnd(N, K, seed=7), rnd(N, seed=8)
+    out = o.gemm_simt(x.to(DEV), w.to(DEV), b.to(DEV), torch.empty(M, N, device=DEV)).cpu()
+    want, size = x.double() @ w.double().T + b.double(), x.abs().double() @ w.abs().double().T + b.abs().double()
+    assert ((out.double() - want).abs() <= (K / 4 + 8) * 2.0 ** -24 * size).all()
+    if M > 9:
+        few = o.gemm_simt(x[M - 9:].to(DEV), w.to(DEV), b.to(DEV), torch.empty(9, N, device=DEV)).cpu()
+        assert torch.equal(few, out[M - 9:])
+
+
+@pytest.mark.parametrize("R,E,k,H,I", [(3, 8, 2, 64, 68), (40, 3, 2, 36, 132), (200, 4, 2, 100, 64), (130, 2, 1, 32, 40)])
+@pytest.mark.parametrize("act", [1, 0, -3])
+def test_grouped_gemm_in_16_byte_pieces(R, E, k, H, I, act):
+    """The routed products in 32-bit where a plan's tile of up to 64 rows is cut into the kernel's own (16 or 32 rows)."""
+    o = ops()
+    x, ids = rnd(R, H, seed=3), torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(i))[:k] for i in range(R)]).int()
+    w = rnd(E, I * (2 if act > 0 else 1), H, seed=4, scale=0.2)
+    plan = o.MoePlan(R * k, E, o.simt_tile_rows(), DEV).build(ids.to(DEV))
+    out = o.gemm_simt_grouped(x.to(DEV), plan.sorted_pairs, k, w.to(DEV), torch.empty(R * k, I, device=DEV), plan, act)
+    z = torch.einsum("rkh,rknh->rkn", x.double()[:, None].expand(-1, k, -1), w.double()[ids.long()]).flatten(0, 1)
+    want = (torch.nn.functional.silu(z[:, :I]) * z[:, I:] if act > 0 else z.clamp(min=0) ** 2 if act < 0 else z)
+    got = out.cpu()[plan.pos_of_pair[:R * k].cpu().long()]
+    close(got, want.float(), torch.float32, f"{act}")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("R,E,k,H,I", [(5, 4, 2, 48, 40), (70, 6, 3, 96, 72), (300, 40, 4, 64, 24), (1, 8, 8, 32, 16)])
 def test_router_plan_experts_and_combine(dtype, R, E, k, H, I):
