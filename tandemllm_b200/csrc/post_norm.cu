@@ -33,11 +33,182 @@ struct PostNormParams {
   float pre_eps;
   void* normed;
   const int* gather;
-  int few_rows;              // a step of few rows (few blocks): the form whose loads of a source are all in flight together
+  const void* gate_x;        // or the gate's rows and its vector: logit = gate_x[r] . gate_w (delta_gate is then nullptr)
+  const void* gate_w;
+  long long gate_ld;
+  int gate_bf16;
 };
 
-// FEW: the form for a step of few rows (see `few_rows`), a kernel of its own so that the other keeps its few registers.
-template <typename T, bool FEW>
+// Rows whose length is a multiple of four, VPT 16-byte pieces a thread, held in registers from the first load to the last store.
+// A decode step has a block or a few and their time is the chain of round trips, so what does not depend on another load (the
+// residual, both norms' weights, the gate's row and vector, the dense parts) is asked for before the experts' rows, which are asked
+// for four slots at a time; every warp orders the row's slots itself and no barrier stands in front of them. The gate's logit is
+// taken here because a kernel of its own cost 5.5 us and a launch for one number a row. Measured at two rows of 2048 in a decode
+// step, six slots beside a shared part in ten partial sums: 13.8 us with a number a load, 4.5 us here (with the gate's logit); 1000
+// rows 30.9 and 19.8 us.
+template <typename T, int VPT>
+__global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) add_normed_vec_kernel(PostNormParams p) {
+  __shared__ float red[96];
+  const int hidden = p.hidden, lane = threadIdx.x & 31;
+  const int r = p.gather ? p.gather[blockIdx.x] : (int)blockIdx.x;
+  // the row's slots in ascending expert id (the slot index breaks ties)
+  int slot_src = 0, rank = -1;
+  float slot_w = 0.f;
+  if (p.expert_rows) {
+    const int k = p.top_k, j = lane;
+    const bool mine = j < k;
+    const int e = mine ? p.ids[(long long)r * k + j] : 0x7fffffff;
+    slot_src = mine ? p.pos_of_pair[(long long)r * k + j] : 0;
+    slot_w = mine ? (p.wts ? p.wts[(long long)r * k + j] : 1.f) : 0.f;
+    int before = 0;
+    for (int i = 0; i < k; ++i) {
+      const int ei = __shfl_sync(0xffffffffu, e, i);
+      before += (ei < e) || (ei == e && i < j);
+    }
+    if (mine) rank = before;
+  }
+  float* res = p.residual + (size_t)r * hidden;
+  float4 d[VPT], x[VPT], w[VPT], pw[VPT];
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    const int c = (threadIdx.x + v * blockDim.x) * 4;
+    d[v] = x[v] = w[v] = pw[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < hidden) {
+      x[v] = load4_now(res + c);
+      w[v] = load4_now(p.weight + c);
+      if (p.pre_weight) pw[v] = load4_now(p.pre_weight + c);
+    }
+  }
+  float g = 1.f;
+  if (p.gate_x) {
+    float dot = 0.f;
+    if (p.gate_bf16) {
+      const bf16* gx = reinterpret_cast<const bf16*>(p.gate_x) + (long long)r * p.gate_ld;
+      const bf16* gw = reinterpret_cast<const bf16*>(p.gate_w);
+#pragma unroll
+      for (int v = 0; v < VPT; ++v) {
+        const int c = (threadIdx.x + v * blockDim.x) * 4;
+        if (c < hidden) {
+          const uint2 a = *reinterpret_cast<const uint2*>(gx + c), b = *reinterpret_cast<const uint2*>(gw + c);
+          const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.x));
+          const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.y));
+          const float2 b0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.x));
+          const float2 b1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.y));
+          dot = dot4(make_float4(a0.x, a0.y, a1.x, a1.y), make_float4(b0.x, b0.y, b1.x, b1.y), dot);
+        }
+      }
+    } else {
+      const float* gx = reinterpret_cast<const float*>(p.gate_x) + (long long)r * p.gate_ld;
+      const float* gw = reinterpret_cast<const float*>(p.gate_w);
+#pragma unroll
+      for (int v = 0; v < VPT; ++v) {
+        const int c = (threadIdx.x + v * blockDim.x) * 4;
+        if (c < hidden) dot = dot4(load4_now(gx + c), load4_now(gw + c), dot);
+      }
+    }
+    g = 1.f / (1.f + expf(-block_sum_once(dot, red + 64)));
+  } else if (p.delta_gate) {
+    g = 1.f / (1.f + expf(-p.delta_gate[r]));
+  }
+  constexpr int AT_ONCE = VPT == 1 ? 4 : VPT == 2 ? 2 : 1;
+  if (p.delta) {
+    const float* src = p.delta + (size_t)r * hidden;
+    for (int s0 = 0; s0 < p.parts; s0 += AT_ONCE) {
+      float4 y[AT_ONCE][VPT];
+#pragma unroll
+      for (int s = 0; s < AT_ONCE; ++s)
+#pragma unroll
+        for (int v = 0; v < VPT; ++v) {
+          const int c = (threadIdx.x + v * blockDim.x) * 4;
+          if (s0 + s < p.parts && c < hidden) y[s][v] = load4_now(src + (long long)(s0 + s) * p.part_stride + c);
+          else y[s][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+      for (int s = 0; s < AT_ONCE; ++s)
+        if (s0 + s < p.parts)
+#pragma unroll
+          for (int v = 0; v < VPT; ++v) add4(d[v], y[s][v]);
+    }
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) { d[v].x *= g; d[v].y *= g; d[v].z *= g; d[v].w *= g; }
+  }
+  if (p.expert_rows) {
+    float4 routed[VPT];
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) routed[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j0 = 0; j0 < p.top_k; j0 += AT_ONCE) {
+      float4 y[AT_ONCE][VPT];
+      float ws[AT_ONCE];
+      const float* from[AT_ONCE];
+#pragma unroll
+      for (int j = 0; j < AT_ONCE; ++j) {
+        const unsigned who = __ballot_sync(0xffffffffu, rank == j0 + j);
+        const int at = who ? __ffs(who) - 1 : 0;
+        ws[j] = __shfl_sync(0xffffffffu, slot_w, at);
+        from[j] = p.expert_rows + (long long)__shfl_sync(0xffffffffu, slot_src, at) * hidden;
+#pragma unroll
+        for (int v = 0; v < VPT; ++v) y[j][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      for (int s = 0; s < p.expert_parts; ++s) {
+        float4 t[AT_ONCE][VPT];
+#pragma unroll
+        for (int j = 0; j < AT_ONCE; ++j)
+#pragma unroll
+          for (int v = 0; v < VPT; ++v) {
+            const int c = (threadIdx.x + v * blockDim.x) * 4;
+            if (j0 + j < p.top_k && c < hidden) t[j][v] = load4_now(from[j] + (long long)s * p.expert_part_stride + c);
+            else t[j][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+        for (int j = 0; j < AT_ONCE; ++j)
+#pragma unroll
+          for (int v = 0; v < VPT; ++v) add4(y[j][v], t[j][v]);
+      }
+#pragma unroll
+      for (int j = 0; j < AT_ONCE; ++j)
+        if (j0 + j < p.top_k)
+#pragma unroll
+          for (int v = 0; v < VPT; ++v) {
+            routed[v].x = fmaf(ws[j], y[j][v].x, routed[v].x);
+            routed[v].y = fmaf(ws[j], y[j][v].y, routed[v].y);
+            routed[v].z = fmaf(ws[j], y[j][v].z, routed[v].z);
+            routed[v].w = fmaf(ws[j], y[j][v].w, routed[v].w);
+          }
+    }
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) {
+      add4(routed[v], d[v]);
+      d[v] = routed[v];
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) ss = dot4(d[v], d[v], ss);
+  const float inv = rsqrtf(block_sum_once(ss, red) / (float)hidden + p.eps);
+  float ss2 = 0.f;
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    const int c = (threadIdx.x + v * blockDim.x) * 4;
+    x[v].x += d[v].x * inv * w[v].x;
+    x[v].y += d[v].y * inv * w[v].y;
+    x[v].z += d[v].z * inv * w[v].z;
+    x[v].w += d[v].w * inv * w[v].w;
+    if (!p.gather && c < hidden) store4(res + c, x[v].x, x[v].y, x[v].z, x[v].w);
+    ss2 = dot4(x[v], x[v], ss2);
+  }
+  if (!p.pre_weight) return;
+  const float inv2 = rsqrtf(block_sum_once(ss2, red + 32) / (float)hidden + p.pre_eps);
+  T* out = reinterpret_cast<T*>(p.normed) + (size_t)blockIdx.x * hidden;
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    const int c = (threadIdx.x + v * blockDim.x) * 4;
+    if (c < hidden)
+      store4(out + c, x[v].x * inv2 * pw[v].x, x[v].y * inv2 * pw[v].y, x[v].z * inv2 * pw[v].z, x[v].w * inv2 * pw[v].w);
+  }
+}
+
+// Rows of any other length, or that do not begin at 16 bytes: a number a load, the row in shared memory.
+template <typename T>
 __global__ void __launch_bounds__(256) add_normed_kernel(PostNormParams p) {
   extern __shared__ __align__(16) float row[];          // hidden floats, then 33 for the reductions
   float* scratch = row + p.hidden;
@@ -67,53 +238,6 @@ __global__ void __launch_bounds__(256) add_normed_kernel(PostNormParams p) {
   }
   const float g = p.delta_gate ? 1.f / (1.f + expf(-p.delta_gate[r])) : 1.f;
   float ss = 0.f;
-  constexpr int CPT = 16;           // columns a thread holds in registers in the form for rows of up to 16 x 256 numbers
-  if (FEW && hidden <= CPT * (int)blockDim.x) {
-    // Source by source, a thread's loads of one source all sent before the first is used: a decode step has a handful of
-    // blocks, and their time is the chain of round trips to L2, one a source instead of one a source and column.
-    float d[CPT], routed[CPT];
-#pragma unroll
-    for (int i = 0; i < CPT; ++i) d[i] = routed[i] = 0.f;
-    if (p.delta) {
-      for (int s = 0; s < p.parts; ++s) {
-        const float* src = p.delta + (long long)s * p.part_stride + (size_t)r * hidden;
-#pragma unroll
-        for (int i = 0; i < CPT; ++i) {
-          const int c = threadIdx.x + i * blockDim.x;
-          if (c < hidden) d[i] += src[c];
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < CPT; ++i) d[i] *= g;
-    }
-    if (p.expert_rows) {
-      for (int j = 0; j < p.top_k; ++j) {
-        float v[CPT];
-#pragma unroll
-        for (int i = 0; i < CPT; ++i) v[i] = 0.f;
-        for (int s = 0; s < p.expert_parts; ++s) {
-          const float* src = p.expert_rows + (long long)s * p.expert_part_stride + (long long)s_src[j] * hidden;
-#pragma unroll
-          for (int i = 0; i < CPT; ++i) {
-            const int c = threadIdx.x + i * blockDim.x;
-            if (c < hidden) v[i] += src[c];
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < CPT; ++i) routed[i] = fmaf(s_w[j], v[i], routed[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < CPT; ++i) d[i] = routed[i] + d[i];
-    }
-#pragma unroll
-    for (int i = 0; i < CPT; ++i) {
-      const int c = threadIdx.x + i * blockDim.x;
-      if (c < hidden) {
-        row[c] = d[i];
-        ss += d[i] * d[i];
-      }
-    }
-  } else
   for (int c = threadIdx.x; c < hidden; c += blockDim.x) {
     float d = 0.f;
     if (p.delta) {
@@ -230,11 +354,20 @@ __global__ void add_vector_kernel(float* __restrict__ residual, const float* __r
 
 using namespace tl;
 
+// Whether everything add_normed_vec_kernel reads and writes begins at 16 bytes, row by row.
+static bool add_normed_aligned(const PostNormParams& p) {
+  const uintptr_t all = (uintptr_t)p.residual | (uintptr_t)p.delta | (uintptr_t)p.expert_rows | (uintptr_t)p.weight |
+                        (uintptr_t)p.pre_weight | (uintptr_t)p.normed | (uintptr_t)p.gate_x | (uintptr_t)p.gate_w;
+  return (all & 15) == 0 && (!p.delta || p.parts <= 1 || p.part_stride % 4 == 0) &&
+         (!p.expert_rows || p.expert_parts <= 1 || p.expert_part_stride % 4 == 0) && (!p.gate_x || p.gate_ld % 4 == 0);
+}
+
 extern "C" int tl_add_normed(float* residual, const float* delta, int parts, long long part_stride, const float* delta_gate,
                              const float* expert_rows, int expert_parts, long long expert_part_stride, const int* pos_of_pair,
                              const int* ids, const float* wts, int top_k, const float* weight, float eps,
-                             const float* pre_weight, float pre_eps, void* normed, const int* gather, int rows, int hidden,
-                             int dtype, cudaStream_t stream) {
+                             const float* pre_weight, float pre_eps, void* normed, const int* gather, const void* gate_x,
+                             long long gate_ld, const void* gate_w, int gate_dtype, int rows, int hidden, int dtype,
+                             cudaStream_t stream) {
   if (rows == 0) return 0;
   TL_REQUIRE(rows > 0 && hidden > 0 && hidden <= 16384, "add_normed: %d rows of %d", rows, hidden);
   TL_REQUIRE(residual && weight && (delta || expert_rows), "add_normed: a residual, a weight and a branch output are needed");
@@ -248,21 +381,31 @@ extern "C" int tl_add_normed(float* residual, const float* delta, int parts, lon
   p.expert_rows = expert_rows; p.expert_parts = expert_parts; p.expert_part_stride = expert_part_stride;
   p.pos_of_pair = pos_of_pair; p.ids = ids; p.wts = wts; p.top_k = top_k; p.weight = weight; p.eps = eps; p.hidden = hidden;
   p.pre_weight = pre_weight; p.pre_eps = pre_eps; p.normed = normed; p.gather = gather;
-  p.few_rows = rows <= 2 * sm_count() ? 1 : 0;
+  p.gate_x = gate_x; p.gate_w = gate_w; p.gate_ld = gate_ld; p.gate_bf16 = gate_dtype == TL_BF16;
+  if (hidden % 4 == 0 && hidden <= 8192 && add_normed_aligned(p)) {
+    const int pieces = hidden / 4, threads = pieces >= 512 ? 512 : ceil_div(pieces, 32) * 32, vpt = ceil_div(pieces, threads);
+#define TL_ADD_NORMED_VEC(V_)                                                                     \
+  do {                                                                                            \
+    if (dtype == TL_FP32) add_normed_vec_kernel<float, V_><<<rows, threads, 0, stream>>>(p);      \
+    else add_normed_vec_kernel<bf16, V_><<<rows, threads, 0, stream>>>(p);                        \
+  } while (0)
+    if (vpt == 1) TL_ADD_NORMED_VEC(1);
+    else if (vpt == 2) TL_ADD_NORMED_VEC(2);
+    else TL_ADD_NORMED_VEC(4);
+#undef TL_ADD_NORMED_VEC
+    TL_LAUNCH_CHECK();
+    return 0;
+  }
+  TL_REQUIRE(!gate_x, "add_normed: rows of %d that are not laid out for 16-byte loads take the gate's logits, not its rows", hidden);
   const size_t smem = (size_t)(hidden + 33) * sizeof(float);
-#define TL_ADD_NORMED(T_, FEW_)                                                                                         \
+#define TL_ADD_NORMED(T_)                                                                                               \
   do {                                                                                                                  \
     if (smem > 48 * 1024)                                                                                               \
-      cudaFuncSetAttribute(add_normed_kernel<T_, FEW_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
-    add_normed_kernel<T_, FEW_><<<rows, 256, smem, stream>>>(p);                                                        \
+      cudaFuncSetAttribute(add_normed_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);              \
+    add_normed_kernel<T_><<<rows, 256, smem, stream>>>(p);                                                              \
   } while (0)
-  if (dtype == TL_FP32) {
-    if (p.few_rows) TL_ADD_NORMED(float, true);
-    else TL_ADD_NORMED(float, false);
-  } else {
-    if (p.few_rows) TL_ADD_NORMED(bf16, true);
-    else TL_ADD_NORMED(bf16, false);
-  }
+  if (dtype == TL_FP32) TL_ADD_NORMED(float);
+  else TL_ADD_NORMED(bf16);
 #undef TL_ADD_NORMED
   TL_LAUNCH_CHECK();
   return 0;

@@ -120,7 +120,8 @@ _SIGNATURES = {
     "tl_moe_combine": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "tl_argmax": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p],
     "tl_add_normed": [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_void_p,
-                      c_int, c_void_p, c_float, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+                      c_int, c_void_p, c_float, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int,
+                      c_int, c_int, c_int, c_void_p],
     "tl_add_vector": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "tl_row_dot": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "tl_causal_conv_act": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -300,9 +301,19 @@ class ExpertRows:
         return out
 
 
+class RowDot:
+    """One number a row, x[r] . w, that has not been computed yet (the logit of a gate a row): the kernel that uses it takes it."""
+
+    def __init__(self, x: torch.Tensor, w: torch.Tensor):
+        self.x, self.w = x, w
+
+    def materialize(self) -> torch.Tensor:
+        return row_dot(self.x, self.w, torch.empty(self.x.shape[0], 1, dtype=torch.float32, device=self.x.device))
+
+
 class GatedSum:
     """A branch output in three pieces: dense [rows, hidden] (a tensor or `PartialSums`) times sigmoid(gate[r]) (float32
-    [rows, 1] logits; None: no gate), plus the weighed rows of `experts` (`ExpertRows` or None)."""
+    [rows, 1] logits or a `RowDot`; None: no gate), plus the weighed rows of `experts` (`ExpertRows` or None)."""
 
     def __init__(self, dense, gate: torch.Tensor | None, experts: "ExpertRows | None"):
         self.dense, self.gate, self.experts = dense, gate, experts
@@ -310,7 +321,8 @@ class GatedSum:
     def materialize(self) -> torch.Tensor:
         total = materialize(self.dense).float()
         if self.gate is not None:
-            total = total * torch.sigmoid(self.gate.view(-1, 1))
+            gate = self.gate.materialize() if isinstance(self.gate, RowDot) else self.gate
+            total = total * torch.sigmoid(gate.view(-1, 1))
         return total if self.experts is None else total + self.experts.materialize()
 
 
@@ -529,10 +541,10 @@ def add_layernorm(residual: torch.Tensor, delta, weight: torch.Tensor, bias: tor
     return out
 
 
-def add_normed(residual: torch.Tensor, delta, weight: torch.Tensor, eps: float, gate: torch.Tensor | None = None,
+def add_normed(residual: torch.Tensor, delta, weight: torch.Tensor, eps: float, gate: "torch.Tensor | RowDot | None" = None,
                experts: "ExpertRows | None" = None, then: tuple | None = None) -> torch.Tensor | None:
     """The norm behind a branch, fused with the residual add: d = delta (None, a float32 tensor or `PartialSums`), times
-    sigmoid(gate[r]) where `gate` (float32 [rows] logits) is given, plus the weighed rows of `experts`;
+    sigmoid(gate[r]) where `gate` (float32 [rows] logits, or a `RowDot` whose number the kernel takes itself) is given, plus the weighed rows of `experts`;
     residual += weight * d / rms(d). `then` = (next norm's weight, its eps, out, gather or None): the kernel also writes
     the next norm's rows of the new residual into `out` (with `gather`, only of those rows, whose residual then stays as it
     was); returns `out` or None."""
@@ -554,14 +566,24 @@ def add_normed(residual: torch.Tensor, delta, weight: torch.Tensor, eps: float, 
         rows_ptr, pos, ids, wts, top_k = experts.rows, experts.pos_of_pair, experts.ids, experts.wts, experts.ids.shape[1]
         if experts.parts > 1:
             eparts, estride = experts.parts, experts.rows.shape[1] * experts.rows.shape[2]
-    if gate is not None:
-        _need(gate, torch.float32, "gate logits")
     hidden = residual.shape[-1]
     pre_w, pre_eps, out, gather = then if then is not None else (None, 0.0, None, None)
     rows = residual.shape[0] if gather is None else out.shape[0]
+    gate_x = gate_w = None
+    gate_ld, gate_dtype = 0, FP32
+    if isinstance(gate, RowDot):
+        x, w = gate.x, gate.w
+        at = [ptr(t) for t in (residual, weight, pre_w, out, rows_ptr, x, w) if t is not None] + [dense or 0]
+        if (hidden % 4 or hidden > 8192 or x.shape[1] != hidden or w.numel() != hidden or x.dtype != w.dtype or x.stride(1) != 1
+                or x.stride(0) % 4 or not w.is_contiguous() or any(a % 16 for a in at)):
+            gate = gate.materialize()           # what the kernel's form for 16-byte loads does not take
+        else:
+            gate_x, gate_w, gate_ld, gate_dtype, gate = ptr(x), ptr(w), x.stride(0), dtype_code(x.dtype), None
+    if gate is not None:
+        _need(gate, torch.float32, "gate logits")
     check(core().tl_add_normed(ptr(residual), dense, parts, stride, ptr(gate), ptr(rows_ptr), eparts, estride, ptr(pos), ptr(ids),
                                ptr(wts), top_k, ptr(weight), float(eps), ptr(pre_w), float(pre_eps), ptr(out), ptr(gather),
-                               rows, hidden, dtype_code(out.dtype) if out is not None else FP32, stream()), "add_normed")
+                               gate_x, gate_ld, gate_w, gate_dtype, rows, hidden, dtype_code(out.dtype) if out is not None else FP32, stream()), "add_normed")
     return out
 
 

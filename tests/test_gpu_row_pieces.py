@@ -39,3 +39,30 @@ def test_layer_norm_of_partial_sums(dtype, width, parts):
     some = torch.empty(2, width, dtype=DT[dtype], device=DEV)
     ops.add_layernorm(r, None, w.to(DEV), b.to(DEV), 1e-5, some, torch.tensor([4, 0], dtype=torch.int32, device=DEV))
     assert torch.equal(some, out[[4, 0]])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width,top,parts", [(4, 1, 1), (132, 5, 3), (2048, 6, 10), (2052, 4, 2), (4096, 9, 1), (8192, 2, 3), (8196, 3, 2),
+                                             (2050, 3, 2)])
+def test_norm_behind_a_branch_with_a_gate_that_is_not_computed_yet(dtype, width, top, parts):
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(width + top)
+    R = 3
+    res, sums = draw(g, R, width), draw(g, parts, R, width)
+    w, w2 = 1 + draw(g, width, scale=0.2), 1 + draw(g, width, scale=0.2)
+    x, wg = draw(g, R, width, dtype=DT[dtype]), draw(g, 1, width, scale=2.0 / width ** 0.5, dtype=DT[dtype])
+    rows = draw(g, 2, R * top, width)
+    ids = torch.stack([torch.randperm(40, generator=g)[:top] for _ in range(R)]).to(torch.int32)
+    wts, pos = torch.rand(R, top, generator=g), torch.randperm(R * top, generator=g).to(torch.int32)
+    experts = ops.ExpertRows(rows.to(DEV), pos.to(DEV), ids.to(DEV), wts.to(DEV), parts=2)
+    gate = torch.sigmoid((x.double() * wg.double()).sum(-1, keepdim=True))
+    d = sums.double().sum(0) * gate
+    for r in range(R):
+        for j in range(top):
+            d[r] += wts[r, j].double() * rows[:, pos[r * top + j]].double().sum(0)
+    new = res.double() + w.double() * d / (d.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()
+    r1, out = res.to(DEV), torch.empty(R, width, dtype=DT[dtype], device=DEV)
+    ops.add_normed(r1, ops.PartialSums(sums.to(DEV).reshape(-1), parts, R, width), w.to(DEV), 1e-5, ops.RowDot(x.to(DEV), wg.to(DEV)),
+                   experts, (w2.to(DEV), 1e-4, out, None))
+    assert rel(r1, new) < 1e-5
+    assert rel(out.float(), w2.double() * new / (new.pow(2).mean(-1, keepdim=True) + 1e-4).sqrt()) < TOL[dtype]
