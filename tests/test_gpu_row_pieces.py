@@ -66,3 +66,38 @@ def test_norm_behind_a_branch_with_a_gate_that_is_not_computed_yet(dtype, width,
                    experts, (w2.to(DEV), 1e-4, out, None))
     assert rel(r1, new) < 1e-5
     assert rel(out.float(), w2.double() * new / (new.pow(2).mean(-1, keepdim=True) + 1e-4).sqrt()) < TOL[dtype]
+
+
+@pytest.mark.parametrize("Hq,Hk,D,VD,rot,turn_values", [(4, 2, 16, 8, 16, False), (3, 1, 64, 64, 32, True), (16, 4, 128, 128, 128, False),
+                                                        (40, 8, 128, 64, 64, True), (2, 2, 24, 16, 0, False), (4, 2, 16, 8, 8, False)])
+def test_turned_heads_and_their_pages(Hq, Hk, D, VD, rot, turn_values):
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + rot)
+    R, page, pad = 5, 16, 8
+    q_col, k_col = pad, pad + Hq * D
+    v_col = k_col + Hk * D
+    qkv = draw(g, R, v_col + Hk * VD, dtype=torch.bfloat16)
+    pos, req = torch.tensor([3, 1000, 17, 250, 31]), torch.tensor([0, 1, 0, 1, 0])
+    table = torch.stack([torch.randperm(64, generator=g), 64 + torch.randperm(64, generator=g)]).to(torch.int32)
+    inv, inv_v = torch.rand(max(rot // 2, 1), generator=g), torch.rand(VD // 2, generator=g)
+    q_out = torch.empty(R, Hq, D, dtype=torch.bfloat16, device=DEV)
+    kc = torch.zeros(128, Hk, page, D, dtype=torch.bfloat16, device=DEV)
+    vc = torch.zeros(128, Hk, page, VD, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ops.qkv_rotate_store(qkv.to(DEV), q_col, k_col, v_col, inv.to(DEV) if rot else None, rot, inv_v.to(DEV) if turn_values else None,
+                         pos.to(**i32), req.to(**i32), table.to(DEV), page, q_out, kc, vc, Hq, Hk, D, VD, status, rot_magnitude=0.75)
+    assert int(status.item()) == 0
+
+    def turned(x, freq, n, magnitude):              # x [R, heads, size]; angles in 32-bit as the kernel's are
+        angle = (pos.float()[:, None] * freq[None, :n // 2]).double()[:, None]
+        c, s = angle.cos() * magnitude, angle.sin() * magnitude
+        a, b = x[..., :n // 2], x[..., n // 2:n]
+        return torch.cat([a * c - b * s, b * c + a * s, x[..., n:]], -1)
+
+    q, k, v = (qkv[:, at:at + h * d].double().view(R, h, d) for at, h, d in ((q_col, Hq, D), (k_col, Hk, D), (v_col, Hk, VD)))
+    assert rel(q_out.float(), turned(q, inv, rot, 0.75)) < TOL["bfloat16"]
+    where = [(int(table[req[r], pos[r] // page]), int(pos[r] % page)) for r in range(R)]
+    assert rel(torch.stack([kc[p, :, o] for p, o in where]).float(), turned(k, inv, rot, 0.75)) < TOL["bfloat16"]
+    assert rel(torch.stack([vc[p, :, o] for p, o in where]).float(), turned(v, inv_v, VD, 1.0) if turn_values else v) < TOL["bfloat16"]
+    assert int((kc != 0).any(-1).sum()) == R * Hk
