@@ -101,3 +101,56 @@ def test_turned_heads_and_their_pages(Hq, Hk, D, VD, rot, turn_values):
     assert rel(torch.stack([kc[p, :, o] for p, o in where]).float(), turned(k, inv, rot, 0.75)) < TOL["bfloat16"]
     assert rel(torch.stack([vc[p, :, o] for p, o in where]).float(), turned(v, inv_v, VD, 1.0) if turn_values else v) < TOL["bfloat16"]
     assert int((kc != 0).any(-1).sum()) == R * Hk
+
+
+@pytest.mark.parametrize("halves", [False, True])
+@pytest.mark.parametrize("H,D,L,Rr,dims", [(1, 8, 8, 16, 16), (32, 128, 512, 64, 64), (20, 16, 520, 32, 16), (3, 0, 2048, 8, 0),
+                                           (4, 16, 64, 0, 0), (2, 8, 24, 12, 8)])
+def test_latent_rows_and_turned_queries(H, D, L, Rr, dims, halves):
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(L + Rr)
+    R, page, at, Dk = 3, 16, 16, L + Rr
+    q, down = draw(g, R, H * (D + Rr), dtype=torch.bfloat16), draw(g, R, at + Dk, dtype=torch.bfloat16)
+    w, inv = 1 + draw(g, L, scale=0.2), torch.rand(max(dims // 2, 1), generator=g)
+    pos = torch.tensor([5, 130, 77])
+    table = torch.randperm(16, generator=g).to(torch.int32)[None]
+    cache = torch.zeros(16, 1, page, Dk, dtype=torch.bfloat16, device=DEV)
+    qa = torch.zeros(R, H, Dk, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.latent_prepare(q.to(DEV), down.to(DEV)[:, at:], w.to(DEV), 1e-5, inv.to(DEV), dims, pos.to(DEV, torch.int32),
+                       torch.zeros(R, dtype=torch.int32, device=DEV), table.to(DEV), page, cache, qa, H, D, L, Rr, status, halves)
+    assert int(status.item()) == 0
+
+    def turned(x):                                  # x [R, heads, Rr]
+        n = dims // 2
+        angle = (pos.float()[:, None] * inv[None, :n]).double()[:, None]
+        c, s = angle.cos(), angle.sin()
+        a, b = (x[..., :n], x[..., n:dims]) if halves else (x[..., 0:dims:2], x[..., 1:dims:2])
+        y = x.clone()
+        if halves:
+            y[..., :n], y[..., n:dims] = a * c - b * s, b * c + a * s
+        else:
+            y[..., 0:dims:2], y[..., 1:dims:2] = a * c - b * s, b * c + a * s
+        return y
+
+    kv = down[:, at:].double()
+    c = kv[:, :L] / (kv[:, :L].pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * w.double()
+    got = torch.stack([cache[int(table[0, p // page]), 0, p % page] for p in pos.tolist()]).float()
+    assert rel(got[:, :L], c) < TOL["bfloat16"]
+    if Rr:
+        assert rel(got[:, L:], turned(kv[:, None, L:])[:, 0]) < TOL["bfloat16"]
+        want = turned(q.double().view(R, H, D + Rr)[..., D:])
+        # (a turned number is a difference of two products and may be small beside them: held to the head's largest)
+        assert rel(qa[..., L:], want) < 1e-5
+    assert not qa[..., :L].any()
+
+
+@pytest.mark.parametrize("n", [8, 264, 1024, 2048, 2056, 8192, 8200, 1028])
+def test_norm_of_the_first_columns(n):
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(n)
+    x, w = draw(g, 3, n + 8 - n % 8, dtype=torch.bfloat16), 1 + draw(g, n, scale=0.2)
+    out = torch.empty(3, n, dtype=torch.bfloat16, device=DEV)
+    ops.rmsnorm_rows(x.to(DEV), n, w.to(DEV), 1e-5, out)
+    v = x[:, :n].double()
+    assert rel(out.float(), v / (v.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * w.double()) < TOL["bfloat16"]
