@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
   bf16* sK = sQ + LM_ROWS * p.qs;                                // two buffers of [32][qs], then some slack (see the launcher)
   __shared__ int s_pos[LM_ROWS], s_lo[LM_ROWS], s_page[2][LM_KEYS];
   __shared__ int s_tile[4];                                      // request, its first row, its rows, first pair of the tile
+  __shared__ __align__(16) float sS[CPB == 2 ? 2 * 128 * 8 : 4];    // the scores the two groups of warps hand each other
   const int H = p.H, L = p.L, Dk = p.Dk, qs = p.qs;
   const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int chunk_index = blockIdx.y * CPB + (threadIdx.x >> 7);
@@ -113,18 +114,6 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
     key_hi = min(key_hi, ((int)blockIdx.z + 1) * p.span_keys - 1);
   }
   if (key_lo > key_hi) return;          // none of the tile's rows sees a key of this span: the join never asks for it
-  for (int i = threadIdx.x; i < LM_ROWS * (qs / 2); i += blockDim.x) {
-    const int m = i / (qs / 2), c = 2 * (i - m * (qs / 2));
-    const int f = f0 + m;
-    float x = 0.f, y = 0.f;
-    if (f < pairs) {
-      const float* src = p.q + ((long long)row_base * H + f) * Dk;
-      if (c < Dk) x = src[c];
-      if (c + 1 < Dk) y = src[c + 1];
-    }
-    reinterpret_cast<uint32_t*>(sQ + (size_t)m * qs)[c >> 1] = pack_bf16(x, y);
-  }
-  __syncthreads();
   float o[NT][4];
 #pragma unroll
   for (int n = 0; n < NT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
@@ -181,6 +170,44 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
   lookup(j_first, 0);
   __syncthreads();
   fetch(j_first, 0);
+  // The query rows, rounded to bfloat16 (zero beyond the pairs and Dk). They are asked for behind the first key tile, eight
+  // entries and several pieces a thread at a time: with an entry a load their round trips were a third of a decode step's kernel.
+  if ((Dk & 7) == 0 && ((uintptr_t)p.q & 15) == 0) {
+    const int per_row = qs >> 3, pieces = LM_ROWS * per_row;
+    constexpr int AT_ONCE = 4;
+    for (int i0 = threadIdx.x; i0 < pieces; i0 += AT_ONCE * blockDim.x) {
+      float4 x[AT_ONCE], y[AT_ONCE];
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u) {
+        const int i = i0 + u * blockDim.x, m = i / per_row, c = (i - m * per_row) << 3;
+        x[u] = y[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < pieces && f0 + m < pairs && c < Dk) {
+          const float* src = p.q + ((long long)row_base * H + f0 + m) * Dk + c;
+          x[u] = load4_now(src);
+          y[u] = load4_now(src + 4);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u) {
+        const int i = i0 + u * blockDim.x, m = i / per_row, c = (i - m * per_row) << 3;
+        if (i < pieces)
+          *reinterpret_cast<uint4*>(sQ + (size_t)m * qs + c) =
+              make_uint4(pack_bf16(x[u].x, x[u].y), pack_bf16(x[u].z, x[u].w), pack_bf16(y[u].x, y[u].y), pack_bf16(y[u].z, y[u].w));
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < LM_ROWS * (qs / 2); i += blockDim.x) {
+      const int m = i / (qs / 2), c = 2 * (i - m * (qs / 2));
+      const int f = f0 + m;
+      float x = 0.f, y = 0.f;
+      if (f < pairs) {
+        const float* src = p.q + ((long long)row_base * H + f) * Dk;
+        if (c < Dk) x = src[c];
+        if (c + 1 < Dk) y = src[c + 1];
+      }
+      reinterpret_cast<uint32_t*>(sQ + (size_t)m * qs)[c >> 1] = pack_bf16(x, y);
+    }
+  }
   int which = 0;
   for (int j0 = j_first; j0 <= key_hi; j0 += LM_KEYS, which ^= 1) {
     const bool more = j0 + LM_KEYS <= key_hi;
@@ -195,22 +222,46 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
     __syncthreads();            // this tile's rows have landed, for every thread
     const bf16* tK = sK + (size_t)which * LM_KEYS * qs;
     const int* t_page = s_page[which];
-    // S = Q K^T for the warp's 16 pairs and the tile's 32 keys
+    // S = Q K^T for the warp's 16 pairs and the tile's 32 keys, both operands by ldmatrix (A: rows 0..7 and 8..15 of the block's
+    // first and last eight entries; B: eight keys' first and last eight entries, two groups of keys a load). With two groups of
+    // warps on the same pairs each takes 16 of the keys and hands its scores to the other through shared memory. (Prompts of 300
+    // and 700 rows, 32 heads, a latent of 512: 447 us with 32-bit operand loads and every score made twice, 319 us so.)
     float s[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-    const uint32_t* q_lo = reinterpret_cast<const uint32_t*>(sQ + (size_t)(warp * 16 + g) * qs);
-    const uint32_t* q_hi = reinterpret_cast<const uint32_t*>(sQ + (size_t)(warp * 16 + g + 8) * qs);
+    const uint32_t qa = (uint32_t)__cvta_generic_to_shared(sQ + (size_t)(warp * 16 + (lane & 15)) * qs + (lane >> 4) * 8);
+    const int group = CPB == 2 ? (int)(threadIdx.x >> 7) : 0;
+    const uint32_t ka = (uint32_t)__cvta_generic_to_shared(tK + (size_t)(group * 16 + (lane >> 4) * 8 + (lane & 7)) * qs + ((lane >> 3) & 1) * 8);
+#pragma unroll 4
     for (int ks = 0; ks < ksteps; ++ks) {
       uint32_t a[4];
-      a[0] = q_lo[ks * 8 + t];
-      a[1] = q_hi[ks * 8 + t];
-      a[2] = q_lo[ks * 8 + 4 + t];
-      a[3] = q_hi[ks * 8 + 4 + t];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(qa + ks * 32));
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const uint32_t* kr = reinterpret_cast<const uint32_t*>(tK + (size_t)(n * 8 + g) * qs);
-        mma_bf16(s[n], a, kr[ks * 8 + t], kr[ks * 8 + 4 + t]);
+      for (int n = 0; n < 4 / CPB; n += 2) {
+        uint32_t b0, b1, b2, b3;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(ka + n * 8 * qs * 2 + ks * 32));
+        mma_bf16(s[n], a, b0, b1);
+        mma_bf16(s[n + 1], a, b2, b3);
+      }
+    }
+    if (CPB == 2) {
+      // (a slot of eight numbers a thread: thread (warp, lane) of the other group holds the same pairs and columns)
+      float4* mine = reinterpret_cast<float4*>(sS) + threadIdx.x * 2;
+      mine[0] = make_float4(s[0][0], s[0][1], s[0][2], s[0][3]);
+      mine[1] = make_float4(s[1][0], s[1][1], s[1][2], s[1][3]);
+      __syncthreads();
+      const float4* theirs = reinterpret_cast<const float4*>(sS) + (threadIdx.x ^ 128) * 2;
+      const float4 o0 = theirs[0], o1 = theirs[1];
+      if (group == 0) {
+        s[2][0] = o0.x; s[2][1] = o0.y; s[2][2] = o0.z; s[2][3] = o0.w;
+        s[3][0] = o1.x; s[3][1] = o1.y; s[3][2] = o1.z; s[3][3] = o1.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { s[2][e] = s[0][e]; s[3][e] = s[1][e]; }
+        s[0][0] = o0.x; s[0][1] = o0.y; s[0][2] = o0.z; s[0][3] = o0.w;
+        s[1][0] = o1.x; s[1][1] = o1.y; s[1][2] = o1.z; s[1][3] = o1.w;
       }
     }
     // scale, mask, running maximum and sum; thread (g, t) holds rows g and g + 8, keys 8 n + 2 t + {0, 1}
@@ -311,32 +362,63 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
   }
 }
 
-// grid (rows * H), 128 threads: the spans of a pair joined in ascending order
+// grid (rows * H), 128 threads: the spans of a pair joined in ascending order. Every warp takes the spans' maxima and sums itself, a
+// lane a span (the sum is then taken in the order of the spans), and the spans' rows are asked for four at a time: with a span a
+// round trip the kernel took 17 us for 12 spans of 64 pairs, 3.7 us here.
 __global__ void __launch_bounds__(128) latent_join_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                           const int* __restrict__ positions, int window, bf16* __restrict__ out,
                                                           int H, int L, int n_spans, int span_keys,
                                                           const float* __restrict__ sinks) {
   const long long pair = blockIdx.x;
+  const int lane = threadIdx.x & 31;
   const int pos = positions[pair / H];
   const int lo = window > 0 ? max(0, pos - window + 1) : 0;
   const int s0 = lo / span_keys, s1 = min(pos / span_keys, n_spans - 1);
+  const float* ml = part_ml + pair * n_spans * 2;
   float m = -INFINITY;
-  for (int s = s0; s <= s1; ++s) m = fmaxf(m, part_ml[(pair * n_spans + s) * 2]);
+  for (int s = s0 + lane; s <= s1; s += 32) m = fmaxf(m, ml[2 * s]);
+  m = warp_max(m);
   float sum = 0.f;
-  for (int s = s0; s <= s1; ++s) {
-    const float ms = part_ml[(pair * n_spans + s) * 2];
-    if (ms != -INFINITY) sum += expf(ms - m) * part_ml[(pair * n_spans + s) * 2 + 1];
+  for (int b = s0; b <= s1; b += 32) {
+    const float ms = b + lane <= s1 ? ml[2 * (b + lane)] : -INFINITY;
+    const float share = ms != -INFINITY ? expf(ms - m) * ml[2 * (b + lane) + 1] : 0.f;
+    for (int s = 0; s < min(32, s1 - b + 1); ++s) sum += __shfl_sync(0xffffffffu, share, s);
   }
   float keep, inv;
   latent_finish(m, sum, sinks, (int)(pair % H), &keep, &inv);
   inv *= keep;
-  for (int c = threadIdx.x; c < L; c += blockDim.x) {
-    float acc = 0.f;
-    for (int s = s0; s <= s1; ++s) {
-      const float ms = part_ml[(pair * n_spans + s) * 2];
-      if (ms != -INFINITY) acc += expf(ms - m) * part_o[(pair * n_spans + s) * L + c];
+  const float* rows = part_o + pair * n_spans * L;
+  for (int c0 = 0; c0 < L; c0 += 512) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};                // columns c0 + threadIdx.x + 128 i
+    for (int b = s0; b <= s1; b += 32) {
+      const float mine = b + lane <= s1 ? ml[2 * (b + lane)] : -INFINITY;
+      const float factor = mine != -INFINITY ? expf(mine - m) : 0.f;
+      const unsigned live = __ballot_sync(0xffffffffu, mine != -INFINITY);      // spans in which the pair sees a key
+      const int n = min(32, s1 - b + 1);
+      for (int s = 0; s < n; s += 4) {
+        float v[4][4], f[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          f[u] = __shfl_sync(0xffffffffu, factor, (s + u) & 31);
+          const bool seen = s + u < n && (live >> ((s + u) & 31) & 1u);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int c = c0 + threadIdx.x + 128 * i;
+            v[u][i] = seen && c < L ? rows[(long long)(b + s + u) * L + c] : 0.f;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (s + u < n && (live >> ((s + u) & 31) & 1u))
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] += f[u] * v[u][i];
+      }
     }
-    out[pair * L + c] = __float2bfloat16_rn(acc * inv);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = c0 + threadIdx.x + 128 * i;
+      if (c < L) out[pair * L + c] = __float2bfloat16_rn(acc[i] * inv);
+    }
   }
 }
 

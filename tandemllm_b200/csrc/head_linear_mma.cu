@@ -93,6 +93,69 @@ __global__ void __launch_bounds__(128) head_linear_mma_kernel(const bf16* __rest
   }
 }
 
+// A decode step's rows (up to 8 NT): the heads' weights are all there is to read, so no shared memory and no barrier stands between
+// them and the tensor cores. The weights are the M side (16 outputs a CTA), the rows the N side; a thread's 16 bytes of a weight row
+// or of a row hold what it feeds to two `mma.sync` (both operands in the same order of k, so the sum is over the same pairs), a warp
+// has all its loads in flight at once, and long reductions are cut among the CTA's KW warps and added in their order.
+// 32 heads of 128 x 512 with two rows took 24.6 us and 512 x 128 8.0 us on tiles of 64 rows, 3.4 and 3.5 us here.
+// grid (ceil(N / 16), H), 32 KW threads; K a multiple of 32 KW
+template <typename TO, int NT, int KW>
+__global__ void __launch_bounds__(32 * KW) head_linear_few_kernel(const bf16* __restrict__ a, long long ld_a, long long a_head,
+                                                                  const bf16* __restrict__ w, TO* __restrict__ out, long long ld_out,
+                                                                  long long out_head, int rows, int N, int K,
+                                                                  const bf16* __restrict__ gate, long long ld_gate, int gate_heads) {
+  __shared__ float part[KW][NT * 8][16];
+  const int h = blockIdx.y, n0 = blockIdx.x * 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int span = K / KW, k0 = warp * span + t * 8;
+  // (an output or a row beyond the last one reads the last one's numbers; what it makes is not stored)
+  const bf16* w_lo = w + ((long long)h * N + min(n0 + g, N - 1)) * K + k0;
+  const bf16* w_hi = w + ((long long)h * N + min(n0 + g + 8, N - 1)) * K + k0;
+  const bf16* ar[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) ar[n] = a + (long long)min(n * 8 + g, rows - 1) * ld_a + (long long)h * a_head + k0;
+  float acc[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+  constexpr int AT_ONCE = 4;                        // pieces of 32 k in flight a warp
+  for (int k = 0; k < span; k += 32 * AT_ONCE) {
+    uint4 lo[AT_ONCE], hi[AT_ONCE], b[AT_ONCE][NT];
+#pragma unroll
+    for (int u = 0; u < AT_ONCE; ++u) {
+      const int at = min(k + 32 * u, span - 32);
+      lo[u] = load16_now(w_lo + at);
+      hi[u] = load16_now(w_hi + at);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) b[u][n] = load16_now(ar[n] + at);
+    }
+#pragma unroll
+    for (int u = 0; u < AT_ONCE; ++u) {
+      if (k + 32 * u >= span) break;
+      const uint32_t first[4] = {lo[u].x, hi[u].x, lo[u].y, hi[u].y}, second[4] = {lo[u].z, hi[u].z, lo[u].w, hi[u].w};
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        hm_mma(acc[n], first, b[u][n].x, b[u][n].y);
+        hm_mma(acc[n], second, b[u][n].z, b[u][n].w);
+      }
+    }
+  }
+  // thread (g, t) holds outputs g and g + 8 of rows 2 t and 2 t + 1 of every eight
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) part[warp][n * 8 + 2 * t + (e & 1)][g + 8 * (e >> 1)] = acc[n][e];
+  __syncthreads();
+  for (int i = threadIdx.x; i < NT * 8 * 16; i += 32 * KW) {
+    const int row = i >> 4, col = n0 + (i & 15);
+    if (row >= rows || col >= N) continue;
+    float v = part[0][row][i & 15];
+#pragma unroll
+    for (int s = 1; s < KW; ++s) v += part[s][row][i & 15];
+    if (gate) v *= 1.f / (1.f + expf(-to_f32(gate[(long long)row * ld_gate + (gate_heads ? (long long)h : (long long)h * N + col)])));
+    out[(long long)row * ld_out + (long long)h * out_head + col] = from_f32<TO>(v);
+  }
+}
+
 }  // namespace tl
 
 using namespace tl;
@@ -107,6 +170,30 @@ extern "C" int tl_head_linear_mma(const void* a, long long ld_a, long long a_hea
   TL_REQUIRE(rows > 0 && H > 0 && H <= 65535 && N > 0 && K > 0, "head product: %d rows, %d heads, %d x %d", rows, H, N, K);
   TL_REQUIRE(ceil_div(rows, HM_TILE) <= 65535, "head product: %d rows in one launch", rows);
   const int vec = (K % 8 == 0 && ld_a % 8 == 0 && a_head % 8 == 0 && ((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0) ? 1 : 0;
+  // (a row's sums are taken in another order than on the tiles of 64 rows: the same products, 32-bit sums)
+  if (rows <= 16 && vec && K % 32 == 0) {
+    const dim3 few(ceil_div(N, 16), H);
+#define TL_HL_FEW(T_, NT_, KW_)                                                                                           \
+  head_linear_few_kernel<T_, NT_, KW_><<<few, 32 * KW_, 0, stream>>>((const bf16*)a, ld_a, a_head, (const bf16*)w, (T_*)out, ld_out,  \
+                                                                     out_head, rows, N, K, (const bf16*)gate, ld_gate, gate_heads)
+#define TL_HL_FEW_ROWS(T_, KW_)                     \
+  do {                                              \
+    if (rows <= 8) TL_HL_FEW(T_, 1, KW_);           \
+    else TL_HL_FEW(T_, 2, KW_);                     \
+  } while (0)
+    const bool cut = K >= 256 && K % 128 == 0;
+    if (out_dtype == TL_FP32) {
+      if (cut) TL_HL_FEW_ROWS(float, 4);
+      else TL_HL_FEW_ROWS(float, 1);
+    } else {
+      if (cut) TL_HL_FEW_ROWS(bf16, 4);
+      else TL_HL_FEW_ROWS(bf16, 1);
+    }
+#undef TL_HL_FEW_ROWS
+#undef TL_HL_FEW
+    TL_LAUNCH_CHECK();
+    return 0;
+  }
   const dim3 grid(ceil_div(N, HM_TILE), ceil_div(rows, HM_TILE), H);
   if (out_dtype == TL_FP32)
     head_linear_mma_kernel<float><<<grid, 128, 0, stream>>>((const bf16*)a, ld_a, a_head, (const bf16*)w, (float*)out, ld_out,

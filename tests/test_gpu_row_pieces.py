@@ -154,3 +154,25 @@ def test_norm_of_the_first_columns(n):
     ops.rmsnorm_rows(x.to(DEV), n, w.to(DEV), 1e-5, out)
     v = x[:, :n].double()
     assert rel(out.float(), v / (v.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * w.double()) < TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17])
+@pytest.mark.parametrize("N,K,gate", [(16, 32, None), (24, 160, "entries"), (512, 128, None), (128, 512, "heads"), (40, 384, None), (10, 48, None)])
+def test_a_product_a_head_for_a_few_rows(rows, N, K, gate):
+    """32-bit sums of K products of bfloat16 numbers: 1e-5 of the row's largest in a 32-bit result, plus a last place in a bfloat16 one."""
+    from tandemllm_b200.kernels import tensorcore
+    from tandemllm_b200.parts.base import Runtime
+    tc = tensorcore.enable(Runtime(torch.device(DEV), torch.bfloat16))
+    g = torch.Generator().manual_seed(N + K + rows)
+    H, pad = 3, 8
+    a, w = draw(g, rows, H, K + pad, dtype=torch.bfloat16), draw(g, H, N, K, scale=K ** -0.5, dtype=torch.bfloat16)
+    logits = {None: None, "entries": draw(g, rows, H * N, dtype=torch.bfloat16), "heads": draw(g, rows, H, dtype=torch.bfloat16)}[gate]
+    want = torch.einsum("rhk,hnk->rhn", a[..., :K].double(), w.double())
+    if gate:
+        want = want * torch.sigmoid(logits.double().view(rows, H, -1))
+    for dtype in ("float32", "bfloat16"):
+        out = torch.zeros(rows, H, N + 4, dtype=DT[dtype], device=DEV)
+        assert tc.head_linear(a.to(DEV), H * (K + pad), K + pad, w.to(DEV), out, H * (N + 4), N + 4, rows,
+                              logits.to(DEV) if gate else None, gate == "heads")
+        assert rel(out[..., :N].float(), want) < TOL[dtype] + 1e-5
+        assert not out[..., N:].any()
