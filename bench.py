@@ -360,7 +360,8 @@ class LaunchTimer:
             return "dense products (tcgen05, pairs of SMs, activation in the epilogue)"
         if name == "tl_gemm_skinny_grouped":
             return "experts gate/up + SwiGLU (register-only)" if args[11] else "experts down (register-only)"
-        return {"tl_gemm_skinny_mma": "dense products (register-only)", "tl_gemm_skinny_conv": "in-projection + short conv",
+        return {"tl_gemm_skinny_mma": "dense products (register-only)", "tl_gemm_skinny_mma_runs": "dense products (register-only)",
+                "tl_gemm_skinny_conv": "in-projection + short conv",
                 "tl_add_rmsnorm": "residual add + norm (+ router, + deferred sums)",
                 "tl_add_rmsnorm_streams": "residual add + norm (+ router, + deferred sums)", "tl_embed_rows_copies": "embedding",
                 "tl_embed_token_pairs": "embedding",

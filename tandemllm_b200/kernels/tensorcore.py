@@ -39,6 +39,7 @@ from .build import load
 SKINNY_TOKENS = 32              # up to this many token rows ...
 SKINNY_K = 2048                 # ... of at most this many elements (one round of loads a warp) ...
 SKINNY_BYTES = 64 << 20         # ... against at most this many bytes of weights go to the register-only kernel
+SKINNY_RUN_ROWS = 16            # rows up to which a longer reduction whose sums may stay in parts goes there too, in runs of k
 SKINNY_ROWS = 16                # rows of a step up to which the experts go to its grouped form, over plan tiles of 8 (an
                                 # expert with more pairs has two tiles, and the second reads its weights from L2); measured
                                 # against the tcgen05 form: 8 % faster a step at 16 rows, even at 24, 4 % slower at 32
@@ -134,6 +135,9 @@ def lib():
         l.tl_gemm_skinny_mma.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int,
                                          c_int, c_int, c_int, c_void_p]
         l.tl_gemm_skinny_mma.restype = c_int
+        l.tl_gemm_skinny_mma_runs.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int,
+                                              c_int, c_int, c_int, c_int, c_void_p]
+        l.tl_gemm_skinny_mma_runs.restype = c_int
         l.tl_gemm_skinny_grouped.argtypes = [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_void_p,
                                              c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                              c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
@@ -300,6 +304,18 @@ class TensorCore:
                                             out.data_ptr(), out.stride(0), M, N, K, ops.dtype_code(out.dtype),
                                             ops.stream()), "gemm_skinny_mma")
             return True
+        if (defer and (out.dtype == torch.float32 or defer == "rounded") and M <= SKINNY_RUN_ROWS and K > SKINNY_K
+                and N * K * 2 <= SKINNY_BYTES and lib().tl_gemm_skinny_supported(M, N, K, x.stride(0), w.stride(0))):
+            # a long reduction whose partial sums the consumer adds: as many runs of k as fill the GPU with four CTAs an SM
+            runs = min(4 * self.sm_count // -(-N // 16), 16)
+            run = -(-K // (128 * max(runs, 1))) * 128
+            runs = -(-K // run)
+            if runs > 1:
+                partial = self.workspace(runs * M * N)
+                _check(lib().tl_gemm_skinny_mma_runs(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), ops.ptr(bias),
+                                                     partial.data_ptr(), N, M, N, K, run, ops.FP32, ops.stream()),
+                       "gemm_skinny_mma_runs")
+                return ops.PartialSums(partial, runs, M, N, None if out.dtype == torch.float32 else out.dtype)
         return self.gemm(x, w, bias, out, defer=defer) or True
 
     def linear_act(self, x, w, act: int, a0: float = 0.0, a1: float = 0.0):

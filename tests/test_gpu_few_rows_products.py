@@ -1,0 +1,64 @@
+"""The products that a step of a few rows takes straight from registers: runs of k, and the experts' grouped form over pairs without
+a plan, at the edges of their chunks (32 numbers of k, 4 or 8 chunks a warp and round, 16 outputs, 8 rows, 32 and 256 pairs). Sums
+of bfloat16 products in 32-bit: 1e-5 of a row's largest for rows of a few thousand numbers."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def tensor_core():
+    from tandemllm_b200.kernels import tensorcore
+    from tandemllm_b200.parts.base import Runtime
+    return tensorcore.enable(Runtime(torch.device(DEV), torch.bfloat16))
+
+
+def rel(a, b):
+    a, b = a.double().cpu(), b.double().cpu()
+    return float(((a - b).abs() / b.abs().amax(dim=-1, keepdim=True).clamp_min(1e-30)).max())
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17])
+@pytest.mark.parametrize("N,K", [(2048, 4096), (2048, 8192), (40, 2056), (24, 11776), (9472, 2304), (512, 7168)])
+def test_long_reductions_in_runs_of_k(M, N, K):
+    from tandemllm_b200.kernels import ops
+    tc = tensor_core()
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g).to(torch.bfloat16), (torch.randn(N, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(N, generator=g)
+    out = torch.empty(M, N, device=DEV)
+    got = tc.linear(x.to(DEV), w.to(DEV), bias.to(DEV), out, defer=True)
+    want = x.double() @ w.double().T + bias.double()
+    assert rel(ops.materialize(got) if isinstance(got, ops.PartialSums) else out, want) < 1e-5
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("R,k,E", [(1, 4, 32), (5, 6, 64), (8, 4, 5), (8, 32, 64), (7, 5, 1000)])
+@pytest.mark.parametrize("N,K", [(16, 32), (40, 264), (136, 1792), (24, 1536), (16, 2048)])
+def test_grouped_products_of_pairs_without_a_plan(R, k, E, N, K, gated):
+    from tandemllm_b200.kernels import ops, tensorcore
+    tensor_core()
+    k = min(k, E)
+    g = torch.Generator().manual_seed(R * k + N)
+    P = R * k
+    ids = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(R)]).to(torch.int32)
+    used = sorted(set(ids.view(-1).tolist()))       # (only the experts that are used get numbers)
+    w = torch.zeros(E, (2 if gated else 1) * N, K, dtype=torch.bfloat16)
+    for e in used:
+        w[e] = (torch.randn(w.shape[1], K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    x = torch.randn(R if gated else P, K, generator=g).to(torch.bfloat16)
+    out = torch.zeros(P, N, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    xd, wd, idd = x.to(DEV), w.to(DEV), ids.to(DEV)
+    tensorcore._check(tensorcore.lib().tl_gemm_skinny_grouped(
+        xd.data_ptr(), K, None, k if gated else 1, wd.data_ptr(), K, w.shape[1], out.data_ptr(), N, N, K, int(gated), ops.FP32, None,
+        None, None, None, 0, idd.data_ptr(), P, E, status.data_ptr(), None, None, ops.stream()), "grouped")
+    want = torch.empty(P, N, dtype=torch.float64)
+    for p in range(P):
+        y = w[int(ids.view(-1)[p])].double() @ x[p // k if gated else p].double()
+        want[p] = torch.nn.functional.silu(y[:N]) * y[N:] if gated else y
+    assert int(status.item()) == 0
+    assert rel(out, want) < 1e-5
