@@ -100,13 +100,16 @@ __global__ void short_conv_kernel(const T* __restrict__ bcx, const float* __rest
   store_run<T, V>(y + (long long)r * hidden + c, cv);
 }
 
-// The same for a prompt's many rows: a thread walks CONV_RUN consecutive rows for its 8 channels with the last KT - 1
+// The same for a prompt's many rows: a thread walks RUN consecutive rows for its 8 channels with the last KT - 1
 // inputs bx in registers, so every B, C and x is read once, and the loads of four rows are sent before the first is
 // used. Rows of a run that belong to several requests (a run across a request's edge) go the way of the kernel above,
 // row by row. Same results: a tap whose input lies before the sequence's first token multiplies a zero here and is
 // left out there.
-constexpr int CONV_RUN = 8;
-template <typename T, int KT>
+// Runs of eight rows where those alone give the GPU two blocks an SM, else of two: a block's time is a chain of round trips and, in
+// a run of several requests, one such chain a row (hidden 2048, runs of eight -> two: 535 rows of 24 requests 17.9 -> 8.2 us, 969 rows
+// of 5 11.4 -> 7.9 us, 37 rows 6.5 -> 4.2 us; at 2048 rows the inputs that are then read twice cost more than that).
+constexpr int CONV_RUN = 8, CONV_SHORT_RUN = 2;
+template <typename T, int KT, int RUN>
 __global__ void __launch_bounds__(128) short_conv_run_kernel(const T* __restrict__ bcx, const float* __restrict__ taps,
                                                              const float* __restrict__ bias, const float* __restrict__ state,
                                                              const int* __restrict__ state_slot,
@@ -117,10 +120,10 @@ __global__ void __launch_bounds__(128) short_conv_run_kernel(const T* __restrict
   constexpr int V = 8, S = KT - 1;
   chain_next();
   chain_wait();
-  const int r0 = blockIdx.x * CONV_RUN;
+  const int r0 = blockIdx.x * RUN;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
   if (c >= hidden) return;
-  const int n = min(CONV_RUN, rows - r0);
+  const int n = min(RUN, rows - r0);
   const long long ld = 3LL * hidden;
   float tp[KT][V], bs[V];
 #pragma unroll
@@ -185,7 +188,7 @@ __global__ void __launch_bounds__(128) short_conv_run_kernel(const T* __restrict
       }
     }
   }
-  constexpr int AHEAD = 4;
+  constexpr int AHEAD = RUN < 4 ? RUN : 4;
   for (int q0 = 0; q0 < n; q0 += AHEAD) {
     float bv[AHEAD][V], cv[AHEAD][V], xv[AHEAD][V];
 #pragma unroll
@@ -331,10 +334,16 @@ extern "C" int tl_short_conv(const void* bcx, const float* taps, const float* bi
   TL_REQUIRE(grid.y <= 65535, "short_conv: hidden size %d exceeds the grid limit", hidden);
   // many rows, 16-byte accesses, 2 to 4 taps: the form that walks runs of rows
   if (wide && rows >= 4 * CONV_RUN && K <= 4) {
-    dim3 run_grid(ceil_div(rows, CONV_RUN), grid.y);
-#define TL_RUN(T_, K_)                                                                                                     \
-  return (int)launch_chained(short_conv_run_kernel<T_, K_>, run_grid, dim3(128), 0, stream, (const T_*)bcx, taps, bias,   \
+    const bool brief = (long long)ceil_div(rows, CONV_RUN) * grid.y < 2LL * sm_count();
+    dim3 run_grid(ceil_div(rows, brief ? CONV_SHORT_RUN : CONV_RUN), grid.y);
+#define TL_RUN_(T_, K_, R_)                                                                                                \
+  return (int)launch_chained(short_conv_run_kernel<T_, K_, R_>, run_grid, dim3(128), 0, stream, (const T_*)bcx, taps, bias, \
                              state, state_slot, req_of_row, row_start, positions, (T_*)y, rows, hidden)
+#define TL_RUN(T_, K_)                          \
+  do {                                          \
+    if (brief) TL_RUN_(T_, K_, CONV_SHORT_RUN); \
+    TL_RUN_(T_, K_, CONV_RUN);                  \
+  } while (0)
     if (dtype == TL_FP32) {
       if (K == 2) TL_RUN(float, 2);
       if (K == 3) TL_RUN(float, 3);
@@ -344,6 +353,7 @@ extern "C" int tl_short_conv(const void* bcx, const float* taps, const float* bi
     if (K == 3) TL_RUN(bf16, 3);
     TL_RUN(bf16, 4);
 #undef TL_RUN
+#undef TL_RUN_
   }
 #define TL_CONV(T_, V_)                                                                                                   \
   return (int)launch_chained(short_conv_kernel<T_, V_>, grid, dim3(128), 0, stream, (const T_*)bcx, taps, bias, state,    \
