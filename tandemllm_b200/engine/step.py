@@ -22,6 +22,7 @@ new one is captured).
 
 from __future__ import annotations
 
+from array import array
 from collections import OrderedDict
 from dataclasses import dataclass
 
@@ -63,6 +64,15 @@ def context_bucket(longest: int) -> int:
     while g * 16 <= longest:
         g *= 2
     return -(-longest // g) * g
+
+
+def _int32s(values):
+    """A list of whole numbers as int32, through `array` (a third of the time numpy takes to look at each of a prompt's ids);
+    anything `array` does not take goes to numpy as it is."""
+    try:
+        return np.frombuffer(array("i", values), dtype=np.int32)
+    except TypeError:
+        return values
 
 
 class _Staging:
@@ -159,8 +169,8 @@ class StepFunction:
         for b, e in enumerate(entries):
             n = len(e.tokens)
             start = cache.length_of(e.request)
-            host[o["tok"] + r:o["tok"] + r + n] = e.tokens
-            host[o["pos"] + r:o["pos"] + r + n] = range(start, start + n)
+            host[o["tok"] + r:o["tok"] + r + n] = _int32s(e.tokens)
+            host[o["pos"] + r:o["pos"] + r + n] = np.arange(start, start + n, dtype=np.int32)
             host[o["req"] + r:o["req"] + r + n] = b
             host[o["start"] + b] = r
             host[o["slot"] + b] = cache.slot_of(e.request)
