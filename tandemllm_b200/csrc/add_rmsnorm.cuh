@@ -654,7 +654,7 @@ static int launch_add_rmsnorm(NormParams p, int dtype, cudaStream_t stream) {
   if (rows_per_block == 1 && router_w && E >= 16 && (hidden & 3) == 0 && MODE != NORM_STREAMS)
     p.split = out_rows <= ROUTER_SPLIT_ROWS ? ROUTER_SPLIT : (out_rows <= 37 ? 4 : (out_rows <= 74 ? 2 : 1));
   const dim3 grid(ceil_div(out_rows, rows_per_block) * p.split);
-  const int per = !router_w ? 0 : (E <= 32 ? 1 : (E <= 128 ? 4 : MAX_EXPERTS / 32));
+  const int per = !router_w ? 0 : (E <= 32 ? 1 : (E <= 64 ? 2 : (E <= 128 ? 4 : MAX_EXPERTS / 32)));
 #define TL_NORM1(T_, PER_, ONE_)                                                                                        \
   do {                                                                                                                  \
     if (smem > 48 * 1024)                                                                                               \
@@ -671,11 +671,13 @@ static int launch_add_rmsnorm(NormParams p, int dtype, cudaStream_t stream) {
   if (dtype == TL_FP32) {
     if (per == 0) TL_NORM(float, 0);
     if (per == 1) TL_NORM(float, 1);
+    if (per == 2) TL_NORM(float, 2);
     if (per == 4) TL_NORM(float, 4);
     TL_NORM(float, MAX_EXPERTS / 32);
   }
   if (per == 0) TL_NORM(bf16, 0);
   if (per == 1) TL_NORM(bf16, 1);
+  if (per == 2) TL_NORM(bf16, 2);
   if (per == 4) TL_NORM(bf16, 4);
   TL_NORM(bf16, MAX_EXPERTS / 32);
 #undef TL_NORM
