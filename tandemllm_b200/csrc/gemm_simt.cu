@@ -243,19 +243,22 @@ __global__ void __launch_bounds__(256) gemm_tall_narrow_kernel(GemmParams p) {
 // The kernels above fetch a number at a time, wait for a tile before they multiply it and were what a 32-bit prompt
 // consisted of. These take 16 bytes a load and keep four stages of 32 k-elements in flight (cp.async).
 //
-// CTA: BM rows by 64 outputs (gated: 32 gate rows and the 32 up rows of the same outputs), eight warps that all hold the whole
-// tile and take one of a stage's eight k-quads each; their sums meet in shared memory at the end. What bounds such a
-// kernel is the multiply-adds and what shared memory hands to the registers, 128 bytes a clock: a 16-byte load feeds 16
-// multiply-adds with 8 x 8 outputs a thread, as many as the SM does meanwhile, and a warp on a tile of its own is what
-// makes 8 x 8 possible with tiles small enough to fill the GPU. Measured at 150 rows: 14336 outputs of 2048 in 281 us
-// (31 TFLOP/s), the eleven plain products of a three-layer pass 364 -> 168 us each on average, the experts' gate/up of
-// 600 pairs 1135 -> 448 us. A thread's rows lie 4 and its columns 8 apart, so a quarter of a warp reads one row or eight neighbouring ones:
+// CTA: BM rows by 64 outputs (gated: 32 gate rows and the 32 up rows of the same outputs), four warps that all hold the whole
+// tile and take two of a stage's eight k-quads each; their sums meet in shared memory at the end. What bounds such a
+// kernel is the multiply-adds and what shared memory hands to the registers, 128 bytes a clock. The multiply-adds go two an
+// instruction (fma.rn.f32x2) on neighbouring k of one output, so both operands lie in registers as they were loaded, and an output
+// is two sums, of the even k and of the odd. A 16-byte load feeds 16 multiply-adds with 8 x 8 outputs a thread, as many as the SM
+// does meanwhile, and a warp on a tile of its own is what makes 8 x 8 possible with tiles small enough to fill the GPU. Two CTAs of
+// four warps share an SM (240 registers a thread); the multiply-add pipe is then 58 % busy, what is lost is two warps a scheduler
+// waiting for shared memory and for one another. Measured at 150 rows, eight warps of single multiply-adds -> this: 14336 outputs of
+// 2048 281 -> 252 us, 6144 of 2048 144 -> 130 us, 2048 of 2048 and of 7168 140 -> 128 us on average, the experts' gate/up of
+// 600 pairs 448 -> 403 us. A thread's rows lie 4 and its columns 8 apart, so a quarter of a warp reads one row or eight neighbouring ones:
 // with 36 floats a row the eight meet no bank twice.
 //
-// An output is the sum of eight chains, chain q in ascending order over the quads q, q + 8, ..., added in order: which k
-// a chain has depends on k alone, whatever the tile's height, so a row still does not depend on the others, and eight
-// short chains lose less than one long one.
-constexpr int FK = 32, FPITCH = FK + 4, FSTAGES = 4, FN = 64, FWARPS = 8;
+// An output is the sum of eight chains, a warp's even and odd k in ascending order over the quads q = warp (mod 4), added in
+// order: which k a chain has depends on k alone, whatever the tile's height, so a row still does not depend on the others, and
+// eight short chains lose less than one long one.
+constexpr int FK = 32, FPITCH = FK + 4, FSTAGES = 4, FN = 64, FWARPS = 4;
 
 template <int BM_>
 struct F32Tile {
@@ -263,7 +266,8 @@ struct F32Tile {
   static constexpr int STAGE = (BM_ + FN) * FPITCH;                   // floats
   static constexpr int RED = FWARPS * BM_ * FN;                       // the warps' sums
   static constexpr int SMEM = (FSTAGES * STAGE > RED ? FSTAGES * STAGE : RED) * 4;
-  static constexpr int LOADS = (BM_ + FN + 31) / 32;                  // 16-byte pieces a thread and stage
+  static constexpr int ROWS_A_PASS = FWARPS * 4;                      // rows of [A tile; W tile] that the CTA's threads load at a time
+  static constexpr int LOADS = (BM_ + FN + ROWS_A_PASS - 1) / ROWS_A_PASS;     // 16-byte pieces a thread and stage
 };
 
 __device__ __forceinline__ void cp16(uint32_t dst, const float* src, bool valid) {
@@ -279,7 +283,7 @@ __device__ __forceinline__ float both(unsigned long long v) {
 
 // `sub`: how many CTA tiles a tile of the plan is cut into (grouped)
 template <int BM_, bool GATED>
-__global__ void __launch_bounds__(256, 2) gemm_f32_kernel(GemmParams p, int sub) {
+__global__ void __launch_bounds__(FWARPS * 32, BM_ == 32 ? 2 : 3) gemm_f32_kernel(GemmParams p, int sub) {
   using T = F32Tile<BM_>;
   constexpr int TM_ = T::TM;
   extern __shared__ float4 f32_smem[];
@@ -301,13 +305,13 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(GemmParams p, int sub)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ty = lane >> 3, tx = lane & 7;
 
-  // what this thread loads: 16 bytes at k offset 4 (tid % 8) of rows tid / 8, + 32, ... of [A tile; W tile]
+  // what this thread loads: 16 bytes at k offset 4 (tid % 8) of rows tid / 8, + 16, ... of [A tile; W tile]
   const int lk = (tid & 7) * 4;
   const float* src[T::LOADS];
   bool ok[T::LOADS];
 #pragma unroll
   for (int i = 0; i < T::LOADS; ++i) {
-    const int r = (tid >> 3) + 32 * i;
+    const int r = (tid >> 3) + T::ROWS_A_PASS * i;
     src[i] = W;
     ok[i] = false;
     if (r < BM_) {
@@ -333,39 +337,39 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(GemmParams p, int sub)
       const uint32_t at = smem0 + (uint32_t)((step % FSTAGES) * T::STAGE * 4);
 #pragma unroll
       for (int i = 0; i < T::LOADS; ++i)
-        if ((tid >> 3) + 32 * i < BM_ + FN) {
+        if ((tid >> 3) + T::ROWS_A_PASS * i < BM_ + FN) {
           const bool in = ok[i] && k < p.K;          // (K is a multiple of 4)
-          cp16(at + (uint32_t)(32 * i * FPITCH * 4), in ? src[i] + k : W, in);
+          cp16(at + (uint32_t)(T::ROWS_A_PASS * i * FPITCH * 4), in ? src[i] + k : W, in);
         }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  float acc[TM_][8];
+  unsigned long long acc[TM_][8];                     // (sum over even k, sum over odd k)
 #pragma unroll
   for (int i = 0; i < TM_; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
 
   for (int s = 0; s < FSTAGES - 1; ++s) load(s);
   for (int step = 0; step < steps; ++step) {
     asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
     __syncthreads();                                  // the stage is here, and everybody is done with the one before
     load(step + FSTAGES - 1);
-    const float* st = tiles + (step % FSTAGES) * T::STAGE + warp * 4;
-    const float* a_at = st + ty * FPITCH, * w_at = st + (BM_ + tx) * FPITCH;
-    float4 w[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(w_at + j * 8 * FPITCH);
+    for (int half = 0; half < 2; ++half) {
+      const float* st = tiles + (step % FSTAGES) * T::STAGE + (warp + FWARPS * half) * 4;
+      const float* a_at = st + ty * FPITCH, * w_at = st + (BM_ + tx) * FPITCH;
+      ulonglong2 w[8];
 #pragma unroll
-    for (int m = 0; m < TM_; ++m) {
-      const float4 a = *reinterpret_cast<const float4*>(a_at + m * 4 * FPITCH);
+      for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_at + j * 8 * FPITCH);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        acc[m][j] = fmaf(a.x, w[j].x, acc[m][j]);
-        acc[m][j] = fmaf(a.y, w[j].y, acc[m][j]);
-        acc[m][j] = fmaf(a.z, w[j].z, acc[m][j]);
-        acc[m][j] = fmaf(a.w, w[j].w, acc[m][j]);
+      for (int m = 0; m < TM_; ++m) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_at + m * 4 * FPITCH);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) fma2(acc[m][j], a.x, w[j].x);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) fma2(acc[m][j], a.y, w[j].y);
       }
     }
   }
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(GemmParams p, int sub)
 #pragma unroll
   for (int m = 0; m < TM_; ++m)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) red[((warp * TM_ + m) * 8 + j) * 32 + lane] = acc[m][j];
+    for (int j = 0; j < 8; ++j) red[((warp * TM_ + m) * 8 + j) * 32 + lane] = both(acc[m][j]);
   __syncthreads();
   auto sum = [&](int m, int j) {
     float v = 0.f;
@@ -384,11 +388,11 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(GemmParams p, int sub)
     return v;
   };
   float* C = (float*)p.C;
-  // a warp stores column block `warp` (gated: rows of either parity of the outputs' block warp % 4)
+  // a warp stores column blocks `warp` and (plain) `warp` + 4
 #pragma unroll
-  for (int i = 0; i < (GATED ? TM_ / 2 : TM_); ++i) {
-    const int m = GATED ? 2 * i + (warp >> 2) : i;
-    const int j = GATED ? warp & 3 : warp;
+  for (int i = 0; i < (GATED ? TM_ : 2 * TM_); ++i) {
+    const int m = GATED ? i : i >> 1;
+    const int j = GATED ? warp : warp + 4 * (i & 1);
     const int lr = ty + 4 * m, n = col0 + tx + 8 * j;
     const float v = sum(m, j), u = GATED ? sum(m, j + 4) : 0.f;
     if (lr >= rows || n >= p.N) continue;
@@ -461,7 +465,7 @@ static int launch_f32(const GemmParams& p, int max_tiles, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BM_>::SMEM);
   if (e != cudaSuccess) return (int)e;
   const unsigned y = p.tile_group ? (unsigned)(max_tiles * sub) : (unsigned)ceil_div(p.M, BM_);
-  kernel<<<dim3(ceil_div(p.N, GATED ? FN / 2 : FN), y), 256, F32Tile<BM_>::SMEM, stream>>>(p, sub);
+  kernel<<<dim3(ceil_div(p.N, GATED ? FN / 2 : FN), y), FWARPS * 32, F32Tile<BM_>::SMEM, stream>>>(p, sub);
   return 0;
 }
 
