@@ -144,16 +144,17 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
   auto fetch = [&](int j0, int which) {
     bf16* dst = sK + (size_t)which * LM_KEYS * qs;
     if (vec) {
+      // (a warp a key: what a key's place costs, two divisions among it, is paid once a row and not once a piece)
       const int per_row = Dk >> 3;                               // 16-byte pieces of a cached row
-      for (int i = threadIdx.x; i < LM_KEYS * per_row; i += blockDim.x) {
-        const int kk = i / per_row, c = (i - kk * per_row) << 3;
+      for (int kk = threadIdx.x >> 5; kk < LM_KEYS; kk += blockDim.x >> 5) {
         const int page = s_page[which][kk];
-        bf16* to = dst + (size_t)kk * qs + c;
-        if (page >= 0) {
-          const bf16* from = p.cache + ((long long)page * p.page_size + (j0 + kk) % p.page_size) * Dk + c;
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
-        } else {
-          *reinterpret_cast<uint4*>(to) = make_uint4(0u, 0u, 0u, 0u);
+        bf16* to = dst + (size_t)kk * qs;
+        const bf16* from = p.cache + ((long long)page * p.page_size + (j0 + kk) % p.page_size) * Dk;
+        for (int c = lane; c < per_row; c += 32) {
+          if (page >= 0)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 8 * c)), "l"(from + 8 * c) : "memory");
+          else
+            *reinterpret_cast<uint4*>(to + 8 * c) = make_uint4(0u, 0u, 0u, 0u);
         }
       }
     } else {
@@ -173,15 +174,15 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
   // The query rows, rounded to bfloat16 (zero beyond the pairs and Dk). They are asked for behind the first key tile, eight
   // entries and several pieces a thread at a time: with an entry a load their round trips were a third of a decode step's kernel.
   if ((Dk & 7) == 0 && ((uintptr_t)p.q & 15) == 0) {
-    const int per_row = qs >> 3, pieces = LM_ROWS * per_row;
-    constexpr int AT_ONCE = 4;
+    const int per_row = qs >> 3, mine = min(LM_ROWS, pairs - f0), pieces = mine * per_row;
+    constexpr int AT_ONCE = 6;
     for (int i0 = threadIdx.x; i0 < pieces; i0 += AT_ONCE * blockDim.x) {
       float4 x[AT_ONCE], y[AT_ONCE];
 #pragma unroll
       for (int u = 0; u < AT_ONCE; ++u) {
         const int i = i0 + u * blockDim.x, m = i / per_row, c = (i - m * per_row) << 3;
         x[u] = y[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < pieces && f0 + m < pairs && c < Dk) {
+        if (i < pieces && c < Dk) {
           const float* src = p.q + ((long long)row_base * H + f0 + m) * Dk + c;
           x[u] = load4_now(src);
           y[u] = load4_now(src + 4);
@@ -195,6 +196,8 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
               make_uint4(pack_bf16(x[u].x, x[u].y), pack_bf16(x[u].z, x[u].w), pack_bf16(y[u].x, y[u].y), pack_bf16(y[u].z, y[u].w));
       }
     }
+    for (int i = mine * per_row + threadIdx.x; i < LM_ROWS * per_row; i += blockDim.x)      // (no pair: zeros)
+      *reinterpret_cast<uint4*>(sQ + (size_t)i * 8) = make_uint4(0u, 0u, 0u, 0u);
   } else {
     for (int i = threadIdx.x; i < LM_ROWS * (qs / 2); i += blockDim.x) {
       const int m = i / (qs / 2), c = 2 * (i - m * (qs / 2));
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
     // S = Q K^T for the warp's 16 pairs and the tile's 32 keys, both operands by ldmatrix (A: rows 0..7 and 8..15 of the block's
     // first and last eight entries; B: eight keys' first and last eight entries, two groups of keys a load). With two groups of
     // warps on the same pairs each takes 16 of the keys and hands its scores to the other through shared memory. (Prompts of 300
-    // and 700 rows, 32 heads, a latent of 512: 447 us with 32-bit operand loads and every score made twice, 319 us so.)
+    // and 700 rows, 32 heads, a latent of 512: 447 us with 32-bit operand loads and every score made twice, 319 us so, 272 us with a warp a key in front.)
     float s[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
@@ -347,13 +350,21 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
         }
     } else {
       const long long at = pair * p.n_spans + blockIdx.z;
+      if ((L & 1) == 0) {
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int c = chunk0 + n * 8 + 2 * t + e;
-          if (c < L) p.part_o[at * L + c] = o[n][2 * r + e];
+        for (int n = 0; n < NT; ++n) {
+          const int c = chunk0 + n * 8 + 2 * t;
+          if (c < L) *reinterpret_cast<float2*>(p.part_o + at * L + c) = make_float2(o[n][2 * r], o[n][2 * r + 1]);
         }
+      } else {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int c = chunk0 + n * 8 + 2 * t + e;
+            if (c < L) p.part_o[at * L + c] = o[n][2 * r + e];
+          }
+      }
       if (chunk_index == 0 && t == 0) {
         p.part_ml[at * 2] = m_run[r];
         p.part_ml[at * 2 + 1] = l_run[r];
