@@ -112,7 +112,10 @@ __device__ __noinline__ float activation_any(float v, int act) { return gate_act
 
 __device__ __forceinline__ float plain_result(float v, int act) { return act < 0 ? gate_activation(v, -act) : v; }
 
-template <int BN, bool SWAP, bool SWIGLU>
+// DEEP: the swapped plain product where its CTAs are at most one an SM and have more k-blocks than the three stages that let three
+// CTAs share an SM: as many as fit (64 rows against 14336 x 2048, 112 CTAs 21.0 -> 18.7 us; 37 rows against 6144 x 2048, 48 CTAs
+// 16.7 -> 14.6 us).
+template <int BN, bool SWAP, bool SWIGLU, bool DEEP = false>
 struct Smem {
   static constexpr int A_BYTES = TILE_M * TILE_K * 2;                  // the M-side tile
   static constexpr int B_BYTES = BN * TILE_K * 2;                      // the N-side tile
@@ -125,7 +128,7 @@ struct Smem {
   // expert tiles (a few hundred CTAs) into one wave.
   // The swapped plain product keeps to a third: its CTAs stream little each (a decode step's down projections are a
   // few hundred CTAs of half a MB), and three an SM put them into one wave.
-  static constexpr int BUDGET = SWAP ? (SWIGLU ? 110 * 1024 : 74 * 1024) : 100 * 1024;
+  static constexpr int BUDGET = DEEP ? 200 * 1024 : SWAP ? (SWIGLU ? 110 * 1024 : 74 * 1024) : 100 * 1024;
   static constexpr int FIT = BUDGET / STAGE_BYTES;
   static constexpr int STAGES = FIT > 8 ? 8 : (FIT < 2 ? 2 : FIT);
   static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
@@ -134,10 +137,10 @@ struct Smem {
                                    : TMEM_COLS_RAW <= 256 ? 256 : 512;
 };
 
-template <int BN, bool SWAP, bool SWIGLU, typename TOut>
+template <int BN, bool SWAP, bool SWIGLU, typename TOut, bool DEEP = false>
 __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW,
                                                       const __grid_constant__ CUtensorMap tmX, TcParams p) {
-  using S = Smem<BN, SWAP, SWIGLU>;
+  using S = Smem<BN, SWAP, SWIGLU, DEEP>;
   // Chained launches: the weights are written by no kernel, so a product without a tile map sets itself up and
   // requests its first weight tiles before it waits for the kernels in front of it; only the token rows, and
   // everything a grouped product reads through the tile map, have to wait.
@@ -666,10 +669,10 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const bf16* __restrict
 }
 
 // ------------------------------------------------------------------------------------------ host side
-template <int BN, bool SWAP, bool SWIGLU, typename TOut>
-static int launch_one(const CUtensorMap& tmW, const CUtensorMap& tmX, const TcParams& p, dim3 grid, cudaStream_t stream) {
-  using S = Smem<BN, SWAP, SWIGLU>;
-  auto kernel = gemm_tc_kernel<BN, SWAP, SWIGLU, TOut>;
+template <int BN, bool SWAP, bool SWIGLU, typename TOut, bool DEEP>
+static int launch_form(const CUtensorMap& tmW, const CUtensorMap& tmX, const TcParams& p, dim3 grid, cudaStream_t stream) {
+  using S = Smem<BN, SWAP, SWIGLU, DEEP>;
+  auto kernel = gemm_tc_kernel<BN, SWAP, SWIGLU, TOut, DEEP>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
@@ -677,6 +680,15 @@ static int launch_one(const CUtensorMap& tmW, const CUtensorMap& tmX, const TcPa
     configured = true;
   }
   return (int)launch_chained(kernel, grid, dim3(192), S::TOTAL, stream, tmW, tmX, p);
+}
+
+template <int BN, bool SWAP, bool SWIGLU, typename TOut>
+static int launch_one(const CUtensorMap& tmW, const CUtensorMap& tmX, const TcParams& p, dim3 grid, cudaStream_t stream) {
+  if constexpr (SWAP && !SWIGLU && BN <= 128) {
+    if (!p.tile_group && (long long)grid.x * grid.y * grid.z <= sm_count() && p.k_blocks_per_split > Smem<BN, SWAP, SWIGLU>::STAGES)
+      return launch_form<BN, SWAP, SWIGLU, TOut, true>(tmW, tmX, p, grid, stream);
+  }
+  return launch_form<BN, SWAP, SWIGLU, TOut, false>(tmW, tmX, p, grid, stream);
 }
 
 template <bool SWIGLU, typename TOut>
