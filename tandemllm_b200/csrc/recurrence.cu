@@ -544,6 +544,54 @@ __global__ void __launch_bounds__(128) group_norm_gate_warp_kernel(const float* 
   }
 }
 
+// The same for groups of more than 256 entries whose rows, gates and weights lie in 16-byte pieces, up to two a thread: everything
+// a row needs is asked for before its squares are summed. Four rows of 2048 took 8.6 us with a number a load and the gate and the weight
+// behind the sum, 2.3 us here; 1997 rows 20.6 and 12.9 us.
+__device__ __forceinline__ float4 load_gate4(const float* p) { return load4_now(p); }
+__device__ __forceinline__ float4 load_gate4(const bf16* p) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename T, typename G>
+__global__ void __launch_bounds__(512) group_norm_gate_vec_kernel(const float* __restrict__ y, const G* __restrict__ gate,
+                                                                  long long ld_gate, const float* __restrict__ weight, float eps,
+                                                                  float scale, T* __restrict__ out, long long ld_out, int width,
+                                                                  int group, int silu_gate, int shared_weight) {
+  __shared__ float red[32];
+  constexpr int MOST = 2;
+  const int r = blockIdx.x, c0 = blockIdx.y * group;
+  const float* yr = y + (long long)r * width + c0;
+  float4 v[MOST], g[MOST], w[MOST];
+  float ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < MOST; ++e) {
+    const int i = (threadIdx.x + e * blockDim.x) * 4;
+    v[e] = g[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    w[e] = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (i < group) {
+      v[e] = load4_now(yr + i);
+      g[e] = load_gate4(gate + (long long)r * ld_gate + c0 + i);
+      if (weight) w[e] = load4_now(weight + (shared_weight ? 0 : c0) + i);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < MOST; ++e) ss = dot4(v[e], v[e], ss);
+  const float inv = 1.f / sqrtf(block_sum_once(ss, red) / (float)group + eps);
+  auto made = [&](float x, float z, float m) {
+    const float a = silu_gate ? z / (1.f + expf(-z)) : 1.f / (1.f + expf(-z));
+    return x * inv * m * a * scale;
+  };
+#pragma unroll
+  for (int e = 0; e < MOST; ++e) {
+    const int i = (threadIdx.x + e * blockDim.x) * 4;
+    if (i < group)
+      store4(out + (long long)r * ld_out + c0 + i, made(v[e].x, g[e].x, w[e].x), made(v[e].y, g[e].y, w[e].y),
+             made(v[e].z, g[e].z, w[e].z), made(v[e].w, g[e].w, w[e].w));
+  }
+}
+
 }  // namespace tl
 
 using namespace tl;
@@ -673,8 +721,15 @@ extern "C" int tl_group_norm_gate(const float* y, const void* gate, long long ld
   const int group = width / groups;
   const int threads = group >= 1024 ? 256 : (group >= 256 ? 128 : (group > 32 ? 64 : 32));
   dim3 grid(rows, groups);
+  const uintptr_t all = (uintptr_t)y | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out;
+  const bool pieces = group > 256 && group <= 4096 && group % 4 == 0 && ld_gate % 4 == 0 && ld_out % 4 == 0 && (all & 15) == 0;
+  const int vthreads = group >= 2048 ? 512 : ceil_div(group / 4, 32) * 32;
 #define TL_GNG(T_, G_)                                                                                                   \
-  if (group <= 256)                                                                                                      \
+  if (pieces)                                                                                                            \
+    group_norm_gate_vec_kernel<T_, G_><<<grid, vthreads, 0, stream>>>(y, (const G_*)gate, ld_gate, weight, eps, scale,    \
+                                                                      (T_*)out, ld_out, width, group, silu_gate,         \
+                                                                      shared_weight);                                    \
+  else if (group <= 256)                                                                                                      \
     group_norm_gate_warp_kernel<T_, G_><<<(unsigned)(((long long)rows * groups + 3) / 4), 128, 0, stream>>>(              \
         y, (const G_*)gate, ld_gate, weight, eps, scale, (T_*)out, ld_out, rows, groups, group, silu_gate, shared_weight); \
   else                                                                                                                   \

@@ -176,3 +176,22 @@ def test_a_product_a_head_for_a_few_rows(rows, N, K, gate):
                               logits.to(DEV) if gate else None, gate == "heads")
         assert rel(out[..., :N].float(), want) < TOL[dtype] + 1e-5
         assert not out[..., N:].any()
+
+
+@pytest.mark.parametrize("dtype,gate_dtype", [("float32", "float32"), ("bfloat16", "float32"), ("bfloat16", "bfloat16")])
+@pytest.mark.parametrize("group,parts", [(260, 3), (2048, 1), (2052, 2), (4096, 1), (4100, 1), (258, 1)])
+def test_norm_of_parts_times_a_gate(group, parts, dtype, gate_dtype):
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(group)
+    width = group * parts
+    y, w = draw(g, 3, width), 1 + draw(g, width, scale=0.2)
+    gate = draw(g, 3, width + 4, dtype=DT[gate_dtype])
+    for silu, weight in ((False, w), (True, None)):
+        out = torch.zeros(3, width + 4, dtype=DT[dtype], device=DEV)
+        ops.group_norm_gate(y.to(DEV), gate.to(DEV), width + 4, None if weight is None else weight.to(DEV), 1e-5, parts, 0.75,
+                            out[:, :width], "silu" if silu else "sigmoid")
+        v, z = y.double().view(3, parts, group), gate[:, :width].double()
+        want = (v / (v.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()).view(3, width) * (1 if weight is None else weight.double())
+        want = want * (z if silu else 1) * torch.sigmoid(z) * 0.75
+        assert rel(out[:, :width].float(), want) < TOL[dtype]
+        assert not out[:, width:].any()
