@@ -43,6 +43,7 @@ SKINNY_RUN_ROWS = 16            # rows up to which a longer reduction whose sums
 SKINNY_ROWS = 16                # rows of a step up to which the experts go to its grouped form, over plan tiles of 8 (an
                                 # expert with more pairs has two tiles, and the second reads its weights from L2); measured
                                 # against the tcgen05 form: 8 % faster a step at 16 rows, even at 24, 4 % slower at 32
+FEW_ACT_ROWS = 8                # rows up to which a dense feed-forward's activation is in its product's epilogue
 SKINNY_PAIRS = 24               # routed pairs of such a step up to which its products run without a routing plan
 PROMPT_ATTENTION = "tcgen05"    # prompt portions of head size 64: the tcgen05 kernel (csrc/attention_tc.cu), or "mma" for the
                                 # mma.sync kernel that also takes them (kept for head size 128 and for comparison)
@@ -179,6 +180,7 @@ class TensorCore:
         self.branch = 0             # which of several chains of products that keep partial sums for one norm is running
         self._workspaces = {}
         self._pair_order = None
+        self._counts = None
         self._pairs = None
         self._outgrown = []
 
@@ -295,6 +297,32 @@ class TensorCore:
         self.gemm(x, w_gate_up, bias, out, swiglu=act, swap=False, n_out=inter)
         return True
 
+    def gated_few_rows(self, x, w_gate_up, out, act: int = 1, bias=None) -> bool:
+        """`gated` for a decode step of up to FEW_ACT_ROWS rows, without a bias; False for anything else."""
+        inter = w_gate_up.shape[0] // 2
+        if bias is not None or out.stride(-1) != 1 or out.dtype != torch.bfloat16 or not self._few_rows_through(x, w_gate_up, inter):
+            return False
+        self._few_rows_act(x, w_gate_up, out, act, inter)
+        return True
+
+    def _few_rows_through(self, x, w, n_out: int) -> bool:
+        """Whether a feed-forward's first product and its activation go through the experts' register-only kernel as one group:
+        up to 8 rows (what its CTAs take), the weights `linear` sends to the register-only product, and outputs for two CTAs an SM
+        (7168 gated outputs of 2048: 12.5 us against 11.1 us and 2.1 us for the activation behind it, and a launch less; 1536, 96
+        CTAs: 7.5 us against 4.5 and 2.0). The activation then meets 32-bit sums, not rounded ones."""
+        M, K = x.shape
+        return (1 <= M <= FEW_ACT_ROWS and K <= SKINNY_K and w.numel() * 2 <= SKINNY_BYTES and -(-n_out // 16) >= 2 * self.sm_count
+                and usable(x, w))
+
+    def _few_rows_act(self, x, w, out, act: int, n_out: int) -> None:
+        M, K = x.shape
+        if self._counts is None:
+            self._counts = torch.arange(FEW_ACT_ROWS + 1, dtype=torch.int32, device=self.device)
+        at = self._counts.data_ptr()                    # 0, 1, 2, ...: one tile, group 0, from row 0, of M rows
+        _check(lib().tl_gemm_skinny_grouped(x.data_ptr(), x.stride(0), None, 1, w.data_ptr(), w.stride(0), w.shape[0], out.data_ptr(),
+                                            out.stride(0), n_out, K, int(act), ops.dtype_code(out.dtype), at, at, at + 4 * M, at + 4,
+                                            1, None, 0, 1, self.status.data_ptr(), None, None, ops.stream()), "gemm_skinny_grouped")
+
     def linear(self, x, w, bias, out, defer: bool = False):
         """False when the kernels do not take these operands; else True, or the deferred partial sums."""
         if not usable(x, w) or out.stride(-1) != 1:
@@ -323,10 +351,15 @@ class TensorCore:
         return self.gemm(x, w, bias, out, defer=defer) or True
 
     def linear_act(self, x, w, act: int, a0: float = 0.0, a1: float = 0.0):
-        """act(x @ w^T) in bfloat16 with the activation in the epilogue of the prompt-sized product (pairs of SMs), or None
-        when that kernel does not take these operands: a decode step's few rows, strides TMA cannot box (the caller then
-        runs the product and the activation one after the other, as a gated feed-forward does for a decode step)."""
+        """act(x @ w^T) in bfloat16 with the activation in the epilogue of the prompt-sized product (pairs of SMs) or, for up to
+        FEW_ACT_ROWS rows, of the experts' register-only one (which has the gates' four activations without constants), or None when
+        neither takes these operands: rows in between, strides TMA cannot box (the caller then runs the product and the activation
+        one after the other)."""
         M, N = x.shape[0], w.shape[0]
+        if 1 <= act <= ops.ACTIVATIONS["identity"] and self._few_rows_through(x, w, N):
+            out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+            self._few_rows_act(x, w, out, -act, N)
+            return out
         if M <= 128 or PROMPT_PRODUCT != "pair" or not usable(x, w) or N % 8:
             return None
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)

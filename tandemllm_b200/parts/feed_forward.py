@@ -79,8 +79,9 @@ class SwiGLU(Part):
         tc = self.runtime.tensorcore
         if self.gate_constants is not None:
             ops.gate_constants(*self.gate_constants)
-        # prompts: gate, up and act(gate) * up in one kernel
-        if tc is None or not tc.gated(x, self.w_gate_up, act, self.act, self.b_gate_up):
+        # prompts and steps of up to eight rows: gate, up and act(gate) * up in one kernel
+        if tc is None or not (tc.gated_few_rows(x, self.w_gate_up, act, self.act, self.b_gate_up)
+                              or tc.gated(x, self.w_gate_up, act, self.act, self.b_gate_up)):
             gu = linear(self.runtime, x, self.w_gate_up, self.b_gate_up)
             ops.gated_mul(gu, act, self.act)
         return linear(self.runtime, act, self.w_down, self.b_down, out_dtype=torch.float32, defer=True)

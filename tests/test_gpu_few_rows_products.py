@@ -62,3 +62,25 @@ def test_grouped_products_of_pairs_without_a_plan(R, k, E, N, K, gated):
         want[p] = torch.nn.functional.silu(y[:N]) * y[N:] if gated else y
     assert int(status.item()) == 0
     assert rel(out, want) < 1e-5
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9])
+@pytest.mark.parametrize("inter,K", [(2368, 32), (4736, 264), (4760, 2048), (40, 264)])
+def test_feed_forward_activations_in_the_products_epilogue(M, inter, K):
+    """32-bit sums, activated in 32-bit and rounded once: a last place of bfloat16. Nine rows, other activations and products of
+    fewer than two CTAs of 16 outputs an SM go elsewhere."""
+    tc = tensor_core()
+    gates, plain = (M <= 8 and -(-n // 16) >= 2 * tc.sm_count for n in (inter, 2 * inter))
+    g = torch.Generator().manual_seed(M + inter)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16)
+    w = (torch.randn(2 * inter, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    z = x.double() @ w.double().T
+    out = torch.empty(M, inter, dtype=torch.bfloat16, device=DEV)
+    assert tc.gated_few_rows(x.to(DEV), w.to(DEV), out, 1) == gates
+    if gates:
+        assert rel(out, torch.nn.functional.silu(z[:, :inter]) * z[:, inter:]) < 2.0 ** -8
+    got = tc.linear_act(x.to(DEV), w.to(DEV), 3)
+    assert (got is not None) == plain
+    if plain:
+        assert rel(got, z.clamp(min=0) ** 2) < 2.0 ** -8
+    assert tc.linear_act(x.to(DEV), w.to(DEV), 8) is None          # tanh: not one of the kernel's
