@@ -478,7 +478,9 @@ static bool f32_pieces(const GemmParams& p, int max_tiles) {
 }
 
 static int launch_f32_any(const GemmParams& p, int max_tiles, cudaStream_t stream) {
-  if (!p.tile_group && p.M <= 8) {
+  // (weights of less than a megabyte are not worth a kernel of their own for a few rows, whose other order of additions would be all
+  // that a small model's prompt sees of where it was cut)
+  if (!p.tile_group && p.M <= 8 && (long long)p.N * p.K >= 1 << 18) {
     const int blocks = ceil_div(p.N, 16);
     if (p.M == 1) gemm_f32_few_kernel<1><<<blocks, 256, 0, stream>>>(p);
     else if (p.M <= 4) gemm_f32_few_kernel<4><<<blocks, 256, 0, stream>>>(p);
