@@ -3,10 +3,13 @@
 //
 //   C[m, n] = sum_k A[m, k] * W[n, k] (+ bias[n])            both operands row-major with k contiguous
 //
-// Each output element is accumulated in an order that depends on k alone (ascending, by one thread; the kernels for
-// 16-byte pieces: four such chains, see there), so a row's result
+// The order in which an output's products are added depends on k alone in each kernel: ascending, by one thread, in the tiled kernels;
+// in those for 32-bit operands of whole 16-byte pieces the eight chains described there, whatever the tile's height. So with
+// 32-bit operands of whole pieces and more than 64 outputs, and in every grouped product, a row's result
 // does not depend on how many other rows the call has (the reference's row invariance,
-// engine/models/lfm2_moe/kernels.py:290-306). The same kernel runs the experts: a tile map built on the
+// engine/models/lfm2_moe/kernels.py:290-306). Plain products of up to 64 outputs, of bfloat16 operands and of rows that are not whole
+// pieces have kernels of their own for up to 8 rows, with a warp's or a CTA's lanes along k: there a row's last bits differ between
+// a call of up to 8 rows and one of more. The same kernel runs the experts: a tile map built on the
 // device (moe_route.cu) names, per row tile, the expert whose weights it multiplies by and the rows of
 // the expert-sorted pair list it covers; with `swiglu` the epilogue is silu(gate) * up over the two
 // halves of the expert's fused [2 I, H] matrix (engine/models/lfm2_moe/ref.py:199-205).
@@ -258,16 +261,30 @@ __global__ void __launch_bounds__(256) gemm_tall_narrow_kernel(GemmParams p) {
 // An output is the sum of eight chains, a warp's even and odd k in ascending order over the quads q = warp (mod 4), added in
 // order: which k a chain has depends on k alone, whatever the tile's height, so a row still does not depend on the others, and
 // eight short chains lose less than one long one.
-constexpr int FK = 32, FPITCH = FK + 4, FSTAGES = 4, FN = 64, FWARPS = 4;
+//
+// Up to 8 rows are bound by the weights' bytes: tiles of 1, 2, 4 or 8 rows and so few outputs (8, 16 or 32) that the weights come
+// through as many SMs as there are, a lane an output where it goes (a weight is then read from shared memory once, by one lane), and
+// stages of 128 k-elements, eight of them for the narrow tiles, so that enough is in flight. Same chains, same order: it is what lets
+// a prompt be cut anywhere without a change in its products. 1 and 8 rows, outputs x k: 512 x 256 2.2 and 2.3 us (a warp an output,
+// lanes along k: 3.1 and 4.4), 512 x 1024 3.2 and 3.8 (a CTA an output: 3.3 and 3.7), 2048 x 2048 6.6 and 8.6 (a warp for two outputs: 6.8
+// and 26.5), 65536 x 2048 88 and 118 us (78 and, a warp an output, 265). A CTA an output is still faster only for some hundred outputs of a
+// long k (128 x 1024 2.5 and 2.8 us, 3.2 and 3.7 here).
+constexpr int FWARPS = 4;
+constexpr int FEW_ROWS = 8;
 
-template <int BM_>
+template <int BM_, int FN_>
 struct F32Tile {
-  static constexpr int TM = BM_ / 4;                                  // outputs a thread: TM x 8
-  static constexpr int STAGE = (BM_ + FN) * FPITCH;                   // floats
-  static constexpr int RED = FWARPS * BM_ * FN;                       // the warps' sums
-  static constexpr int SMEM = (FSTAGES * STAGE > RED ? FSTAGES * STAGE : RED) * 4;
-  static constexpr int ROWS_A_PASS = FWARPS * 4;                      // rows of [A tile; W tile] that the CTA's threads load at a time
-  static constexpr int LOADS = (BM_ + FN + ROWS_A_PASS - 1) / ROWS_A_PASS;     // 16-byte pieces a thread and stage
+  static constexpr bool FEW = BM_ <= FEW_ROWS;
+  static constexpr int FK = FEW ? 128 : 32, PITCH = FK + 4, STAGES = FEW && FN_ <= 16 ? 8 : 4;
+  static constexpr int TX = FEW ? FN_ : 8, TY = 32 / TX;              // lanes across outputs and across rows
+  static constexpr int TM = BM_ < TY ? 1 : BM_ / TY, TN = FN_ / TX;   // outputs a thread
+  static constexpr int STAGE = (BM_ + FN_) * PITCH;                   // floats
+  static constexpr int RED = FWARPS * TM * TN * 32;                   // the warps' sums
+  static constexpr int SMEM = (STAGES * STAGE > RED ? STAGES * STAGE : RED) * 4;
+  static constexpr int PIECES = FK / 4;                               // 16-byte pieces of a staged row
+  static constexpr int ROWS_A_PASS = FWARPS * 32 / PIECES;            // rows of [A tile; W tile] that the CTA's threads load at a time
+  static constexpr int LOADS = (BM_ + FN_ + ROWS_A_PASS - 1) / ROWS_A_PASS;    // pieces a thread and stage
+  static constexpr int CTAS = BM_ == 32 ? 2 : BM_ == 16 ? 3 : 2;      // an SM
 };
 
 __device__ __forceinline__ void cp16(uint32_t dst, const float* src, bool valid) {
@@ -282,10 +299,10 @@ __device__ __forceinline__ float both(unsigned long long v) {
 }
 
 // `sub`: how many CTA tiles a tile of the plan is cut into (grouped)
-template <int BM_, bool GATED>
-__global__ void __launch_bounds__(FWARPS * 32, BM_ == 32 ? 2 : 3) gemm_f32_kernel(GemmParams p, int sub) {
-  using T = F32Tile<BM_>;
-  constexpr int TM_ = T::TM;
+template <int BM_, int FN, bool GATED>
+__global__ void __launch_bounds__(FWARPS * 32, F32Tile<BM_, FN>::CTAS) gemm_f32_kernel(GemmParams p, int sub) {
+  using T = F32Tile<BM_, FN>;
+  constexpr int TM_ = T::TM, TN_ = T::TN, TX = T::TX, TY = T::TY, FK = T::FK, FPITCH = T::PITCH, FSTAGES = T::STAGES;
   extern __shared__ float4 f32_smem[];
   float* tiles = reinterpret_cast<float*>(f32_smem);
   int row0 = blockIdx.y * BM_, rows;
@@ -303,15 +320,15 @@ __global__ void __launch_bounds__(FWARPS * 32, BM_ == 32 ? 2 : 3) gemm_f32_kerne
   constexpr int OUTS = GATED ? FN / 2 : FN;          // outputs a CTA
   const int col0 = blockIdx.x * OUTS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ty = lane >> 3, tx = lane & 7;
+  const int ty = lane / TX, tx = lane % TX;
 
-  // what this thread loads: 16 bytes at k offset 4 (tid % 8) of rows tid / 8, + 16, ... of [A tile; W tile]
-  const int lk = (tid & 7) * 4;
+  // what this thread loads: a piece of row tid / PIECES and of every ROWS_A_PASS-th behind it of [A tile; W tile]
+  const int lrow = tid / T::PIECES, lk = (tid % T::PIECES) * 4;
   const float* src[T::LOADS];
   bool ok[T::LOADS];
 #pragma unroll
   for (int i = 0; i < T::LOADS; ++i) {
-    const int r = (tid >> 3) + T::ROWS_A_PASS * i;
+    const int r = lrow + T::ROWS_A_PASS * i;
     src[i] = W;
     ok[i] = false;
     if (r < BM_) {
@@ -330,14 +347,14 @@ __global__ void __launch_bounds__(FWARPS * 32, BM_ == 32 ? 2 : 3) gemm_f32_kerne
     }
   }
   const int steps = (p.K + FK - 1) / FK;
-  const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)(((tid >> 3) * FPITCH + lk) * 4);
+  const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)((lrow * FPITCH + lk) * 4);
   auto load = [&](int step) {
     if (step < steps) {
       const int k = step * FK + lk;
       const uint32_t at = smem0 + (uint32_t)((step % FSTAGES) * T::STAGE * 4);
 #pragma unroll
       for (int i = 0; i < T::LOADS; ++i)
-        if ((tid >> 3) + T::ROWS_A_PASS * i < BM_ + FN) {
+        if (lrow + T::ROWS_A_PASS * i < BM_ + FN) {
           const bool in = ok[i] && k < p.K;          // (K is a multiple of 4)
           cp16(at + (uint32_t)(T::ROWS_A_PASS * i * FPITCH * 4), in ? src[i] + k : W, in);
         }
@@ -345,11 +362,11 @@ __global__ void __launch_bounds__(FWARPS * 32, BM_ == 32 ? 2 : 3) gemm_f32_kerne
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  unsigned long long acc[TM_][8];                     // (sum over even k, sum over odd k)
+  unsigned long long acc[TM_][TN_];                   // (sum over even k, sum over odd k)
 #pragma unroll
   for (int i = 0; i < TM_; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TN_; ++j) acc[i][j] = 0ull;
 
   for (int s = 0; s < FSTAGES - 1; ++s) load(s);
   for (int step = 0; step < steps; ++step) {
@@ -357,43 +374,44 @@ __global__ void __launch_bounds__(FWARPS * 32, BM_ == 32 ? 2 : 3) gemm_f32_kerne
     __syncthreads();                                  // the stage is here, and everybody is done with the one before
     load(step + FSTAGES - 1);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const float* st = tiles + (step % FSTAGES) * T::STAGE + (warp + FWARPS * half) * 4;
-      const float* a_at = st + ty * FPITCH, * w_at = st + (BM_ + tx) * FPITCH;
-      ulonglong2 w[8];
+    for (int part = 0; part < FK / 16; ++part) {
+      const float* st = tiles + (step % FSTAGES) * T::STAGE + (warp + FWARPS * part) * 4;
+      const float* a_at = st + (BM_ < TY ? ty % BM_ : ty) * FPITCH, * w_at = st + (BM_ + tx) * FPITCH;
+      ulonglong2 w[TN_];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_at + j * 8 * FPITCH);
+      for (int j = 0; j < TN_; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_at + j * TX * FPITCH);
 #pragma unroll
       for (int m = 0; m < TM_; ++m) {
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_at + m * 4 * FPITCH);
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_at + m * TY * FPITCH);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) fma2(acc[m][j], a.x, w[j].x);
+        for (int j = 0; j < TN_; ++j) fma2(acc[m][j], a.x, w[j].x);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) fma2(acc[m][j], a.y, w[j].y);
+        for (int j = 0; j < TN_; ++j) fma2(acc[m][j], a.y, w[j].y);
       }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  float* red = tiles;                                // [warps][8 TM][32]
+  float* red = tiles;                                // [warps][TM][TN][32]
 #pragma unroll
   for (int m = 0; m < TM_; ++m)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) red[((warp * TM_ + m) * 8 + j) * 32 + lane] = both(acc[m][j]);
+    for (int j = 0; j < TN_; ++j) red[((warp * TM_ + m) * TN_ + j) * 32 + lane] = both(acc[m][j]);
   __syncthreads();
   auto sum = [&](int m, int j) {
     float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < FWARPS; ++w) v += red[((w * TM_ + m) * 8 + j) * 32 + lane];
+    for (int w = 0; w < FWARPS; ++w) v += red[((w * TM_ + m) * TN_ + j) * 32 + lane];
     return v;
   };
   float* C = (float*)p.C;
-  // a warp stores column blocks `warp` and (plain) `warp` + 4
+  // a warp stores every fourth of the TM x TN blocks of outputs (gated: the gate's column blocks are the first four)
+  constexpr int BLOCKS = GATED ? 4 : TN_;
 #pragma unroll
-  for (int i = 0; i < (GATED ? TM_ : 2 * TM_); ++i) {
-    const int m = GATED ? i : i >> 1;
-    const int j = GATED ? warp : warp + 4 * (i & 1);
-    const int lr = ty + 4 * m, n = col0 + tx + 8 * j;
+  for (int i = 0; i < (TM_ * BLOCKS + FWARPS - 1) / FWARPS; ++i) {
+    const int m = (warp + FWARPS * i) / BLOCKS, j = (warp + FWARPS * i) % BLOCKS;
+    if (m >= TM_) break;
+    const int lr = ty + TY * m, n = col0 + tx + TX * j;
     const float v = sum(m, j), u = GATED ? sum(m, j + 4) : 0.f;
     if (lr >= rows || n >= p.N) continue;
     const long long r = row0 + lr;
@@ -407,90 +425,49 @@ __global__ void __launch_bounds__(FWARPS * 32, BM_ == 32 ? 2 : 3) gemm_f32_kerne
   }
 }
 
-// Up to 8 rows: bound by the weights' bytes. A warp takes two outputs, each lane 16 bytes of either weight row, four k-steps in
-// flight. Four chains a lane and row (one a component), then the lanes. The head of one row (65536 x 2048, 537 MB):
-// 231 -> 78 us, 6.9 TB/s.
-template <int MAXM>
-__global__ void __launch_bounds__(256) gemm_f32_few_kernel(GemmParams p) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int n0 = 2 * warp;
-  if (n0 >= p.N) return;
-  const float* A = (const float*)p.A;
-  const float* w0 = (const float*)p.W + (long long)n0 * p.ldw;
-  const float* w1 = n0 + 1 < p.N ? w0 + p.ldw : w0;
-  unsigned long long acc[MAXM][2][2];
-#pragma unroll
-  for (int m = 0; m < MAXM; ++m) acc[m][0][0] = acc[m][0][1] = acc[m][1][0] = acc[m][1][1] = 0ull;
-  constexpr int U = 4;
-  for (int k0 = lane * 4; k0 < p.K; k0 += 128 * U) {
-    ulonglong2 a[U], b[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = k0 + 128 * u;
-      a[u] = b[u] = make_ulonglong2(0ull, 0ull);
-      if (k < p.K) {
-        a[u] = *reinterpret_cast<const ulonglong2*>(w0 + k);
-        b[u] = *reinterpret_cast<const ulonglong2*>(w1 + k);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = k0 + 128 * u;
-      if (k >= p.K) break;
-#pragma unroll
-      for (int m = 0; m < MAXM; ++m) {
-        if (m >= p.M) break;
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(A + (long long)m * p.lda + k);
-        fma2(acc[m][0][0], x.x, a[u].x);
-        fma2(acc[m][0][1], x.y, a[u].y);
-        fma2(acc[m][1][0], x.x, b[u].x);
-        fma2(acc[m][1][1], x.y, b[u].y);
-      }
-    }
-  }
-  float* C = (float*)p.C;
-#pragma unroll
-  for (int m = 0; m < MAXM; ++m) {
-    if (m >= p.M) break;
-    const float v0 = warp_sum(both(acc[m][0][0]) + both(acc[m][0][1])), v1 = warp_sum(both(acc[m][1][0]) + both(acc[m][1][1]));
-    if (lane < 2 && n0 + lane < p.N)
-      C[(long long)m * p.ldc + n0 + lane] = (lane ? v1 : v0) + (p.bias ? p.bias[n0 + lane] : 0.f);
-  }
-}
-
-template <int BM_, bool GATED>
+template <int BM_, int FN, bool GATED>
 static int launch_f32(const GemmParams& p, int max_tiles, cudaStream_t stream) {
   const int sub = p.tile_group ? BM / BM_ : 1;       // (a plan's tiles hold at most BM rows)
-  auto kernel = gemm_f32_kernel<BM_, GATED>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BM_>::SMEM);
-  if (e != cudaSuccess) return (int)e;
+  constexpr int SMEM = F32Tile<BM_, FN>::SMEM;
+  auto kernel = gemm_f32_kernel<BM_, FN, GATED>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
   const unsigned y = p.tile_group ? (unsigned)(max_tiles * sub) : (unsigned)ceil_div(p.M, BM_);
-  kernel<<<dim3(ceil_div(p.N, GATED ? FN / 2 : FN), y), FWARPS * 32, F32Tile<BM_>::SMEM, stream>>>(p, sub);
+  kernel<<<dim3(ceil_div(p.N, GATED ? FN / 2 : FN), y), FWARPS * 32, SMEM, stream>>>(p, sub);
   return 0;
 }
 
-// Whether the 16-byte kernels take these operands: rows that are whole pieces, a grid within its limit, and not one of the
-// narrow products (a router's), which have kernels of their own.
+// Tiles of 8, 16 or 32 outputs: the widest of which there is one for every SM (16 in place of 32: 6144 x 2048 14.3 us for a row, 11.8 so;
+// 64 in place of 32: 65536 x 2048 93 us, 88 so).
+template <int BM_>
+static int launch_f32_few(const GemmParams& p, cudaStream_t stream) {
+  if (p.N <= 8 * sm_count()) return launch_f32<BM_, 8, false>(p, 0, stream);
+  if (p.N <= 32 * sm_count()) return launch_f32<BM_, 16, false>(p, 0, stream);
+  return launch_f32<BM_, 32, false>(p, 0, stream);
+}
+
+// Whether the 16-byte kernels take these operands: rows that are whole pieces, a grid within its limit, and not a product of so few
+// outputs (a router's) that it has kernels of its own.
 static bool f32_pieces(const GemmParams& p, int max_tiles) {
   if (p.K % 4 || p.lda % 4 || p.ldw % 4 || p.w_group_stride % 4 || ((uintptr_t)p.A & 15) || ((uintptr_t)p.W & 15)) return false;
   if (p.tile_group) return (long long)max_tiles * (BM / 16) <= 65535;
-  return p.N > 64 && ceil_div(p.M, 16) <= 65535 && (p.M > 8 || p.N > 512 || p.K < 512);
+  return p.N > 64 && ceil_div(p.M, 16) <= 65535;
 }
 
 static int launch_f32_any(const GemmParams& p, int max_tiles, cudaStream_t stream) {
-  // (weights of less than a megabyte are not worth a kernel of their own for a few rows, whose other order of additions would be all
-  // that a small model's prompt sees of where it was cut)
-  if (!p.tile_group && p.M <= 8 && (long long)p.N * p.K >= 1 << 18) {
-    const int blocks = ceil_div(p.N, 16);
-    if (p.M == 1) gemm_f32_few_kernel<1><<<blocks, 256, 0, stream>>>(p);
-    else if (p.M <= 4) gemm_f32_few_kernel<4><<<blocks, 256, 0, stream>>>(p);
-    else gemm_f32_few_kernel<8><<<blocks, 256, 0, stream>>>(p);
-    return 0;
+  if (!p.tile_group && p.M <= FEW_ROWS) {
+    if (p.M == 1) return launch_f32_few<1>(p, stream);
+    if (p.M == 2) return launch_f32_few<2>(p, stream);
+    return p.M <= 4 ? launch_f32_few<4>(p, stream) : launch_f32_few<8>(p, stream);
   }
   // tiles of 16 rows for what fits one; grouped, where an expert has as few on average (max_tiles: the experts or more)
   const bool low = p.tile_group ? p.M <= 10 * max_tiles : p.M <= 16;
-  if (p.swiglu > 0) return low ? launch_f32<16, true>(p, max_tiles, stream) : launch_f32<32, true>(p, max_tiles, stream);
-  return low ? launch_f32<16, false>(p, max_tiles, stream) : launch_f32<32, false>(p, max_tiles, stream);
+  if (p.swiglu > 0) return low ? launch_f32<16, 64, true>(p, max_tiles, stream) : launch_f32<32, 64, true>(p, max_tiles, stream);
+  return low ? launch_f32<16, 64, false>(p, max_tiles, stream) : launch_f32<32, 64, false>(p, max_tiles, stream);
 }
 
 template <typename TIn, typename TOut>

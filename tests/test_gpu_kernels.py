@@ -423,6 +423,18 @@ def test_gemm_simt_in_16_byte_pieces(M, N, K):
         assert torch.equal(few, out[M - 9:])
 
 
+@pytest.mark.parametrize("N,K", [(65, 4), (128, 256), (513, 36), (128, 1024), (513, 1024), (70, 2052), (1030, 520), (2048, 2048)])
+def test_gemm_simt_in_16_byte_pieces_row_by_row(N, K):
+    """More than 64 outputs: a row has the same bits alone, among up to eight rows (a kernel of their own) and in the tiles of 16
+    and 32 rows, so where a prompt is cut changes no product."""
+    o = ops()
+    x, w, b = rnd(33, K, seed=6).to(DEV), rnd(N, K, seed=7).to(DEV), rnd(N, seed=8).to(DEV)
+    made = lambda n: o.gemm_simt(x[:n], w, b, torch.empty(n, N, device=DEV))
+    whole = made(33)
+    for n in (1, 2, 4, 5, 8, 9, 16, 17):
+        assert torch.equal(made(n), whole[:n]), n
+
+
 @pytest.mark.parametrize("R,E,k,H,I", [(3, 8, 2, 64, 68), (40, 3, 2, 36, 132), (200, 4, 2, 100, 64), (130, 2, 1, 32, 40)])
 @pytest.mark.parametrize("act", [1, 0, -3])
 def test_grouped_gemm_in_16_byte_pieces(R, E, k, H, I, act):
