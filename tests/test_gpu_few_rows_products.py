@@ -84,3 +84,44 @@ def test_feed_forward_activations_in_the_products_epilogue(M, inter, K):
     if plain:
         assert rel(got, z.clamp(min=0) ** 2) < 2.0 ** -8
     assert tc.linear_act(x.to(DEV), w.to(DEV), 8) is None          # tanh: not one of the kernel's
+
+
+@pytest.mark.parametrize("M", [1, 8, 33, 37, 64, 65, 127, 128])
+@pytest.mark.parametrize("N,K", [(5000, 4104), (9480, 2056), (14400, 2056), (18900, 1096), (4096, 2560)])
+def test_swapped_products_cut_and_uncut(M, N, K):
+    """Fewer tiles than SMs: the ring as deep as it goes where k is not cut, partial sums that a kernel of its own adds where it is,
+    or that are left to the consumer; last tiles, k-blocks and blocks of 16 rows that are not full. 32-bit sums of bfloat16 products, plus the rounding of a
+    bfloat16 result; rows behind the last one are not written."""
+    from tandemllm_b200.kernels import ops
+    tc = tensor_core()
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x, w = (torch.randn(n, K, generator=g, device=DEV).to(torch.bfloat16) for n in (M, N))
+    w = (w.float() * K ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device=DEV)
+    want = x.double() @ w.double().T + bias.double()
+    for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 1e-5 + 2.0 ** -8)):
+        for defer in (False, "rounded"):
+            whole = torch.full((M + 1, N), 7.0, dtype=dtype, device=DEV)
+            got = tc.gemm(x, w, bias, whole[:M], defer=defer)
+            assert got is None or defer
+            assert rel((whole[:M] if got is None else ops.materialize(got)).float(), want) < tol, (dtype, defer)
+            assert bool((whole[M] == 7).all())
+
+
+@pytest.mark.parametrize("act,name", [(3, "relu2"), (1, "silu")])
+@pytest.mark.parametrize("M", [1, 17, 40])
+def test_swapped_grouped_products_with_an_activation(act, name, M):
+    """An ungated activation in the swapped epilogue (experts without a gate), rows of a group that are not a multiple of 16."""
+    from tandemllm_b200.kernels import ops
+    tc = tensor_core()
+    g = torch.Generator(device=DEV).manual_seed(M)
+    E, N, K = 3, 264, 520
+    x = torch.randn(2 * M, K, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    ids = torch.tensor([[0]] * M + [[2]] * M, dtype=torch.int32, device=DEV)
+    plan = ops.MoePlan(2 * M, E, 64, DEV).build(ids)
+    out = torch.empty(2 * M, N, dtype=torch.bfloat16, device=DEV)
+    tc.gemm(x, w.view(E * N, K), None, out, rows_per_group=N, plan=plan, swiglu=-act, swap=True, bn=64, n_out=N)
+    z = torch.cat([x[:M].double() @ w[0].double().T, x[M:].double() @ w[2].double().T])
+    want = z.clamp(min=0) ** 2 if name == "relu2" else torch.nn.functional.silu(z)
+    assert rel(out.float(), want) < 1e-5 + 2.0 ** -8
