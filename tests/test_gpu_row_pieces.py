@@ -68,6 +68,33 @@ def test_norm_behind_a_branch_with_a_gate_that_is_not_computed_yet(dtype, width,
     assert rel(out.float(), w2.double() * new / (new.pow(2).mean(-1, keepdim=True) + 1e-4).sqrt()) < TOL[dtype]
 
 
+@pytest.mark.parametrize("width,top", [(50, 1), (2050, 6), (4094, 3), (4098, 2), (131, 0)])
+def test_norm_behind_a_branch_at_widths_four_does_not_divide(width, top):
+    """A number a load: the form of a step of few rows (up to two a SM, rows of up to 4096 numbers) and the other give a row the same
+    bits, and those of the formula."""
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(width)
+    R = 400
+    res, dense = draw(g, R, width), draw(g, R, width)
+    w, w2 = 1 + draw(g, width, scale=0.2), 1 + draw(g, width, scale=0.2)
+    experts, d = None, dense.double()
+    if top:
+        rows = draw(g, R * top, width)
+        ids = torch.stack([torch.randperm(40, generator=g)[:top] for _ in range(R)]).to(torch.int32)
+        wts, pos = torch.rand(R, top, generator=g), torch.arange(R * top, dtype=torch.int32)
+        d = d + (wts.double()[..., None] * rows.double().view(R, top, width)).sum(1)
+        experts = lambda n: ops.ExpertRows(rows[:n * top].to(DEV), pos[:n * top].to(DEV), ids[:n].to(DEV), wts[:n].to(DEV))
+    new = res.double() + w.double() * d / (d.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()
+    made = []
+    for n in (R, 3):
+        r, out = res[:n].to(DEV), torch.empty(n, width, device=DEV)
+        ops.add_normed(r, dense[:n].to(DEV), w.to(DEV), 1e-5, None, experts(n) if top else None, (w2.to(DEV), 1e-4, out, None))
+        assert rel(r, new[:n]) < 1e-5
+        assert rel(out, w2.double() * new[:n] / (new[:n].pow(2).mean(-1, keepdim=True) + 1e-4).sqrt()) < 1e-5
+        made.append((r[:3], out[:3]))
+    assert torch.equal(made[0][0], made[1][0]) and torch.equal(made[0][1], made[1][1])
+
+
 @pytest.mark.parametrize("Hq,Hk,D,VD,rot,turn_values", [(4, 2, 16, 8, 16, False), (3, 1, 64, 64, 32, True), (16, 4, 128, 128, 128, False),
                                                         (40, 8, 128, 64, 64, True), (2, 2, 24, 16, 0, False), (4, 2, 16, 8, 8, False)])
 def test_turned_heads_and_their_pages(Hq, Hk, D, VD, rot, turn_values):
