@@ -47,15 +47,20 @@ struct PostNormParams {
 // taken here because a kernel of its own cost 5.5 us and a launch for one number a row. Measured at two rows of 2048 in a decode
 // step, six slots beside a shared part in ten partial sums: 13.8 us with a number a load, 4.5 us here (with the gate's logit); 1000
 // rows 30.9 and 19.8 us.
-template <typename T, int VPT>
-__global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) add_normed_vec_kernel(PostNormParams p) {
+//
+// PLAIN: one dense source, no slots, no gate's rows, and more rows than the other form lets stand on the GPU at once (1024
+// threads an SM with a piece a thread; with more, two rounds of rows): with no loads to send ahead, an instantiation without their registers keeps more
+// rows on an SM and reads the norms' weights where they are used. 2000 and 6000 rows of 1536 13.1 and 39.1 -> 6.5 and 16.0 us (a
+// number a load 11.6 and 29.8), of 2048 15.4 and 53.9 -> 8.3 and 27.6 (13.5 and 50.4), of 2560 20.3 and 88.8 -> 8.5 and 33.0 (16.3 and 73.6).
+template <typename T, int VPT, bool PLAIN>
+__global__ void __launch_bounds__(512, PLAIN ? (VPT == 1 ? 3 : VPT == 2 ? 2 : 1) : VPT == 1 ? 2 : 1) add_normed_vec_kernel(PostNormParams p) {
   __shared__ float red[96];
   const int hidden = p.hidden, lane = threadIdx.x & 31;
   const int r = p.gather ? p.gather[blockIdx.x] : (int)blockIdx.x;
   // the row's slots in ascending expert id (the slot index breaks ties)
   int slot_src = 0, rank = -1;
   float slot_w = 0.f;
-  if (p.expert_rows) {
+  if (!PLAIN && p.expert_rows) {
     const int k = p.top_k, j = lane;
     const bool mine = j < k;
     const int e = mine ? p.ids[(long long)r * k + j] : 0x7fffffff;
@@ -76,12 +81,14 @@ __global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) add_normed_vec_kernel(P
     d[v] = x[v] = w[v] = pw[v] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < hidden) {
       x[v] = load4_now(res + c);
-      w[v] = load4_now(p.weight + c);
-      if (p.pre_weight) pw[v] = load4_now(p.pre_weight + c);
+      if (!PLAIN) {
+        w[v] = load4_now(p.weight + c);
+        if (p.pre_weight) pw[v] = load4_now(p.pre_weight + c);
+      }
     }
   }
   float g = 1.f;
-  if (p.gate_x) {
+  if (!PLAIN && p.gate_x) {
     float dot = 0.f;
     if (p.gate_bf16) {
       const bf16* gx = reinterpret_cast<const bf16*>(p.gate_x) + (long long)r * p.gate_ld;
@@ -111,7 +118,7 @@ __global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) add_normed_vec_kernel(P
   } else if (p.delta_gate) {
     g = 1.f / (1.f + expf(-p.delta_gate[r]));
   }
-  constexpr int AT_ONCE = VPT == 1 ? 4 : VPT == 2 ? 2 : 1;
+  constexpr int AT_ONCE = PLAIN ? 1 : VPT == 1 ? 4 : VPT == 2 ? 2 : 1;
   if (p.delta) {
     const float* src = p.delta + (size_t)r * hidden;
     for (int s0 = 0; s0 < p.parts; s0 += AT_ONCE) {
@@ -133,7 +140,7 @@ __global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) add_normed_vec_kernel(P
 #pragma unroll
     for (int v = 0; v < VPT; ++v) { d[v].x *= g; d[v].y *= g; d[v].z *= g; d[v].w *= g; }
   }
-  if (p.expert_rows) {
+  if (!PLAIN && p.expert_rows) {
     float4 routed[VPT];
 #pragma unroll
     for (int v = 0; v < VPT; ++v) routed[v] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -190,6 +197,7 @@ __global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) add_normed_vec_kernel(P
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     const int c = (threadIdx.x + v * blockDim.x) * 4;
+    if (PLAIN && c < hidden) w[v] = *reinterpret_cast<const float4*>(p.weight + c);
     x[v].x += d[v].x * inv * w[v].x;
     x[v].y += d[v].y * inv * w[v].y;
     x[v].z += d[v].z * inv * w[v].z;
@@ -203,6 +211,7 @@ __global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1) add_normed_vec_kernel(P
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     const int c = (threadIdx.x + v * blockDim.x) * 4;
+    if (PLAIN && c < hidden) pw[v] = *reinterpret_cast<const float4*>(p.pre_weight + c);
     if (c < hidden)
       store4(out + c, x[v].x * inv2 * pw[v].x, x[v].y * inv2 * pw[v].y, x[v].z * inv2 * pw[v].z, x[v].w * inv2 * pw[v].w);
   }
@@ -433,15 +442,24 @@ extern "C" int tl_add_normed(float* residual, const float* delta, int parts, lon
   p.pre_weight = pre_weight; p.pre_eps = pre_eps; p.normed = normed; p.gather = gather;
   p.gate_x = gate_x; p.gate_w = gate_w; p.gate_ld = gate_ld; p.gate_bf16 = gate_dtype == TL_BF16;
   if (hidden % 4 == 0 && hidden <= 8192 && add_normed_aligned(p)) {
-    const int pieces = hidden / 4, threads = pieces >= 512 ? 512 : ceil_div(pieces, 32) * 32, vpt = ceil_div(pieces, threads);
-#define TL_ADD_NORMED_VEC(V_)                                                                     \
-  do {                                                                                            \
-    if (dtype == TL_FP32) add_normed_vec_kernel<float, V_><<<rows, threads, 0, stream>>>(p);      \
-    else add_normed_vec_kernel<bf16, V_><<<rows, threads, 0, stream>>>(p);                        \
+    // (as few pieces a thread as 512 threads allow, and then as few threads as those need: 640 pieces are two for each of 320)
+    const int pieces = hidden / 4, vpt = ceil_div(pieces, 512), threads = ceil_div(ceil_div(pieces, vpt), 32) * 32;
+    const bool plain = !expert_rows && parts <= 1 && !gate_x && rows * (long long)threads > 1024LL * sm_count();
+#define TL_ADD_NORMED_VEC_(T_, V_, P_) add_normed_vec_kernel<T_, V_, P_><<<rows, threads, 0, stream>>>(p)
+#define TL_ADD_NORMED_VEC(V_)                               \
+  do {                                                      \
+    if (dtype == TL_FP32) {                                 \
+      if (plain) TL_ADD_NORMED_VEC_(float, V_, true);       \
+      else TL_ADD_NORMED_VEC_(float, V_, false);            \
+    } else {                                                \
+      if (plain) TL_ADD_NORMED_VEC_(bf16, V_, true);        \
+      else TL_ADD_NORMED_VEC_(bf16, V_, false);             \
+    }                                                       \
   } while (0)
     if (vpt == 1) TL_ADD_NORMED_VEC(1);
     else if (vpt == 2) TL_ADD_NORMED_VEC(2);
     else TL_ADD_NORMED_VEC(4);
+#undef TL_ADD_NORMED_VEC_
 #undef TL_ADD_NORMED_VEC
     TL_LAUNCH_CHECK();
     return 0;

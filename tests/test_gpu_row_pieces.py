@@ -222,3 +222,25 @@ def test_norm_of_parts_times_a_gate(group, parts, dtype, gate_dtype):
         want = want * (z if silu else 1) * torch.sigmoid(z) * 0.75
         assert rel(out[:, :width].float(), want) < TOL[dtype]
         assert not out[:, width:].any()
+
+
+@pytest.mark.parametrize("width", [4, 1536, 2048, 2052, 2560, 4100, 8192])
+def test_norm_behind_a_branch_of_many_rows(width):
+    """More rows than the form for few keeps on the GPU, one dense source and none of the rest: an instantiation of its own, the same bits a row."""
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(width)
+    R = 2500 if width > 512 else 160000
+    res, dense = torch.randn(R, width, generator=g, device=DEV), torch.randn(R, width, generator=g, device=DEV)
+    w, w2 = (1 + 0.2 * torch.randn(width, generator=g, device=DEV) for _ in range(2))
+    logits = torch.randn(R, generator=g, device=DEV)
+    for gate in (None, logits):
+        d = dense.double() * (1 if gate is None else torch.sigmoid(gate.double())[:, None])
+        new = res.double() + w.double() * d / (d.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()
+        made = []
+        for n in (R, 5):
+            r, out = res[:n].clone(), torch.empty(n, width, dtype=torch.bfloat16, device=DEV)
+            ops.add_normed(r, dense[:n].contiguous(), w, 1e-5, None if gate is None else gate[:n].contiguous(), None, (w2, 1e-4, out, None))
+            made.append((r[:5], out[:5]))
+            assert rel(r, new[:n]) < 1e-5
+            assert rel(out.float(), w2.double() * new[:n] / (new[:n].pow(2).mean(-1, keepdim=True) + 1e-4).sqrt()) < TOL["bfloat16"]
+        assert all(torch.equal(a, b) for a, b in zip(*made))
