@@ -15,8 +15,14 @@ namespace tl {
 // chain of round trips: the row and its sources are asked for together, up to eight partial sums at a time, and the norm's own
 // numbers before the first reduction. Measured at four rows of 2048 in a decode step with ten partial sums every other time:
 // 11.3 us with a number a load and a load a round trip, 3.3 us here; 1997 rows without partial sums 19.2 and 17.4 us.
-template <typename T, int VPT>
-__global__ void __launch_bounds__(512) add_layernorm_vec_kernel(float* __restrict__ residual, const float* __restrict__ delta,
+//
+// PLAIN: one source at most and more rows than the other form lets stand on the GPU at once (1024 threads an SM with a piece a thread;
+// with more pieces the line lies at two rounds of rows): with no loads to send ahead of others, an instantiation without their registers keeps more rows on an SM and
+// reads the norm's numbers where they are used. One source, 2000 and 6000 rows: of 2048 15.8 and 52.1 -> 10.7 and 36.1 us (a number a load
+// 16.8 and 57.1), of 2560 24.7 and 100.6 -> 11.0 and 39.6 (20.0 and 69.2; the 640 pieces of a row also went to 512 threads, 384 of which idled
+// through the second).
+template <typename T, int VPT, bool PLAIN>
+__global__ void __launch_bounds__(512, PLAIN ? (VPT == 1 ? 3 : VPT == 2 ? 2 : 1) : 0) add_layernorm_vec_kernel(float* __restrict__ residual, const float* __restrict__ delta,
                                                                 int parts, long long part_stride,
                                                                 const float* __restrict__ weight, const float* __restrict__ bias,
                                                                 float eps, T* __restrict__ out, const int* __restrict__ gather,
@@ -33,7 +39,7 @@ __global__ void __launch_bounds__(512) add_layernorm_vec_kernel(float* __restric
     x[v] = w[v] = b[v] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < hidden) x[v] = load4_now(res + c);
   }
-  constexpr int AT_ONCE = VPT == 1 ? 8 : VPT == 2 ? 4 : 1;
+  constexpr int AT_ONCE = PLAIN ? 1 : VPT == 1 ? 8 : VPT == 2 ? 4 : 1;
   for (int p0 = 0; p0 < parts; p0 += AT_ONCE) {
     float4 d[AT_ONCE][VPT];
 #pragma unroll
@@ -44,7 +50,7 @@ __global__ void __launch_bounds__(512) add_layernorm_vec_kernel(float* __restric
         if (p0 + p < parts && c < hidden) d[p][v] = load4_now(src + (size_t)(p0 + p) * part_stride + c);
         else d[p][v] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-    if (p0 == 0)
+    if (!PLAIN && p0 == 0)
 #pragma unroll
       for (int v = 0; v < VPT; ++v) {
         const int c = (threadIdx.x + v * blockDim.x) * 4;
@@ -59,7 +65,7 @@ __global__ void __launch_bounds__(512) add_layernorm_vec_kernel(float* __restric
 #pragma unroll
         for (int v = 0; v < VPT; ++v) add4(x[v], d[p][v]);
   }
-  if (parts == 0)
+  if (!PLAIN && parts == 0)
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
       const int c = (threadIdx.x + v * blockDim.x) * 4;
@@ -91,6 +97,10 @@ __global__ void __launch_bounds__(512) add_layernorm_vec_kernel(float* __restric
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     const int c = (threadIdx.x + v * blockDim.x) * 4;
+    if (PLAIN && c < hidden) {
+      w[v] = *reinterpret_cast<const float4*>(weight + c);
+      b[v] = *reinterpret_cast<const float4*>(bias + c);
+    }
     if (c < hidden)
       store4(o + c, fmaf(x[v].x * inv, w[v].x, b[v].x), fmaf(x[v].y * inv, w[v].y, b[v].y), fmaf(x[v].z * inv, w[v].z, b[v].z),
              fmaf(x[v].w * inv, w[v].w, b[v].w));
@@ -100,12 +110,20 @@ __global__ void __launch_bounds__(512) add_layernorm_vec_kernel(float* __restric
 template <typename T>
 void launch_layernorm_vec(float* residual, const float* delta, int parts, long long part_stride, const float* weight,
                           const float* bias, float eps, T* out, const int* gather, int rows, int hidden, cudaStream_t stream) {
-  const int pieces = hidden / 4, threads = pieces >= 512 ? 512 : ceil_div(pieces, 32) * 32, vpt = ceil_div(pieces, threads);
-#define TL_LN(V_) add_layernorm_vec_kernel<T, V_><<<rows, threads, 0, stream>>>(residual, delta, parts, part_stride, weight, bias, eps, out, gather, hidden)
+  // (as few pieces a thread as 512 threads allow, and then as few threads as those need: 640 pieces are two for each of 320)
+  const int pieces = hidden / 4, vpt = ceil_div(pieces, 512), threads = ceil_div(ceil_div(pieces, vpt), 32) * 32;
+  const bool plain = parts <= 1 && rows * (long long)threads > 1024LL * sm_count();
+#define TL_LN_(V_, P_) add_layernorm_vec_kernel<T, V_, P_><<<rows, threads, 0, stream>>>(residual, delta, parts, part_stride, weight, bias, eps, out, gather, hidden)
+#define TL_LN(V_)               \
+  do {                          \
+    if (plain) TL_LN_(V_, true); \
+    else TL_LN_(V_, false);     \
+  } while (0)
   if (vpt == 1) TL_LN(1);
   else if (vpt == 2) TL_LN(2);
   else if (vpt <= 4) TL_LN(4);
   else TL_LN(6);
+#undef TL_LN_
 #undef TL_LN
 }
 

@@ -244,3 +244,25 @@ def test_norm_behind_a_branch_of_many_rows(width):
             assert rel(r, new[:n]) < 1e-5
             assert rel(out.float(), w2.double() * new[:n] / (new[:n].pow(2).mean(-1, keepdim=True) + 1e-4).sqrt()) < TOL["bfloat16"]
         assert all(torch.equal(a, b) for a, b in zip(*made))
+
+
+@pytest.mark.parametrize("width", [4, 1536, 2052, 2560, 8192, 11264])
+def test_layer_norm_of_many_rows(width):
+    """The same for the layer norm, with one source and with none."""
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(width)
+    R = 2500 if width > 512 else 160000
+    res, dense = torch.randn(R, width, generator=g, device=DEV) + 2, torch.randn(R, width, generator=g, device=DEV)
+    w, b = (torch.randn(width, generator=g, device=DEV) for _ in range(2))
+    for delta in (dense, None):
+        x = res.double() + (0 if delta is None else delta.double())
+        d = x - x.mean(-1, keepdim=True)
+        want = d / (d.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * w.double() + b.double()
+        made = []
+        for n in (R, 5):
+            r, out = res[:n].clone(), torch.empty(n, width, dtype=torch.bfloat16, device=DEV)
+            ops.add_layernorm(r, None if delta is None else delta[:n].contiguous(), w, b, 1e-5, out)
+            made.append((r[:5], out[:5]))
+            assert rel(r, x[:n]) < 1e-6
+            assert rel(out.float(), want[:n]) < TOL["bfloat16"]
+        assert all(torch.equal(a, b) for a, b in zip(*made))
