@@ -105,10 +105,11 @@ __global__ void short_conv_kernel(const T* __restrict__ bcx, const float* __rest
 // used. Rows of a run that belong to several requests (a run across a request's edge) go the way of the kernel above,
 // row by row. Same results: a tap whose input lies before the sequence's first token multiplies a zero here and is
 // left out there.
-// Runs of eight rows where those alone give the GPU two blocks an SM, else of two: a block's time is a chain of round trips and, in
-// a run of several requests, one such chain a row (hidden 2048, runs of eight -> two: 535 rows of 24 requests 17.9 -> 8.2 us, 969 rows
-// of 5 11.4 -> 7.9 us, 37 rows 6.5 -> 4.2 us; at 2048 rows the inputs that are then read twice cost more than that).
-constexpr int CONV_RUN = 8, CONV_SHORT_RUN = 2;
+// Runs of eight rows where those alone give the GPU two blocks an SM, of four where they give it one and a row is 1024 channels or
+// more, else of two: a block's time is a chain of round trips and, in a run of several requests, one such chain a row, while a short
+// run reads more inputs twice. Hidden 2048, runs of 8 | 4 | 2 rows: 37 rows 6.5 | - | 4.2 us, 535 rows of 24 requests 17.9 | - | 8.2, 600
+// rows of one request 5.8 | 5.2 | 5.6, 969 rows of one 6.0 | 6.0 | 7.0, of five 9.2 | 7.4 | 7.4; hidden 512, 1200 rows of 24 requests 8.0 | 5.8 | 4.1.
+constexpr int CONV_RUN = 8, CONV_MIDDLE_RUN = 4, CONV_SHORT_RUN = 2;
 template <typename T, int KT, int RUN>
 __global__ void __launch_bounds__(128) short_conv_run_kernel(const T* __restrict__ bcx, const float* __restrict__ taps,
                                                              const float* __restrict__ bias, const float* __restrict__ state,
@@ -334,15 +335,17 @@ extern "C" int tl_short_conv(const void* bcx, const float* taps, const float* bi
   TL_REQUIRE(grid.y <= 65535, "short_conv: hidden size %d exceeds the grid limit", hidden);
   // many rows, 16-byte accesses, 2 to 4 taps: the form that walks runs of rows
   if (wide && rows >= 4 * CONV_RUN && K <= 4) {
-    const bool brief = (long long)ceil_div(rows, CONV_RUN) * grid.y < 2LL * sm_count();
-    dim3 run_grid(ceil_div(rows, brief ? CONV_SHORT_RUN : CONV_RUN), grid.y);
+    const long long blocks = (long long)ceil_div(rows, CONV_RUN) * grid.y;
+    const int run = blocks >= 2LL * sm_count() ? CONV_RUN : blocks >= sm_count() && hidden >= 1024 ? CONV_MIDDLE_RUN : CONV_SHORT_RUN;
+    dim3 run_grid(ceil_div(rows, run), grid.y);
 #define TL_RUN_(T_, K_, R_)                                                                                                \
   return (int)launch_chained(short_conv_run_kernel<T_, K_, R_>, run_grid, dim3(128), 0, stream, (const T_*)bcx, taps, bias, \
                              state, state_slot, req_of_row, row_start, positions, (T_*)y, rows, hidden)
-#define TL_RUN(T_, K_)                          \
-  do {                                          \
-    if (brief) TL_RUN_(T_, K_, CONV_SHORT_RUN); \
-    TL_RUN_(T_, K_, CONV_RUN);                  \
+#define TL_RUN(T_, K_)                                                  \
+  do {                                                                  \
+    if (run == CONV_SHORT_RUN) TL_RUN_(T_, K_, CONV_SHORT_RUN);         \
+    if (run == CONV_MIDDLE_RUN) TL_RUN_(T_, K_, CONV_MIDDLE_RUN);       \
+    TL_RUN_(T_, K_, CONV_RUN);                                          \
   } while (0)
     if (dtype == TL_FP32) {
       if (K == 2) TL_RUN(float, 2);

@@ -595,6 +595,51 @@ def test_short_conv_of_long_portions_walks_runs_of_rows(dtype, K, H, use_bias):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("K,H,use_bias", [(3, 2048, False), (4, 2048, True), (2, 4096, False)])
+@pytest.mark.parametrize("run", [2, 4, 8])
+def test_short_conv_in_runs_of_two_four_and_eight_rows(dtype, K, H, use_bias, run):
+    """The kernel takes runs of eight rows where those give the GPU two blocks an SM, of four where they give it one, else of two:
+    rows for each, with requests' edges inside runs, sequences shorter than the taps, a last run that is not full, portions behind
+    earlier tokens; against the plain formula and, for short requests, bit for bit against the row-by-row kernel."""
+    o = ops()
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    per_run = H // 1024                                                # blocks a run: 128 threads of eight channels each
+    rows = {2: 8 * (sm // per_run) - 9, 4: 8 * (sm // per_run) + 8 * 20 + 3, 8: 2 * 8 * (sm // per_run) + 8 * 20 + 5}[run]
+    blocks = -(-rows // 8) * per_run
+    assert (2 if blocks < sm else 4 if blocks < 2 * sm else 8) == run
+    short = [1, 2, 29, 3, 11]
+    lens = short + [37] + [rows - sum(short) - 37 - 13] + [13]
+    starts, slots = [0, 0, 7, 1, 4, 0, 9, 2], [2, 0, 3, 5, 1, 6, 8, 4]
+    R = sum(lens)
+    assert R == rows
+    bcx = rnd(R, 3 * H, seed=20).to(dtype)
+    taps_w, bias = rnd(H, K, seed=21), (rnd(H, seed=22) if use_bias else None)
+    state = rnd(9, K - 1, H, seed=23)
+    row_start = [0]
+    for n in lens:
+        row_start.append(row_start[-1] + n)
+    req_of_row = sum(([b] * n for b, n in enumerate(lens)), [])
+    positions = sum((list(range(s0, s0 + n)) for s0, n in zip(starts, lens)), [])
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    dev = lambda t: None if t is None else t.to(DEV)
+    y = torch.full((R, H), float("nan"), dtype=dtype, device=DEV)
+    fixed = (dev(taps_w), dev(bias), dev(state))
+    o.short_conv(dev(bcx), *fixed, i32(slots), i32(req_of_row), i32(row_start), i32(positions), y)
+    for b in range(len(lens)):
+        old = state[slots[b]].clone()
+        if starts[b] < K - 1:
+            old[:K - 1 - starts[b]] = 0
+        rows_b = slice(row_start[b], row_start[b + 1])
+        want_y, _ = plain_conv_with_state(bcx[rows_b].float(), taps_w, bias, old, K)
+        close(y[rows_b], want_y, dtype, f"request {b}")
+    for b in (0, 1, 2, 3, 4, 7):
+        rows_b = slice(row_start[b], row_start[b + 1])
+        alone = torch.empty(lens[b], H, dtype=dtype, device=DEV)
+        o.short_conv(dev(bcx[rows_b]), *fixed, i32([slots[b]]), i32([0] * lens[b]), i32([0, lens[b]]), i32(positions[rows_b]), alone)
+        assert torch.equal(alone, y[rows_b]), b
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("K,H,use_bias", [(3, 200, False), (4, 96, True), (2, 64, False), (7, 300, True)])
 def test_short_conv_of_single_rows_in_one_kernel(dtype, K, H, use_bias):
     """A step of one row a request (decoding) runs one kernel for the convolution and the state's shift: the same
