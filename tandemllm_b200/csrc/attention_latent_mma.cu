@@ -6,8 +6,8 @@
 //
 // A CTA of four warps takes 64 consecutive (row, head) pairs of one request (a warp 16 of them) and walks the visible keys
 // in tiles of 32 aligned to absolute positions. A key tile is copied as it lies into one of two buffers in shared memory
-// (cp.async, 16 bytes a copy) while the tile before it is computed on; it is the B operand of Q K^T as it lies (plain
-// 32-bit loads) and, through ldmatrix with .trans, the B operand of P C. `mma.sync` m16n8k16; rows padded so that the
+// (cp.async, 16 bytes a copy) while the tile before it is computed on; it is the B operand of Q K^T as it lies
+// (ldmatrix) and, through ldmatrix with .trans, the B operand of P C. `mma.sync` m16n8k16; rows padded so that the
 // eight rows a load touches fall into different banks. The latent's
 // columns are taken in chunks of up to 256 (a CTA a chunk: the accumulators of one chunk are all a thread can hold), and,
 // for steps of few rows, the keys in spans aligned to absolute positions, each span a CTA of its own; a second kernel
@@ -144,13 +144,15 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
   auto fetch = [&](int j0, int which) {
     bf16* dst = sK + (size_t)which * LM_KEYS * qs;
     if (vec) {
-      // (a warp a key: what a key's place costs, two divisions among it, is paid once a row and not once a piece)
+      // (eight lanes a key, 128 bytes at a time: what a key's place costs, two divisions among it, is paid once a thread and key and
+      // not once a piece, and short rows leave no lane without work; a warp a key: two portions of 500 rows, 32 heads of 512 + 64 354 us, four
+      // heads of 64 + 16 81 us, a piece a thread 571 and 64, this 321 and 56)
       const int per_row = Dk >> 3;                               // 16-byte pieces of a cached row
-      for (int kk = threadIdx.x >> 5; kk < LM_KEYS; kk += blockDim.x >> 5) {
+      for (int kk = threadIdx.x >> 3; kk < LM_KEYS; kk += blockDim.x >> 3) {
         const int page = s_page[which][kk];
         bf16* to = dst + (size_t)kk * qs;
         const bf16* from = p.cache + ((long long)page * p.page_size + (j0 + kk) % p.page_size) * Dk;
-        for (int c = lane; c < per_row; c += 32) {
+        for (int c = lane & 7; c < per_row; c += 8) {
           if (page >= 0)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 8 * c)), "l"(from + 8 * c) : "memory");
           else
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(128 * CPB) latent_mma_kernel(LatentMmaParams p
     // S = Q K^T for the warp's 16 pairs and the tile's 32 keys, both operands by ldmatrix (A: rows 0..7 and 8..15 of the block's
     // first and last eight entries; B: eight keys' first and last eight entries, two groups of keys a load). With two groups of
     // warps on the same pairs each takes 16 of the keys and hands its scores to the other through shared memory. (Prompts of 300
-    // and 700 rows, 32 heads, a latent of 512: 447 us with 32-bit operand loads and every score made twice, 319 us so, 272 us with a warp a key in front.)
+    // and 700 rows, 32 heads, a latent of 512: 447 us with 32-bit operand loads and every score made twice, 319 us so.)
     float s[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
