@@ -68,7 +68,9 @@ def context_bucket(longest: int) -> int:
 
 def _int32s(values):
     """A list of whole numbers as int32, through `array` (a third of the time numpy takes to look at each of a prompt's ids);
-    anything `array` does not take goes to numpy as it is."""
+    anything else, and what `array` does not take, goes to numpy as it is."""
+    if not isinstance(values, (list, tuple)):
+        return values
     try:
         return np.frombuffer(array("i", values), dtype=np.int32)
     except TypeError:
