@@ -147,8 +147,8 @@ __device__ __forceinline__ int nth_set_bit(uint32_t m, int n) {
 }
 
 // WEIGHED: a row's sums are multiplied by its pair's own weight (a kernel of its own, so that the others stay as lean as they are).
-template <bool SWIGLU, bool WEIGHED, int UNROLL, typename TOut>
-__global__ void __launch_bounds__(GROUPED_WARPS * 32, !SWIGLU && UNROLL == 4 ? 6 : 4) gemm_skinny_grouped_kernel(
+template <bool SWIGLU, bool WEIGHED, int UNROLL, typename TOut, int WARPS = GROUPED_WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS > GROUPED_WARPS ? 2 : !SWIGLU && UNROLL == 4 ? 6 : 4) gemm_skinny_grouped_kernel(
     const bf16* __restrict__ x, long long ldx, const int* __restrict__ row_index, int row_div, const bf16* __restrict__ w,
     long long ldw, long long rows_per_group, TOut* __restrict__ out, long long ldc, int N, int K,
     const int* __restrict__ tile_group, const int* __restrict__ tile_row0, const int* __restrict__ tile_rows,
@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(GROUPED_WARPS * 32, !SWIGLU && UNROLL == 4 ? 6
     int* __restrict__ status, int act, float ga0, float ga1, const float* __restrict__ row_weight,
     const int* __restrict__ weight_index, uint32_t zero) {
   constexpr int W_TILES = SWIGLU ? 2 : 1;
-  constexpr int WORDS = GROUPED_MAX_PAIRS / 32, WORDS_A_WARP = WORDS / GROUPED_WARPS;
-  __shared__ float part[GROUPED_WARPS][W_TILES][16][8 + 1];
+  constexpr int WORDS = GROUPED_MAX_PAIRS / 32, WORDS_A_WARP = WORDS / WARPS;
+  __shared__ float part[WARPS][W_TILES][16][8 + 1];
   __shared__ uint32_t s_match[WORDS];
   __shared__ int s_pair[8];
   __shared__ float s_weight[WEIGHED ? 8 : 1];
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(GROUPED_WARPS * 32, !SWIGLU && UNROLL == 4 ? 6
     uint32_t match[WORDS_A_WARP];                      // the pairs of 32 that belong to the group, a word after another
 #pragma unroll
     for (int i = 0; i < WORDS_A_WARP; ++i) {
-      const int word = warp + i * GROUPED_WARPS, p = word * 32 + lane;
+      const int word = warp + i * WARPS, p = word * 32 + lane;
       match[i] = __ballot_sync(0xffffffffu, (p < n_pairs ? pair_group[p] : -1) == group);
       if (lane == 0) s_match[word] = match[i];
     }
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(GROUPED_WARPS * 32, !SWIGLU && UNROLL == 4 ? 6
     if (earlier) return;
 #pragma unroll
     for (int i = 0; i < WORDS_A_WARP; ++i) {
-      const int word = warp + i * GROUPED_WARPS;
+      const int word = warp + i * WARPS;
       int before = __popc(match[i] & ((1u << lane) - 1u));         // matching pairs before this lane's
       for (int e = 0; e < word; ++e) before += __popc(s_match[e]);
       if ((match[i] >> lane & 1u) && before < 8) s_pair[before] = word * 32 + lane;
@@ -250,12 +250,12 @@ __global__ void __launch_bounds__(GROUPED_WARPS * 32, !SWIGLU && UNROLL == 4 ? 6
     if (warp == 0 && t == 0 && x_ok) my_weight = pair_weight(row_weight, weight_index, pos);
 
   const int chunks = (K + 31) / 32;
-  for (int c0 = warp; c0 < chunks; c0 += GROUPED_WARPS * UNROLL) {
+  for (int c0 = warp; c0 < chunks; c0 += WARPS * UNROLL) {
     uint4 a_lo[UNROLL][W_TILES], a_hi[UNROLL][W_TILES], b[UNROLL];
     uint32_t all = 0u;
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
-      const int c = c0 + u * GROUPED_WARPS;
+      const int c = c0 + u * WARPS;
       const bool in = c < chunks && c * 32 + t * 8 < K;
 #pragma unroll
       for (int j = 0; j < W_TILES; ++j) {
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(GROUPED_WARPS * 32, !SWIGLU && UNROLL == 4 ? 6
   }
   if (WEIGHED && warp == 0 && t == 0) s_weight[g] = my_weight;
   __syncthreads();
-  for (int i = threadIdx.x; i < 16 * 8; i += GROUPED_WARPS * 32) {
+  for (int i = threadIdx.x; i < 16 * 8; i += WARPS * 32) {
     const int row = i & 15, m = i >> 4;
     if (m >= rows || n0 + row >= N) continue;
     float v[W_TILES];
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(GROUPED_WARPS * 32, !SWIGLU && UNROLL == 4 ? 6
     for (int j = 0; j < W_TILES; ++j) {
       v[j] = 0.f;
 #pragma unroll
-      for (int s = 0; s < GROUPED_WARPS; ++s) v[j] += part[s][j][row][m];
+      for (int s = 0; s < WARPS; ++s) v[j] += part[s][j][row][m];
     }
     if constexpr (WEIGHED) {
 #pragma unroll
@@ -516,14 +516,18 @@ extern "C" int tl_gemm_skinny_grouped(const void* x, long long ldx, const int* r
   TL_REQUIRE(swiglu <= 0 ? swiglu >= -TL_ACT_IDENTITY : tl_is_gate(swiglu),
              "skinny grouped product: gate activation %d is none (nor an ungated one, negated)", swiglu);
   TL_REQUIRE(!row_weight || swiglu > 0, "skinny grouped product: row weights need the gated form (activation %d)", swiglu);
-  const dim3 grid(ceil_div(N, 16), max_tiles), block(GROUPED_WARPS * 32);
+  const dim3 grid(ceil_div(N, 16), max_tiles);
   // Plain products: eight chunks of k in flight a warp where a warp has more than eight and the last round is nearly full, else
   // four and more CTAs an SM (2048 of 1792, 14 chunks: 29.7 us with eight and 30.0 with four, one row 8.2 and 9.6; 2048 of 1536,
   // 12 chunks: 47.5 and 42.1 us).
   const int mine = ceil_div(ceil_div(K, 32), GROUPED_WARPS);
   const bool eight = mine > 8 && ceil_div(mine, 8) * 8 - mine <= 2;
-#define TL_GROUPED(SW_, WE_, U_, T_)                                                                                          \
-  return (int)launch_chained(gemm_skinny_grouped_kernel<SW_, WE_, U_, T_>, grid, block, 0, stream, (const bf16*)x, ldx, row_index,  \
+  // Eight warps where a warp of four would have more than two rounds of eight and the CTAs are at most two an SM (both products of top-2 of 8
+  // experts of 4096 x 1024, one and two rows: 17.0 and 24.4 us with four, 15.3 and 22.2 so; of 8192 x 1024 27.6 and 37.9, 24.4 and 34.4).
+  const bool wide = mine > 16 && (long long)grid.x * grid.y <= 2LL * sm_count();
+#define TL_GROUPED(SW_, WE_, U_, T_) TL_GROUPED_(SW_, WE_, U_, T_, GROUPED_WARPS)
+#define TL_GROUPED_(SW_, WE_, U_, T_, W_)                                                                                     \
+  return (int)launch_chained(gemm_skinny_grouped_kernel<SW_, WE_, U_, T_, W_>, grid, dim3(W_ * 32), 0, stream, (const bf16*)x, ldx, row_index,  \
                              row_div, (const bf16*)w, ldw, rows_per_group, (T_*)out, ldc, N, K, tile_group, tile_row0,    \
                              tile_rows, n_tiles, pair_group, n_pairs, n_groups, status, swiglu, tl_gate_constants[0], tl_gate_constants[1],     \
                              row_weight, weight_index, 0u)
@@ -536,11 +540,13 @@ extern "C" int tl_gemm_skinny_grouped(const void* x, long long ldx, const int* r
     TL_GROUPED(true, false, 4, bf16);
   }
   if (out_dtype == TL_FP32) {
+    if (wide) TL_GROUPED_(false, false, 8, float, 8);
     if (eight) TL_GROUPED(false, false, 8, float);
     TL_GROUPED(false, false, 4, float);
   }
   if (eight) TL_GROUPED(false, false, 8, bf16);
   TL_GROUPED(false, false, 4, bf16);
+#undef TL_GROUPED_
 #undef TL_GROUPED
 }
 

@@ -64,6 +64,13 @@ def test_grouped_products_of_pairs_without_a_plan(R, k, E, N, K, gated):
     assert rel(out, want) < 1e-5
 
 
+@pytest.mark.parametrize("R,k,E", [(1, 2, 8), (2, 3, 8), (8, 4, 40)])
+@pytest.mark.parametrize("N,K", [(1024, 4096), (40, 2056), (24, 2600), (1000, 11776)])
+def test_grouped_products_of_long_reductions(R, k, E, N, K):
+    """The same with k above 2048, where a few CTAs have eight warps."""
+    test_grouped_products_of_pairs_without_a_plan(R, k, E, N, K, False)
+
+
 @pytest.mark.parametrize("M", [1, 7, 8, 9])
 @pytest.mark.parametrize("inter,K", [(2368, 32), (4736, 264), (4760, 2048), (40, 264)])
 def test_feed_forward_activations_in_the_products_epilogue(M, inter, K):
