@@ -2,9 +2,10 @@
 // of latent attention (the query's unrotated part through a head's key matrix, the weighted latents through its value
 // matrix). A CTA of four warps makes 64 rows x 64 outputs of one head; k comes in blocks of 64 through shared memory
 // (16-byte loads where rows and heads are aligned for them, else element by element), rows padded so that the eight rows
-// an operand load touches fall into different banks; `mma.sync` m16n8k16 with 32-bit accumulators, k in ascending order,
-// so a row's result does not depend on the rows beside it. A decode step's few rows leave most of a tile's rows empty;
-// the kernel is then bound by the heads' weights, which it reads once.
+// an operand load touches fall into different banks; `mma.sync` m16n8k16 with 32-bit accumulators, k in ascending order.
+// Up to 16 rows (a decode step's) with k in whole blocks of 32 go to a form of their own, which adds the same products in another
+// order: between a call of up to 16 rows and one of more a row's 32-bit sum differs by rounding, within either kind it does not depend on
+// the rows beside it.
 #include "common.cuh"
 
 namespace tl {
