@@ -4,11 +4,12 @@
 //   C[m, n] = sum_k A[m, k] * W[n, k] (+ bias[n])            both operands row-major with k contiguous
 //
 // The order in which an output's products are added depends on k alone in each kernel: ascending, by one thread, in the tiled kernels;
-// in those for 32-bit operands of whole 16-byte pieces the eight chains described there, whatever the tile's height. So with
-// 32-bit operands of whole pieces and more than 64 outputs, and in every grouped product, a row's result
+// in those for 32-bit operands of whole 16-byte pieces the eight chains described there. So in every grouped product, and with 32-bit
+// operands of whole pieces, more than 64 outputs and a k of up to 256, a row's result
 // does not depend on how many other rows the call has (the reference's row invariance,
-// engine/models/lfm2_moe/kernels.py:290-306). Plain products of up to 64 outputs, of bfloat16 operands and of rows that are not whole
-// pieces have kernels of their own for up to 8 rows, with a warp's or a CTA's lanes along k: there a row's last bits differ between
+// engine/models/lfm2_moe/kernels.py:290-306). Up to 8 rows of a longer k are added more exactly, and plain products of up to 64 outputs,
+// of bfloat16 operands and of rows that are not whole pieces have kernels of their own for up to 8 rows, with a warp's or a CTA's lanes
+// along k: there a row's last bits differ between
 // a call of up to 8 rows and one of more. The same kernel runs the experts: a tile map built on the
 // device (moe_route.cu) names, per row tile, the expert whose weights it multiplies by and the rows of
 // the expert-sorted pair list it covers; with `swiglu` the epilogue is silu(gate) * up over the two
@@ -264,13 +265,16 @@ __global__ void __launch_bounds__(256) gemm_tall_narrow_kernel(GemmParams p) {
 //
 // Up to 8 rows are bound by the weights' bytes: tiles of 1, 2, 4 or 8 rows and so few outputs (8, 16 or 32) that the weights come
 // through as many SMs as there are, a lane an output where it goes (a weight is then read from shared memory once, by one lane), and
-// stages of 128 k-elements, eight of them for the narrow tiles, so that enough is in flight. Same chains, same order: it is what lets
-// a prompt be cut anywhere without a change in its products. 1 and 8 rows, outputs x k: 512 x 256 2.2 and 2.3 us (a warp an output,
-// lanes along k: 3.1 and 4.4), 512 x 1024 3.2 and 3.8 (a CTA an output: 3.3 and 3.7), 2048 x 2048 6.6 and 8.6 (a warp for two outputs: 6.8
-// and 26.5), 65536 x 2048 88 and 118 us (78 and, a warp an output, 265). A CTA an output is still faster only for some hundred outputs of a
-// long k (128 x 1024 2.5 and 2.8 us, 3.2 and 3.7 here).
+// stages of 128 k-elements, eight of them for the narrow tiles, so that enough is in flight. Up to a k of WHOLE the chains and their order are
+// the same, and a row's bits do not depend on the rows beside it. Of a longer k the chains are folded into one sum with its rounding
+// errors kept beside it, at WHOLE and at every 128 behind, which loses a quarter of what whole chains lose (a head of k 2048); the taller tiles
+// have no registers for that, and folding in shared memory cost them 9 % (512 rows against 6144 x 2048 338 -> 370 us).
+// 1 and 8 rows, outputs x k: 512 x 256 2.2 and 2.3 us (a warp an output, lanes along k: 3.1 and 4.4), 512 x 1024 3.5 and 4.1 (a CTA an
+// output: 3.3 and 3.7), 2048 x 2048 6.9 and 9.1 (a warp for two outputs: 6.8 and 26.5), 65536 x 2048 87 and 126 (81 and 186). Still faster are a CTA an output for some hundred
+// outputs of a long k (128 x 1024 2.5 and 2.9 us, 3.4 and 4.0 here) and, for one row alone, a warp for two outputs of many (6144 x 2048 10.6 us, 12.0).
 constexpr int FWARPS = 4;
 constexpr int FEW_ROWS = 8;
+constexpr int WHOLE = 256;              // k up to which a few rows' chains are not folded
 
 template <int BM_, int FN_>
 struct F32Tile {
@@ -368,8 +372,31 @@ __global__ void __launch_bounds__(FWARPS * 32, F32Tile<BM_, FN>::CTAS) gemm_f32_
 #pragma unroll
     for (int j = 0; j < TN_; ++j) acc[i][j] = 0ull;
 
+  // (few rows: what the chains have been folded to, and what the folding lost)
+  float high[T::FEW ? TM_ : 1][T::FEW ? TN_ : 1], low[T::FEW ? TM_ : 1][T::FEW ? TN_ : 1];
+  auto fold = [&](int m, int j) {
+    const float v = both(acc[m][j]), sum = high[m][j] + v, part = sum - high[m][j];
+    low[m][j] += (high[m][j] - (sum - part)) + (v - part);
+    high[m][j] = sum;
+    acc[m][j] = 0ull;
+  };
+  if constexpr (T::FEW) {
+#pragma unroll
+    for (int i = 0; i < TM_; ++i)
+#pragma unroll
+      for (int j = 0; j < TN_; ++j) high[i][j] = low[i][j] = 0.f;
+  }
+
   for (int s = 0; s < FSTAGES - 1; ++s) load(s);
   for (int step = 0; step < steps; ++step) {
+    if constexpr (T::FEW) {
+      if (step >= WHOLE / FK) {
+#pragma unroll
+        for (int m = 0; m < TM_; ++m)
+#pragma unroll
+          for (int j = 0; j < TN_; ++j) fold(m, j);
+      }
+    }
     asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
     __syncthreads();                                  // the stage is here, and everybody is done with the one before
     load(step + FSTAGES - 1);
@@ -396,7 +423,16 @@ __global__ void __launch_bounds__(FWARPS * 32, F32Tile<BM_, FN>::CTAS) gemm_f32_
 #pragma unroll
   for (int m = 0; m < TM_; ++m)
 #pragma unroll
-    for (int j = 0; j < TN_; ++j) red[((warp * TM_ + m) * TN_ + j) * 32 + lane] = both(acc[m][j]);
+    for (int j = 0; j < TN_; ++j) {
+      float v = both(acc[m][j]);
+      if constexpr (T::FEW) {
+        if (steps > WHOLE / FK) {
+          fold(m, j);
+          v = fabsf(high[m][j]) < INFINITY ? high[m][j] + low[m][j] : high[m][j];      // (an infinity loses no finite rest)
+        }
+      }
+      red[((warp * TM_ + m) * TN_ + j) * 32 + lane] = v;
+    }
   __syncthreads();
   auto sum = [&](int m, int j) {
     float v = 0.f;

@@ -423,16 +423,28 @@ def test_gemm_simt_in_16_byte_pieces(M, N, K):
         assert torch.equal(few, out[M - 9:])
 
 
-@pytest.mark.parametrize("N,K", [(65, 4), (128, 256), (513, 36), (128, 1024), (513, 1024), (70, 2052), (1030, 520), (2048, 2048)])
+@pytest.mark.parametrize("N,K", [(65, 4), (128, 256), (513, 36), (128, 1024), (513, 1024), (70, 2052), (1030, 260), (1030, 520), (2048, 2048)])
 def test_gemm_simt_in_16_byte_pieces_row_by_row(N, K):
-    """More than 64 outputs: a row has the same bits alone, among up to eight rows (a kernel of their own) and in the tiles of 16
-    and 32 rows, so where a prompt is cut changes no product."""
+    """More than 64 outputs: up to a k of 256 a row has the same bits alone, among up to eight rows (tiles of their own) and in the tiles
+    of 16 and 32 rows, so where a prompt is cut changes no product; of a longer k up to eight rows have the same bits among themselves, and so
+    have more. Eight rows of a longer k fold their chains of at most 32 products (16 behind the first 256) into sums that keep their rounding errors: off by
+    at most 32 + 8 roundings of the sum of absolute values, whatever k."""
     o = ops()
     x, w, b = rnd(33, K, seed=6).to(DEV), rnd(N, K, seed=7).to(DEV), rnd(N, seed=8).to(DEV)
     made = lambda n: o.gemm_simt(x[:n], w, b, torch.empty(n, N, device=DEV))
-    whole = made(33)
-    for n in (1, 2, 4, 5, 8, 9, 16, 17):
+    few, whole = made(8), made(33)
+    for n in (1, 2, 3, 4, 5, 7):
+        assert torch.equal(made(n), few[:n]), n
+    for n in (9, 16, 17):
         assert torch.equal(made(n), whole[:n]), n
+    if K <= 256:
+        assert torch.equal(few, whole[:8])
+    want, size = x[:8].double() @ w.double().T + b.double(), x[:8].double().abs() @ w.double().abs().T + b.double().abs()
+    assert ((few.double() - want).abs() <= 40 * 2.0 ** -24 * size).all()
+    x[0], x[1], x[2, 1] = 3e38, -3e38, float("nan")                 # (sums that overflow stay infinities, as in the tiles)
+    ones = torch.ones(N, K, device=DEV)
+    few, whole = (o.gemm_simt(x[:n], ones, None, torch.empty(n, N, device=DEV))[:3] for n in (8, 33))
+    assert torch.equal(few.isnan(), whole.isnan()) and torch.equal(few[:2], whole[:2]) and bool((few[0] == float("inf")).all()) == (K > 1)
 
 
 @pytest.mark.parametrize("R,E,k,H,I", [(3, 8, 2, 64, 68), (40, 3, 2, 36, 132), (200, 4, 2, 100, 64), (130, 2, 1, 32, 40)])
