@@ -2,11 +2,11 @@
 //
 //   C[m, n] = sum_k X[m, k] * W[n, k] (+ bias[n])      or, gated:  C[m, n] = act(X . Wgate[n]) * (X . Wup[n])
 //
-// A cluster of two CTAs works on one output tile: 256 outputs (weight rows) by up to 256 token rows. The weights are the MMA's M side: each CTA brings its own 128 weight rows (gated: its 128 gate rows and the
-// 128 up rows of the same outputs) and gets their accumulator rows in its own tensor memory. The token rows are the N
-// side, which the pair shares: each CTA brings half of them, and one tcgen05.mma issued by the pair's first CTA reads
-// both halves, so a token row crosses from L2 into shared memory once per 256 outputs instead of once per 128. That
-// path, not the tensor pipe, is what bounds the one-CTA kernel at these sizes.
+// A cluster of two CTAs works on one output tile: 256 weight rows (256 outputs; gated: 128 outputs, 8 gate rows and the 8 up rows of the
+// same outputs in turn) by up to 256 token rows. The weights are the MMA's M side: each CTA brings its own 128 weight rows and gets
+// their accumulator rows in its own tensor memory. The token rows are the N side, which the pair shares: each CTA brings half of them,
+// and one tcgen05.mma issued by the pair's first CTA reads both halves, so a token row crosses from L2 into shared memory once per 256
+// weight rows instead of once per 128. That path, not the tensor pipe, is what bounds the one-CTA kernel at these sizes.
 //
 // The N side of an MMA is a run-time number (a multiple of 16 up to 256): a tile of the routed experts' products that
 // holds 40 rows costs an MMA of N = 48 and not a padded 128-row one, and its token rows come as a box of 64 rows a CTA
@@ -15,13 +15,17 @@
 // Roles in each CTA, as in the one-CTA persistent kernel (tc_gemm.cu): warp 0, one thread, keeps a ring of stages full
 // by TMA (plain loads, each CTA its own; their bytes are counted on the first CTA's barrier); warp 1 of the first CTA,
 // one thread, issues the MMAs into one of two accumulators and releases stages and accumulators in both CTAs with
-// tcgen05.commit; warps 2..9 read a finished accumulator (one output a thread, 16 tokens a load), apply the bias or
-// the gate, turn the block through shared memory and store 16 outputs of a token at a time. The plain product has two
-// accumulators of 256 columns, so that the next tile's MMAs run under a tile's epilogue; the gated product's gate and
-// up accumulators fill all 512 columns, and its MMAs wait for the epilogue while the ring goes on filling: what the
-// pair saves on the way from L2 (48 KB a CTA for 2 x 128 x 256 x 64 multiply-adds, against 40 KB for half of them
-// with tiles of 128 token rows) is worth more than the overlap. The kernel is persistent: as many clusters as fit the
-// GPU walk over the tiles.
+// tcgen05.commit; the epilogue warps (from warp 2 on) read a finished accumulator (one accumulator row a thread, 16 tokens a load), turn
+// the block through shared memory, apply the bias and the activation or gate, and store 8 or 16 outputs of a token at a time. Tensor
+// memory holds two accumulators or more, so that the next tile's MMAs run under a tile's epilogue. The kernel is persistent: as many
+// clusters as fit the GPU walk over the tiles.
+//
+// The gated product once took 256 gate and 256 up rows a tile, whose two accumulators filled tensor memory: its MMAs waited for the
+// epilogue, and its tiles, twice as large, left the last round of clusters emptier (7168 outputs of 2048 rows are 3.03 rounds of such
+// tiles and 6.05 of these). A tile here loads 64 KB for what cost 48, which larger products feel (11776 outputs of 2048 rows 146 -> 150
+// us, 150 rows 32 -> 37 us) and all others gain more than: 7168 outputs of 2048, 150 rows 29 -> 24 us, 535 rows 53 -> 48, 2048 rows
+// 115 -> 105; 32 experts of 1792 x 2048, 535 rows 99 -> 95 us, 1400 rows 114 -> 103; 64 experts of 768 x 2048, top 6, 1000 rows 118 -> 93
+// us, 2000 rows 156 -> 117.
 //
 // Every wait on an mbarrier is bounded: when a bound is hit the CTA records status 11 and tells its peer, both stop
 // issuing work, the first CTA waits (bounded again) for the copies in flight, the pair meets at the cluster barrier,
@@ -65,31 +69,28 @@ inline int& skip_kb_for_test() {
   return kb;
 }
 
-// PER_SM: CTAs an SM. One: the forms described above. Two: half the shared memory and half the tensor memory each (the
-// gated product then takes tiles of 128 token rows, gate and up accumulators of 128 columns; one accumulator set, so the
-// other CTA of the SM is what runs under an epilogue). Twice the pairs are resident, which is what a product bound by
-// its weights wants: its work items all cost the same (what their weight tiles take to load), and when the last round
-// leaves an SM with one CTA instead of two, that CTA loads at the SM's full rate. Measured on the experts' two products
-// of 128 to 512 tokens (32 experts, 16 to 64 rows each): 170 to 176 us -> 158 to 164 us; from 128 rows an expert on the
-// form with one CTA an SM and its deeper ring is faster again.
+// PER_SM 2 is the form for products bound by their weights. Plain: two CTAs an SM, half the shared memory and half the tensor memory
+// each and one accumulator, so the other CTA of the SM is what runs under an epilogue; twice the pairs are resident, and when the last
+// round leaves an SM with one CTA instead of two, that CTA loads at the SM's full rate. Gated: tiles of up to 128 token rows, one CTA an
+// SM with a ring of eight stages and four accumulators (two CTAs of four stages each took 107 us where this takes 92: 400 rows of
+// top-4 of 32 experts of 1792 x 2048).
 template <bool GATED, int PER_SM>
 struct Smem {
   static constexpr int TOKENS = (GATED && PER_SM == 2) ? 128 : 256;  // token rows a tile at most
-  static constexpr int W_TILES = GATED ? 2 : 1;
-  static constexpr int ACC_BUFS = (GATED || PER_SM == 2) ? 1 : 2;  // accumulators (sets of them) in tensor memory
-  static constexpr int TMEM_COLS = PER_SM == 2 ? 256 : 512;
-  static constexpr int UP_COL = TOKENS;                            // the gated product's second accumulator
-  // Epilogue warps: one a quarter of the accumulator's lanes, or, where the MMAs wait for the epilogue, two that take
-  // every other block of 16 tokens (measured: the plain product is a little slower with eight)
+  static constexpr int OUTS = GATED ? ROWS / 2 : ROWS;             // outputs a CTA
+  static constexpr int CTAS = GATED ? 1 : PER_SM;                  // CTAs an SM
+  static constexpr int TMEM_COLS = CTAS == 2 ? 256 : 512;
+  static constexpr int ACC_BUFS = TMEM_COLS / TOKENS;              // accumulators in tensor memory
+  // Epilogue warps: one a quarter of the accumulator's lanes, or two that take every other block of 16 tokens
   static constexpr int EPI_WARPS = GATED ? 8 : 4;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int A_BYTES = ROWS * TILE_K * 2;                // one box of weights
   static constexpr int B_BYTES = (TOKENS / 2) * TILE_K * 2;        // this CTA's half of the token rows, at most
-  static constexpr int STAGE_BYTES = W_TILES * A_BYTES + B_BYTES;
-  static constexpr int STAGES = PER_SM == 2 ? (GATED ? 2 : 3) : (GATED ? 4 : 6);
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = PER_SM == 2 ? (GATED ? 8 : 3) : 6;
   static constexpr int TURN_BYTES = EPI_WARPS * 16 * 32 * 4;       // the epilogue warps' blocks
   static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */ + TURN_BYTES;
-  static_assert(PER_SM * TOTAL <= 227 * 1024, "the CTAs of an SM share its shared memory");
+  static_assert(CTAS * TOTAL <= 227 * 1024, "the CTAs of an SM share its shared memory");
 };
 
 // K-major tile with 128-byte rows and the 128-byte swizzle: 8-row groups 1024 bytes apart, descriptor version 1.
@@ -160,6 +161,14 @@ __device__ __forceinline__ void load_2d(void* dst, const CUtensorMap* map, uint3
       : "memory");
 }
 
+// One box of gate and up rows (`gate_up_map`) from (column x, block of 8 outputs, group), counted as the box above.
+__device__ __forceinline__ void load_gate_up(void* dst, const CUtensorMap* map, uint32_t bar_addr, int x, int block, int group) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(bar_addr), "r"(x), "r"(0), "r"(block), "r"(group)
+      : "memory");
+}
+
 __device__ __forceinline__ void ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
   asm volatile(
@@ -180,7 +189,7 @@ template <> __device__ __forceinline__ void put<bf16>(bf16* p, float v) { *p = _
 // evaluations 1000 rows of six experts of 768 x 2048 took 125 us, 100 us so, and as one more branch of the other gates' kernel it
 // cost those 1.5 %.
 template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false>
-__global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
+__global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_SM>::CTAS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
                                                            const __grid_constant__ CUtensorMap tmX16,
                                                            const __grid_constant__ CUtensorMap tmX64,
                                                            const __grid_constant__ CUtensorMap tmX128, Params p) {
@@ -189,9 +198,9 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(tiles + S::STAGES * S::STAGE_BYTES);   // used in the first CTA: both CTAs' bytes
   uint64_t* empty = full + S::STAGES;                                  // in each CTA: the MMAs have read the stage
-  uint64_t* acc_full = empty + S::STAGES;                              // [2] in each CTA: a tile's accumulator is done
-  uint64_t* acc_empty = acc_full + 2;                                  // [2] used in the first CTA: both epilogues read it
-  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  uint64_t* acc_full = empty + S::STAGES;                              // [ACC_BUFS] in each CTA: a tile's accumulator is done
+  uint64_t* acc_empty = acc_full + 4;                                  // [ACC_BUFS] used in the first CTA: both epilogues read it
+  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 4);
   volatile uint32_t* aborted = tmem_slot + 1;
   float* turns = (float*)(tiles + S::STAGES * S::STAGE_BYTES + 256);   // [warps][16 tokens][32 outputs]: see the epilogue
 
@@ -203,7 +212,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < S::ACC_BUFS; ++b) {
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 2 * S::EPI_WARPS);         // one arrival an epilogue warp of either CTA
     }
@@ -229,7 +238,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
     atomicExch(p.status, 11);
   };
 
-  const int tiles_n = (p.N + 2 * ROWS - 1) / (2 * ROWS);
+  const int tiles_n = (p.N + 2 * S::OUTS - 1) / (2 * S::OUTS);
   const int tiles_m = p.tile_group ? *p.n_tiles : (p.M + S::TOKENS - 1) / S::TOKENS;
   const int work = tiles_m * tiles_n * p.splits;
   const int all_kb = (p.K + TILE_K - 1) / TILE_K;
@@ -237,21 +246,21 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
 
   // work item w: token tile w / tiles_n, weight tile w % tiles_n (neighbouring clusters share token rows); with runs of
   // k-blocks, run w / (tiles_m tiles_n) of that tile
-  auto tile_of = [&](int w, int& tok0, int& tok_rows, long long& w_base, int& n0, int& kb0, int& num_kb) {
+  auto tile_of = [&](int w, int& tok0, int& tok_rows, int& group, int& n0, int& kb0, int& num_kb) {
     const int run = w / (tiles_m * tiles_n);
     w -= run * tiles_m * tiles_n;
     kb0 = run * p.kb_per_split;
     num_kb = p.splits > 1 ? min(p.kb_per_split, all_kb - kb0) : all_kb;
     const int tm = w / tiles_n;
-    n0 = (w - tm * tiles_n) * 2 * ROWS;
+    n0 = (w - tm * tiles_n) * 2 * S::OUTS;
     if (p.tile_group) {
       tok0 = p.tile_row0[tm];
       tok_rows = min(p.tile_rows[tm], S::TOKENS);
-      w_base = (long long)p.tile_group[tm] * p.rows_per_group;
+      group = p.tile_group[tm];
     } else {
       tok0 = tm * S::TOKENS;
       tok_rows = min(S::TOKENS, p.M - tok0);
-      w_base = 0;
+      group = 0;
     }
   };
 
@@ -259,18 +268,18 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
     // ---- producer (each CTA for its own shared memory) ----
     int it = 0, issued = 0;
     for (int w = cluster; w < work && !*aborted; w += clusters) {
-      int tok0, tok_rows, n0, kb0, num_kb;
-      long long w_base;
-      tile_of(w, tok0, tok_rows, w_base, n0, kb0, num_kb);
+      int tok0, tok_rows, group, n0, kb0, num_kb;
+      tile_of(w, tok0, tok_rows, group, n0, kb0, num_kb);
       if (tok_rows <= 0) continue;
       const int n_mma = (tok_rows + 15) & ~15;
       const int half = n_mma >> 1;
       const int my_tok = tok0 + (int)rank * half;                    // this CTA's half of the N side
-      const int my_row = (int)(w_base + n0) + (int)rank * ROWS;      // this CTA's 128 outputs
+      const int my_out = n0 + (int)rank * S::OUTS;                   // this CTA's outputs
+      const int my_row = (int)(group * p.rows_per_group) + my_out;
       // the smallest box that holds the half; rows of it behind the half are read and never used
       const int box = half <= 16 ? 16 : (half <= 64 ? 64 : 128);      // (a half is at most TOKENS / 2 rows)
       const CUtensorMap* tmX = box == 16 ? &tmX16 : (box == 64 ? &tmX64 : &tmX128);
-      const uint32_t cta_bytes = (uint32_t)(S::W_TILES * S::A_BYTES + box * TILE_K * 2);
+      const uint32_t cta_bytes = (uint32_t)(S::A_BYTES + box * TILE_K * 2);
       for (int kb = 0; kb < num_kb; ++kb, ++it) {
         const int s = it % S::STAGES;
         if (it >= S::STAGES && !mbar_wait(&empty[s], ((it / S::STAGES) - 1) & 1)) give_up();
@@ -280,9 +289,9 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
           const uint32_t bar = in_cta(&full[s], 0);
           if (first) mbar_expect_tx(&full[s], 2 * cta_bytes);
           const int kx = (kb0 + kb) * TILE_K;
-          load_2d(st, &tmW, bar, kx, my_row);
-          if (GATED) load_2d(st + S::A_BYTES, &tmW, bar, kx, my_row + p.N);
-          load_2d(st + S::W_TILES * S::A_BYTES, tmX, bar, kx, my_tok);
+          if (GATED) load_gate_up(st, &tmW, bar, kx, my_out >> 3, group);
+          else load_2d(st, &tmW, bar, kx, my_row);
+          load_2d(st + S::A_BYTES, tmX, bar, kx, my_tok);
         }
         issued = it + 1;
       }
@@ -296,9 +305,8 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
     // ---- MMA issuer (the first CTA for the pair) ----
     int it = 0, n = 0;
     for (int w = cluster; w < work && !*aborted; w += clusters) {
-      int tok0, tok_rows, n0, kb0, num_kb;
-      long long w_base;
-      tile_of(w, tok0, tok_rows, w_base, n0, kb0, num_kb);
+      int tok0, tok_rows, group, n0, kb0, num_kb;
+      tile_of(w, tok0, tok_rows, group, n0, kb0, num_kb);
       if (tok_rows <= 0) continue;
       const int n_mma = (tok_rows + 15) & ~15;
       const uint32_t id = idesc(n_mma);
@@ -308,7 +316,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t acc = tmem_base + buf * 256;
+      const uint32_t acc = tmem_base + buf * S::TOKENS;
       for (int kb = 0; kb < num_kb; ++kb, ++it) {
         const int s = it % S::STAGES;
         if (!mbar_wait(&full[s], (it / S::STAGES) & 1)) {
@@ -316,12 +324,11 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(tiles + s * S::STAGE_BYTES), b0 = a0 + S::W_TILES * S::A_BYTES;
+        const uint32_t a0 = smem_u32(tiles + s * S::STAGE_BYTES), b0 = a0 + S::A_BYTES;
 #pragma unroll
         for (int k = 0; k < TILE_K / UMMA_K; ++k) {
           const uint32_t more = (kb > 0 || k > 0) ? 1u : 0u, koff = k * UMMA_K * 2;
           mma2(acc, desc(a0 + koff), desc(b0 + koff), id, more);
-          if (GATED) mma2(acc + S::UP_COL, desc(a0 + S::A_BYTES + koff), desc(b0 + koff), id, more);
         }
         commit_both(&empty[s]);
       }
@@ -339,15 +346,15 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
     int n = 0;
     if (p.tile_group && p.plan_rows > S::TOKENS && threadIdx.x == 64) atomicExch(p.status, 5);   // taller tiles than the kernel takes
     for (int w = cluster; w < work && !*aborted; w += clusters) {
-      int tok0, tok_rows, n0, kb0, num_kb;
-      long long w_base;
-      tile_of(w, tok0, tok_rows, w_base, n0, kb0, num_kb);
+      int tok0, tok_rows, group, n0, kb0, num_kb;
+      tile_of(w, tok0, tok_rows, group, n0, kb0, num_kb);
       if (tok_rows <= 0) continue;
       const int n_mma = (tok_rows + 15) & ~15;
       const int buf = n % S::ACC_BUFS, round = n / S::ACC_BUFS;
       // The weights of the pairs that the warp's blocks of 16 tokens stand for (at most eight blocks: two a register, a block a half of
       // the lanes) are on their way while the MMAs run.
       constexpr int STEP = 16 * (S::EPI_WARPS / 4);
+      static_assert(!GATED || S::TOKENS <= 8 * STEP, "four registers of weights hold eight blocks");
       float rw[4] = {1.f, 1.f, 1.f, 1.f};
       if (GATED && p.row_weight) {
 #pragma unroll
@@ -361,62 +368,32 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * 256;
-      const int col = n0 + (int)rank * ROWS + m_row;                 // this thread's output
-      const float b = (p.bias && col < p.N && kb0 == 0) ? p.bias[col] : 0.f;
-      const float b_up = (GATED && p.bias && col < p.N) ? p.bias[p.N + col] : 0.f;      // (gated: N gate biases, then N of the up rows)
-      const int j_tok = lane >> 1, c_half = (lane & 1) * 16;        // after the turn: token c0 + j_tok, 16 outputs
-      const int out0 = n0 + (int)rank * ROWS + quad * 32 + c_half;
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * S::TOKENS;
+      const int j_tok = lane >> 1, c_half = (lane & 1) * 16;        // after the turn: token c0 + j_tok, 16 accumulator rows
+      // This thread's accumulator row stands for output `col`; gated: rows come as 8 gates, then the up rows of the same outputs.
+      const int cta0 = n0 + (int)rank * S::OUTS;
+      const int col = cta0 + (GATED ? (m_row >> 4) * 8 + (m_row & 7) : m_row);
+      const bool up_row = GATED && (m_row & 8);
+      const float b = (p.bias && col < p.N && kb0 == 0) ? p.bias[up_row ? p.N + col : col] : 0.f;
+      constexpr int STORED = GATED ? 8 : 16;                        // outputs a thread stores of a token
+      const int out0 = cta0 + (quad * 32 + c_half) / (GATED ? 2 : 1);
 #pragma unroll 1
-      for (int c0 = 16 * turn_of; c0 < n_mma; c0 += 16 * (S::EPI_WARPS / 4)) {
-        float v[16], u[16];
+      for (int c0 = 16 * turn_of; c0 < n_mma; c0 += STEP) {
+        float v[16];
         if (num_kb > 0) {
           ld16(taddr + c0, v);
-          if (GATED) ld16(taddr + S::UP_COL + c0, u);
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = u[j] = 0.f;
+          for (int j = 0; j < 16; ++j) v[j] = 0.f;
         }
-        // The thread holds 16 tokens of one output; a store wants 16 outputs of one token. The warp turns its block of
-        // 16 tokens by 32 outputs through shared memory: row j (a token) is 32 words, rotated by 4 j words so that
-        // neither the writes (a row a time, a word a lane) nor the 16-byte reads meet in a bank.
-        if (GATED) {
-          // The gated product's MMAs wait for this loop, so it is written for speed: the choice of the activation
-          // stands outside the 16 independent evaluations, and SiLU, the usual one, takes the fast exponential and
-          // division (the result is rounded to bfloat16, far coarser than their error).
-          if (p.row_weight) {
-            const int block = c0 / STEP;
-            const float mine = (block >> 1) == 0 ? rw[0] : ((block >> 1) == 1 ? rw[1] : ((block >> 1) == 2 ? rw[2] : rw[3]));
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float wj = __shfl_sync(0xffffffffu, mine, 16 * (block & 1) + j);
-              v[j] *= wj;
-              u[j] *= wj;
-            }
-          }
-          if (p.bias) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              v[j] += b;
-              u[j] += b_up;
-            }
-          }
-          if constexpr (CLAMPED) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = gated(v[j], u[j], TL_ACT_CLAMPED_SWISH, p.ga0, p.ga1);
-          } else if (p.act == TL_ACT_SILU) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __fdividef(v[j], 1.f + __expf(-v[j])) * u[j];
-          } else if (p.act == TL_ACT_GELU_TANH) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __fdividef(v[j], 1.f + __expf(-gelu_tanh_argument(v[j]))) * u[j];
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = gated(v[j], u[j], p.act, p.ga0, p.ga1);
-          }
-        } else {
+        // The thread holds 16 tokens of one accumulator row; a store wants neighbouring outputs of one token, a gate its up row. The
+        // warp turns its block of 16 tokens by 32 rows through shared memory: row j (a token) is 32 words, rotated by 4 j words
+        // so that neither the writes (a row a time, a word a lane) nor the 16-byte reads meet in a bank.
+        if (!GATED || p.bias) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] += b;
+        }
+        if (!GATED) {
           if (p.unary == TL_ACT_XIELU) {
             // written for speed, as the gated epilogue is: both branches from the fast exponential, one select (the
             // result is rounded to bfloat16, far coarser than exp(z) - 1 - z loses near 0 beside the z / 2 it is added to)
@@ -447,27 +424,53 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, PER_SM) gemm_tc_
           const float4 q = *reinterpret_cast<const float4*>(turn + j_tok * 32 + ((c_half + 4 * i + 4 * j_tok) & 31));
           r[4 * i] = q.x; r[4 * i + 1] = q.y; r[4 * i + 2] = q.z; r[4 * i + 3] = q.w;
         }
+        if constexpr (GATED) {
+          // r: eight gates, then the eight up numbers of the same outputs. The choice of the activation stands outside the
+          // independent evaluations, and SiLU, the usual one, takes the fast exponential and division (the result is rounded
+          // to bfloat16, far coarser than their error).
+          if (p.row_weight) {
+            const int block = c0 / STEP;
+            const float four = (block >> 1) == 0 ? rw[0] : ((block >> 1) == 1 ? rw[1] : ((block >> 1) == 2 ? rw[2] : rw[3]));
+            const float mine = __shfl_sync(0xffffffffu, four, 16 * (block & 1) + j_tok);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] *= mine;
+          }
+          if constexpr (CLAMPED) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = gated(r[j], r[8 + j], TL_ACT_CLAMPED_SWISH, p.ga0, p.ga1);
+          } else if (p.act == TL_ACT_SILU) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = __fdividef(r[j], 1.f + __expf(-r[j])) * r[8 + j];
+          } else if (p.act == TL_ACT_GELU_TANH) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = __fdividef(r[j], 1.f + __expf(-gelu_tanh_argument(r[j]))) * r[8 + j];
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = gated(r[j], r[8 + j], p.act, p.ga0, p.ga1);
+          }
+        }
         const int t = c0 + j_tok;
         if (t < tok_rows && out0 < p.N) {
           TOut* dst = C + (kb0 / p.kb_per_split) * p.part_stride + (long long)(tok0 + t) * p.ldc + out0;
-          if (out0 + 16 <= p.N && (((uintptr_t)dst) & 15) == 0) {
+          if (out0 + STORED <= p.N && (((uintptr_t)dst) & 15) == 0) {
             if constexpr (sizeof(TOut) == 2) {
-              uint4 lo, hi;
-              __nv_bfloat162 h2;
+#pragma unroll
+              for (int i = 0; i < STORED; i += 8) {
+                uint4 q;
+                __nv_bfloat162 h2;
 #define TL_PACK(dst_, a_, b_) h2 = __floats2bfloat162_rn(a_, b_); dst_ = *reinterpret_cast<uint32_t*>(&h2)
-              TL_PACK(lo.x, r[0], r[1]); TL_PACK(lo.y, r[2], r[3]); TL_PACK(lo.z, r[4], r[5]); TL_PACK(lo.w, r[6], r[7]);
-              TL_PACK(hi.x, r[8], r[9]); TL_PACK(hi.y, r[10], r[11]); TL_PACK(hi.z, r[12], r[13]); TL_PACK(hi.w, r[14], r[15]);
+                TL_PACK(q.x, r[i], r[i + 1]); TL_PACK(q.y, r[i + 2], r[i + 3]); TL_PACK(q.z, r[i + 4], r[i + 5]); TL_PACK(q.w, r[i + 6], r[i + 7]);
 #undef TL_PACK
-              reinterpret_cast<uint4*>(dst)[0] = lo;
-              reinterpret_cast<uint4*>(dst)[1] = hi;
+                reinterpret_cast<uint4*>(dst)[i / 8] = q;
+              }
             } else {
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
+              for (int i = 0; i < STORED / 4; ++i)
                 reinterpret_cast<float4*>(dst)[i] = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
+            for (int i = 0; i < STORED; ++i)
               if (out0 + i < p.N) put<TOut>(dst + i, r[i]);
           }
         }
@@ -506,7 +509,7 @@ static int resident_pairs() {
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(2 * PER_SM * (sm_count() / 2));
+  cfg.gridDim = dim3(2 * S::CTAS * (sm_count() / 2));
   cfg.blockDim = dim3(S::THREADS);
   cfg.dynamicSmemBytes = S::TOTAL;
   cfg.attrs = attr;
@@ -518,7 +521,7 @@ static int resident_pairs() {
   // Two CTAs an SM: the query answers as if a pair had the two SMs to itself (74), yet two pairs do share them
   // (ncu: 296 CTAs are one wave, 20 warps active an SM). No pair waits for another in this kernel, so a grid of twice
   // the pairs is safe either way: on a GPU that held only one CTA an SM the others would simply start later.
-  if (PER_SM == 2 && n >= 1) clusters = 2 * (sm_count() / 2);
+  if (S::CTAS == 2 && n >= 1) clusters = 2 * (sm_count() / 2);
   return clusters;
 }
 
@@ -594,7 +597,15 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   const int tokens = (gated && per_sm == 2) ? 128 : 256;
   TL_REQUIRE(!tile_group || plan_rows <= tokens, "pair product: a tile map with tiles of %d rows; at most %d", plan_rows, tokens);
   CUtensorMap tmW, tmX[3];
-  if (int e = tensor_map(W, w_rows, K, ldw, pair::ROWS, &tmW)) return e;
+  if (gated) {
+    const long long per_group = tile_group ? rows_per_group : 2 * (long long)N;
+    TL_REQUIRE(N % 8 == 0 && per_group >= 2 * (long long)N && w_rows >= per_group,
+               "pair product: %d gated outputs (a multiple of 8) need as many gate and up rows a group (%lld rows a group, %lld in all)", N,
+               per_group, w_rows);
+    if (int e = gate_up_map(W, w_rows, per_group, N, K, ldw, pair::ROWS, &tmW)) return e;
+  } else if (int e = tensor_map(W, w_rows, K, ldw, pair::ROWS, &tmW)) {
+    return e;
+  }
   if (int e = tensor_map(X, x_rows, K, ldx, 16, &tmX[0])) return e;
   if (int e = tensor_map(X, x_rows, K, ldx, 64, &tmX[1])) return e;
   if (int e = tensor_map(X, x_rows, K, ldx, 128, &tmX[2])) return e;
@@ -608,7 +619,7 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   p.unary = unary; p.a0 = a0; p.a1 = a1;
   p.skip_kb = pair::skip_kb_for_test();
   p.splits = splits; p.kb_per_split = kb_per_split; p.part_stride = splits > 1 ? (long long)M * ldc : 0;
-  const long long work = (long long)ceil_div(N, 2 * pair::ROWS) * (tile_group ? max_tiles : ceil_div(M, tokens)) * splits;
+  const long long work = (long long)ceil_div(N, gated ? pair::ROWS : 2 * pair::ROWS) * (tile_group ? max_tiles : ceil_div(M, tokens)) * splits;
 #define TL_PAIR(G_, P_) \
   (out_dtype == TL_BF16 ? pair::launch<G_, P_, bf16>(tmW, tmX, p, work, stream) : pair::launch<G_, P_, float>(tmW, tmX, p, work, stream))
   if (gated == TL_ACT_CLAMPED_SWISH && out_dtype == TL_BF16)

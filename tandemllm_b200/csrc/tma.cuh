@@ -80,24 +80,25 @@ struct MapKey {
   const void* ptr;
   long long rows, cols, ld;
   int box_rows;
+  long long outputs, per_group;      // of a `gate_up_map`; 0 for a 2D map
   bool operator==(const MapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows;
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && outputs == o.outputs &&
+           per_group == o.per_group;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = (size_t)k.ptr;
     h ^= (size_t)k.rows * 0x9E3779B97F4A7C15ULL + (size_t)k.cols * 0xBF58476D1CE4E5B9ULL + (size_t)k.ld * 31 + k.box_rows;
-    return h;
+    return h ^ ((size_t)k.outputs * 0x94D049BB133111EBULL + (size_t)k.per_group);
   }
 };
 
-// A 2D bf16 tensor [rows, cols] with row stride ld (elements), box [box_rows, 64 columns], 128-byte swizzle. Maps are
-// kept by (pointer, shape, box): the same weights and caches come back every step.
-inline int tensor_map(const void* ptr, long long rows, long long cols, long long ld, int box_rows, CUtensorMap* out) {
+// The map of `key`, made by `encode` where it is not kept yet: the same weights and caches come back every step.
+template <typename Encode>
+inline int kept_map(const MapKey& key, CUtensorMap* out, Encode encode) {
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   static std::mutex mu;
-  MapKey key{ptr, rows, cols, ld, box_rows};
   std::lock_guard<std::mutex> g(mu);
   auto it = cache.find(key);
   if (it != cache.end()) {
@@ -106,18 +107,41 @@ inline int tensor_map(const void* ptr, long long rows, long long cols, long long
   }
   EncodeTiledFn fn = encode_fn();
   TL_REQUIRE(fn != nullptr, "tensor map: the driver does not export cuTensorMapEncodeTiled (%d)", 0);
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)TMA_BOX_COLS, (cuuint32_t)box_rows};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = encode(fn);
   TL_REQUIRE(r == CUDA_SUCCESS, "tensor map: cuTensorMapEncodeTiled failed with %d (rows %lld cols %lld ld %lld box %d)",
-             (int)r, rows, cols, ld, box_rows);
+             (int)r, key.rows, key.cols, key.ld, key.box_rows);
   if (cache.size() > 8192) cache.clear();
   cache.emplace(key, *out);
   return 0;
+}
+
+// A 2D bf16 tensor [rows, cols] with row stride ld (elements), box [box_rows, 64 columns], 128-byte swizzle.
+inline int tensor_map(const void* ptr, long long rows, long long cols, long long ld, int box_rows, CUtensorMap* out) {
+  return kept_map(MapKey{ptr, rows, cols, ld, box_rows, 0, 0}, out, [&](EncodeTiledFn fn) {
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    cuuint32_t box[2] = {(cuuint32_t)TMA_BOX_COLS, (cuuint32_t)box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
+}
+
+// Weights of gated products, [rows / per_group groups][`outputs` gate rows, as many up rows][cols] with row stride ld, as a 5D
+// tensor (k, row of 8, gate or up, block of 8 outputs, group): a box of 8 x 2 x box_rows / 16 rows lands in shared memory with 8
+// gate rows and the 8 up rows of the same outputs in turn. `outputs` is a multiple of 8; blocks past the last read as zero.
+inline int gate_up_map(const void* ptr, long long rows, long long per_group, long long outputs, long long cols, long long ld,
+                       int box_rows, CUtensorMap* out) {
+  return kept_map(MapKey{ptr, rows, cols, ld, box_rows, outputs, per_group}, out, [&](EncodeTiledFn fn) {
+    cuuint64_t dims[5] = {(cuuint64_t)cols, 8, 2, (cuuint64_t)(outputs / 8), (cuuint64_t)(rows / per_group)};
+    cuuint64_t strides[4] = {(cuuint64_t)ld * 2, (cuuint64_t)(outputs * ld) * 2, (cuuint64_t)ld * 16, (cuuint64_t)(per_group * ld) * 2};
+    cuuint32_t box[5] = {(cuuint32_t)TMA_BOX_COLS, 8, 2, (cuuint32_t)(box_rows / 16), 1};
+    cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
 }
 
 }  // namespace tl

@@ -53,7 +53,7 @@ PROMPT_PRODUCT = SETTINGS.get("PROMPT_PRODUCT")
 if PROMPT_PRODUCT not in ("pair", "single"):
     raise ValueError(f"TANDEMLLM_PROMPT_PRODUCT={PROMPT_PRODUCT!r}: pair or single")
 HEADMIX_PROMPT_ROWS = 8         # rows a request must bring for a step's head-mixed attention to run on the tensor cores
-PAIR_HALF_ROWS = 64             # rows an expert (on average) up to which the experts' pair products run two CTAs an SM
+PAIR_HALF_ROWS = 64             # rows an expert (on average) up to which the experts' pair products take the form bound by weights
 _lib = None
 
 
@@ -272,10 +272,10 @@ class TensorCore:
 
     def gemm_pair(self, x, w2d, bias, out, *, rows_per_group=0, plan=None, gated: int = 0, n_out=None,
                   rows: int | None = None, per_sm: int | None = None, splits: int = 1, weights=None) -> None:
-        """The product on pairs of SMs (csrc/tc_gemm_pair.cu): 256 outputs by up to 256 token rows a pair, the N side
-        of its MMAs as many rows as a tile holds. `plan`: tiles of any height up to 256 rows. `per_sm` 2: two CTAs an
-        SM, each with half the shared and tensor memory (gated: tiles of up to 128 rows), the form for products bound
-        by their weights; default: 2 for a plan with tiles of up to 128 rows, else 1. `splits` > 1: `out` is
+        """The product on pairs of SMs (csrc/tc_gemm_pair.cu): 256 weight rows by up to 256 token rows a pair, the N side
+        of its MMAs as many rows as a tile holds. `plan`: tiles of any height up to 256 rows. `per_sm` 2: the form for
+        products bound by their weights (plain: two CTAs an SM, each with half the shared and tensor memory; gated: tiles of
+        up to 128 rows behind a deeper ring); default: 2 for a plan with tiles of up to 128 rows, else 1. `splits` > 1: `out` is
         [splits, M, N] 32-bit and receives the partial results of as many runs of k-blocks (plain product only). A `bias` of
         the gated form (no plan) holds the gate's numbers, then the up rows'. `weights` (gated, with a plan): as in `gemm`."""
         M, K = (rows if rows is not None else x.shape[0]), x.shape[1]
