@@ -9,8 +9,8 @@
 // weight rows instead of once per 128. That path, not the tensor pipe, is what bounds the one-CTA kernel at these sizes.
 //
 // The N side of an MMA is a run-time number (a multiple of 16 up to 256): a tile of the routed experts' products that
-// holds 40 rows costs an MMA of N = 48 and not a padded 128-row one, and its token rows come as a box of 64 rows a CTA
-// and not of 128 (three box heights are kept: 16, 64 and 128), so ragged expert sizes cost about what they hold.
+// holds 40 rows costs an MMA of N = 48 and not a padded 128-row one, and its token rows come as a box of 32 rows a CTA
+// and not of 128 (four box heights are kept: 16, 32, 64 and 128), so ragged expert sizes cost about what they hold.
 //
 // Roles in each CTA, as in the one-CTA persistent kernel (tc_gemm.cu): warp 0, one thread, keeps a ring of stages full
 // by TMA (plain loads, each CTA its own; their bytes are counted on the first CTA's barrier); warp 1 of the first CTA,
@@ -72,7 +72,7 @@ inline int& skip_kb_for_test() {
 // PER_SM 2 is the form for products bound by their weights. Plain: two CTAs an SM, half the shared memory and half the tensor memory
 // each and one accumulator, so the other CTA of the SM is what runs under an epilogue; twice the pairs are resident, and when the last
 // round leaves an SM with one CTA instead of two, that CTA loads at the SM's full rate. Gated: tiles of up to 128 token rows, one CTA an
-// SM with a ring of eight stages and four accumulators (two CTAs of four stages each took 107 us where this takes 92: 400 rows of
+// SM with a ring of nine stages and four accumulators (two CTAs of four stages each took 107 us where this takes 91: 400 rows of
 // top-4 of 32 experts of 1792 x 2048).
 template <bool GATED, int PER_SM>
 struct Smem {
@@ -82,12 +82,12 @@ struct Smem {
   static constexpr int TMEM_COLS = CTAS == 2 ? 256 : 512;
   static constexpr int ACC_BUFS = TMEM_COLS / TOKENS;              // accumulators in tensor memory
   // Epilogue warps: one a quarter of the accumulator's lanes, or two that take every other block of 16 tokens
-  static constexpr int EPI_WARPS = GATED ? 8 : 4;
+  static constexpr int EPI_WARPS = GATED && PER_SM == 1 ? 8 : 4;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int A_BYTES = ROWS * TILE_K * 2;                // one box of weights
   static constexpr int B_BYTES = (TOKENS / 2) * TILE_K * 2;        // this CTA's half of the token rows, at most
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = PER_SM == 2 ? (GATED ? 8 : 3) : 6;
+  static constexpr int STAGES = PER_SM == 2 ? (GATED ? 9 : 3) : 6;
   static constexpr int TURN_BYTES = EPI_WARPS * 16 * 32 * 4;       // the epilogue warps' blocks
   static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */ + TURN_BYTES;
   static_assert(CTAS * TOTAL <= 227 * 1024, "the CTAs of an SM share its shared memory");
@@ -191,6 +191,7 @@ template <> __device__ __forceinline__ void put<bf16>(bf16* p, float v) { *p = _
 template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false>
 __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_SM>::CTAS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
                                                            const __grid_constant__ CUtensorMap tmX16,
+                                                           const __grid_constant__ CUtensorMap tmX32,
                                                            const __grid_constant__ CUtensorMap tmX64,
                                                            const __grid_constant__ CUtensorMap tmX128, Params p) {
   using S = Smem<GATED, PER_SM>;
@@ -277,8 +278,8 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
       const int my_out = n0 + (int)rank * S::OUTS;                   // this CTA's outputs
       const int my_row = (int)(group * p.rows_per_group) + my_out;
       // the smallest box that holds the half; rows of it behind the half are read and never used
-      const int box = half <= 16 ? 16 : (half <= 64 ? 64 : 128);      // (a half is at most TOKENS / 2 rows)
-      const CUtensorMap* tmX = box == 16 ? &tmX16 : (box == 64 ? &tmX64 : &tmX128);
+      const int box = half <= 16 ? 16 : (half <= 32 ? 32 : (half <= 64 ? 64 : 128));      // (a half is at most TOKENS / 2 rows)
+      const CUtensorMap* tmX = box == 16 ? &tmX16 : (box == 32 ? &tmX32 : (box == 64 ? &tmX64 : &tmX128));
       const uint32_t cta_bytes = (uint32_t)(S::A_BYTES + box * TILE_K * 2);
       for (int kb = 0; kb < num_kb; ++kb, ++it) {
         const int s = it % S::STAGES;
@@ -543,7 +544,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap* tmX, const Params& 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED>, tmW, tmX[0], tmX[1], tmX[2], p);
+  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED>, tmW, tmX[0], tmX[1], tmX[2], tmX[3], p);
 }
 
 }  // namespace pair
@@ -596,7 +597,7 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
              splits);
   const int tokens = (gated && per_sm == 2) ? 128 : 256;
   TL_REQUIRE(!tile_group || plan_rows <= tokens, "pair product: a tile map with tiles of %d rows; at most %d", plan_rows, tokens);
-  CUtensorMap tmW, tmX[3];
+  CUtensorMap tmW, tmX[4];
   if (gated) {
     const long long per_group = tile_group ? rows_per_group : 2 * (long long)N;
     TL_REQUIRE(N % 8 == 0 && per_group >= 2 * (long long)N && w_rows >= per_group,
@@ -606,9 +607,9 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   } else if (int e = tensor_map(W, w_rows, K, ldw, pair::ROWS, &tmW)) {
     return e;
   }
-  if (int e = tensor_map(X, x_rows, K, ldx, 16, &tmX[0])) return e;
-  if (int e = tensor_map(X, x_rows, K, ldx, 64, &tmX[1])) return e;
-  if (int e = tensor_map(X, x_rows, K, ldx, 128, &tmX[2])) return e;
+  const int boxes[4] = {16, 32, 64, 128};
+  for (int i = 0; i < 4; ++i)
+    if (int e = tensor_map(X, x_rows, K, ldx, boxes[i], &tmX[i])) return e;
   pair::Params p = {};
   p.C = C; p.bias = bias; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
   p.rows_per_group = rows_per_group;
