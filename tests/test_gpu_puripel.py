@@ -166,6 +166,52 @@ def test_long_portions_in_chunks_that_run_side_by_side():
     assert torch.equal(dev_state[1].cpu(), state[1]) and torch.equal(dev_state[:, :offset].cpu(), state[:, :offset])
 
 
+@pytest.mark.parametrize("H,Pc,N,G", [(3, 20, 64, 1), (4, 64, 128, 2), (2, 68, 132, 1), (1, 8, 256, 1)])
+def test_long_portions_in_matrix_form(H, Pc, N, G):
+    """States of 64 keys and more: chunks of 64 rows as products (csrc/chunk_matrix.cuh), requests of 1, 64, 65 and 330 rows side by
+    side, against the plain recurrence in 64 bits (32-bit sums of up to 330 + N terms: 1e-5 of the result); and an infinite value
+    late in a portion reaches no row before it."""
+    from tandemllm_b200.kernels import ops
+    from tandemllm_b200.parts.base import Runtime
+    rt = Runtime(torch.device(DEV), torch.float32)
+    g = torch.Generator().manual_seed(H * 1000 + N)
+    inner, lengths, slots = H * Pc, [64, 330, 1, 65], [2, 0, 3, 1]
+    T = sum(lengths)
+    xbc = torch.randn(T, inner + 2 * G * N, generator=g)
+    dt = torch.randn(T, H, generator=g) - 1.0
+    dt_bias, a_log, d = 0.5 * torch.randn(H, generator=g), 0.7 * torch.randn(H, generator=g) - 2.0, 1 + torch.randn(H, generator=g)
+    state = torch.randn(5, H * Pc * N, generator=g)
+    starts = [0, 64, 394, 395, 460]
+
+    def run(x):
+        dev_state, y = state.clone().to(DEV), torch.empty(T, inner, device=DEV)
+        assert ops.core().tl_ssm_scan_chunk(Pc, N, x.shape[1], 0) == 64
+        ops.ssm_scan(x.to(DEV), dt.to(DEV), dt_bias.to(DEV), a_log.to(DEV), d.to(DEV), dev_state, 0, i32(slots), i32(starts), 4, y, H, Pc,
+                     N, G, max_rows_per_request=330, runtime=rt)
+        return y.cpu(), dev_state.cpu()
+    y, after = run(xbc)
+    group = torch.arange(H) // (H // G)
+    for b, (n, slot) in enumerate(zip(lengths, slots)):
+        rows = xbc[starts[b]:starts[b] + n].double()
+        x, B, Cm = rows[:, :inner].view(n, H, Pc), rows[:, inner:inner + G * N].view(n, G, N), rows[:, inner + G * N:].view(n, G, N)
+        step = P.softplus(dt[starts[b]:starts[b] + n].double() + dt_bias.double())
+        decay = torch.exp(-torch.exp(a_log.double()) * step)
+        S = state[slot].double().view(H, Pc, N).transpose(1, 2).clone()
+        want = torch.zeros(n, H, Pc, dtype=torch.float64)
+        for t in range(n):
+            S = decay[t, :, None, None] * S + step[t, :, None, None] * B[t, group][:, :, None] * x[t, :, None, :]
+            want[t] = torch.einsum("hnp,hn->hp", S, Cm[t, group]) + d.double()[:, None] * x[t]
+        assert rel(y[starts[b]:starts[b] + n], want.view(n, inner)) < 1e-5, b
+        assert rel(after[slot].view(1, -1), S.transpose(1, 2).reshape(1, -1)) < 1e-5, b
+    assert torch.equal(after[4], state[4])
+    wild = xbc.clone()
+    wild[64 + 150, 3] = float("inf")
+    y2, _ = run(wild)
+    keep = [r for r in range(T) if not 64 + 150 <= r < 394]
+    assert rel(y2[keep], y[keep].double()) < 1e-5 and bool(torch.isfinite(y2[keep]).all())
+    assert not bool(torch.isfinite(y2[64 + 150, 3]))
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_the_gate_comes_before_the_norm_of_each_part(dtype):
     from tandemllm_b200.kernels import ops
