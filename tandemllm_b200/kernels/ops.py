@@ -111,6 +111,8 @@ _SIGNATURES = {
     "tl_paged_attention_split": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_int,
                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "tl_attention_join": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "tl_attention_join_tiles": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                                c_void_p],
     "tl_router_topk": [c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p,
                        c_void_p],
     "tl_moe_max_tiles": [c_int, c_int, c_int],
@@ -873,6 +875,14 @@ def attention_join(scratch, positions, window, out, n_spans: int, span_keys: int
     check(core().tl_attention_join(ptr(scratch), ptr(positions), int(window or 0), ptr(out), rows, Hq, D, int(n_spans),
                                    int(span_keys), dtype_code(out.dtype), stream()), "attention_join",
           kernels=1 if n_spans > 1 else 0)
+
+
+def attention_join_tiles(scratch, positions, window, out, n_spans: int, span_keys: int, tiles, tile_rows: int) -> None:
+    """`attention_join` for the rows of `tiles` (int32 [n, 3] = (request, first row, rows), at most `tile_rows` rows each) alone."""
+    rows, Hq, D = out.shape
+    check(core().tl_attention_join_tiles(ptr(scratch), ptr(positions), int(window or 0), ptr(out), rows, Hq, D, int(n_spans),
+                                         int(span_keys), dtype_code(out.dtype), ptr(tiles), tiles.shape[0], int(tile_rows), stream()),
+          "attention_join_tiles", kernels=1 if n_spans > 1 else 0)
 
 
 def qkv_rotate_store(qkv, q_col: int, k_col: int, v_col: int, inv_freq, rot: int, inv_freq_v, positions, req_of_row, table,

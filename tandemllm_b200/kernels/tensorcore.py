@@ -654,10 +654,12 @@ def _attention_flex(self, part, q, cache, table, step, gate, ld_gate: int, out_s
     return True
 
 
-def _split_tiles(self, step, big_rows: int, small_rows: int):
+def _split_tiles(self, step, big_rows: int, small_rows: int, from_first: bool = False):
     """(tiles of requests that bring more than `small_rows` rows, cut into `big_rows` rows; one tile for each of the other
-    requests), each int32 [n, 3] = (request, first row, rows) on the device, or None. Kept on the step."""
-    key = ("split_tiles", big_rows, small_rows)
+    requests; the most rows of those), tiles int32 [n, 3] = (request, first row, rows) on the device, or None. With `from_first`
+    the other requests' rows are counted from their first one; where that lies, how many rows there are up to their last one and
+    their longest context is at ("small_rows", small_rows). Kept on the step."""
+    key = ("split_tiles", big_rows, small_rows, from_first)
     if key not in step.host:
         starts = step.host["row_start"]
         big, small = [], []
@@ -667,6 +669,11 @@ def _split_tiles(self, step, big_rows: int, small_rows: int):
                 small.append((b, starts[b], n))
             else:
                 big += [(b, r0, min(big_rows, starts[b + 1] - r0)) for r0 in range(starts[b], starts[b + 1], big_rows)]
+        if from_first and small:
+            first, at = small[0][1], step.host.get("start_pos")
+            longest = max(at[b] + n for b, _, n in small) if at else step.max_context
+            step.host["small_rows", small_rows] = (first, small[-1][1] + small[-1][2] - first, longest)
+            small = [(b, r0 - first, n) for b, r0, n in small]
         both = torch.tensor(big + small, dtype=torch.int32).reshape(-1, 3).to(self.device, non_blocking=True)
         step.host[key] = (both[:len(big)] if big else None, both[len(big):] if small else None,
                           max((t[2] for t in small), default=0))
@@ -676,40 +683,65 @@ def _split_tiles(self, step, big_rows: int, small_rows: int):
 def _prompt_attention(self, q, cache, table, step, scale, window, out, runtime) -> bool:
     """A step with prompt portions. Requests that bring many rows go to the tcgen05 kernel in tiles of 128 M rows (128 / G
     query rows), two CTAs an SM; requests that bring a row or a few (the decode rows of a mixed step) go to the mma.sync
-    kernel's form for small tiles, which splits each key tile among its warps. Both cut the keys into the same spans, so
-    one join serves the step; the keys are split only when the tiles alone would leave half of the GPU idle."""
+    kernel's form for small tiles, which splits each key tile among its warps. Each cuts its keys into spans of its own and joins
+    its own rows; the keys of many-row tiles are split only when the tiles alone would leave half of the GPU idle."""
     R, Hq, D = q.shape
     Hk = cache.k.shape[1]
     G = Hq // Hk
     tile_rows = lib().tl_attention_tc_tile_rows(Hq, Hk)
-    big, small, small_max = self._split_tiles(step, tile_rows, 16 // G)
+    big, small, small_max = self._split_tiles(step, tile_rows, 16 // G, from_first=True)
     n_big = 0 if big is None else big.shape[0]
     n_small = 0 if small is None else small.shape[0]
-    ctas, slots = (n_big + n_small) * Hk, 2 * self.sm_count
-    span_keys, spans = 0, 1
-    if step.max_context > 1024 and 2 * ctas <= slots:
-        # (only then: the join reads and writes every row's partial results, which for a prompt's many rows costs as
-        # much as the attention of a short context itself)
-        want = slots // ctas                                           # spans that fill the GPU once
-        span_keys = max(1024, -(-(-(-step.max_context // want)) // 128) * 128)
-        spans = -(-step.max_context // span_keys)
-        if spans <= 1:
-            span_keys, spans = 0, 1
-    scratch = runtime.scratch("attention", ops.attention_scratch_floats(R, Hq, D, spans)) if span_keys else None
-    common = (step.positions.data_ptr(), float(scale), int(window or 0), out.data_ptr(), ops.ptr(scratch), R, Hq, Hk, D, spans,
-              span_keys, self.status.data_ptr(), ops.stream())
-    head = (q.data_ptr(), cache.k.data_ptr(), cache.v.data_ptr(), table.data_ptr(), table.shape[1], cache.page_size,
-            cache.k.shape[0])
+    kv = (cache.k.data_ptr(), cache.v.data_ptr(), table.data_ptr(), table.shape[1], cache.page_size, cache.k.shape[0])
+
+    def run(kernel, what, tiles, most, first, rows, spans, span_keys, scratch):
+        at = first * Hq * D * q.element_size()
+        _check(kernel(q.data_ptr() + at, *kv, tiles.data_ptr(), tiles.shape[0], most, step.positions.data_ptr() + 4 * first, float(scale),
+                      int(window or 0), out.data_ptr() + at, ops.ptr(scratch), rows, Hq, Hk, D, spans, span_keys,
+                      self.status.data_ptr(), ops.stream()), what)
     if n_big:
-        _check(lib().tl_paged_attention_tc(*head, big.data_ptr(), n_big, min(tile_rows, step.max_rows_per_request), *common),
-               "attention_tc")
+        ctas, slots = n_big * Hk, 2 * self.sm_count
+        span_keys, spans = 0, 1
+        if step.max_context > 1024 and 2 * (ctas + n_small * Hk) <= slots:
+            # (only then: the join reads and writes every row's partial results, which for a prompt's many rows costs as
+            # much as the attention of a short context itself)
+            want = slots // (ctas + n_small * Hk)                          # spans that fill the GPU once
+            span_keys = max(1024, -(-(-(-step.max_context // want)) // 128) * 128)
+            spans = -(-step.max_context // span_keys)
+            if spans <= 1:
+                span_keys, spans = 0, 1
+        scratch = runtime.scratch("attention", ops.attention_scratch_floats(R, Hq, D, spans)) if span_keys else None
+        run(lib().tl_paged_attention_tc, "attention_tc", big, min(tile_rows, step.max_rows_per_request), 0, R, spans, span_keys, scratch)
+        if span_keys and n_small:
+            ops.attention_join_tiles(scratch, step.positions, window, out, spans, span_keys, big, tile_rows)
+        elif span_keys:
+            ops.attention_join(scratch, step.positions, window, out, spans, span_keys)
     if n_small:
-        _check(lib().tl_paged_attention_mma(*head, small.data_ptr(), n_small, small_max, *common), "attention_mma")
-    if span_keys:
-        ops.attention_join(scratch, step.positions, window, out, spans, span_keys)
+        # A row a request, and contexts of any length: without spans the longest context is one CTA's chain (23 rows at 201 to 4100
+        # keys, 184 CTAs: 57 us a layer; a step of 512 rows beside them 2360 -> 2271 us with the gated products, two layers of eight).
+        first, rows, longest = step.host[("small_rows", 16 // G)]
+        spans, span_keys = self._row_spans(n_small * Hk, longest) if rows <= 16 * n_small + 64 else (1, 0)
+        scratch = runtime.scratch("attention_rows", ops.attention_scratch_floats(rows, Hq, D, spans)) if span_keys else None
+        run(lib().tl_paged_attention_mma, "attention_mma", small, small_max, first, rows, spans, span_keys, scratch)
+        if span_keys:
+            ops.attention_join_tiles(scratch, step.positions[first:first + rows], window, out[first:first + rows], spans, span_keys, small,
+                                     small_max)
     return True
 
 
+def _row_spans(self, ctas: int, longest: int) -> tuple[int, int]:
+    """(spans, keys a span) of the keys of `ctas` small tiles whose longest context is `longest`: spans of 256 keys, doubled while the
+    longest contexts alone would still be four CTAs an SM; (1, 0) where the tiles fill the GPU or the contexts are short."""
+    if longest <= 512 or ctas >= 8 * self.sm_count:
+        return 1, 0
+    span = 256
+    while span < 2048 and ctas * -(-longest // (2 * span)) >= 4 * self.sm_count:
+        span *= 2
+    spans = -(-longest // span)
+    return (spans, span) if spans > 1 else (1, 0)
+
+
+TensorCore._row_spans = _row_spans
 TensorCore._split_tiles = _split_tiles
 TensorCore.attention_flex = _attention_flex
 TensorCore._prompt_attention = _prompt_attention

@@ -418,6 +418,40 @@ def test_a_mixed_step_sends_portions_and_decode_rows_to_their_kernels_over_the_s
         at += n
 
 
+@pytest.mark.parametrize("Hq,Hk,window,lead", [(32, 8, None, 300), (4, 4, 700, 0), (8, 2, None, 20)])
+def test_decode_rows_beside_a_portion_cut_their_keys_into_spans_of_their_own(Hq, Hk, window, lead):
+    """Decode rows that lie together behind a portion's rows (`lead` rows; 0: every request brings a few): contexts of one to
+    thousands of keys, at the edges of a span and inside the first one."""
+    import types
+
+    from tests.test_gpu_kernels import paged_setup, plain_attention
+    impl, rt = tc()
+    few = 16 // (Hq // Hk)
+    seqs, news = [1, 255, 256, 257, 513, 1024, 3000, 2100], [1, 1, min(2, few), 1, 1, 1, 1, few]
+    if lead:
+        seqs, news = [400] + seqs, [lead] + news
+    else:
+        seqs, news = seqs + [900], news + [40]
+    kc, vc, table, ks, vs = paged_setup(seqs, Hk, 64, 16, torch.bfloat16, seed=90)
+    R = sum(news)
+    q = rnd(R, Hq, 64, seed=91)
+    positions = sum((list(range(L - n, L)) for L, n in zip(seqs, news)), [])
+    starts = [0]
+    for n in news:
+        starts.append(starts[-1] + n)
+    step = types.SimpleNamespace(n_requests=len(seqs), max_rows_per_request=max(news), max_context=max(seqs),
+                                 positions=torch.tensor(positions, dtype=torch.int32, device=DEV),
+                                 host={"row_start": starts, "start_pos": [L - n for L, n in zip(seqs, news)]})
+    cache = types.SimpleNamespace(k=kc.to(DEV), v=vc.to(DEV), page_size=16)
+    out = torch.full((R, Hq, 64), float("nan"), dtype=torch.bfloat16, device=DEV)
+    assert impl.attention(q.to(DEV), cache, table.to(DEV), step, 0.125, window, out, rt)
+    torch.cuda.synchronize()
+    assert int(rt.status) == 0
+    for b, (L, n) in enumerate(zip(seqs, news)):
+        want = plain_attention(q[starts[b]:starts[b] + n].float(), ks[b], vs[b], 0.125, window)
+        assert rel(out[starts[b]:starts[b] + n], want) < 2e-2, f"sequence {b}"
+
+
 def attention_against_plain(seqs, news, split, Hq, Hk, D, page, window, kernel="mma"):
     if kernel == "tc":
         # both forms of the tcgen05 kernel: P back in tensor memory (the default), and P through shared memory
