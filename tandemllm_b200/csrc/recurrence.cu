@@ -296,95 +296,102 @@ __global__ void __launch_bounds__(128) recurrence_prepare_kernel(
 
 constexpr int REC_GROUP = 8;
 constexpr int REC_CHUNK = 16;     // the most tokens a stage holds; a column's values of a stage lie this far apart
-// REC_GROUP tokens (FULL) or the first n of them for one lane: the lane's KPL keys of its column go through the tokens, the
-// outputs wait in registers and cross the lanes together. Everything a token needs lies at offsets the compiler knows
-// (`tok`: the lane's first four floats of the group's first prepared token; `vcol`: the column's values, a token a float),
-// so the group is straight-line code whose loads the compiler moves ahead of the chain.
-template <int RULE, int KPL, int DP, bool FULL>
-__device__ __forceinline__ void rec_group(float (&s)[KPL], const float* __restrict__ tok, const float* __restrict__ vcol,
-                                          float* __restrict__ yg, long long ldy, int n, int part, bool owns, float c_h) {
+// REC_GROUP tokens (FULL) or the first n of them for one lane: the lane's KPL keys of its CPL neighbouring columns go through the
+// tokens, the outputs wait in registers and cross the lanes together. Everything a token needs lies at offsets the compiler knows
+// (`tok`: the lane's first four floats of the group's first prepared token; `vcol`: its first column's values, a token a float),
+// so the group is straight-line code whose loads the compiler moves ahead of the chain. `owned`: how many of its columns exist.
+template <int RULE, int KPL, int CPL, int DP, bool FULL>
+__device__ __forceinline__ void rec_group(float (&s)[CPL][KPL], const float* __restrict__ tok, const float* __restrict__ vcol,
+                                          float* __restrict__ yg, long long ldy, int n, int part, int owned, float c_h) {
   constexpr bool DELTA = RULE == RULE_DELTA, GATED = RULE == RULE_GATED;
   constexpr int P = DP / KPL, M = KPL / 4, tok_floats = rec_arrays(RULE) * DP, Q = DP / 4;
-  float o[REC_GROUP];
+  float o[CPL][REC_GROUP];
 #pragma unroll
   for (int tt = 0; tt < REC_GROUP; ++tt) {
-    o[tt] = 0.f;
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) o[c][tt] = 0.f;
     if (FULL || tt < n) {
       const float4* a = reinterpret_cast<const float4*>(tok + tt * tok_floats);
-      const float vj = vcol[tt];
-      float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+      float us[CPL], vj[CPL], sum[CPL][4];
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        vj[c] = vcol[c * REC_CHUNK + tt];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[c][i] = 0.f;
+      }
       if (DELTA) {
-        float us0 = 0.f, us1 = 0.f, us2 = 0.f, us3 = 0.f;      // four short chains of additions instead of one long one
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
+        for (int m = 0; m < M; ++m) {             // four short chains of additions a column instead of one long one
           const float4 u = a[3 * Q + P * m];
-          us0 = fmaf(u.x, s[4 * m], us0);
-          us1 = fmaf(u.y, s[4 * m + 1], us1);
-          us2 = fmaf(u.z, s[4 * m + 2], us2);
-          us3 = fmaf(u.w, s[4 * m + 3], us3);
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) {
+            sum[c][0] = fmaf(u.x, s[c][4 * m], sum[c][0]);
+            sum[c][1] = fmaf(u.y, s[c][4 * m + 1], sum[c][1]);
+            sum[c][2] = fmaf(u.z, s[c][4 * m + 2], sum[c][2]);
+            sum[c][3] = fmaf(u.w, s[c][4 * m + 3], sum[c][3]);
+          }
         }
-        float us = (us0 + us1) + (us2 + us3);
 #pragma unroll
-        for (int off = P >> 1; off > 0; off >>= 1) us += __shfl_xor_sync(0xffffffffu, us, off);
+        for (int c = 0; c < CPL; ++c) {
+          us[c] = (sum[c][0] + sum[c][1]) + (sum[c][2] + sum[c][3]);
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-          const float4 q = a[P * m], k = a[Q + P * m], d = a[2 * Q + P * m], au = a[4 * Q + P * m];
-          s[4 * m] = fmaf(d.x, s[4 * m], fmaf(-au.x, us, k.x * vj));
-          s[4 * m + 1] = fmaf(d.y, s[4 * m + 1], fmaf(-au.y, us, k.y * vj));
-          s[4 * m + 2] = fmaf(d.z, s[4 * m + 2], fmaf(-au.z, us, k.z * vj));
-          s[4 * m + 3] = fmaf(d.w, s[4 * m + 3], fmaf(-au.w, us, k.w * vj));
-          o0 = fmaf(s[4 * m], q.x, o0);
-          o1 = fmaf(s[4 * m + 1], q.y, o1);
-          o2 = fmaf(s[4 * m + 2], q.z, o2);
-          o3 = fmaf(s[4 * m + 3], q.w, o3);
+          for (int i = 0; i < 4; ++i) sum[c][i] = 0.f;
         }
-      } else if (GATED) {
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-          const float4 q = a[P * m], k = a[Q + P * m], d = a[2 * Q + P * m];
-          s[4 * m] = fmaf(d.x, s[4 * m], k.x * vj);
-          s[4 * m + 1] = fmaf(d.y, s[4 * m + 1], k.y * vj);
-          s[4 * m + 2] = fmaf(d.z, s[4 * m + 2], k.z * vj);
-          s[4 * m + 3] = fmaf(d.w, s[4 * m + 3], k.w * vj);
-          o0 = fmaf(s[4 * m], q.x, o0);
-          o1 = fmaf(s[4 * m + 1], q.y, o1);
-          o2 = fmaf(s[4 * m + 2], q.z, o2);
-          o3 = fmaf(s[4 * m + 3], q.w, o3);
-        }
-      } else {
+        for (int off = P >> 1; off > 0; off >>= 1)
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-          const float4 q = a[P * m], k = a[Q + P * m];
-          s[4 * m] = fmaf(c_h, s[4 * m], k.x * vj);
-          s[4 * m + 1] = fmaf(c_h, s[4 * m + 1], k.y * vj);
-          s[4 * m + 2] = fmaf(c_h, s[4 * m + 2], k.z * vj);
-          s[4 * m + 3] = fmaf(c_h, s[4 * m + 3], k.w * vj);
-          o0 = fmaf(s[4 * m], q.x, o0);
-          o1 = fmaf(s[4 * m + 1], q.y, o1);
-          o2 = fmaf(s[4 * m + 2], q.z, o2);
-          o3 = fmaf(s[4 * m + 3], q.w, o3);
+          for (int c = 0; c < CPL; ++c) us[c] += __shfl_xor_sync(0xffffffffu, us[c], off);
+      }
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const float4 q = a[P * m], k = a[Q + P * m];
+        float4 d, au;
+        if (DELTA || GATED) d = a[2 * Q + P * m];
+        if (DELTA) au = a[4 * Q + P * m];
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          float* sc = s[c] + 4 * m;
+          if (DELTA) {
+            sc[0] = fmaf(d.x, sc[0], fmaf(-au.x, us[c], k.x * vj[c]));
+            sc[1] = fmaf(d.y, sc[1], fmaf(-au.y, us[c], k.y * vj[c]));
+            sc[2] = fmaf(d.z, sc[2], fmaf(-au.z, us[c], k.z * vj[c]));
+            sc[3] = fmaf(d.w, sc[3], fmaf(-au.w, us[c], k.w * vj[c]));
+          } else {
+            sc[0] = fmaf(GATED ? d.x : c_h, sc[0], k.x * vj[c]);
+            sc[1] = fmaf(GATED ? d.y : c_h, sc[1], k.y * vj[c]);
+            sc[2] = fmaf(GATED ? d.z : c_h, sc[2], k.z * vj[c]);
+            sc[3] = fmaf(GATED ? d.w : c_h, sc[3], k.w * vj[c]);
+          }
+          sum[c][0] = fmaf(sc[0], q.x, sum[c][0]);
+          sum[c][1] = fmaf(sc[1], q.y, sum[c][1]);
+          sum[c][2] = fmaf(sc[2], q.z, sum[c][2]);
+          sum[c][3] = fmaf(sc[3], q.w, sum[c][3]);
         }
       }
-      o[tt] = (o0 + o1) + (o2 + o3);
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) o[c][tt] = (sum[c][0] + sum[c][1]) + (sum[c][2] + sum[c][3]);
     }
   }
-  rec_reduce_scatter<REC_GROUP, P>(o, part);
-  if (!owns) return;
-  if (P <= REC_GROUP) {
-    constexpr int each = P <= REC_GROUP ? REC_GROUP / P : 1;
 #pragma unroll
-    for (int i = 0; i < each; ++i) {
-      const int t = part * each + i;
-      if (FULL || t < n) yg[t * ldy] = o[i];
+  for (int c = 0; c < CPL; ++c) {
+    rec_reduce_scatter<REC_GROUP, P>(o[c], part);
+    if (c >= owned) continue;
+    if (P <= REC_GROUP) {
+      constexpr int each = P <= REC_GROUP ? REC_GROUP / P : 1;
+#pragma unroll
+      for (int i = 0; i < each; ++i) {
+        const int t = part * each + i;
+        if (FULL || t < n) yg[t * ldy + c] = o[c][i];
+      }
+    } else {
+      constexpr int share = P > REC_GROUP ? P / REC_GROUP : 1;
+      const int t = part / share;
+      if (part % share == 0 && (FULL || t < n)) yg[t * ldy + c] = o[c][0];
     }
-  } else {
-    constexpr int share = P > REC_GROUP ? P / REC_GROUP : 1;
-    const int t = part / share;
-    if (part % share == 0 && (FULL || t < n)) yg[t * ldy] = o[0];
   }
 }
 
-// The scan over prepared tokens. Block: cols_per_block * P computing threads (a multiple of 32) and one more warp, the
+// The scan over prepared tokens. Block: cols_per_block * P / CPL computing threads (a multiple of 32) and one more warp, the
 // producer, which does nothing but fetch: it keeps STAGES - 1 chunks of TC tokens in flight (each token's NARR * Dp prepared
 // floats, then the chunk's values, a column's REC_CHUNK apart) and meets the computing warps at one barrier a chunk, when the next
 // chunk has landed and the last one has been read.
@@ -392,8 +399,12 @@ __device__ __forceinline__ void rec_group(float (&s)[KPL], const float* __restri
 // third of the instructions, at the price of two more lane crossings a sum; the launcher takes 4 where the GPU would
 // otherwise stand idle. DP: the keys a head, filled up to a power of two (16 at least); sizes known to the compiler keep
 // the loop free of address arithmetic.
+// CPL neighbouring columns a lane (2 with 16 keys): a token's numbers are read from shared memory once for both, and those reads (five
+// arrays of a token in 16-byte pieces, four cycles a warp each) are what the scan is bound by with a column a lane. With the preparation:
+// 4 requests of 120 to 1100 rows, 16 heads of 128 x 128, 942 -> 605 us with the delta rule, 448 -> 377 with fixed decays, 582 -> 385 with
+// a decay a channel; 8 of 250 rows 495 -> 372, 268 -> 224 and 321 -> 283.
 constexpr int REC_STAGES = 3;
-template <int RULE, int KPL, int DP>
+template <int RULE, int KPL, int CPL, int DP>
 __global__ void __launch_bounds__(REC_THREADS + 32) recurrence_scan_staged_kernel(
     const float* __restrict__ prep, const float* __restrict__ vsrc, long long ld_v, int v_col, const float* __restrict__ head_decay,
     float* __restrict__ state, long long slot_floats, const int* __restrict__ state_slot, const int* __restrict__ row_start,
@@ -406,8 +417,8 @@ __global__ void __launch_bounds__(REC_THREADS + 32) recurrence_scan_staged_kerne
   const int b = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * cols_per_block;
   const int tid = threadIdx.x, nth = blockDim.x - 32;
   const bool producer = tid >= nth;
-  const int part = tid % P, jl = tid / P, j = col0 + jl;
-  const bool owns = !producer && j < VD;
+  const int part = tid % P, jl = tid / P * CPL, j = col0 + jl;
+  const int owned = producer ? 0 : max(0, min(CPL, VD - j));
   const int r0 = row_start[b], r1 = row_start[b + 1];
   if (r1 <= r0) return;
   float* S = state + (long long)state_slot[b] * slot_floats + (long long)h * D * VD;
@@ -431,7 +442,7 @@ __global__ void __launch_bounds__(REC_THREADS + 32) recurrence_scan_staged_kerne
       else vb[c * REC_CHUNK + t] = 0.f;
     }
   };
-  float s[KPL];
+  float s[CPL][KPL];
   if (producer) {
 #pragma unroll
     for (int s0 = 0; s0 < STAGES - 1; ++s0) {
@@ -443,10 +454,12 @@ __global__ void __launch_bounds__(REC_THREADS + 32) recurrence_scan_staged_kerne
 #pragma unroll
     for (int m = 0; m < M; ++m)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int i = 4 * (part + P * m) + c;
-        s[4 * m + c] = (owns && i < D) ? S[(long long)i * VD + j] : 0.f;
-      }
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          const int i = 4 * (part + P * m) + e;
+          s[c][4 * m + e] = (c < owned && i < D) ? S[(long long)i * VD + j + c] : 0.f;
+        }
   }
   __syncthreads();
 
@@ -465,19 +478,21 @@ __global__ void __launch_bounds__(REC_THREADS + 32) recurrence_scan_staged_kerne
       float* yg = y + (long long)t0 * ldy + (long long)h * VD + j;
       int g = 0;
       for (; g + REC_GROUP <= nt; g += REC_GROUP)
-        rec_group<RULE, KPL, DP, true>(s, tok + g * tok_floats, vcol + g, yg + g * ldy, ldy, REC_GROUP, part, owns, c_h);
-      if (g < nt) rec_group<RULE, KPL, DP, false>(s, tok + g * tok_floats, vcol + g, yg + g * ldy, ldy, nt - g, part, owns, c_h);
+        rec_group<RULE, KPL, CPL, DP, true>(s, tok + g * tok_floats, vcol + g, yg + g * ldy, ldy, REC_GROUP, part, owned, c_h);
+      if (g < nt) rec_group<RULE, KPL, CPL, DP, false>(s, tok + g * tok_floats, vcol + g, yg + g * ldy, ldy, nt - g, part, owned, c_h);
     }
     __syncthreads();
   }
-  if (write_state && owns) {
+  if (write_state) {
 #pragma unroll
     for (int m = 0; m < M; ++m)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int i = 4 * (part + P * m) + c;
-        if (i < D) S[(long long)i * VD + j] = s[4 * m + c];
-      }
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          const int i = 4 * (part + P * m) + e;
+          if (c < owned && i < D) S[(long long)i * VD + j + c] = s[c][4 * m + e];
+        }
   }
 }
 
@@ -606,12 +621,13 @@ extern "C" long long tl_recurrence_scratch_floats(long long rows, int H, int D, 
 
 // positions [rows], inv_freq [rot / 2], rot, k_scale: with a fixed decay, see the top of the file (rot 0: nothing turns).
 // scratch: null runs the one-kernel form (steps of a few rows a request); else tl_recurrence_scratch_floats(rows, ...) floats.
+// longest: the most rows a request brings (0: not known).
 extern "C" int tl_recurrence_scan(const float* proj, long long ld, int q_col, int k_col, int v_col, int a_col, const float* wl,
                                   long long ld_w, const float* w0, const float* a_bias, const float* head_decay, float rate,
                                   float key_eps, int silu_inputs, float* state, long long slot_floats, const int* state_slot,
                                   const int* row_start, int requests, float* y, int H, int D, int VD, int write_state,
                                   float* scratch, long long rows, int sm_count, int rule, float q_scale, const int* positions,
-                                  const float* inv_freq, int rot, float k_scale, cudaStream_t stream) {
+                                  const float* inv_freq, int rot, float k_scale, int longest, cudaStream_t stream) {
   if (requests == 0) return 0;
   TL_REQUIRE(rule >= RULE_FIXED && rule <= RULE_GATED, "recurrence_scan: rule %d is not one of 0..2", rule);
   const bool delta = rule == RULE_DELTA, fixed = rule == RULE_FIXED;
@@ -627,14 +643,20 @@ extern "C" int tl_recurrence_scan(const float* proj, long long ld, int q_col, in
   while (16 * P < D) P <<= 1;
   const int P16 = P;
   const int sms = sm_count > 0 ? sm_count : 148;
-  // the staged form gives a column to four times as many lanes (4 keys a lane) until the GPU has two warps a scheduler
-  int kpl = 16;
-  if (scratch && 4 * P <= 32 && (long long)requests * H * VD * P < 256LL * sms) {
+  // The staged form's lanes take two columns each, or where those would be few warps, one column by four times as many lanes (4 keys a
+  // lane): the delta rule over 1100 rows, 16 heads of 128 x 128 376 us with 4 keys, 402 with two columns, 32 heads 712 and 457. Its
+  // blocks are sized for requests as long as the longest (`longest` rows), because the others are over before it.
+  const long long alike = scratch ? (longest > 0 ? max(1LL, min((long long)requests, (rows + longest / 2) / longest)) : requests) : 0;
+  int kpl = 16, cpl = 1;
+  if (scratch && (long long)requests * H * VD * P >= 128LL * sms) {
+    cpl = 2;
+  } else if (scratch && 4 * P <= 32) {
     kpl = 4;
     P *= 4;
   }
   int threads, cols_per_block;
-  recurrence_block(requests, H, VD, P, scratch ? (3LL * sms) / 4 : 2LL * sms, &threads, &cols_per_block);
+  recurrence_block(scratch ? (int)alike : requests, H, ceil_div(VD, cpl), P, scratch ? (3LL * sms) / 4 : 2LL * sms, &threads, &cols_per_block);
+  cols_per_block *= cpl;
   const int tiles = ceil_div(VD, cols_per_block);
   TL_REQUIRE(tiles <= 65535, "recurrence_scan: %d tiles of value columns exceed the grid limit", tiles);
   dim3 grid(requests, H, tiles);
@@ -660,19 +682,20 @@ extern "C" int tl_recurrence_scan(const float* proj, long long ld, int q_col, in
     const float* vsrc = fixed ? vact : proj;
     const long long ld_v = fixed ? (long long)H * VD : ld;
     const int vc = fixed ? 0 : v_col;
-#define TL_RSS(DELTA_, KPL_, DP_)                                                                                               \
+#define TL_RSS(DELTA_, KPL_, CPL_, DP_)                                                                                               \
   do {                                                                                                                          \
     if (smem > 48 * 1024)                                                                                                       \
-      cudaFuncSetAttribute(recurrence_scan_staged_kernel<DELTA_, KPL_, DP_>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+      cudaFuncSetAttribute(recurrence_scan_staged_kernel<DELTA_, KPL_, CPL_, DP_>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
                            96 * 1024);                                                                                          \
-    recurrence_scan_staged_kernel<DELTA_, KPL_, DP_><<<grid, threads + 32, smem, stream>>>(                                     \
+    recurrence_scan_staged_kernel<DELTA_, KPL_, CPL_, DP_><<<grid, threads + 32, smem, stream>>>(                                     \
         prep, vsrc, ld_v, vc, head_decay, state, slot_floats, state_slot, row_start, y, rows, H, D, VD, cols_per_block, TC,           \
         write_state);                                                                                                           \
   } while (0)
 #define TL_RSS_D(DELTA_, DP_)                   \
   do {                                          \
-    if (kpl == 16) TL_RSS(DELTA_, 16, DP_);     \
-    else if (DP_ <= 128) TL_RSS(DELTA_, 4, (DP_ <= 128 ? DP_ : 128)); \
+    if (cpl == 2) TL_RSS(DELTA_, 16, 2, DP_);   \
+    else if (kpl == 16) TL_RSS(DELTA_, 16, 1, DP_); \
+    else if (DP_ <= 128) TL_RSS(DELTA_, 4, 1, (DP_ <= 128 ? DP_ : 128)); \
   } while (0)
 #define TL_RSS_ALL(DELTA_)                      \
   do {                                          \

@@ -151,7 +151,7 @@ _SIGNATURES = {
     "tl_recurrence_scan": [c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                            c_float, c_float, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
                            c_int, c_int, c_void_p, c_longlong, c_int, c_int, c_float, c_void_p, c_void_p, c_int, c_float,
-                           c_void_p],
+                           c_int, c_void_p],
     "tl_recurrence_scratch_floats": [c_longlong, c_int, c_int, c_int, c_int],
     "tl_gated_delta_scan": [c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_float,
                             c_float, c_void_p, c_int, c_int, c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_int,
@@ -962,7 +962,7 @@ def recurrence_scan(proj, q_col: int, k_col: int, v_col: int, state, state_slot,
                                     float(key_eps), int(silu_inputs), ptr(state), state[0].numel(), ptr(state_slot),
                                     ptr(row_start), int(requests), ptr(y), heads, key_dim, value_dim, int(write_state),
                                     ptr(scratch), rows, sm_count(), rule, float(q_scale), ptr(turn[0]) if turn else None,
-                                    ptr(turn[1]) if turn else None, int(turn[2]) if turn else 0, float(k_scale), stream()),
+                                    ptr(turn[1]) if turn else None, int(turn[2]) if turn else 0, float(k_scale), int(max_rows), stream()),
           "recurrence_scan",
           kernels=2 if scratch is not None else 1)
     return y

@@ -490,3 +490,50 @@ def test_models_drawn_at_random(seed, dtype):
     schedule = [[("a", 40), ("b", 1)], [("a", 2), ("b", 17), ("c", 2)], [("a", 1), ("b", 1)], [("a", 31), ("b", 11)],
                 [("a", 23)]]
     held_to_the_plain_model(engine, cfg, W, toks, schedule, dtype, f"random {seed}", slack=2.0 if dtype == "bfloat16" else 1.0)
+
+
+@pytest.mark.parametrize("rule,H,D,VD,lengths", [
+    ("fixed", 3, 64, 32, [200, 64, 1, 65]), ("fixed", 2, 132, 68, [193, 10]), ("fixed", 16, 128, 65, [70, 9, 33]),
+    ("delta", 16, 128, 65, [70, 9, 33]), ("delta", 8, 200, 67, [40, 17, 16]), ("delta", 2, 64, 33, [37]),
+    ("gated", 16, 128, 65, [70, 9, 33]), ("gated", 8, 200, 67, [40, 17, 16])])
+def test_recurrences_of_portions_in_every_form_of_their_scan(rule, H, D, VD, lengths):
+    """The scan over prepared tokens with two columns a lane (an odd number of columns among them) and with four keys a lane, unequal
+    requests side by side with states from before, against the plain recurrence in 64 bits: sums of up to max(lengths) + D terms in 32 bits, 2e-5 of the result."""
+    from tandemllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(D * 7 + VD)
+    R, n = sum(lengths), len(lengths)
+    proj = torch.randn(R, H * (3 * D + VD), generator=g) * 0.3
+    q_col, k_col, a_col, v_col = 0, H * D, 2 * H * D, 3 * H * D
+    state = torch.randn(n + 1, H, D, VD, generator=g)
+    decay = 1 - torch.rand(H, generator=g) * 0.1
+    w, w0, bias = torch.randn(R, H * D, generator=g), torch.randn(H * D, generator=g), torch.randn(H * D, generator=g)
+    starts = [0]
+    for x in lengths:
+        starts.append(starts[-1] + x)
+    slots = list(range(n, 0, -1))
+    kw = {"fixed": dict(head_decay=decay.to(DEV)), "delta": dict(a_col=a_col, w=w.to(DEV), w0=w0.to(DEV), a_bias=bias.to(DEV), rate=0.6, key_eps=1e-6),
+          "gated": dict(w=w.to(DEV), w0=w0.to(DEV), rate=0.0625)}[rule]
+    dev, y = state.clone().to(DEV), torch.full((R, H * VD), float("nan"), device=DEV)
+    ids = torch.tensor(slots, dtype=torch.int32, device=DEV), torch.tensor(starts, dtype=torch.int32, device=DEV)
+    ops.recurrence_scan(proj.to(DEV), q_col, k_col, v_col, dev, *ids, n, y, H, D, VD, max_rows=max(lengths), q_scale=0.5, **kw)
+    p = proj.double()
+    q, k, a = (p[:, c:c + H * D].view(R, H, D) for c in (q_col, k_col, a_col))
+    q, v = 0.5 * q, p[:, v_col:].view(R, H, VD)
+    logits = (w + w0).double().view(R, H, D)
+    d = {"fixed": decay.double()[None, :, None].expand(R, H, D), "delta": torch.exp(-0.6 * torch.sigmoid(logits)),
+         "gated": torch.sigmoid(logits) ** 0.0625}[rule]
+    u = k * torch.rsqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    au = torch.sigmoid(a + bias.double().view(H, D)) * u
+    for b, slot in enumerate(slots):
+        S, want = state[slot].double(), []
+        for t in range(starts[b], starts[b + 1]):
+            new = d[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            if rule == "delta":
+                new = new - au[t][:, :, None] * (u[t][:, :, None] * S).sum(1)[:, None, :]
+            S = new
+            want.append((S * q[t][:, :, None]).sum(1).flatten())
+        want = torch.stack(want)
+        got = y[starts[b]:starts[b + 1]].cpu().double()
+        assert float((got - want).norm() / want.norm()) < 2e-5, (b, float((got - want).norm() / want.norm()))
+        assert float((dev[slot].cpu().double() - S).norm() / S.norm()) < 2e-5, b
+    assert torch.equal(dev[0].cpu(), state[0])
