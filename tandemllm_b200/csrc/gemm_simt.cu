@@ -39,6 +39,8 @@ struct GemmParams {
   float ga0, ga1;          // the constants of a gate form that has some
   int swiglu;              // a gate activation TL_ACT_* (1: SiLU): W holds 2 N rows per group; C = act(A W[0:N]^T) * (A W[N:2N]^T)
                            // (negative: N rows per group, C = act(A W^T) with the code's activation; grouped products only)
+  int k_run;                  // > 0: k is cut into runs of so many elements, a CTA each; run z's result begins part_stride floats behind
+  long long part_stride;      // the one before it
 };
 
 template <typename TIn, typename TOut, bool SWIGLU>
@@ -259,6 +261,9 @@ __global__ void __launch_bounds__(256) gemm_tall_narrow_kernel(GemmParams p) {
 // 600 pairs 448 -> 403 us. A thread's rows lie 4 and its columns 8 apart, so a quarter of a warp reads one row or eight neighbouring ones:
 // with 36 floats a row the eight meet no bank twice.
 //
+// A product of few tiles (150 rows against 2048 outputs are 160 CTAs on 148 SMs: twelve SMs with two, and the others wait for them)
+// whose sums may stay in parts is cut into runs of k, a CTA each (`simt_runs` in kernels/ops.py).
+//
 // An output is the sum of eight chains, a warp's even and odd k in ascending order over the quads q = warp (mod 4), added in
 // order: which k a chain has depends on k alone, whatever the tile's height, so a row still does not depend on the others, and
 // eight short chains lose less than one long one.
@@ -350,7 +355,12 @@ __global__ void __launch_bounds__(FWARPS * 32, F32Tile<BM_, FN>::CTAS) gemm_f32_
       }
     }
   }
-  const int steps = (p.K + FK - 1) / FK;
+  // (a run of k: its sums go to a result of their own, the bias into the first's)
+  const int k0 = p.k_run ? (int)blockIdx.z * p.k_run : 0, k_len = p.k_run ? min(p.k_run, p.K - k0) : p.K;
+#pragma unroll
+  for (int i = 0; i < T::LOADS; ++i)
+    if (ok[i]) src[i] += k0;
+  const int steps = (k_len + FK - 1) / FK;
   const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)((lrow * FPITCH + lk) * 4);
   auto load = [&](int step) {
     if (step < steps) {
@@ -359,7 +369,7 @@ __global__ void __launch_bounds__(FWARPS * 32, F32Tile<BM_, FN>::CTAS) gemm_f32_
 #pragma unroll
       for (int i = 0; i < T::LOADS; ++i)
         if (lrow + T::ROWS_A_PASS * i < BM_ + FN) {
-          const bool in = ok[i] && k < p.K;          // (K is a multiple of 4)
+          const bool in = ok[i] && k < k_len;        // (K and a run are multiples of 4)
           cp16(at + (uint32_t)(T::ROWS_A_PASS * i * FPITCH * 4), in ? src[i] + k : W, in);
         }
     }
@@ -440,7 +450,8 @@ __global__ void __launch_bounds__(FWARPS * 32, F32Tile<BM_, FN>::CTAS) gemm_f32_
     for (int w = 0; w < FWARPS; ++w) v += red[((w * TM_ + m) * TN_ + j) * 32 + lane];
     return v;
   };
-  float* C = (float*)p.C;
+  float* C = (float*)p.C + (long long)blockIdx.z * p.part_stride;
+  const float* bias = blockIdx.z == 0 ? p.bias : nullptr;
   // a warp stores every fourth of the TM x TN blocks of outputs (gated: the gate's column blocks are the first four)
   constexpr int BLOCKS = GATED ? 4 : TN_;
 #pragma unroll
@@ -455,7 +466,7 @@ __global__ void __launch_bounds__(FWARPS * 32, F32Tile<BM_, FN>::CTAS) gemm_f32_
       const float rw = pair_weight(p.pair_weight, p.weight_index, r);
       C[r * p.ldc + n] = gated(rw * v, rw * u, p.swiglu, p.ga0, p.ga1);
     } else {
-      const float x = v + (p.bias ? p.bias[n] : 0.f);
+      const float x = v + (bias ? bias[n] : 0.f);
       C[r * p.ldc + n] = p.swiglu < 0 ? gate_activation(x, -p.swiglu) : x;
     }
   }
@@ -473,7 +484,7 @@ static int launch_f32(const GemmParams& p, int max_tiles, cudaStream_t stream) {
     configured = true;
   }
   const unsigned y = p.tile_group ? (unsigned)(max_tiles * sub) : (unsigned)ceil_div(p.M, BM_);
-  kernel<<<dim3(ceil_div(p.N, GATED ? FN / 2 : FN), y), FWARPS * 32, SMEM, stream>>>(p, sub);
+  kernel<<<dim3(ceil_div(p.N, GATED ? FN / 2 : FN), y, p.k_run ? ceil_div(p.K, p.k_run) : 1), FWARPS * 32, SMEM, stream>>>(p, sub);
   return 0;
 }
 
@@ -553,6 +564,22 @@ extern "C" int tl_gemm_simt(const void* A, long long lda, const void* W, long lo
   else if (in_dtype == TL_BF16 && out_dtype == TL_FP32) e = launch<bf16, float>(p, 0, stream);
   else TL_REQUIRE(false, "gemm: input dtype %d with output dtype %d is not implemented", in_dtype, out_dtype);
   if (e) return e;
+  TL_LAUNCH_CHECK();
+  return 0;
+}
+
+// The 32-bit product in runs of `run` k-elements (a multiple of 32; 32-bit operands whose rows are whole 16-byte pieces, more than 64
+// outputs): C receives every run's sums, [runs][M][ldc], for the caller to add in order; the bias is in the first.
+extern "C" int tl_gemm_simt_runs(const float* A, long long lda, const float* W, long long ldw, const float* bias, float* C, long long ldc,
+                                 int M, int N, int K, int run, cudaStream_t stream) {
+  if (M == 0 || N == 0) return 0;
+  TL_REQUIRE(M > 0 && N > 0 && K > 0 && run > 0 && run % 32 == 0, "gemm in runs: M %d N %d K %d, runs of %d", M, N, K, run);
+  TL_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm in runs: strides lda %lld ldw %lld ldc %lld for M %d N %d K %d", lda, ldw, ldc, M, N, K);
+  GemmParams p = {};
+  p.A = A; p.W = W; p.bias = bias; p.C = C; p.lda = lda; p.ldw = ldw; p.ldc = ldc;
+  p.M = M; p.N = N; p.K = K; p.a_div = 1; p.k_run = run; p.part_stride = (long long)M * ldc;
+  TL_REQUIRE(f32_pieces(p, 0) && M > FEW_ROWS && ceil_div(K, run) <= 65535, "gemm in runs: %d rows of %d against %d outputs", M, K, N);
+  if (int e = launch_f32_any(p, 0, stream)) return e;
   TL_LAUNCH_CHECK();
   return 0;
 }

@@ -423,6 +423,20 @@ def test_gemm_simt_in_16_byte_pieces(M, N, K):
         assert torch.equal(few, out[M - 9:])
 
 
+@pytest.mark.parametrize("M,N,K,run", [(9, 65, 36, 32), (16, 130, 1024, 256), (33, 257, 1028, 288), (150, 2048, 2048, 512), (65, 192, 260, 96)])
+def test_gemm_simt_in_runs_of_k(M, N, K, run):
+    """The 32-bit product cut into runs of k: the parts add up to the product (bias included) as closely as whole chains must, the last
+    run shorter than the others; rows that are no whole pieces are left to the caller."""
+    o = ops()
+    x, w, b = rnd(M, K, seed=6), rnd(N, K, seed=7), rnd(N, seed=8)
+    got = o.gemm_simt_runs(x.to(DEV), w.to(DEV), b.to(DEV), run)
+    assert got.parts == -(-K // run)
+    out = got.materialize().cpu()
+    want, size = x.double() @ w.double().T + b.double(), x.abs().double() @ w.abs().double().T + b.abs().double()
+    assert ((out.double() - want).abs() <= (run / 4 + 8 + got.parts) * 2.0 ** -24 * size).all()
+    assert o.gemm_simt_runs(x[:, 1:].to(DEV), w[:, 1:].to(DEV), None, run) is None
+
+
 @pytest.mark.parametrize("N,K", [(65, 4), (128, 256), (513, 36), (128, 1024), (513, 1024), (70, 2052), (1030, 260), (1030, 520), (2048, 2048)])
 def test_gemm_simt_in_16_byte_pieces_row_by_row(N, K):
     """More than 64 outputs: up to a k of 256 a row has the same bits alone, among up to eight rows (tiles of their own) and in the tiles
