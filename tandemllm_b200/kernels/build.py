@@ -17,10 +17,14 @@ from __future__ import annotations
 import ctypes
 import fcntl
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
+import platform
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -164,5 +168,64 @@ def load(name: str) -> ctypes.CDLL:
         return _loaded[name]
 
 
+_KINDS = {ctypes.c_void_p: "p", ctypes.c_longlong: "l", ctypes.c_int: "i", ctypes.c_uint: "i", ctypes.c_float: "f"}
+
+
+def build_fastcall() -> str | None:
+    """The extension that calls launchers (csrc/fastcall.c), compiled if its file is not there yet; None where there is no C compiler or
+    no Python header, or on another platform than the one it is written for (launches then go through ctypes, as they are)."""
+    include = sysconfig.get_paths()["include"]
+    cc = shutil.which("cc") or shutil.which("gcc")
+    source = os.path.join(CSRC, "fastcall.c")
+    with open(source, "rb") as fh:
+        tag = hashlib.sha1(fh.read() + sys.version.encode()).hexdigest()[:12]
+    folder = build_dir()
+    out = os.path.join(folder, f"fastcall-{tag}.so")
+    if os.path.isfile(out):
+        return out
+    if platform.machine() != "x86_64" or not sys.platform.startswith("linux") or not cc or not os.path.isfile(os.path.join(include, "Python.h")):
+        return None
+    tmp = out + f".tmp{os.getpid()}"
+    r = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, source, "-o", tmp], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise ExtensionError(f"{cc} failed on fastcall.c:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, out)
+    return out
+
+
+def _launcher_type():
+    global _launcher
+    if _launcher is None:
+        path = build_fastcall()
+        if path is None:
+            _launcher = False
+        else:
+            loader = importlib.machinery.ExtensionFileLoader("fastcall", path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("fastcall", path, loader=loader))
+            loader.exec_module(module)
+            _launcher = module.Launcher
+    return _launcher
+
+
+_launcher = None
+
+
+class Launchers:
+    """A library whose functions with declared parameters that return an int are called through csrc/fastcall.c; everything else is
+    the library's own."""
+
+    def __init__(self, library: ctypes.CDLL, names):
+        self._library = library
+        launcher = _launcher_type()
+        for name in names if launcher else ():
+            fn = getattr(library, name)
+            kinds = "".join(_KINDS.get(t, "?") for t in fn.argtypes or ("?",))
+            if "?" not in kinds and kinds.count("f") <= 8 and len(kinds) - kinds.count("f") <= 48 and fn.restype is ctypes.c_int:
+                setattr(self, name, launcher(ctypes.cast(fn, ctypes.c_void_p).value, kinds, fn))
+
+    def __getattr__(self, name):
+        return getattr(self._library, name)
+
+
 def build_all() -> list[str]:
-    return [build(name) for name in LIBRARIES]
+    return [build(name) for name in LIBRARIES] + [path for path in (build_fastcall(),) if path]

@@ -12,7 +12,7 @@ from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
 
-from .build import load
+from .build import Launchers, load
 
 FP32, BF16 = 0, 1
 TL_BAD_ARGUMENT = 100001
@@ -200,7 +200,7 @@ def core():
         lib.tl_cuda_error_string.restype = ctypes.c_char_p
         lib.tl_ssm_scan_chunk.argtypes, lib.tl_ssm_scan_chunk.restype = [c_int, c_int, c_longlong, c_void_p], c_int
         lib.tl_cuda_error_string.argtypes = [c_int]
-        _core = lib
+        _core = Launchers(lib, _SIGNATURES)
     return _core
 
 

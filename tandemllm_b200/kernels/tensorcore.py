@@ -34,7 +34,7 @@ import torch
 
 from ..settings import SETTINGS
 from . import ops
-from .build import load
+from .build import Launchers, load
 
 SKINNY_TOKENS = 32              # up to this many token rows ...
 SKINNY_K = 2048                 # ... of at most this many elements (one round of loads a warp) ...
@@ -146,7 +146,7 @@ def lib():
         l.tl_gemm_skinny_conv.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
                                           c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
         l.tl_gemm_skinny_conv.restype = c_int
-        _lib = l
+        _lib = Launchers(l, [name for name, fn in vars(l).items() if name.startswith("tl_") and fn.argtypes])
     return _lib
 
 
