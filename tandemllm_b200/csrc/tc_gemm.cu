@@ -115,7 +115,11 @@ __device__ __forceinline__ float plain_result(float v, int act) { return act < 0
 // DEEP: the swapped plain product where its CTAs are at most one an SM and have more k-blocks than the three stages that let three
 // CTAs share an SM: as many as fit (64 rows against 14336 x 2048, 112 CTAs 21.0 -> 18.7 us; 37 rows against 6144 x 2048, 48 CTAs
 // 16.7 -> 14.6 us).
-template <int BN, bool SWAP, bool SWIGLU, bool DEEP = false>
+// FOUR: the swapped plain product of up to 16 rows with more CTAs than three an SM hold: three stages each, so that four share an SM
+// with as many bytes on their way (65536 outputs of 2048 are 512 CTAs: 444 and a second round of 68 at three an SM; a step of 8 rows at
+// 8192 tokens 890 -> 868 us with it, of 64 rows, whose experts' down products are as many CTAs, 1374 -> 1346).
+constexpr int USUAL = 0, DEEP = 1, FOUR = 2;
+template <int BN, bool SWAP, bool SWIGLU, int FORM = USUAL>
 struct Smem {
   static constexpr int A_BYTES = TILE_M * TILE_K * 2;                  // the M-side tile
   static constexpr int B_BYTES = BN * TILE_K * 2;                      // the N-side tile
@@ -128,7 +132,7 @@ struct Smem {
   // expert tiles (a few hundred CTAs) into one wave.
   // The swapped plain product keeps to a third: its CTAs stream little each (a decode step's down projections are a
   // few hundred CTAs of half a MB), and three an SM put them into one wave.
-  static constexpr int BUDGET = DEEP ? 200 * 1024 : SWAP ? (SWIGLU ? 110 * 1024 : 74 * 1024) : 100 * 1024;
+  static constexpr int BUDGET = FORM == DEEP ? 200 * 1024 : FORM == FOUR ? 55 * 1024 : SWAP ? (SWIGLU ? 110 * 1024 : 74 * 1024) : 100 * 1024;
   static constexpr int FIT = BUDGET / STAGE_BYTES;
   static constexpr int STAGES = FIT > 8 ? 8 : (FIT < 2 ? 2 : FIT);
   static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
@@ -137,10 +141,10 @@ struct Smem {
                                    : TMEM_COLS_RAW <= 256 ? 256 : 512;
 };
 
-template <int BN, bool SWAP, bool SWIGLU, typename TOut, bool DEEP = false>
+template <int BN, bool SWAP, bool SWIGLU, typename TOut, int FORM = USUAL>
 __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW,
                                                       const __grid_constant__ CUtensorMap tmX, TcParams p) {
-  using S = Smem<BN, SWAP, SWIGLU, DEEP>;
+  using S = Smem<BN, SWAP, SWIGLU, FORM>;
   // Chained launches: the weights are written by no kernel, so a product without a tile map sets itself up and
   // requests its first weight tiles before it waits for the kernels in front of it; only the token rows, and
   // everything a grouped product reads through the tile map, have to wait.
@@ -669,10 +673,10 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const bf16* __restrict
 }
 
 // ------------------------------------------------------------------------------------------ host side
-template <int BN, bool SWAP, bool SWIGLU, typename TOut, bool DEEP>
+template <int BN, bool SWAP, bool SWIGLU, typename TOut, int FORM>
 static int launch_form(const CUtensorMap& tmW, const CUtensorMap& tmX, const TcParams& p, dim3 grid, cudaStream_t stream) {
-  using S = Smem<BN, SWAP, SWIGLU, DEEP>;
-  auto kernel = gemm_tc_kernel<BN, SWAP, SWIGLU, TOut, DEEP>;
+  using S = Smem<BN, SWAP, SWIGLU, FORM>;
+  auto kernel = gemm_tc_kernel<BN, SWAP, SWIGLU, TOut, FORM>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
@@ -686,9 +690,11 @@ template <int BN, bool SWAP, bool SWIGLU, typename TOut>
 static int launch_one(const CUtensorMap& tmW, const CUtensorMap& tmX, const TcParams& p, dim3 grid, cudaStream_t stream) {
   if constexpr (SWAP && !SWIGLU && BN <= 128) {
     if (!p.tile_group && (long long)grid.x * grid.y * grid.z <= sm_count() && p.k_blocks_per_split > Smem<BN, SWAP, SWIGLU>::STAGES)
-      return launch_form<BN, SWAP, SWIGLU, TOut, true>(tmW, tmX, p, grid, stream);
+      return launch_form<BN, SWAP, SWIGLU, TOut, DEEP>(tmW, tmX, p, grid, stream);
+    if constexpr (BN == 16)
+      if ((long long)grid.x * grid.y * grid.z > 3 * sm_count()) return launch_form<BN, SWAP, SWIGLU, TOut, FOUR>(tmW, tmX, p, grid, stream);
   }
-  return launch_form<BN, SWAP, SWIGLU, TOut, false>(tmW, tmX, p, grid, stream);
+  return launch_form<BN, SWAP, SWIGLU, TOut, USUAL>(tmW, tmX, p, grid, stream);
 }
 
 template <bool SWIGLU, typename TOut>
