@@ -2,6 +2,10 @@
 // launcher, instantiated in rows.cu (one residual, several residual streams) and in rows_pair.cu (two branches, two norms).
 #pragma once
 
+#include <map>
+#include <mutex>
+#include <tuple>
+
 #include "route.cuh"
 
 namespace tl {
@@ -614,6 +618,37 @@ static cudaError_t launch_clustered(void (*kernel)(KernelArgs...), dim3 grid, di
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KernelArgs>(args)...);
 }
 
+// How many clusters of `cluster` CTAs of a kernel the GPU holds at a time (asked once a kernel, size and device): fewer than its SMs
+// divided by the cluster, because a cluster lies within one of the GPU's partitions of SMs.
+static int active_clusters(const void* kernel, int threads, size_t smem, int cluster) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, size_t, int, int>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> g(mu);
+  auto [it, fresh] = known.try_emplace({kernel, threads, smem, cluster, dev}, 0);
+  if (fresh) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(cluster * (sm_count() / cluster)));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    it->second = n;
+  }
+  return it->second;
+}
+
 // Checks `p` and launches the norm of `p.out_rows` rows in the form its rows, its width and its router want.
 template <int MODE>
 static int launch_add_rmsnorm(NormParams p, int dtype, cudaStream_t stream) {
@@ -647,18 +682,21 @@ static int launch_add_rmsnorm(NormParams p, int dtype, cudaStream_t stream) {
   // experts of 2048: a third of the kernel's time). A cluster of CTAs a row shares them out; every CTA of the cluster
   // puts the row together for itself, which a step of many rows no longer pays (measured: 2.415 -> 2.374 ms a step at
   // batch 8, 773 -> 797 tok/s at batch 1, but 13.2 k -> 12.5 k tok/s at batch 64). Above 16 rows the cluster shrinks so
-  // that all CTAs still run at once, one an SM (37 rows x 4, 74 rows x 2: 8119 -> 8246 tok/s at batch 32, 13.2 k -> 13.5 k
-  // at batch 64).
+  // that all CTAs still run at once, one an SM (4 up to 37 rows, 2 up to 74: 8119 -> 8246 tok/s at batch 32, 13.2 k -> 13.5 k
+  // at batch 64) and every cluster has its place: 37 clusters of four are 148 SMs, but the GPU does not hold them all at a time,
+  // and 35 to 37 rows took two rounds (with a launch, 14.4 us, 12.3 in clusters of two), 16 rows in clusters of eight as well (14.4 and 10.3).
   p.split = 1;
   // (not over several streams: the row's first CTA would rewrite them while the others still read them)
   if (rows_per_block == 1 && router_w && E >= 16 && (hidden & 3) == 0 && MODE != NORM_STREAMS)
     p.split = out_rows <= ROUTER_SPLIT_ROWS ? ROUTER_SPLIT : (out_rows <= 37 ? 4 : (out_rows <= 74 ? 2 : 1));
-  const dim3 grid(ceil_div(out_rows, rows_per_block) * p.split);
   const int per = !router_w ? 0 : (E <= 32 ? 1 : (E <= 64 ? 2 : (E <= 128 ? 4 : MAX_EXPERTS / 32)));
 #define TL_NORM1(T_, PER_, ONE_)                                                                                        \
   do {                                                                                                                  \
     if (smem > 48 * 1024)                                                                                               \
       cudaFuncSetAttribute(add_rmsnorm_kernel<T_, PER_, ONE_, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    while (p.split > 1 && out_rows > active_clusters((const void*)add_rmsnorm_kernel<T_, PER_, ONE_, MODE>, threads, smem, p.split)) \
+      p.split /= 2;                                                                                                     \
+    const dim3 grid(ceil_div(out_rows, rows_per_block) * p.split);                                                      \
     if (p.split > 1)                                                                                                    \
       return (int)launch_clustered(add_rmsnorm_kernel<T_, PER_, ONE_, MODE>, grid, dim3(threads), smem, stream, p.split, p); \
     return (int)launch_chained(add_rmsnorm_kernel<T_, PER_, ONE_, MODE>, grid, dim3(threads), smem, stream, p);         \
