@@ -34,13 +34,12 @@ struct ChunkMatrix {
   const float* v;            // v + r * ld_v + h * P
   long long ld_qk, group_qk, ld_v;
   int heads_per_group;       // heads that share q and k
-  const float* decay;        // a_t of (row, head) at r * H + h, or null: `head_decay[h]`
-  const float* head_decay;
-  const float* weight;       // w_t of (row, head), or null: 1
-  const float* skip;         // o_t += skip[h] v_t, or null
+  const float* decay;        // a_t of (row, head) at r * H + h
+  const float* weight;       // w_t of (row, head)
+  const float* skip;         // o_t += skip[h] v_t
   const int* row_start;
   float* scores;             // [places][groups][64][64]
-  float* chunk_state;        // [places][H][N P]
+  float* chunk_state;        // [places][H][P][N]
   float* chunk_decay;        // [places][H]
   float* y;                  // [rows, H P]
   int H, P, N, max_chunks;
@@ -71,26 +70,36 @@ __device__ __forceinline__ void cm_stage(float* dst, int pitch, int width, const
 }
 
 // The 64 x 64 products of a block: two halves of 64 threads take a half of the sum each, a thread rows ti + 8 i of `a` against rows tj
-// + 8 j of `b` (i, j < 8), so that 16 reads of 16 bytes feed 256 multiply-adds.
+// + 8 j of `b` (i, j < 8), so that 16 reads of 16 bytes feed 256 multiply-adds. Sixteen products are added up in a row before their
+// sum joins the others (CM_RUN pieces): chains as long as the keys lost half as much again as the scan token by token does.
 struct CmPlace {
   int half, ti, tj;
   __device__ __forceinline__ CmPlace() : half(threadIdx.x >> 6), ti((threadIdx.x & 63) >> 3), tj(threadIdx.x & 7) {}
 };
-__device__ __forceinline__ void cm_dots(float (&acc)[8][8], const CmPlace& at, const float* a, const float* b, int pitch, int pieces) {
+constexpr int CM_RUN = 4;
+__device__ __forceinline__ void cm_dots(float (&sum)[8][8], const CmPlace& at, const float* a, const float* b, int pitch, int pieces) {
   const int mid = (pieces + 1) >> 1, e1 = at.half ? pieces : mid;
   a += at.ti * pitch;
   b += at.tj * pitch;
 #pragma unroll 1
-  for (int e = at.half ? mid : 0; e < e1; ++e) {
-    float4 x[8];
+  for (int e0 = at.half ? mid : 0; e0 < e1; e0 += CM_RUN) {
+    float acc[8][8] = {};
+#pragma unroll 1
+    for (int e = e0; e < min(e0 + CM_RUN, e1); ++e) {
+      float4 x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(a + i * 8 * pitch + 4 * e);
+      for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(a + i * 8 * pitch + 4 * e);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float4 z = *reinterpret_cast<const float4*>(b + j * 8 * pitch + 4 * e);
+      for (int j = 0; j < 8; ++j) {
+        const float4 z = *reinterpret_cast<const float4*>(b + j * 8 * pitch + 4 * e);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i][j] = dot4(x[i], z, acc[i][j]);
+        for (int i = 0; i < 8; ++i) acc[i][j] = dot4(x[i], z, acc[i][j]);
+      }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[i][j] += acc[i][j];
   }
 }
 // Adds the halves: the first half's threads keep rows i < 4, the second's i >= 4, in r[i & 3][j]. `buf`: 4096 floats nobody reads.
@@ -140,9 +149,7 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_score_kernel(ChunkMatrix m) 
 }
 
 // grid (H, chunks, tiles of 64 columns x tiles of 128 keys): what the chunk adds to a zero state. A thread holds 8 columns and 8 keys.
-// VALUES_LAST: a state is [N][P] (else [P][N]).
-template <bool VALUES_LAST>
-__global__ void __launch_bounds__(CM_THREADS) chunk_end_kernel(ChunkMatrix m) {
+static __global__ void __launch_bounds__(CM_THREADS) chunk_end_kernel(ChunkMatrix m) {
   extern __shared__ __align__(16) float sm[];
   float* sk = sm;                                    // [64][128]
   float* sv = sk + CM_TOKENS * CM_KEYS;              // [64][64], weighed
@@ -154,7 +161,7 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_end_kernel(ChunkMatrix m) {
   const int p0 = (blockIdx.z / key_tiles) * CM_COLS, n0 = (blockIdx.z % key_tiles) * CM_KEYS;
   const int keys = min(CM_KEYS, m.N - n0), cols = min(CM_COLS, m.P - p0);
   const int group = h / m.heads_per_group;
-  if (tid < CM_TOKENS) sa[tid] = tid < n ? (m.decay ? m.decay[(long long)(first + tid) * m.H + h] : m.head_decay[h]) : 1.f;
+  if (tid < CM_TOKENS) sa[tid] = tid < n ? m.decay[(long long)(first + tid) * m.H + h] : 1.f;
   cm_stage(sk, CM_KEYS, CM_KEYS, m.k + (long long)first * m.ld_qk + (long long)group * m.group_qk + n0, m.ld_qk, n, keys);
   cm_stage(sv, CM_COLS, CM_COLS, m.v + (long long)first * m.ld_v + (long long)h * m.P + p0, m.ld_v, n, cols);
   __syncthreads();
@@ -163,7 +170,7 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_end_kernel(ChunkMatrix m) {
     left = 1.f;
     for (int u = tid + 1; u < n; ++u) left *= sa[u];
     if (tid == 0 && blockIdx.z == 0) m.chunk_decay[(long long)b * m.H + h] = left * sa[0];
-    if (tid < n && m.weight) left *= m.weight[(long long)(first + tid) * m.H + h];
+    if (tid < n) left *= m.weight[(long long)(first + tid) * m.H + h];
   }
   __syncthreads();
   if (tid < CM_TOKENS) sa[tid] = tid < n ? left : 0.f;
@@ -195,22 +202,9 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_end_kernel(ChunkMatrix m) {
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int key = n0 + 4 * tn + 64 * j;
-      if (!VALUES_LAST && p < m.P && key < m.N)
+      if (p < m.P && key < m.N)
         *reinterpret_cast<float4*>(out + (long long)p * m.N + key) =
             make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
-    }
-  }
-  if (VALUES_LAST) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int key = n0 + 4 * tn + 64 * (j >> 2) + (j & 3);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int p = p0 + 4 * tp + 32 * i;
-        if (p < m.P && key < m.N)
-          *reinterpret_cast<float4*>(out + (long long)key * m.P + p) =
-              make_float4(acc[4 * i][j], acc[4 * i + 1][j], acc[4 * i + 2][j], acc[4 * i + 3][j]);
-      }
     }
   }
 }
@@ -218,8 +212,7 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_end_kernel(ChunkMatrix m) {
 constexpr int CM_OUT_FLOATS = 2 * CM_TOKENS * (CM_KEYS + 4) + CM_TOKENS * (CM_TOKENS + 4) + CM_COLS * (CM_TOKENS + 4) + 2 * CM_TOKENS;
 
 // grid (H, chunks, tiles of 64 columns): the chunk's outputs from the state it starts from.
-template <bool VALUES_LAST>
-__global__ void __launch_bounds__(CM_THREADS) chunk_out_kernel(ChunkMatrix m) {
+static __global__ void __launch_bounds__(CM_THREADS) chunk_out_kernel(ChunkMatrix m) {
   extern __shared__ __align__(16) float sm[];
   constexpr int PITCH = CM_KEYS + 4, SHORT = CM_TOKENS + 4;
   float* sq = sm;                                    // [64 tokens][128]
@@ -232,7 +225,7 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_out_kernel(ChunkMatrix m) {
   int b, first, n;
   if (!cm_chunk(m, blockIdx.y, b, first, n)) return;
   const int cols = min(CM_COLS, m.P - p0), group = h / m.heads_per_group, groups = m.H / m.heads_per_group;
-  if (tid < CM_TOKENS) sa[tid] = tid < n ? (m.decay ? m.decay[(long long)(first + tid) * m.H + h] : m.head_decay[h]) : 1.f;
+  if (tid < CM_TOKENS) sa[tid] = tid < n ? m.decay[(long long)(first + tid) * m.H + h] : 1.f;
   cm_stage(sg, SHORT, CM_TOKENS, m.scores + ((long long)b * groups + group) * (CM_TOKENS * CM_TOKENS), CM_TOKENS, n, CM_TOKENS);
   const float* v = m.v + (long long)first * m.ld_v + (long long)h * m.P + p0;
   bool wild = false;
@@ -245,7 +238,7 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_out_kernel(ChunkMatrix m) {
   wild = __syncthreads_or(wild);     // then a token's zero share of a later one would not be nothing
   if (tid < CM_TOKENS) {             // a thread a token s: its share of every later token's output
     const int s = tid;
-    float d = m.weight && s < n ? m.weight[(long long)(first + s) * m.H + h] : 1.f;
+    float d = s < n ? m.weight[(long long)(first + s) * m.H + h] : 1.f;
     for (int t = 0; t < n; ++t) {
       if (t > s) d *= sa[t];
       sg[t * SHORT + s] = t >= s ? d * sg[t * SHORT + s] : 0.f;
@@ -263,39 +256,35 @@ __global__ void __launch_bounds__(CM_THREADS) chunk_out_kernel(ChunkMatrix m) {
     const int keys = min(CM_KEYS, m.N - n0);
     if (n0) __syncthreads();
     cm_stage(sq, PITCH, CM_KEYS, m.q + (long long)first * m.ld_qk + (long long)group * m.group_qk + n0, m.ld_qk, n, keys);
-    if (!VALUES_LAST) {
-      cm_stage(ss, PITCH, CM_KEYS, state + (long long)p0 * m.N + n0, m.N, cols, keys);
-    } else {
-      for (int i = tid; i < CM_KEYS * CM_COLS; i += CM_THREADS) {
-        const int key = i / CM_COLS, c = i - key * CM_COLS;
-        ss[c * PITCH + key] = (key < keys && c < cols) ? state[(long long)(n0 + key) * m.P + p0 + c] : 0.f;
-      }
-    }
+    cm_stage(ss, PITCH, CM_KEYS, state + (long long)p0 * m.N + n0, m.N, cols, keys);
     __syncthreads();
     cm_dots(acc, place, sq, ss, PITCH, keys >> 2);
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float d = sd[place.ti + 8 * i];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] *= d;
-  }
-  if (!wild) cm_dots(acc, place, sg, sv, SHORT, ceil_div(n, 4));
+  // The two sums are joined one after the other and meet in one multiply-add: every addition less at the size of the result is felt in
+  // its last bits.
+  float r0[4][8], r[4][8];
   __syncthreads();                   // sq has been read
-  float r[4][8];
+  cm_join(acc, r0, place, sq);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  if (!wild) cm_dots(acc, place, sg, sv, SHORT, ceil_div(n, 4));
+  __syncthreads();                   // the first sums have been read
   cm_join(acc, r, place, sq);
-  const float skip = m.skip ? m.skip[h] : 0.f;
+  const float skip = m.skip[h];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int t = place.ti + 8 * (i + 4 * place.half);
     if (t >= n) continue;
+    const float d = sd[t];
     float* out = m.y + (long long)(first + t) * ((long long)m.H * m.P) + (long long)h * m.P + p0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int c = place.tj + 8 * j;
       if (wild)
         for (int s = 0; s <= t; ++s) r[i][j] = fmaf(sg[t * SHORT + s], sv[c * SHORT + s], r[i][j]);
-      if (c < cols) out[c] = m.skip ? fmaf(skip, sv[c * SHORT + t], r[i][j]) : r[i][j];
+      if (c < cols) out[c] = fmaf(skip, sv[c * SHORT + t], fmaf(d, r0[i][j], r[i][j]));
     }
   }
 }
@@ -359,21 +348,21 @@ static int chunk_walk(float* chunk_state, const float* chunk_decay, float* state
 }
 
 // The three kernels' sizes and launches; `walk` puts the states the chunks start from in the place of what they add.
-template <bool VALUES_LAST, typename Walk>
+template <typename Walk>
 static int chunk_matrix_run(const ChunkMatrix& m, int chunks, Walk walk, cudaStream_t stream) {
   const int groups = m.H / m.heads_per_group, key_tiles = ceil_div(m.N, CM_KEYS), col_tiles = ceil_div(m.P, CM_COLS);
   constexpr int score_bytes = 2 * CM_TOKENS * (CM_KEYS + 4) * 4;
   constexpr int end_bytes = (CM_TOKENS * (CM_KEYS + CM_COLS) + CM_TOKENS) * 4, out_bytes = CM_OUT_FLOATS * 4;
   cudaError_t e = cudaFuncSetAttribute(chunk_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, score_bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_end_kernel<VALUES_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, end_bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<VALUES_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_end_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, end_bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, out_bytes);
   if (e != cudaSuccess) return (int)e;
   chunk_score_kernel<<<dim3(groups, chunks), CM_THREADS, score_bytes, stream>>>(m);
   TL_LAUNCH_CHECK();
-  chunk_end_kernel<VALUES_LAST><<<dim3(m.H, chunks, col_tiles * key_tiles), CM_THREADS, end_bytes, stream>>>(m);
+  chunk_end_kernel<<<dim3(m.H, chunks, col_tiles * key_tiles), CM_THREADS, end_bytes, stream>>>(m);
   TL_LAUNCH_CHECK();
   if (int err = walk()) return err;
-  chunk_out_kernel<VALUES_LAST><<<dim3(m.H, chunks, col_tiles), CM_THREADS, out_bytes, stream>>>(m);
+  chunk_out_kernel<<<dim3(m.H, chunks, col_tiles), CM_THREADS, out_bytes, stream>>>(m);
   TL_LAUNCH_CHECK();
   return 0;
 }

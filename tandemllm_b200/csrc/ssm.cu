@@ -365,7 +365,7 @@ extern "C" int tl_ssm_scan(const float* xbc, long long ld_xbc, const float* dt, 
     const long long count = (long long)rows * H;
     ssm_rates_kernel<<<(unsigned)ceil_div64(count, 256), 256, 0, stream>>>(dt, ld_dt, dt_bias, a_log, step, decay, count, H);
     TL_LAUNCH_CHECK();
-    return chunk_matrix_run<false>(m, requests * max_chunks, [&]() {
+    return chunk_matrix_run(m, requests * max_chunks, [&]() {
       return chunk_walk(m.chunk_state, m.chunk_decay, state, state_stride, state_slot, row_start, requests, H, P * N, CM_TOKENS,
                         max_chunks, write_state, 1, stream);
     }, stream);
