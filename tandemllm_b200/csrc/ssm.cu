@@ -11,8 +11,14 @@
 // A step's rows are several requests' portions side by side (one row for a decoding request): every kernel takes the
 // row's request from req_of_row / row_start and never looks at another request's rows. The recurrence is sequential in
 // a request and parallel over requests, heads and the state's columns, with a fixed order of additions, so a position's
-// result does not depend on how the sequence was cut into steps or on what else is in the batch.
-#include "chunk_matrix.cuh"
+// result does not depend on how the sequence was cut into steps or on what else is in the batch, except where a step's
+// longest portion is cut into chunks: a state that crosses a chunk's end (and a request's last one) is then decay * start
+// + the chunk's own, rounded once, and not once a token.
+//
+// The chunks' outputs as products (scores C B^T of a chunk times its values, and the state's share) were measured and taken back: a turn of
+// two requests of 300 and 700 rows took 10773 us instead of 11559, but a scan's error against 64 bits grew by a tenth to a sixth
+// (6.0e-8 -> 6.6e-8), and the other order of additions is enough to change a router's choice for a row some layers on.
+#include "common.cuh"
 
 namespace tl {
 
@@ -86,7 +92,7 @@ struct ScanParams {
   int write_state;
   // Long portions are cut into chunks of `chunk_tokens` rows that run side by side (0: a request's rows one after the other):
   //   mode 1: every chunk runs from a zero state, writes no y, and leaves its last state and the product of its decays;
-  //   (chunk_walk then walks a request's chunks: each chunk's slot receives the state the chunk starts from,
+  //   (ssm_chunk_states_kernel then walks a request's chunks: each chunk's slot receives the state the chunk starts from,
   //   S <- decay_c S + last_c, and the request's slot the state after the last chunk)
   //   mode 2: every chunk runs from the state it starts from and writes its y.
   int mode, chunk_tokens, max_chunks;
@@ -94,7 +100,6 @@ struct ScanParams {
   float* chunk_decay;        // [requests * max_chunks, H]
 };
 
-constexpr int SSM_MATRIX_KEYS = 64; // a state's keys from which long portions take the matrix form (chunk_matrix.cuh)
 constexpr int SCAN_LANES = 8;       // lanes that share a column of the state: lane l holds n = l, l + 8, ...
 constexpr int SCAN_COLS = 16;       // columns (values of p) a block
 constexpr int SCAN_TOKENS = 16;     // tokens staged at a time
@@ -263,17 +268,27 @@ __global__ void __launch_bounds__(SCAN_COLS * SCAN_LANES) ssm_scan_kernel(ScanPa
   if (p.mode == 1 && blockIdx.x == 0 && threadIdx.x == 0) *chunk_decay = decay_product;
 }
 
-// dt and the decay of every row and head, [rows, H] each, for the matrix form
-__global__ void __launch_bounds__(256) ssm_rates_kernel(const float* __restrict__ dt, long long ld_dt, const float* __restrict__ dt_bias,
-                                                        const float* __restrict__ a_log, float* __restrict__ step,
-                                                        float* __restrict__ decay, long long count, int H) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const long long r = i / H;
-  const int h = (int)(i - r * H);
-  const float d = softplus_f(dt[r * ld_dt + h] + dt_bias[h]);
-  step[i] = d;
-  decay[i] = expf(-expf(a_log[h]) * d);
+// grid (ceil(H P N / 256), requests): a thread an entry of the state walks the request's chunks in order
+__global__ void __launch_bounds__(256) ssm_chunk_states_kernel(float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
+                                                               float* __restrict__ state, long long state_stride,
+                                                               const int* __restrict__ state_slot, const int* __restrict__ row_start,
+                                                               int H, int PN, int chunk_tokens, int max_chunks, int write_state) {
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int b = blockIdx.y;
+  const long long per = (long long)H * PN;
+  if (e >= per) return;
+  const int h = (int)(e / PN);
+  const int chunks = ceil_div(row_start[b + 1] - row_start[b], chunk_tokens);
+  if (chunks <= 0) return;
+  float* slot = state + (long long)state_slot[b] * state_stride + e;
+  float S = *slot;
+  for (int c = 0; c < chunks; ++c) {
+    float* at = chunk_state + ((long long)b * max_chunks + c) * per + e;
+    const float last = *at;
+    *at = S;
+    S = fmaf(chunk_decay[((long long)b * max_chunks + c) * H + h], S, last);
+  }
+  if (write_state) *slot = S;
 }
 
 // grid (groups, rows): out[r, part] = w * v / rms(v), v = y * silu(z)
@@ -331,7 +346,7 @@ extern "C" int tl_conv_state(const float* in, long long ld_in, float* state, lon
 extern "C" int tl_ssm_scan(const float* xbc, long long ld_xbc, const float* dt, long long ld_dt, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, long long state_stride,
                            const int* state_slot, const int* row_start, float* y, int requests, int H, int P, int N, int G,
-                           int write_state, int chunk_tokens, int max_chunks, float* chunk_scratch, int rows, cudaStream_t stream) {
+                           int write_state, int chunk_tokens, int max_chunks, float* chunk_scratch, cudaStream_t stream) {
   if (requests == 0) return 0;
   TL_REQUIRE(requests > 0 && requests <= 65535 && H > 0 && H <= 65535 && P > 0 && N > 0 && G > 0 && H % G == 0,
              "ssm scan: %d requests, %d heads in %d groups, columns %d, state %d", requests, H, G, P, N);
@@ -347,28 +362,6 @@ extern "C" int tl_ssm_scan(const float* xbc, long long ld_xbc, const float* dt, 
   if (chunked) {
     p.chunk_state = chunk_scratch;
     p.chunk_decay = chunk_scratch + (long long)requests * max_chunks * H * P * N;
-  }
-  if (chunked && chunk_tokens == CM_TOKENS && N >= SSM_MATRIX_KEYS) {
-    TL_REQUIRE(rows > 0 && rows <= requests * max_chunks * CM_TOKENS, "ssm scan: %d rows in %d chunks of 64", rows, requests * max_chunks);
-    const long long places = chunk_places(rows, requests);
-    ChunkMatrix m = {};
-    m.chunk_state = chunk_scratch;
-    m.scores = m.chunk_state + places * H * P * N;
-    float* step = m.scores + places * G * CM_TOKENS * CM_TOKENS;
-    float* decay = step + (long long)rows * H;
-    m.chunk_decay = decay + (long long)rows * H;
-    m.v = xbc; m.k = xbc + (long long)H * P; m.q = m.k + (long long)G * N;
-    m.ld_v = ld_xbc; m.ld_qk = ld_xbc; m.group_qk = N; m.heads_per_group = H / G;
-    m.decay = decay; m.weight = step; m.skip = d_skip; m.row_start = row_start; m.y = y;
-    m.H = H; m.P = P; m.N = N; m.max_chunks = max_chunks;
-    TL_REQUIRE(chunk_matrix_fits(m), "ssm scan: chunks of 64 want 16-byte pieces (columns %d, state %d, row stride %lld)", P, N, ld_xbc);
-    const long long count = (long long)rows * H;
-    ssm_rates_kernel<<<(unsigned)ceil_div64(count, 256), 256, 0, stream>>>(dt, ld_dt, dt_bias, a_log, step, decay, count, H);
-    TL_LAUNCH_CHECK();
-    return chunk_matrix_run(m, requests * max_chunks, [&]() {
-      return chunk_walk(m.chunk_state, m.chunk_decay, state, state_stride, state_slot, row_start, requests, H, P * N, CM_TOKENS,
-                        max_chunks, write_state, 1, stream);
-    }, stream);
   }
   const dim3 grid(ceil_div(P, SCAN_COLS), H, chunked ? requests * max_chunks : requests), block(SCAN_COLS * SCAN_LANES);
   const size_t smem = 2 * (size_t)(2 * SCAN_TOKENS * N + SCAN_TOKENS * SCAN_COLS + 3 * SCAN_TOKENS) * sizeof(float);
@@ -399,9 +392,9 @@ extern "C" int tl_ssm_scan(const float* xbc, long long ld_xbc, const float* dt, 
   p.mode = 1;
   TL_SCAN_ANY();
   TL_LAUNCH_CHECK();
-  if (int e = chunk_walk(p.chunk_state, p.chunk_decay, state, state_stride, state_slot, row_start, requests, H, P * N, chunk_tokens,
-                         max_chunks, write_state, 0, stream))
-    return e;
+  ssm_chunk_states_kernel<<<dim3((unsigned)ceil_div64((long long)H * P * N, 256), requests), 256, 0, stream>>>(
+      p.chunk_state, p.chunk_decay, state, state_stride, state_slot, row_start, H, P * N, chunk_tokens, max_chunks, write_state);
+  TL_LAUNCH_CHECK();
   p.mode = 2;
   TL_SCAN_ANY();
 #undef TL_SCAN_ANY
@@ -410,19 +403,9 @@ extern "C" int tl_ssm_scan(const float* xbc, long long ld_xbc, const float* dt, 
   return 0;
 }
 
-// Floats of scratch a chunked scan needs: the chunks' states and decays; in the matrix form (64 tokens a chunk) for the chunks there
-// are, with every row's step and decay and the chunks' scores.
-extern "C" long long tl_ssm_scan_scratch(int requests, int max_chunks, int H, int P, int N, int G, int chunk_tokens, int rows) {
-  const long long state = (long long)H * P * N + H;
-  const long long scan = (long long)requests * max_chunks * state;
-  if (chunk_tokens != CM_TOKENS || N < SSM_MATRIX_KEYS) return scan;
-  return chunk_places(rows, requests) * (state + (long long)G * CM_TOKENS * CM_TOKENS) + 2LL * rows * H;
-}
-
-// Rows a chunk of long portions has: 64 where the states have keys enough for the matrix form and everything lies in 16-byte pieces,
-// else 128.
-extern "C" int tl_ssm_scan_chunk(int P, int N, long long ld_xbc, const float* xbc) {
-  return N >= SSM_MATRIX_KEYS && N % 4 == 0 && P % 4 == 0 && ld_xbc % 4 == 0 && ((uintptr_t)xbc & 15) == 0 ? CM_TOKENS : 2 * CM_TOKENS;
+// Floats of scratch a chunked scan needs.
+extern "C" long long tl_ssm_scan_scratch(int requests, int max_chunks, int H, int P, int N) {
+  return (long long)requests * max_chunks * ((long long)H * P * N + H);
 }
 
 extern "C" int tl_gated_group_norm(const float* y, const float* z, long long ld_z, const float* w, float eps, void* out,

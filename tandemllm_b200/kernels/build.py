@@ -45,7 +45,7 @@ LIBRARIES: dict[str, list[str]] = {
     "tensorcore": ["tc_gemm.cu", "tc_gemm_pair.cu", "attention_mma.cu", "attention_tc.cu", "attention_headmix_mma.cu",
                    "attention_latent_mma.cu", "attention_flex_mma.cu", "head_linear_mma.cu", "gemm_skinny_mma.cu"],
 }
-HEADERS = ["common.cuh", "route.cuh", "add_rmsnorm.cuh", "recurrence.cuh", "chunk_matrix.cuh", "attention_noalloc.h", "tma.cuh"]
+HEADERS = ["common.cuh", "route.cuh", "add_rmsnorm.cuh", "recurrence.cuh", "attention_noalloc.h", "tma.cuh"]
 
 _loaded: dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()

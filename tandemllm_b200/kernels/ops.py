@@ -132,7 +132,7 @@ _SIGNATURES = {
                            c_longlong, c_int, c_int, c_int, c_int, c_void_p],
     "tl_conv_state": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "tl_ssm_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
-                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
+                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "tl_gated_group_norm": [c_void_p, c_void_p, c_longlong, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "tl_latent_prepare": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_float, c_void_p, c_int, c_void_p, c_void_p,
                           c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
@@ -194,11 +194,10 @@ def core():
         lib.tl_headmix_scratch_floats.restype = c_longlong
         lib.tl_recurrence_scratch_floats.restype = c_longlong
         lib.tl_write_scan_scratch_floats.restype = c_longlong
-        lib.tl_ssm_scan_scratch.argtypes = [c_int] * 8
+        lib.tl_ssm_scan_scratch.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.tl_ssm_scan_scratch.restype = c_longlong
         lib.tl_last_error.restype = ctypes.c_char_p
         lib.tl_cuda_error_string.restype = ctypes.c_char_p
-        lib.tl_ssm_scan_chunk.argtypes, lib.tl_ssm_scan_chunk.restype = [c_int, c_int, c_longlong, c_void_p], c_int
         lib.tl_cuda_error_string.argtypes = [c_int]
         _core = Launchers(lib, _SIGNATURES)
     return _core
@@ -644,27 +643,23 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias, a_log, d_skip, state:
     """The selective state-space recurrence of csrc/ssm.cu over each request's rows. `xbc` float32 [rows, H P + 2 G N];
     `dt` a float32 view [rows, H] of the raw step sizes; a slot's recurrent state [H, P, N] begins `state_offset` floats
     into its row of `state`; `y` float32 [rows, H P]. With `max_rows_per_request` (the step's longest portion) of
-    SCAN_CHUNKED_FROM rows or more and a `runtime` to keep the scratch, portions are cut into chunks of SCAN_CHUNK rows (64 where
-    the states have keys enough for the matrix form, csrc/chunk_matrix.cuh): every chunk's own contribution from a zero state, the
-    states the chunks start from, then every chunk's outputs."""
+    SCAN_CHUNKED_FROM rows or more and a `runtime` to keep the scratch, portions are cut into chunks of SCAN_CHUNK rows:
+    every chunk's own contribution from a zero state, the states the chunks start from, then every chunk's outputs."""
     _need(xbc, torch.float32, "xbc"); _need(y, torch.float32, "y"); _need(state, torch.float32, "state")
     if dt.dtype != torch.float32 or dt.stride(-1) != 1:
         raise KernelError("ssm scan: float32 step sizes with unit stride")
     chunk = chunks = 0
     scratch = None
     if runtime is not None and max_rows_per_request >= SCAN_CHUNKED_FROM:
-        chunk = core().tl_ssm_scan_chunk(cols, n_state, xbc.stride(0), ptr(xbc))
-        chunks = -(-max_rows_per_request // chunk)
-        if requests * chunks > 65535 and chunk < SCAN_CHUNK:
-            chunk, chunks = SCAN_CHUNK, -(-max_rows_per_request // SCAN_CHUNK)
+        chunk, chunks = SCAN_CHUNK, -(-max_rows_per_request // SCAN_CHUNK)
         if requests * chunks > 65535:
             chunk = chunks = 0
         else:
-            scratch = runtime.scratch("ssm_chunks", core().tl_ssm_scan_scratch(requests, chunks, heads, cols, n_state, groups, chunk, xbc.shape[0]))
+            scratch = runtime.scratch("ssm_chunks", core().tl_ssm_scan_scratch(requests, chunks, heads, cols, n_state))
     check(core().tl_ssm_scan(ptr(xbc), xbc.stride(0), ptr(dt), dt.stride(0), ptr(dt_bias), ptr(a_log), ptr(d_skip),
                              state.data_ptr() + 4 * state_offset, state.stride(0), ptr(state_slot), ptr(row_start), ptr(y),
-                             requests, heads, cols, n_state, groups, int(write_state), chunk, chunks, ptr(scratch), xbc.shape[0], stream()),
-          "ssm_scan", kernels=(5 if chunk < SCAN_CHUNK else 3) if chunks > 1 else 1)
+                             requests, heads, cols, n_state, groups, int(write_state), chunk, chunks, ptr(scratch), stream()),
+          "ssm_scan", kernels=3 if chunks > 1 else 1)
     return y
 
 
