@@ -657,6 +657,10 @@ extern "C" int tl_recurrence_scan(const float* proj, long long ld, int q_col, in
   int threads, cols_per_block;
   recurrence_block(scratch ? (int)alike : requests, H, ceil_div(VD, cpl), P, scratch ? (3LL * sms) / 4 : 2LL * sms, &threads, &cols_per_block);
   cols_per_block *= cpl;
+  if (cols_per_block > REC_THREADS) {      // (16 keys and fewer, two columns a lane: three stages of 512 columns' values are all of 96 KB)
+    cols_per_block = REC_THREADS;
+    threads = REC_THREADS / cpl * P;
+  }
   const int tiles = ceil_div(VD, cols_per_block);
   TL_REQUIRE(tiles <= 65535, "recurrence_scan: %d tiles of value columns exceed the grid limit", tiles);
   dim3 grid(requests, H, tiles);
@@ -679,6 +683,7 @@ extern "C" int tl_recurrence_scan(const float* proj, long long ld, int q_col, in
     auto bytes = [&](int tc) { return (size_t)REC_STAGES * (tc * narr * Dp + REC_CHUNK * cols_per_block) * sizeof(float); };
     while (TC > 1 && bytes(TC) > 96 * 1024) TC >>= 1;
     const size_t smem = bytes(TC);
+    TL_REQUIRE(smem <= 96 * 1024, "recurrence_scan: stages of %lld bytes for %d keys and %d columns", (long long)smem, D, cols_per_block);
     const float* vsrc = fixed ? vact : proj;
     const long long ld_v = fixed ? (long long)H * VD : ld;
     const int vc = fixed ? 0 : v_col;

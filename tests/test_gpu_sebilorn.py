@@ -495,7 +495,10 @@ def test_models_drawn_at_random(seed, dtype):
 @pytest.mark.parametrize("rule,H,D,VD,lengths", [
     ("fixed", 3, 64, 32, [200, 64, 1, 65]), ("fixed", 2, 132, 68, [193, 10]), ("fixed", 16, 128, 65, [70, 9, 33]),
     ("delta", 16, 128, 65, [70, 9, 33]), ("delta", 8, 200, 67, [40, 17, 16]), ("delta", 2, 64, 33, [37]),
-    ("gated", 16, 128, 65, [70, 9, 33]), ("gated", 8, 200, 67, [40, 17, 16])])
+    ("gated", 16, 128, 65, [70, 9, 33]), ("gated", 8, 200, 67, [40, 17, 16]),
+    # one lane a column: as many columns a block as shared memory holds
+    ("fixed", 112, 16, 512, [20]), ("fixed", 112, 8, 449, [17, 3]), ("delta", 112, 16, 512, [20]), ("delta", 112, 16, 449, [17, 3]),
+    ("gated", 112, 16, 512, [17, 3]), ("gated", 112, 8, 450, [20])])
 def test_recurrences_of_portions_in_every_form_of_their_scan(rule, H, D, VD, lengths):
     """The scan over prepared tokens with two columns a lane (an odd number of columns among them) and with four keys a lane, unequal
     requests side by side with states from before, against the plain recurrence in 64 bits: sums of up to max(lengths) + D terms in 32 bits, 2e-5 of the result."""
