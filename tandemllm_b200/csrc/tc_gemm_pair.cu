@@ -275,9 +275,10 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
     }
   };
 
+  int issued = 0, ahead = 0;      // producer: k-blocks it has gone through, k-blocks whose weights it asked for before that
   if (warp == 0 && lane == 0) {
     // ---- producer (each CTA for its own shared memory) ----
-    int it = 0, issued = 0, ahead = 0;
+    int it = 0;
     auto load_weights = [&](int i, int kx, int my_out, int group) {
       uint8_t* st = tiles + (i % S::STAGES) * S::STAGE_BYTES;
       const uint32_t bar = in_cta(&full[i % S::STAGES], 0);
@@ -504,6 +505,15 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*aborted && first && warp == 0 && lane == 0) {
+    // Weights asked for ahead (by both CTAs alike) at stages the producer did not come to: nobody has announced their bytes yet. Only
+    // here, where the MMA issuer has ended: it takes a stage whose barrier completes.
+    for (int i = issued; i < ahead; ++i)
+      if (i != p.skip_kb) {
+        mbar_expect_tx(&full[i], 2 * S::A_BYTES);
+        mbar_wait(&full[i], 0);
+      }
+  }
   cluster_sync();                                      // neither CTA leaves while the other may still signal it or read its tiles
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == 1) {
