@@ -188,7 +188,9 @@ template <> __device__ __forceinline__ void put<bf16>(bf16* p, float v) { *p = _
 // CLAMPED: the gated form with the clamped swish, an instantiation of its own: with the choice among the gates inside the 16
 // evaluations 1000 rows of six experts of 768 x 2048 took 125 us, 100 us so, and as one more branch of the other gates' kernel it
 // cost those 1.5 %.
-template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false>
+// EIGHTS: gate and up rows come as 2D boxes of eight, for weights that `gate_up_map` does not describe (as a branch of the usual form's
+// producer it cost a prompt of 2048 rows 3286 -> 3416 us).
+template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, bool EIGHTS = false>
 __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_SM>::CTAS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
                                                            const __grid_constant__ CUtensorMap tmX16,
                                                            const __grid_constant__ CUtensorMap tmX32,
@@ -282,7 +284,13 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
     auto load_weights = [&](int i, int kx, int my_out, int group) {
       uint8_t* st = tiles + (i % S::STAGES) * S::STAGE_BYTES;
       const uint32_t bar = in_cta(&full[i % S::STAGES], 0);
-      if (GATED) load_gate_up(st, &tmW, bar, kx, my_out >> 3, group);
+      if (GATED && !EIGHTS) load_gate_up(st, &tmW, bar, kx, my_out >> 3, group);
+      else if (EIGHTS)
+        for (int r = 0; r < S::OUTS; r += 8) {
+          const int y = (int)(group * p.rows_per_group) + my_out + r;
+          load_2d(st + 2 * r * TILE_K * 2, &tmW, bar, kx, y);
+          load_2d(st + (2 * r + 8) * TILE_K * 2, &tmW, bar, kx, y + p.N);
+        }
       else load_2d(st, &tmW, bar, kx, (int)(group * p.rows_per_group) + my_out);
     };
     if (weights_first) {
@@ -522,12 +530,12 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
 }
 
 // How many pairs of this kernel the GPU holds at a time (asked once a kernel); negative: a CUDA error code, negated.
-template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false>
+template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, bool EIGHTS = false>
 static int resident_pairs() {
   using S = Smem<GATED, PER_SM>;
   static int clusters = 0;
   if (clusters != 0) return clusters;
-  auto kernel = gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED>;
+  auto kernel = gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED, EIGHTS>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
   if (e != cudaSuccess) return -(int)e;
   // all of the SM's configurable memory as shared memory: two CTAs an SM need it
@@ -555,10 +563,10 @@ static int resident_pairs() {
   return clusters;
 }
 
-template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false>
+template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, bool EIGHTS = false>
 static int launch(const CUtensorMap& tmW, const CUtensorMap* tmX, const Params& p, long long work, cudaStream_t stream) {
   using S = Smem<GATED, PER_SM>;
-  const int clusters = resident_pairs<GATED, PER_SM, TOut, CLAMPED>();
+  const int clusters = resident_pairs<GATED, PER_SM, TOut, CLAMPED, EIGHTS>();
   if (clusters < 0) return -clusters;
   TL_REQUIRE(clusters >= 1, "pair product: no cluster of two CTAs with %d bytes of shared memory fits this GPU", S::TOTAL);
   cudaLaunchConfig_t cfg = {};
@@ -575,7 +583,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap* tmX, const Params& 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED>, tmW, tmX[0], tmX[1], tmX[2], tmX[3], p);
+  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED, EIGHTS>, tmW, tmX[0], tmX[1], tmX[2], tmX[3], p);
 }
 
 }  // namespace pair
@@ -629,13 +637,13 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   const int tokens = (gated && per_sm == 2) ? 128 : 256;
   TL_REQUIRE(!tile_group || plan_rows <= tokens, "pair product: a tile map with tiles of %d rows; at most %d", plan_rows, tokens);
   CUtensorMap tmW, tmX[4];
-  if (gated) {
-    const long long per_group = tile_group ? rows_per_group : 2 * (long long)N;
-    TL_REQUIRE(N % 8 == 0 && per_group >= 2 * (long long)N && w_rows >= per_group,
-               "pair product: %d gated outputs (a multiple of 8) need as many gate and up rows a group (%lld rows a group, %lld in all)", N,
-               per_group, w_rows);
+  // One box brings a tile's gate and up rows where the outputs are whole blocks of eight and the tensor whole groups; else eight rows a
+  // box, sixteen boxes a stage: box rows past the outputs belong to others and their products are not stored.
+  const long long per_group = tile_group ? rows_per_group : w_rows;
+  const bool by_eights = gated && !(N % 8 == 0 && per_group >= 2 * (long long)N && w_rows % per_group == 0);
+  if (gated && !by_eights) {
     if (int e = gate_up_map(W, w_rows, per_group, N, K, ldw, pair::ROWS, &tmW)) return e;
-  } else if (int e = tensor_map(W, w_rows, K, ldw, pair::ROWS, &tmW)) {
+  } else if (int e = tensor_map(W, w_rows, K, ldw, by_eights ? 8 : pair::ROWS, &tmW)) {
     return e;
   }
   const int boxes[4] = {16, 32, 64, 128};
@@ -654,6 +662,13 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   const long long work = (long long)ceil_div(N, gated ? pair::ROWS : 2 * pair::ROWS) * (tile_group ? max_tiles : ceil_div(M, tokens)) * splits;
 #define TL_PAIR(G_, P_) \
   (out_dtype == TL_BF16 ? pair::launch<G_, P_, bf16>(tmW, tmX, p, work, stream) : pair::launch<G_, P_, float>(tmW, tmX, p, work, stream))
+  if (by_eights) {
+    if (out_dtype == TL_BF16)
+      return per_sm == 2 ? pair::launch<true, 2, bf16, false, true>(tmW, tmX, p, work, stream)
+                         : pair::launch<true, 1, bf16, false, true>(tmW, tmX, p, work, stream);
+    return per_sm == 2 ? pair::launch<true, 2, float, false, true>(tmW, tmX, p, work, stream)
+                       : pair::launch<true, 1, float, false, true>(tmW, tmX, p, work, stream);
+  }
   if (gated == TL_ACT_CLAMPED_SWISH && out_dtype == TL_BF16)
     return per_sm == 2 ? pair::launch<true, 2, bf16, true>(tmW, tmX, p, work, stream)
                        : pair::launch<true, 1, bf16, true>(tmW, tmX, p, work, stream);

@@ -710,6 +710,45 @@ def test_pair_product_with_the_gated_epilogue(M, H, I, act):
     assert rel(out, plain_activation(act, g) * u) < 1e-2
 
 
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("M,H,I,per_sm", [(300, 136, 203, 1), (150, 64, 5, 1), (600, 520, 1, 2), (129, 72, 130, 2), (40, 64, 262, 1)])
+def test_gated_pair_product_of_outputs_that_are_no_blocks_of_eight(M, H, I, per_sm, bias):
+    """Gate and up rows that one box does not describe come eight rows a box; what lies behind the last output is not stored."""
+    impl, rt = tc()
+    x, w, b = rnd(M, H, seed=66), rnd(2 * I, H, seed=67, scale=0.2), torch.randn(2 * I) if bias else None
+    wide = torch.full((M, I + 3), float("nan"), dtype=torch.bfloat16, device=DEV)
+    impl.gemm_pair(x.to(DEV), w.to(DEV), None if b is None else b.to(DEV), wide[:, :I], gated=1, n_out=I, per_sm=per_sm)
+    torch.cuda.synchronize()
+    assert int(rt.status) == 0
+    full = x.float() @ w.float().T + (b if bias else 0.0)
+    assert rel(wide[:, :I], torch.nn.functional.silu(full[:, :I]) * full[:, I:]) < 1e-2
+    assert bool(torch.isnan(wide[:, I:]).all())
+
+
+@pytest.mark.parametrize("tile", [256, 128])
+@pytest.mark.parametrize("I,gap,rest", [(67, 0, 0), (64, 5, 0), (64, 0, 24), (130, 2, 3)])
+def test_gated_pair_product_over_groups_one_box_does_not_describe(I, gap, rest, tile):
+    """Odd outputs a group, rows between the groups, rows behind the last group."""
+    from tandemllm_b200.kernels import ops
+    impl, rt = tc()
+    R, E, H = 200, 5, 136
+    ids = (torch.arange(R, dtype=torch.int32) ** 2 % E).view(R, 1)
+    plan = ops.MoePlan(R, E, tile, torch.device(DEV)).build(ids.to(DEV))
+    order = plan.sorted_pairs[:R].long().cpu()
+    x = rnd(R, H, seed=68)[order]
+    w = rnd(E * (2 * I + gap) + rest, H, seed=69, scale=0.1)
+    out = torch.full((R, I), float("nan"), dtype=torch.bfloat16, device=DEV)
+    impl.gemm_pair(x.to(DEV), w.to(DEV), None, out, rows_per_group=2 * I + gap, plan=plan, gated=1, n_out=I)
+    torch.cuda.synchronize()
+    assert int(rt.status) == 0
+    expert = ids.flatten()[order].long()
+    for e in range(E):
+        mine, at = expert == e, e * (2 * I + gap)
+        full = x[mine].float() @ w[at:at + 2 * I].float().T
+        if bool(mine.any()):
+            assert rel(out[mine.to(DEV)], torch.nn.functional.silu(full[:, :I]) * full[:, I:]) < 1e-2, e
+
+
 @pytest.mark.parametrize("tile", [256, 128, 48])
 @pytest.mark.parametrize("R,E,k,H,I", [(64, 8, 4, 128, 256), (700, 32, 4, 256, 264), (512, 5, 2, 136, 72), (1500, 3, 1, 64, 136)])
 def test_pair_product_over_a_routing_plan_of_ragged_tiles(R, E, k, H, I, tile):
