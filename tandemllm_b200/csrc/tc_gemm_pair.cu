@@ -20,10 +20,9 @@
 // memory holds two accumulators or more, so that the next tile's MMAs run under a tile's epilogue. The kernel is persistent: as many
 // clusters as fit the GPU walk over the tiles.
 //
-// The gated product once took 256 gate and 256 up rows a tile, whose two accumulators filled tensor memory: its MMAs waited for the
-// epilogue, and its tiles, twice as large, left the last round of clusters emptier (7168 outputs of 2048 rows are 3.03 rounds of such
-// tiles and 6.05 of these). A tile here loads 64 KB for what cost 48, which larger products feel (11776 outputs of 2048 rows 146 -> 150
-// us, 150 rows 32 -> 37 us) and all others gain more than: 7168 outputs of 2048, 150 rows 29 -> 24 us, 535 rows 53 -> 48, 2048 rows
+// The gated product's tiles of 256 outputs (256 gate and 256 up rows, whose two accumulators fill tensor memory: its MMAs wait for the
+// epilogue, and the last round of clusters is emptier) are kept where they load less for as many rounds (`wide_pays`). A tile of 128
+// outputs loads 64 KB for what cost 48, and gains elsewhere: 7168 outputs of 2048, 150 rows 29 -> 24 us, 535 rows 53 -> 48, 2048 rows
 // 115 -> 105; 32 experts of 1792 x 2048, 535 rows 99 -> 95 us, 1400 rows 114 -> 103; 64 experts of 768 x 2048, top 6, 1000 rows 118 -> 93
 // us, 2000 rows 156 -> 117.
 //
@@ -74,20 +73,28 @@ inline int& skip_kb_for_test() {
 // round leaves an SM with one CTA instead of two, that CTA loads at the SM's full rate. Gated: tiles of up to 128 token rows, one CTA an
 // SM with a ring of nine stages and four accumulators (two CTAs of four stages each took 107 us where this takes 91: 400 rows of
 // top-4 of 32 experts of 1792 x 2048).
-template <bool GATED, int PER_SM>
+//
+// FORM, gated products: EIGHTS brings gate and up rows as 2D boxes of eight, for weights that `gate_up_map` does not describe (as a
+// branch of the usual form's producer it cost a prompt of 2048 rows 3286 -> 3416 us). WIDE takes tiles of 256 outputs: a CTA brings 128
+// gate rows and the 128 up rows of the same outputs, whose two accumulators fill tensor memory, so the MMAs wait for the epilogue; a
+// stage has 48 KB for what two stages of the usual form need 64 for. Where that pays: `wide_pays`.
+enum Form { USUAL, EIGHTS, WIDE };
+template <bool GATED, int PER_SM, int FORM = USUAL>
 struct Smem {
   static constexpr int TOKENS = (GATED && PER_SM == 2) ? 128 : 256;  // token rows a tile at most
-  static constexpr int OUTS = GATED ? ROWS / 2 : ROWS;             // outputs a CTA
+  static constexpr int W_TILES = FORM == WIDE ? 2 : 1;             // boxes of weight rows a stage, each with an accumulator
+  static constexpr bool IN_TURN = GATED && FORM != WIDE;           // a box holds 8 gate rows and their 8 up rows in turn
+  static constexpr int OUTS = IN_TURN ? ROWS / 2 : ROWS;           // outputs a CTA
   static constexpr int CTAS = GATED ? 1 : PER_SM;                  // CTAs an SM
   static constexpr int TMEM_COLS = CTAS == 2 ? 256 : 512;
-  static constexpr int ACC_BUFS = TMEM_COLS / TOKENS;              // accumulators in tensor memory
+  static constexpr int ACC_BUFS = TMEM_COLS / (W_TILES * TOKENS);  // accumulators (sets of them) in tensor memory
   // Epilogue warps: one a quarter of the accumulator's lanes, or two that take every other block of 16 tokens
   static constexpr int EPI_WARPS = GATED && PER_SM == 1 ? 8 : 4;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int A_BYTES = ROWS * TILE_K * 2;                // one box of weights
   static constexpr int B_BYTES = (TOKENS / 2) * TILE_K * 2;        // this CTA's half of the token rows, at most
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = PER_SM == 2 ? (GATED ? 9 : 3) : 6;
+  static constexpr int STAGE_BYTES = W_TILES * A_BYTES + B_BYTES;
+  static constexpr int STAGES = PER_SM == 2 ? (GATED ? 9 : 3) : (FORM == WIDE ? 4 : 6);
   static constexpr int TURN_BYTES = EPI_WARPS * 16 * 32 * 4;       // the epilogue warps' blocks
   static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */ + TURN_BYTES;
   static_assert(CTAS * TOTAL <= 227 * 1024, "the CTAs of an SM share its shared memory");
@@ -185,18 +192,35 @@ template <typename TOut> __device__ __forceinline__ void put(TOut* p, float v);
 template <> __device__ __forceinline__ void put<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void put<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// g = act(g) * u. The choice of the activation stands outside the independent evaluations, and SiLU, the usual one, takes the fast
+// exponential and division (the result is rounded to bfloat16, far coarser than their error).
+template <bool CLAMPED, int COUNT>
+__device__ __forceinline__ void gate_all(float* g, const float* u, const Params& p) {
+  if constexpr (CLAMPED) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) g[j] = gated(g[j], u[j], TL_ACT_CLAMPED_SWISH, p.ga0, p.ga1);
+  } else if (p.act == TL_ACT_SILU) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) g[j] = __fdividef(g[j], 1.f + __expf(-g[j])) * u[j];
+  } else if (p.act == TL_ACT_GELU_TANH) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) g[j] = __fdividef(g[j], 1.f + __expf(-gelu_tanh_argument(g[j]))) * u[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) g[j] = gated(g[j], u[j], p.act, p.ga0, p.ga1);
+  }
+}
+
 // CLAMPED: the gated form with the clamped swish, an instantiation of its own: with the choice among the gates inside the 16
 // evaluations 1000 rows of six experts of 768 x 2048 took 125 us, 100 us so, and as one more branch of the other gates' kernel it
 // cost those 1.5 %.
-// EIGHTS: gate and up rows come as 2D boxes of eight, for weights that `gate_up_map` does not describe (as a branch of the usual form's
-// producer it cost a prompt of 2048 rows 3286 -> 3416 us).
-template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, bool EIGHTS = false>
-__global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_SM>::CTAS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
+template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, int FORM = USUAL>
+__global__ void __launch_bounds__(Smem<GATED, PER_SM, FORM>::THREADS, Smem<GATED, PER_SM, FORM>::CTAS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
                                                            const __grid_constant__ CUtensorMap tmX16,
                                                            const __grid_constant__ CUtensorMap tmX32,
                                                            const __grid_constant__ CUtensorMap tmX64,
                                                            const __grid_constant__ CUtensorMap tmX128, Params p) {
-  using S = Smem<GATED, PER_SM>;
+  using S = Smem<GATED, PER_SM, FORM>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(tiles + S::STAGES * S::STAGE_BYTES);   // used in the first CTA: both CTAs' bytes
@@ -284,14 +308,18 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
     auto load_weights = [&](int i, int kx, int my_out, int group) {
       uint8_t* st = tiles + (i % S::STAGES) * S::STAGE_BYTES;
       const uint32_t bar = in_cta(&full[i % S::STAGES], 0);
-      if (GATED && !EIGHTS) load_gate_up(st, &tmW, bar, kx, my_out >> 3, group);
-      else if (EIGHTS)
-        for (int r = 0; r < S::OUTS; r += 8) {
+      if (GATED && FORM == USUAL) {
+        load_gate_up(st, &tmW, bar, kx, my_out >> 3, group);
+      } else if (GATED) {
+        constexpr int box = FORM == EIGHTS ? 8 : ROWS;
+        for (int r = 0; r < S::OUTS; r += box) {
           const int y = (int)(group * p.rows_per_group) + my_out + r;
           load_2d(st + 2 * r * TILE_K * 2, &tmW, bar, kx, y);
-          load_2d(st + (2 * r + 8) * TILE_K * 2, &tmW, bar, kx, y + p.N);
+          load_2d(st + (2 * r + box) * TILE_K * 2, &tmW, bar, kx, y + p.N);
         }
-      else load_2d(st, &tmW, bar, kx, (int)(group * p.rows_per_group) + my_out);
+      } else {
+        load_2d(st, &tmW, bar, kx, (int)(group * p.rows_per_group) + my_out);
+      }
     };
     if (weights_first) {
       int tok0, tok_rows, group, n0, kb0, num_kb = 0;
@@ -311,7 +339,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
       // the smallest box that holds the half; rows of it behind the half are read and never used
       const int box = half <= 16 ? 16 : (half <= 32 ? 32 : (half <= 64 ? 64 : 128));      // (a half is at most TOKENS / 2 rows)
       const CUtensorMap* tmX = box == 16 ? &tmX16 : (box == 32 ? &tmX32 : (box == 64 ? &tmX64 : &tmX128));
-      const uint32_t cta_bytes = (uint32_t)(S::A_BYTES + box * TILE_K * 2);
+      const uint32_t cta_bytes = (uint32_t)(S::W_TILES * S::A_BYTES + box * TILE_K * 2);
       for (int kb = 0; kb < num_kb; ++kb, ++it) {
         const int s = it % S::STAGES;
         if (it >= S::STAGES && !mbar_wait(&empty[s], ((it / S::STAGES) - 1) & 1)) give_up();
@@ -320,7 +348,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
           if (first) mbar_expect_tx(&full[s], 2 * cta_bytes);
           const int kx = (kb0 + kb) * TILE_K;
           if (it >= ahead) load_weights(it, kx, my_out, group);
-          load_2d(tiles + s * S::STAGE_BYTES + S::A_BYTES, tmX, in_cta(&full[s], 0), kx, my_tok);
+          load_2d(tiles + s * S::STAGE_BYTES + S::W_TILES * S::A_BYTES, tmX, in_cta(&full[s], 0), kx, my_tok);
         }
         issued = it + 1;
       }
@@ -345,7 +373,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t acc = tmem_base + buf * S::TOKENS;
+      const uint32_t acc = tmem_base + buf * (S::W_TILES * S::TOKENS);
       for (int kb = 0; kb < num_kb; ++kb, ++it) {
         const int s = it % S::STAGES;
         if (!mbar_wait(&full[s], (it / S::STAGES) & 1)) {
@@ -353,11 +381,13 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(tiles + s * S::STAGE_BYTES), b0 = a0 + S::A_BYTES;
+        const uint32_t a0 = smem_u32(tiles + s * S::STAGE_BYTES), b0 = a0 + S::W_TILES * S::A_BYTES;
 #pragma unroll
         for (int k = 0; k < TILE_K / UMMA_K; ++k) {
           const uint32_t more = (kb > 0 || k > 0) ? 1u : 0u, koff = k * UMMA_K * 2;
-          mma2(acc, desc(a0 + koff), desc(b0 + koff), id, more);
+#pragma unroll
+          for (int t = 0; t < S::W_TILES; ++t)
+            mma2(acc + t * S::TOKENS, desc(a0 + t * S::A_BYTES + koff), desc(b0 + koff), id, more);
         }
         commit_both(&empty[s]);
       }
@@ -397,15 +427,16 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * S::TOKENS;
       const int j_tok = lane >> 1, c_half = (lane & 1) * 16;        // after the turn: token c0 + j_tok, 16 accumulator rows
-      // This thread's accumulator row stands for output `col`; gated: rows come as 8 gates, then the up rows of the same outputs.
+      constexpr int STORED = S::IN_TURN ? 8 : 16;                        // outputs a thread stores of a token
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (S::W_TILES * S::TOKENS);
+      // This thread's accumulator row stands for output `col`; gated, but in the WIDE form: 8 gates, then the up rows of the same outputs.
       const int cta0 = n0 + (int)rank * S::OUTS;
-      const int col = cta0 + (GATED ? (m_row >> 4) * 8 + (m_row & 7) : m_row);
-      const bool up_row = GATED && (m_row & 8);
+      const int col = cta0 + (S::IN_TURN ? (m_row >> 4) * 8 + (m_row & 7) : m_row);
+      const bool up_row = S::IN_TURN && (m_row & 8);
       const float b = (p.bias && col < p.N && kb0 == 0) ? p.bias[up_row ? p.N + col : col] : 0.f;
-      constexpr int STORED = GATED ? 8 : 16;                        // outputs a thread stores of a token
-      const int out0 = cta0 + (quad * 32 + c_half) / (GATED ? 2 : 1);
+      const float b_up = (FORM == WIDE && p.bias && col < p.N) ? p.bias[p.N + col] : 0.f;
+      const int out0 = cta0 + (quad * 32 + c_half) / (S::IN_TURN ? 2 : 1);
 #pragma unroll 1
       for (int c0 = 16 * turn_of; c0 < n_mma; c0 += STEP) {
         float v[16];
@@ -443,6 +474,13 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
             for (int j = 0; j < 16; ++j) v[j] = activation(v[j], p.unary, p.a0, p.a1);
           }
         }
+        if constexpr (FORM == WIDE) {
+          float u[16];
+          ld16(taddr + S::TOKENS + c0, u);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) u[j] += b_up;
+          gate_all<CLAMPED, 16>(v, u, p);
+        }
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 16; ++j) turn[j * 32 + ((lane + 4 * j) & 31)] = v[j];
@@ -453,10 +491,8 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
           const float4 q = *reinterpret_cast<const float4*>(turn + j_tok * 32 + ((c_half + 4 * i + 4 * j_tok) & 31));
           r[4 * i] = q.x; r[4 * i + 1] = q.y; r[4 * i + 2] = q.z; r[4 * i + 3] = q.w;
         }
-        if constexpr (GATED) {
-          // r: eight gates, then the eight up numbers of the same outputs. The choice of the activation stands outside the
-          // independent evaluations, and SiLU, the usual one, takes the fast exponential and division (the result is rounded
-          // to bfloat16, far coarser than their error).
+        if constexpr (S::IN_TURN) {
+          // r: eight gates, then the eight up numbers of the same outputs
           if (p.row_weight) {
             const int block = c0 / STEP;
             const float four = (block >> 1) == 0 ? rw[0] : ((block >> 1) == 1 ? rw[1] : ((block >> 1) == 2 ? rw[2] : rw[3]));
@@ -464,19 +500,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
 #pragma unroll
             for (int j = 0; j < 16; ++j) r[j] *= mine;
           }
-          if constexpr (CLAMPED) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) r[j] = gated(r[j], r[8 + j], TL_ACT_CLAMPED_SWISH, p.ga0, p.ga1);
-          } else if (p.act == TL_ACT_SILU) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) r[j] = __fdividef(r[j], 1.f + __expf(-r[j])) * r[8 + j];
-          } else if (p.act == TL_ACT_GELU_TANH) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) r[j] = __fdividef(r[j], 1.f + __expf(-gelu_tanh_argument(r[j]))) * r[8 + j];
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) r[j] = gated(r[j], r[8 + j], p.act, p.ga0, p.ga1);
-          }
+          gate_all<CLAMPED, 8>(r, r + 8, p);
         }
         const int t = c0 + j_tok;
         if (t < tok_rows && out0 < p.N) {
@@ -518,7 +542,7 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
     // here, where the MMA issuer has ended: it takes a stage whose barrier completes.
     for (int i = issued; i < ahead; ++i)
       if (i != p.skip_kb) {
-        mbar_expect_tx(&full[i], 2 * S::A_BYTES);
+        mbar_expect_tx(&full[i], 2 * S::W_TILES * S::A_BYTES);
         mbar_wait(&full[i], 0);
       }
   }
@@ -530,12 +554,12 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM>::THREADS, Smem<GATED, PER_
 }
 
 // How many pairs of this kernel the GPU holds at a time (asked once a kernel); negative: a CUDA error code, negated.
-template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, bool EIGHTS = false>
+template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, int FORM = USUAL>
 static int resident_pairs() {
-  using S = Smem<GATED, PER_SM>;
+  using S = Smem<GATED, PER_SM, FORM>;
   static int clusters = 0;
   if (clusters != 0) return clusters;
-  auto kernel = gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED, EIGHTS>;
+  auto kernel = gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED, FORM>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
   if (e != cudaSuccess) return -(int)e;
   // all of the SM's configurable memory as shared memory: two CTAs an SM need it
@@ -563,10 +587,10 @@ static int resident_pairs() {
   return clusters;
 }
 
-template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, bool EIGHTS = false>
+template <bool GATED, int PER_SM, typename TOut, bool CLAMPED = false, int FORM = USUAL>
 static int launch(const CUtensorMap& tmW, const CUtensorMap* tmX, const Params& p, long long work, cudaStream_t stream) {
-  using S = Smem<GATED, PER_SM>;
-  const int clusters = resident_pairs<GATED, PER_SM, TOut, CLAMPED, EIGHTS>();
+  using S = Smem<GATED, PER_SM, FORM>;
+  const int clusters = resident_pairs<GATED, PER_SM, TOut, CLAMPED, FORM>();
   if (clusters < 0) return -clusters;
   TL_REQUIRE(clusters >= 1, "pair product: no cluster of two CTAs with %d bytes of shared memory fits this GPU", S::TOTAL);
   cudaLaunchConfig_t cfg = {};
@@ -583,7 +607,19 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap* tmX, const Params& 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED, EIGHTS>, tmW, tmX[0], tmX[1], tmX[2], tmX[3], p);
+  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<GATED, PER_SM, TOut, CLAMPED, FORM>, tmW, tmX[0], tmX[1], tmX[2], tmX[3], p);
+}
+
+// Whether an ungrouped gated product of M rows, N outputs and a reduction of K takes the WIDE form's tiles of 256 outputs: where tiles
+// of 128 outputs need twice as many rounds of the GPU's pairs (with one round less the usual form is ahead: 2048 rows, 7168 outputs of
+// 2048 106 against 115 us). In one round always; in several, where no second accumulator hides the epilogue, from a K of 2048 on, and
+// below 4096 only where L2 holds the weights for the next 256 rows. Usual and wide, us: 150 rows, 11776 outputs of 2048 44 and 40; 300
+// rows, 7168 39 and 37; 2048 rows, 11776 156 and 150; 1024 rows, 9472 72 and 68; 2048 rows, 11776 of 4096 333 and 296; against it 2048
+// rows, 11776 of 1024 94 and 98; 1024 rows, 18944 of 2048 (155 MB) 138 and 143.
+static bool wide_pays(int M, int N, int K) {
+  const long long pairs = sm_count() / 2, tall = ceil_div(M, Smem<true, 1>::TOKENS);
+  const long long usual = (ceil_div(N, ROWS) * tall + pairs - 1) / pairs, wide = (ceil_div(N, 2 * ROWS) * tall + pairs - 1) / pairs;
+  return usual >= 2 * wide && (wide == 1 || K >= 4096 || (K >= 2048 && 4LL * N * K <= 120 << 20));
 }
 
 }  // namespace pair
@@ -640,8 +676,9 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   // One box brings a tile's gate and up rows where the outputs are whole blocks of eight and the tensor whole groups; else eight rows a
   // box, sixteen boxes a stage: box rows past the outputs belong to others and their products are not stored.
   const long long per_group = tile_group ? rows_per_group : w_rows;
-  const bool by_eights = gated && !(N % 8 == 0 && per_group >= 2 * (long long)N && w_rows % per_group == 0);
-  if (gated && !by_eights) {
+  const bool wide = gated && !tile_group && per_sm == 1 && pair::wide_pays(M, N, K);
+  const bool by_eights = gated && !wide && !(N % 8 == 0 && per_group >= 2 * (long long)N && w_rows % per_group == 0);
+  if (gated && !wide && !by_eights) {
     if (int e = gate_up_map(W, w_rows, per_group, N, K, ldw, pair::ROWS, &tmW)) return e;
   } else if (int e = tensor_map(W, w_rows, K, ldw, by_eights ? 8 : pair::ROWS, &tmW)) {
     return e;
@@ -659,15 +696,20 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   p.unary = unary; p.a0 = a0; p.a1 = a1;
   p.skip_kb = pair::skip_kb_for_test();
   p.splits = splits; p.kb_per_split = kb_per_split; p.part_stride = splits > 1 ? (long long)M * ldc : 0;
-  const long long work = (long long)ceil_div(N, gated ? pair::ROWS : 2 * pair::ROWS) * (tile_group ? max_tiles : ceil_div(M, tokens)) * splits;
+  const long long work = (long long)ceil_div(N, gated && !wide ? pair::ROWS : 2 * pair::ROWS) * (tile_group ? max_tiles : ceil_div(M, tokens)) * splits;
 #define TL_PAIR(G_, P_) \
   (out_dtype == TL_BF16 ? pair::launch<G_, P_, bf16>(tmW, tmX, p, work, stream) : pair::launch<G_, P_, float>(tmW, tmX, p, work, stream))
   if (by_eights) {
     if (out_dtype == TL_BF16)
-      return per_sm == 2 ? pair::launch<true, 2, bf16, false, true>(tmW, tmX, p, work, stream)
-                         : pair::launch<true, 1, bf16, false, true>(tmW, tmX, p, work, stream);
-    return per_sm == 2 ? pair::launch<true, 2, float, false, true>(tmW, tmX, p, work, stream)
-                       : pair::launch<true, 1, float, false, true>(tmW, tmX, p, work, stream);
+      return per_sm == 2 ? pair::launch<true, 2, bf16, false, pair::EIGHTS>(tmW, tmX, p, work, stream)
+                         : pair::launch<true, 1, bf16, false, pair::EIGHTS>(tmW, tmX, p, work, stream);
+    return per_sm == 2 ? pair::launch<true, 2, float, false, pair::EIGHTS>(tmW, tmX, p, work, stream)
+                       : pair::launch<true, 1, float, false, pair::EIGHTS>(tmW, tmX, p, work, stream);
+  }
+  if (wide) {
+    if (out_dtype == TL_FP32) return pair::launch<true, 1, float, false, pair::WIDE>(tmW, tmX, p, work, stream);
+    return gated == TL_ACT_CLAMPED_SWISH ? pair::launch<true, 1, bf16, true, pair::WIDE>(tmW, tmX, p, work, stream)
+                                         : pair::launch<true, 1, bf16, false, pair::WIDE>(tmW, tmX, p, work, stream);
   }
   if (gated == TL_ACT_CLAMPED_SWISH && out_dtype == TL_BF16)
     return per_sm == 2 ? pair::launch<true, 2, bf16, true>(tmW, tmX, p, work, stream)

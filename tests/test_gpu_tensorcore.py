@@ -710,6 +710,31 @@ def test_pair_product_with_the_gated_epilogue(M, H, I, act):
     assert rel(out, plain_activation(act, g) * u) < 1e-2
 
 
+@pytest.mark.parametrize("act,dtype", [("silu", "bfloat16"), ("relu2", "bfloat16"), ("silu", "float32"), ("clamped_swish", "bfloat16")])
+@pytest.mark.parametrize("M,H,I", [(40, 72, 9480), (300, 136, 4744), (300, 64, 9472), (257, 2048, 9472)])
+def test_gated_pair_product_in_tiles_of_128_and_of_256_outputs(M, H, I, act, dtype):
+    """Outputs for one round of the GPU's pairs in tiles of 256 and two in tiles of 128, and their neighbours that keep the smaller
+    tiles, the last tile ragged; the same rows have the same bits in both (40 rows of I outputs against the first 128 of them)."""
+    from tandemllm_b200.kernels import ops
+    impl, rt = tc()
+    code = ops.activation_code(act)
+    x, w, b = rnd(M, H, seed=66).to(DEV), rnd(2 * I, H, seed=67, scale=0.2).to(DEV), torch.randn(2 * I, device=DEV)
+    out = torch.full((M, I), float("nan"), dtype=getattr(torch, dtype), device=DEV)
+    impl.gemm_pair(x, w, b, out, gated=code, n_out=I)
+    torch.cuda.synchronize()
+    assert int(rt.status) == 0 and bool(torch.isfinite(out).all())
+    for at in (0, I - 120):                      # (two tiles of 128 alone: never the larger tiles)
+        part = torch.cat([w[at:at + 120], w[I + at:I + at + 120]])
+        few = torch.empty(M, 120, dtype=out.dtype, device=DEV)
+        impl.gemm_pair(x, part, torch.cat([b[at:at + 120], b[I + at:I + at + 120]]), few, gated=code, n_out=120)
+        assert torch.equal(few, out[:, at:at + 120]), at
+    full = x.double() @ w.double().T + b.double()
+    g, u = full[:, :I], full[:, I:]
+    if act == "silu":
+        want = torch.nn.functional.silu(g) * u
+        assert float((out.double() - want).abs().max() / want.abs().max()) < 1e-2
+
+
 @pytest.mark.parametrize("bias", [False, True])
 @pytest.mark.parametrize("M,H,I,per_sm", [(300, 136, 203, 1), (150, 64, 5, 1), (600, 520, 1, 2), (129, 72, 130, 2), (40, 64, 262, 1)])
 def test_gated_pair_product_of_outputs_that_are_no_blocks_of_eight(M, H, I, per_sm, bias):
