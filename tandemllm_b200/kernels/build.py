@@ -172,8 +172,9 @@ _KINDS = {ctypes.c_void_p: "p", ctypes.c_longlong: "l", ctypes.c_int: "i", ctype
 
 
 def build_fastcall() -> str | None:
-    """The extension that calls launchers (csrc/fastcall.c), compiled if its file is not there yet; None where there is no C compiler or
-    no Python header, or on another platform than the one it is written for (launches then go through ctypes, as they are)."""
+    """The extension that calls launchers (csrc/fastcall.c), compiled if its file is not there yet; None where there is no C compiler, no
+    Python header or a compiler that fails, or on another platform than the one it is written for (launches then go through ctypes, as
+    they are)."""
     include = sysconfig.get_paths()["include"]
     cc = shutil.which("cc") or shutil.which("gcc")
     source = os.path.join(CSRC, "fastcall.c")
@@ -186,24 +187,27 @@ def build_fastcall() -> str | None:
     if platform.machine() != "x86_64" or not sys.platform.startswith("linux") or not cc or not os.path.isfile(os.path.join(include, "Python.h")):
         return None
     tmp = out + f".tmp{os.getpid()}"
-    r = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, source, "-o", tmp], capture_output=True, text=True)
-    if r.returncode != 0:
-        raise ExtensionError(f"{cc} failed on fastcall.c:\n{r.stdout}\n{r.stderr}")
-    os.replace(tmp, out)
+    try:
+        subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, source, "-o", tmp], capture_output=True, text=True, check=True)
+        os.replace(tmp, out)
+    except (OSError, subprocess.CalledProcessError) as e:
+        say(f"{cc} failed on fastcall.c, launches go through ctypes: {e}\n{getattr(e, 'stderr', '')}")
+        return None
     return out
 
 
 def _launcher_type():
     global _launcher
     if _launcher is None:
-        path = build_fastcall()
-        if path is None:
-            _launcher = False
-        else:
-            loader = importlib.machinery.ExtensionFileLoader("fastcall", path)
-            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("fastcall", path, loader=loader))
-            loader.exec_module(module)
-            _launcher = module.Launcher
+        path, _launcher = build_fastcall(), False
+        if path is not None:
+            try:
+                loader = importlib.machinery.ExtensionFileLoader("fastcall", path)
+                module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("fastcall", path, loader=loader))
+                loader.exec_module(module)
+                _launcher = module.Launcher
+            except (ImportError, OSError) as e:
+                say(f"{path} could not be loaded, launches go through ctypes: {e}")
     return _launcher
 
 

@@ -50,9 +50,39 @@ def test_arguments_of_every_kind_arrive_as_through_ctypes(library):
     assert fast.none() == 7                                                                              # (no declared parameters)
 
 
+def launched_through(libraries):
+    """(functions with declared parameters that return an int, those of them that go through the extension)"""
+    fit, through = [], []
+    for lib in libraries:
+        for name, fn in vars(lib._library).items():
+            if name.startswith("tl_") and fn.argtypes and fn.restype is ctypes.c_int:
+                fit.append(name)
+                if name in vars(lib):
+                    assert type(vars(lib)[name]).__name__ == "Launcher"
+                    through.append(name)
+    return fit, through
+
+
 def test_the_kernel_libraries_are_called_through_it_where_it_was_built():
-    from tandemllm_b200.kernels import ops
-    core = ops.core()
-    through = [n for n in ops._SIGNATURES if n in vars(core)]
-    assert not through or len(through) > len(ops._SIGNATURES) // 2
-    assert os.path.basename(build.build_fastcall() or "fastcall-.so").startswith("fastcall-")
+    from tandemllm_b200.kernels import ops, tensorcore
+    fit, through = launched_through([ops.core(), tensorcore.lib()])
+    assert len(fit) > 60
+    if build.build_fastcall() is None:
+        assert not through
+    else:
+        assert sorted(set(fit) - set(through)) == []
+
+
+@pytest.mark.parametrize("broken", ["compiler fails", "compiler cannot run", "file is no extension"])
+def test_launches_go_through_ctypes_where_the_extension_cannot_be_had(broken, library, tmp_path, monkeypatch):
+    cc = tmp_path / "cc"
+    cc.write_text("#!/bin/sh\nexit 1\n" if broken == "compiler fails" else
+                  "#!/no/such/shell\n" if broken == "compiler cannot run" else
+                  '#!/bin/sh\nfor a in "$@"; do o=$a; done\necho no > "$o"\n')
+    cc.chmod(0o755)
+    monkeypatch.setenv("PATH", f"{tmp_path}:{os.environ['PATH']}")
+    monkeypatch.setattr(build, "build_dir", lambda: str(tmp_path))            # (where no extension has been built)
+    monkeypatch.setattr(build, "_launcher", None)
+    plain = build.Launchers(library, ["mixed"])
+    assert "mixed" not in vars(plain) and plain.mixed(None, 0, 0.0, None, 5, 0, 0.0, 0, None, 0, 0, 0.0, 3) == 2
+    assert not [f for f in os.listdir(tmp_path) if f.endswith(".so")] or broken == "file is no extension"
