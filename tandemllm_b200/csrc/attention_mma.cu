@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(TMA ? 160 : 128, D == 64 ? (TMA ? 3 : 4) : 2) 
     const int* __restrict__ tiles,
     const int* __restrict__ positions, float scale, int window, bf16* __restrict__ out, float* __restrict__ part_o,
     float* __restrict__ part_ml, int n_spans, int split, int Hq, int Hk, int* __restrict__ status,
-    const __grid_constant__ KvMaps maps, int box_rows) {
+    const __grid_constant__ KvMaps maps, int box_rows, int tile_places) {
   constexpr int CH = D / 8;                 // 16-byte chunks per row
   constexpr int TILE_BYTES = 64 * D * 2;
   constexpr int QROWS = KEYSPLIT ? 16 : 64;
@@ -387,11 +387,12 @@ __global__ void __launch_bounds__(TMA ? 160 : 128, D == 64 ? (TMA ? 3 : 4) : 2) 
     } else {
       // a span that holds none of the row's keys writes nothing: the join kernel reads only the spans of lo .. pos
       if (span < lo / span_keys || span > pos / span_keys) return;
-      float* dst = part_o + ((row * Hq + head) * n_spans + span) * D + col;
+      const long long place = ((tile_places ? (long long)t * tile_places + qi : row) * Hq + head) * n_spans + span;
+      float* dst = part_o + place * D + col;
       dst[0] = o0;
       dst[1] = o1;
       if (first) {
-        float* ml = part_ml + ((row * Hq + head) * n_spans + span) * 2;
+        float* ml = part_ml + place * 2;
         ml[0] = mrow * 0.6931471805599453f;             // the join kernel works in natural units
         ml[1] = l;
       }
@@ -452,7 +453,7 @@ template <int D, bool KEYSPLIT, int STAGES, bool TMA>
 static int launch_mma(const void* q, const void* k_cache, const void* v_cache, const int* block_table, int max_pages,
                       int page_size, int num_pages, const int* tiles, int n_tiles, const int* positions, float scale, int window,
                       void* out, float* part_o, float* part_ml, int n_spans, int split, int Hq, int Hk, int* status,
-                      cudaStream_t stream) {
+                      int tile_places, cudaStream_t stream) {
   // with TMA: room to start the tiles on a 1024-byte boundary, and the stages' mbarriers behind them
   constexpr int SMEM = ((KEYSPLIT ? 16 : 64) + 2 * STAGES * 64) * D * 2 + (TMA ? 1024 + 2 * STAGES * 8 : 0);
   static_assert(!KEYSPLIT || 4 * 16 * (D + 2) * 4 <= 2 * STAGES * 64 * D * 2, "the merge buffer reuses the stages");
@@ -479,7 +480,7 @@ static int launch_mma(const void* q, const void* k_cache, const void* v_cache, c
   return (int)launch_chained(attention_mma_kernel<D, KEYSPLIT, STAGES, TMA>, grid, dim3(TMA ? 160 : 128), SMEM, stream,
                              (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, block_table, max_pages, page_size,
                              page_shift, num_pages, tiles, positions, scale, window, (bf16*)out, part_o, part_ml, n_spans, split,
-                             Hq, Hk, status, maps, box_rows);
+                             Hq, Hk, status, maps, box_rows, tile_places);
 }
 
 static int& decode_with_tma() {
@@ -504,12 +505,17 @@ extern "C" int tl_attention_mma_supported(int Hq, int Hk, int D) {
 // tiles: int32 [n_tiles, 3] = (request index, first row, query rows <= tile_rows), rows of a tile consecutive in position.
 // max_tile_rows: the most query rows any tile holds; when they and their heads fit 16 M rows (decoding), the kernel
 // form that splits the keys among the warps runs. With split, scratch holds rows * Hq * n_spans * (D + 2) floats and
-// the caller runs the join afterwards (tl_attention_join) when n_spans > 1.
-extern "C" int tl_paged_attention_mma(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
-                                      int max_pages, int page_size, int num_pages, const int* tiles, int n_tiles, int max_tile_rows,
-                                      const int* positions, float scale, int window, void* out, float* scratch, int rows,
-                                      int Hq, int Hk, int D, int n_spans, int split, int* status, cudaStream_t stream) {
+// the caller runs the join afterwards (tl_attention_join) when n_spans > 1. With `tile_places` (a number no tile has more rows than)
+// scratch has so many places a tile instead of one a row, n_tiles * tile_places for `rows` (tl_attention_join_tiles reads them):
+// tiles whose rows lie far apart, with other rows between them, then want no more of it than tiles side by side.
+extern "C" int tl_paged_attention_mma_tiles(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
+                                            int max_pages, int page_size, int num_pages, const int* tiles, int n_tiles,
+                                            int max_tile_rows, const int* positions, float scale, int window, void* out,
+                                            float* scratch, int rows, int Hq, int Hk, int D, int n_spans, int split, int* status,
+                                            int tile_places, cudaStream_t stream) {
   if (rows == 0 || n_tiles == 0) return 0;
+  TL_REQUIRE(tile_places == 0 || (tile_places >= max_tile_rows && (long long)n_tiles * tile_places <= rows),
+             "attention: %d places a tile for %d tiles of up to %d rows, %d places in all", tile_places, n_tiles, max_tile_rows, rows);
   TL_REQUIRE(tl_attention_mma_supported(Hq, Hk, D), "attention (tensor cores): %d heads over %d KV heads of size %d", Hq, Hk, D);
   TL_REQUIRE(page_size > 0 && max_pages > 0 && window >= 0, "attention: page size %d, table width %d, window %d", page_size,
              max_pages, window);
@@ -528,13 +534,21 @@ extern "C" int tl_paged_attention_mma(const void* q, const void* k_cache, const 
                    (long long)num_pages * Hk * page_size < (1LL << 31);
 #define TL_MMA(D_, KS_, ST_, TMA_)                                                                                          \
   launch_mma<D_, KS_, ST_, TMA_>(q, k_cache, v_cache, block_table, max_pages, page_size, num_pages, tiles, n_tiles, positions, \
-                                 scale, window, out, part_o, part_ml, n_spans, split, Hq, Hk, status, stream)
+                                 scale, window, out, part_o, part_ml, n_spans, split, Hq, Hk, status, tile_places, stream)
   if (D == 64)
     return keysplit ? (tma ? TL_MMA(64, true, 4, true) : TL_MMA(64, true, 4, false))
                     : (tma ? TL_MMA(64, false, 3, true) : TL_MMA(64, false, 2, false));
   return keysplit ? (tma ? TL_MMA(128, true, 3, true) : TL_MMA(128, true, 3, false))
                   : (tma ? TL_MMA(128, false, 2, true) : TL_MMA(128, false, 2, false));
 #undef TL_MMA
+}
+
+extern "C" int tl_paged_attention_mma(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
+                                      int max_pages, int page_size, int num_pages, const int* tiles, int n_tiles, int max_tile_rows,
+                                      const int* positions, float scale, int window, void* out, float* scratch, int rows,
+                                      int Hq, int Hk, int D, int n_spans, int split, int* status, cudaStream_t stream) {
+  return tl_paged_attention_mma_tiles(q, k_cache, v_cache, block_table, max_pages, page_size, num_pages, tiles, n_tiles, max_tile_rows,
+                                      positions, scale, window, out, scratch, rows, Hq, Hk, D, n_spans, split, status, 0, stream);
 }
 
 // 0: keys and values are fetched with cp.async from every thread instead of a producer warp's TMA copies

@@ -280,7 +280,7 @@ constexpr int JOIN_Q = 4;
 template <typename T>
 __global__ void attention_join_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                       const int* __restrict__ positions, int window, T* __restrict__ out, int Hq, int D,
-                                      int n_spans, int span_keys, const int* __restrict__ tiles) {
+                                      int n_spans, int span_keys, const int* __restrict__ tiles, int tile_places) {
   __shared__ float s_o[JOIN_Q][MAX_D];
   __shared__ float s_sum[JOIN_Q];
   chain_next();
@@ -290,12 +290,13 @@ __global__ void attention_join_kernel(const float* __restrict__ part_o, const fl
     if ((int)blockIdx.z >= tiles[3 * r + 2]) return;
     r = tiles[3 * r + 1] + blockIdx.z;
   }
+  const long long place = tile_places ? (long long)blockIdx.x * tile_places + blockIdx.z : r;
   const int h = blockIdx.y;
   const int pos = positions[r];
   const int lo = window > 0 ? max(0, pos - window + 1) : 0;
   const int s0 = lo / span_keys, s1 = min(pos / span_keys, n_spans - 1);      // never past the scratch's last span
   if (s0 >= s1) return;                                 // one span: written directly by the span kernel
-  const long long base = ((long long)r * Hq + h) * n_spans;
+  const long long base = (place * Hq + h) * n_spans;
   const float2* ml2 = reinterpret_cast<const float2*>(part_ml);      // (max, sum) pairs
   const int lane = threadIdx.x & 31;
   const int DT = blockDim.x / JOIN_Q, q = threadIdx.x / DT, dd = threadIdx.x - q * DT;
@@ -370,7 +371,7 @@ static int launch_spans(const void* q, const void* k_cache, const void* v_cache,
   if (n_spans > 1) {
     dim3 join(rows, Hq);
     attention_join_kernel<T><<<join, JOIN_Q * (D <= 64 ? 64 : 128), 0, stream>>>(part_o, part_ml, positions, window, (T*)out, Hq, D,
-                                                                    n_spans, SPAN, nullptr);
+                                                                    n_spans, SPAN, nullptr, 0);
     e = cudaGetLastError();
   }
   return (int)e;
@@ -411,29 +412,31 @@ extern "C" int tl_paged_attention_split(const void* q, const void* k_cache, cons
 
 // Joins the spans that another kernel left in `scratch` (same layout as above, for `rows` rows) into `out`, in ascending order.
 // `span_keys`: the key positions a span covers (the kernel that wrote the spans chose it). `tiles` (or null: every row): int32
-// [n_tiles, 3] = (request, first row, rows), at most `tile_rows` rows each; the rows of other tiles are left alone.
+// [n_tiles, 3] = (request, first row, rows), at most `tile_rows` rows each; the rows of other tiles are left alone. With `by_tile` the
+// scratch has `tile_rows` places a tile (tl_paged_attention_mma_tiles) and not one a row.
 extern "C" int tl_attention_join_tiles(const float* scratch, const int* positions, int window, void* out, int rows, int Hq, int D,
                                        int n_spans, int span_keys, int dtype, const int* tiles, int n_tiles, int tile_rows,
-                                       cudaStream_t stream) {
+                                       int by_tile, cudaStream_t stream) {
   if (rows == 0 || n_spans <= 1 || (tiles && n_tiles == 0)) return 0;
   TL_REQUIRE(scratch != nullptr && Hq > 0 && Hq <= 65535 && D > 0 && span_keys > 0,
              "attention join: %d heads of size %d, spans of %d keys", Hq, D, span_keys);
   TL_REQUIRE(!tiles || (tile_rows >= 1 && tile_rows <= 65535), "attention join: tiles of %d rows", tile_rows);
   const float* part_o = scratch;
-  const float* part_ml = scratch + (long long)rows * Hq * n_spans * D;
+  const int places = tiles && by_tile ? tile_rows : 0;
+  const float* part_ml = scratch + (places ? (long long)n_tiles * places : (long long)rows) * Hq * n_spans * D;
   dim3 join(tiles ? n_tiles : rows, Hq, tiles ? tile_rows : 1);
   cudaError_t e;
   if (dtype == TL_FP32)
     e = launch_chained(attention_join_kernel<float>, join, dim3(JOIN_Q * (D <= 64 ? 64 : 128)), 0, stream, part_o, part_ml, positions,
-                       window, (float*)out, Hq, D, n_spans, span_keys, tiles);
+                       window, (float*)out, Hq, D, n_spans, span_keys, tiles, places);
   else
     e = launch_chained(attention_join_kernel<bf16>, join, dim3(JOIN_Q * (D <= 64 ? 64 : 128)), 0, stream, part_o, part_ml, positions,
-                       window, (bf16*)out, Hq, D, n_spans, span_keys, tiles);
+                       window, (bf16*)out, Hq, D, n_spans, span_keys, tiles, places);
   return (int)e;
 }
 extern "C" int tl_attention_join(const float* scratch, const int* positions, int window, void* out, int rows, int Hq, int D,
                                  int n_spans, int span_keys, int dtype, cudaStream_t stream) {
-  return tl_attention_join_tiles(scratch, positions, window, out, rows, Hq, D, n_spans, span_keys, dtype, nullptr, 0, 0, stream);
+  return tl_attention_join_tiles(scratch, positions, window, out, rows, Hq, D, n_spans, span_keys, dtype, nullptr, 0, 0, 0, stream);
 }
 
 // ------------------------------------------------------------------------------------------------------------------

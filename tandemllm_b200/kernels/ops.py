@@ -114,7 +114,7 @@ _SIGNATURES = {
                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "tl_attention_join": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "tl_attention_join_tiles": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
-                                c_void_p],
+                                c_int, c_void_p],
     "tl_router_topk": [c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p,
                        c_void_p],
     "tl_moe_max_tiles": [c_int, c_int, c_int],
@@ -897,11 +897,12 @@ def attention_join(scratch, positions, window, out, n_spans: int, span_keys: int
           kernels=1 if n_spans > 1 else 0)
 
 
-def attention_join_tiles(scratch, positions, window, out, n_spans: int, span_keys: int, tiles, tile_rows: int) -> None:
-    """`attention_join` for the rows of `tiles` (int32 [n, 3] = (request, first row, rows), at most `tile_rows` rows each) alone."""
+def attention_join_tiles(scratch, positions, window, out, n_spans: int, span_keys: int, tiles, tile_rows: int, by_tile: bool) -> None:
+    """`attention_join` for the rows of `tiles` (int32 [n, 3] = (request, first row, rows), at most `tile_rows` rows each) alone. The
+    scratch has a place a row of the step, or (`by_tile`) `tile_rows` places a tile."""
     rows, Hq, D = out.shape
     check(core().tl_attention_join_tiles(ptr(scratch), ptr(positions), int(window or 0), ptr(out), rows, Hq, D, int(n_spans),
-                                         int(span_keys), dtype_code(out.dtype), ptr(tiles), tiles.shape[0], int(tile_rows), stream()),
+                                         int(span_keys), dtype_code(out.dtype), ptr(tiles), tiles.shape[0], int(tile_rows), int(by_tile), stream()),
           "attention_join_tiles", kernels=1 if n_spans > 1 else 0)
 
 

@@ -100,6 +100,8 @@ def lib():
                                              c_void_p, ctypes.c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                              c_int, c_void_p, c_void_p]
         l.tl_paged_attention_mma.restype = c_int
+        l.tl_paged_attention_mma_tiles.argtypes = l.tl_paged_attention_mma.argtypes[:-1] + [c_int, c_void_p]
+        l.tl_paged_attention_mma_tiles.restype = c_int
         l.tl_paged_attention_tc.argtypes = l.tl_paged_attention_mma.argtypes
         l.tl_paged_attention_tc.restype = c_int
         l.tl_attention_tc_tile_rows.argtypes = [c_int, c_int]
@@ -654,12 +656,11 @@ def _attention_flex(self, part, q, cache, table, step, gate, ld_gate: int, out_s
     return True
 
 
-def _split_tiles(self, step, big_rows: int, small_rows: int, from_first: bool = False):
+def _split_tiles(self, step, big_rows: int, small_rows: int):
     """(tiles of requests that bring more than `small_rows` rows, cut into `big_rows` rows; one tile for each of the other
-    requests; the most rows of those), tiles int32 [n, 3] = (request, first row, rows) on the device, or None. With `from_first`
-    the other requests' rows are counted from their first one; where that lies, how many rows there are up to their last one and
-    their longest context is at ("small_rows", small_rows). Kept on the step."""
-    key = ("split_tiles", big_rows, small_rows, from_first)
+    requests; the most rows of those), tiles int32 [n, 3] = (request, first row, rows) on the device, or None; the other requests'
+    longest context is at ("small_context", small_rows). Kept on the step."""
+    key = ("split_tiles", big_rows, small_rows)
     if key not in step.host:
         starts = step.host["row_start"]
         big, small = [], []
@@ -669,11 +670,8 @@ def _split_tiles(self, step, big_rows: int, small_rows: int, from_first: bool = 
                 small.append((b, starts[b], n))
             else:
                 big += [(b, r0, min(big_rows, starts[b + 1] - r0)) for r0 in range(starts[b], starts[b + 1], big_rows)]
-        if from_first and small:
-            first, at = small[0][1], step.host.get("start_pos")
-            longest = max(at[b] + n for b, _, n in small) if at else step.max_context
-            step.host["small_rows", small_rows] = (first, small[-1][1] + small[-1][2] - first, longest)
-            small = [(b, r0 - first, n) for b, r0, n in small]
+        at = step.host.get("start_pos")
+        step.host["small_context", small_rows] = max((at[b] + n for b, _, n in small), default=0) if at else step.max_context
         both = torch.tensor(big + small, dtype=torch.int32).reshape(-1, 3).to(self.device, non_blocking=True)
         step.host[key] = (both[:len(big)] if big else None, both[len(big):] if small else None,
                           max((t[2] for t in small), default=0))
@@ -689,16 +687,11 @@ def _prompt_attention(self, q, cache, table, step, scale, window, out, runtime) 
     Hk = cache.k.shape[1]
     G = Hq // Hk
     tile_rows = lib().tl_attention_tc_tile_rows(Hq, Hk)
-    big, small, small_max = self._split_tiles(step, tile_rows, 16 // G, from_first=True)
+    big, small, small_max = self._split_tiles(step, tile_rows, 16 // G)
     n_big = 0 if big is None else big.shape[0]
     n_small = 0 if small is None else small.shape[0]
-    kv = (cache.k.data_ptr(), cache.v.data_ptr(), table.data_ptr(), table.shape[1], cache.page_size, cache.k.shape[0])
-
-    def run(kernel, what, tiles, most, first, rows, spans, span_keys, scratch):
-        at = first * Hq * D * q.element_size()
-        _check(kernel(q.data_ptr() + at, *kv, tiles.data_ptr(), tiles.shape[0], most, step.positions.data_ptr() + 4 * first, float(scale),
-                      int(window or 0), out.data_ptr() + at, ops.ptr(scratch), rows, Hq, Hk, D, spans, span_keys,
-                      self.status.data_ptr(), ops.stream()), what)
+    head = (q.data_ptr(), cache.k.data_ptr(), cache.v.data_ptr(), table.data_ptr(), table.shape[1], cache.page_size, cache.k.shape[0])
+    place = (step.positions.data_ptr(), float(scale), int(window or 0), out.data_ptr())
     if n_big:
         ctas, slots = n_big * Hk, 2 * self.sm_count
         span_keys, spans = 0, 1
@@ -711,21 +704,23 @@ def _prompt_attention(self, q, cache, table, step, scale, window, out, runtime) 
             if spans <= 1:
                 span_keys, spans = 0, 1
         scratch = runtime.scratch("attention", ops.attention_scratch_floats(R, Hq, D, spans)) if span_keys else None
-        run(lib().tl_paged_attention_tc, "attention_tc", big, min(tile_rows, step.max_rows_per_request), 0, R, spans, span_keys, scratch)
+        _check(lib().tl_paged_attention_tc(*head, big.data_ptr(), n_big, min(tile_rows, step.max_rows_per_request), *place, ops.ptr(scratch),
+                                           R, Hq, Hk, D, spans, span_keys, self.status.data_ptr(), ops.stream()), "attention_tc")
         if span_keys and n_small:
-            ops.attention_join_tiles(scratch, step.positions, window, out, spans, span_keys, big, tile_rows)
+            ops.attention_join_tiles(scratch, step.positions, window, out, spans, span_keys, big, tile_rows, False)
         elif span_keys:
             ops.attention_join(scratch, step.positions, window, out, spans, span_keys)
     if n_small:
         # A row a request, and contexts of any length: without spans the longest context is one CTA's chain (23 rows at 201 to 4100
         # keys, 184 CTAs: 57 us a layer; a step of 512 rows beside them 2360 -> 2271 us with the gated products, two layers of eight).
-        first, rows, longest = step.host[("small_rows", 16 // G)]
-        spans, span_keys = self._row_spans(n_small * Hk, longest) if rows <= 16 * n_small + 64 else (1, 0)
-        scratch = runtime.scratch("attention_rows", ops.attention_scratch_floats(rows, Hq, D, spans)) if span_keys else None
-        run(lib().tl_paged_attention_mma, "attention_mma", small, small_max, first, rows, spans, span_keys, scratch)
+        # The scratch has a tile's places, wherever the rows lie: behind one portion or on both sides of it.
+        spans, span_keys = self._row_spans(n_small * Hk, step.host["small_context", 16 // G])
+        places = n_small * small_max
+        scratch = runtime.scratch("attention_rows", ops.attention_scratch_floats(places, Hq, D, spans)) if span_keys else None
+        _check(lib().tl_paged_attention_mma_tiles(*head, small.data_ptr(), n_small, small_max, *place, ops.ptr(scratch), places, Hq, Hk, D,
+                                                  spans, span_keys, self.status.data_ptr(), small_max, ops.stream()), "attention_mma")
         if span_keys:
-            ops.attention_join_tiles(scratch, step.positions[first:first + rows], window, out[first:first + rows], spans, span_keys, small,
-                                     small_max)
+            ops.attention_join_tiles(scratch, step.positions, window, out, spans, span_keys, small, small_max, True)
     return True
 
 

@@ -452,6 +452,44 @@ def test_decode_rows_beside_a_portion_cut_their_keys_into_spans_of_their_own(Hq,
         assert rel(out[starts[b]:starts[b] + n], want) < 2e-2, f"sequence {b}"
 
 
+@pytest.mark.parametrize("Hq,Hk,window", [(32, 8, None), (4, 4, 700), (8, 2, None)])
+def test_decode_rows_on_both_sides_of_a_portion_cut_their_keys_as_on_one_side(Hq, Hk, window):
+    """Decode rows first, a portion of 500 rows, then the last rows of another prompt: the same spans and the same bits as with the
+    portion in front of all of them, and scratch for the tiles' rows, not for the rows that lie between them."""
+    import types
+
+    from tandemllm_b200.kernels import ops
+    from tests.test_gpu_kernels import paged_setup, plain_attention
+    impl, _ = tc()
+    few = 16 // (Hq // Hk)
+    seqs, news = [1, 257, 4000, 700, 600, 3001], [1, 1, 1, 500, 2, min(3, few)]
+    kc, vc, table, ks, vs = paged_setup(seqs, Hk, 64, 16, torch.bfloat16, seed=92)
+    cache = types.SimpleNamespace(k=kc.to(DEV), v=vc.to(DEV), page_size=16)
+    q = [rnd(n, Hq, 64, seed=93 + b) for b, n in enumerate(news)]
+
+    def run(order):
+        from tandemllm_b200.parts import Runtime
+        rt = Runtime(torch.device(DEV), torch.bfloat16)
+        starts = [0]
+        for b in order:
+            starts.append(starts[-1] + news[b])
+        positions = sum((list(range(seqs[b] - news[b], seqs[b])) for b in order), [])
+        step = types.SimpleNamespace(n_requests=len(order), max_rows_per_request=max(news), max_context=max(seqs),
+                                     positions=torch.tensor(positions, dtype=torch.int32, device=DEV),
+                                     host={"row_start": starts, "start_pos": [seqs[b] - news[b] for b in order]})
+        out = torch.full((starts[-1], Hq, 64), float("nan"), dtype=torch.bfloat16, device=DEV)
+        assert impl.attention(torch.cat([q[b] for b in order]).to(DEV), cache, table[order].to(DEV), step, 0.125, window, out, rt)
+        torch.cuda.synchronize()
+        sizes = {name: t.numel() for (name, _), t in rt._scratch.items()}
+        return {b: out[starts[i]:starts[i + 1]] for i, b in enumerate(order)}, sizes
+    (one, had), (both, has) = run([3, 0, 1, 2, 4, 5]), run([0, 1, 2, 3, 4, 5])
+    for b in (0, 1, 2, 4, 5):
+        assert torch.equal(one[b], both[b]), b
+    assert had == has and has["attention_rows/0"] <= ops.attention_scratch_floats(5 * min(3, few), Hq, 64, 16)
+    for b in range(6):
+        assert rel(both[b], plain_attention(q[b].float(), ks[b], vs[b], 0.125, window)) < 2e-2, b
+
+
 def attention_against_plain(seqs, news, split, Hq, Hk, D, page, window, kernel="mma"):
     if kernel == "tc":
         # both forms of the tcgen05 kernel: P back in tensor memory (the default), and P through shared memory
