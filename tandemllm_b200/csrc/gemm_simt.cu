@@ -265,8 +265,9 @@ __global__ void __launch_bounds__(256) gemm_tall_narrow_kernel(GemmParams p) {
 // whose sums may stay in parts is cut into runs of k, a CTA each (`simt_runs` in kernels/ops.py).
 //
 // An output is the sum of eight chains, a warp's even and odd k in ascending order over the quads q = warp (mod 4), added in
-// order: which k a chain has depends on k alone, whatever the tile's height, so a row still does not depend on the others, and
-// eight short chains lose less than one long one.
+// order: which k a chain has depends on k alone, whatever the tile's height, so a row does not depend on the others as long as the
+// product is whole; in runs of k, and with up to eight rows of a long k (below), it has other chains. Eight short chains lose less than
+// one long one.
 //
 // Up to 8 rows are bound by the weights' bytes: tiles of 1, 2, 4 or 8 rows and so few outputs (8, 16 or 32) that the weights come
 // through as many SMs as there are, a lane an output where it goes (a weight is then read from shared memory once, by one lane), and

@@ -742,8 +742,22 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, out: 
 def simt_runs(M: int, N: int, K: int) -> int:
     """Elements a run of k of a 32-bit product whose runs' sums the caller adds, 0 where one run is as good: up to 512 rows, so few
     outputs that their tiles fill the GPU a few times at most, and a k of 1024 and more; four runs. (A prompt of 150 rows through three
-    layers 2492 -> 2225 us: its products into 2048 outputs had 160 tiles on 148 SMs, and a shared SM took as long as two rounds.)"""
-    if not 8 < M <= 512 or not 256 <= N <= 4096 or K < 1024 or -(-M // 32) * -(-N // 64) > 4 * sm_count():
+    layers 2492 -> 2225 us: its products into 2048 outputs had 160 tiles on 148 SMs, and a shared SM took as long as two rounds.)
+
+    Whole, a product takes as long as the SM with the most tiles, one alone on an SM a quarter longer than its share of two; in runs
+    the CTAs even out, but each starts a pipeline (64 k-elements' time) and the norm reads four sums. Whole and in runs with the norm,
+    us: k 1024, 2048 outputs, 50 rows 34 and 24, 150 44 and 40, 256 46 and 50, 400 65 and 75; k 2048, 150 rows 75 and 58, 256 75 and
+    75, 400 110 and 118; k 7168, 16 rows 97 and 40, 150 224 and 149, 512 429 and 384. Below a k of 2048 whole products stay where they
+    are faster; from there on few are (257 to 288 and 385 to 416 rows against 2048 outputs, by a tenth), and runs stay, whose shorter
+    chains lie nearer to 64 bits (1.6e-7 -> 1.4e-7 at 150 rows).
+
+    So a row of such a product has other bits beside few rows than beside many, as it has beside up to eight; runs for any number of
+    rows would cost products of 1024 rows and more up to a quarter of their time."""
+    if not 8 < M <= 512 or not 256 <= N <= 4096 or K < 1024:
+        return 0
+    tiles, sms = -(-M // 32) * -(-N // 64), sm_count()
+    rounds = -(-tiles // sms)
+    if rounds > 4 or (K < 2048 and (4 * tiles / sms + 0.4) * (K / 4 + 64) >= (1.25 if rounds == 1 else rounds) * K):
         return 0
     return -(-K // (4 * 32)) * 32
 
