@@ -312,11 +312,6 @@ class CacheManager:
     def table(self, group: int, req) -> list[int]:
         return self.groups[group].tables[req]
 
-    def table_array(self, group: int, req) -> "np.ndarray":
-        """The block table of `req` in `group` as an int32 array (a view: valid until the table next grows)."""
-        g = self.groups[group]
-        return g.row(req)[:len(g.tables[req])]
-
     def max_table_len(self, reqs) -> int:
         return max((len(g.tables[r]) for g in self.groups for r in reqs), default=0)
 

@@ -72,22 +72,20 @@ def _int32s(values):
     if not isinstance(values, (list, tuple)):
         return values
     try:
-        return np.frombuffer(array("i", values), dtype=np.int32)
+        return array("i", values)
     except TypeError:
         return values
 
 
 def _append_int32s(out: array, values) -> None:
     """`values` as `_int32s` takes them, behind `out`."""
-    if isinstance(values, (list, tuple)):
-        try:
-            out.extend(array("i", values))
-            return
-        except TypeError:
-            pass
-    numbers = np.empty(len(values), dtype=np.int32)
-    numbers[:] = values
-    out.frombytes(numbers.tobytes())
+    ids = _int32s(values)
+    if ids is values:
+        numbers = np.empty(len(values), dtype=np.int32)
+        numbers[:] = values
+        out.frombytes(numbers.tobytes())
+    else:
+        out.extend(ids)
 
 
 class _Staging:

@@ -2,6 +2,7 @@
 
 import random
 
+import numpy as np
 import pytest
 
 from tandemllm_b200.cache import CacheManager, OutOfPages
@@ -40,6 +41,53 @@ def test_reserve_free_and_reuse():
     assert m.table(0, "b")[0] == first[-1], "the page freed last is handed out first"
     assert m.groups[0].pool.reused == 1
     m.check()
+
+
+@pytest.mark.parametrize("width", [3, 63, 64, 65, 128, 200])
+def test_tables_copied_in_whole_rows(width):
+    """Below, at and above the width the rows have room for, one request and several in any order, after the rows grew under requests
+    that held pages, after pages were given back, and in a slot that held a longer table before."""
+    m = manager(pages=400, reqs=4, page=16)
+
+    def tables_are_copied():
+        m.check()
+        held = [r for r in "abc" if r in m._slot_of]
+        for reqs in (held, held[::-1], held[-1:]):
+            for i, g in enumerate(m.groups):
+                if max(len(m.table(i, r)) for r in reqs) > width:
+                    continue
+                out = np.full((len(reqs), width), 7, dtype=np.int32)
+                g.copy_rows([m.slot_of(r) for r in reqs], out)
+                for row, r in zip(out.tolist(), reqs):
+                    assert row == m.table(i, r) + [-1] * (width - len(m.table(i, r)))
+    for r, n in (("a", 40), ("b", 16), ("c", 1)):
+        m.admit(r)
+        m.reserve(r, n)
+    tables_are_copied()
+    m.reserve("b", 66 * 16)                   # the rows grow (64 -> 128) while "a" and "c" hold tables
+    m.advance("b", 66 * 16)                   # and the windowed group gives pages back
+    tables_are_copied()
+    m.free("b")
+    m.admit("b")                              # the slot of the longer table
+    m.reserve("b", 17)
+    tables_are_copied()
+    m.reserve("a", 150 * 16)
+    tables_are_copied()
+
+
+def test_pages_for_a_whole_step_or_for_none():
+    needs = [PagedNeed(2, 16), PagedNeed(2, 16, window=40)]
+    m = manager(pages=8, reqs=3, page=16, needs=needs)
+    m.admit("a"); m.admit("b")
+    m.groups[1].pool.take(5, "elsewhere")     # the second group runs short, the first would not
+    before = [(g.pool.free, {r: list(t) for r, t in g.tables.items()}, g.rows.copy()) for g in m.groups]
+    assert not m.reserve_all([("a", 32), ("b", 32)])
+    for g, (free, tables, rows) in zip(m.groups, before):
+        assert g.pool.free == free and g.tables == tables and (g.rows == rows).all()
+    assert m.reserve_all([("a", 32), ("b", 16)])
+    assert [len(m.table(i, r)) for i in range(2) for r in "ab"] == [2, 1, 2, 1] and [g.pool.free for g in m.groups] == [5, 0]
+    assert m.reserve_all([("a", 20), ("b", 9)]) and not m.reserve_all([("a", 33)])      # (what is there already is enough)
+    assert m.groups[0].pool.free == 5
 
 
 def test_all_or_nothing_and_double_free():
