@@ -645,7 +645,9 @@ extern "C" int tl_recurrence_scan(const float* proj, long long ld, int q_col, in
   const int sms = sm_count > 0 ? sm_count : 148;
   // The staged form's lanes take two columns each, or where those would be few warps, one column by four times as many lanes (4 keys a
   // lane): the delta rule over 1100 rows, 16 heads of 128 x 128 376 us with 4 keys, 402 with two columns, 32 heads 712 and 457. Its
-  // blocks are sized for requests as long as the longest (`longest` rows), because the others are over before it.
+  // blocks are sized for requests as long as the longest (`longest` rows), because the others are over before it; the choice of the
+  // lanes counts all requests, whose short ones' blocks share SMs with the long one's while they last (1100 rows beside one row, 16
+  // heads of 128 x 128: two columns 435, 206 and 249 us with the delta rule, fixed decays and a decay a channel, 4 keys 452, 253 and 255).
   const long long alike = scratch ? (longest > 0 ? max(1LL, min((long long)requests, (rows + longest / 2) / longest)) : requests) : 0;
   int kpl = 16, cpl = 1;
   if (scratch && (long long)requests * H * VD * P >= 128LL * sms) {

@@ -14,11 +14,11 @@
 //
 // Roles in each CTA, as in the one-CTA persistent kernel (tc_gemm.cu): warp 0, one thread, keeps a ring of stages full
 // by TMA (plain loads, each CTA its own; their bytes are counted on the first CTA's barrier); warp 1 of the first CTA,
-// one thread, issues the MMAs into one of two accumulators and releases stages and accumulators in both CTAs with
+// one thread, issues the MMAs into a free accumulator and releases stages and accumulators in both CTAs with
 // tcgen05.commit; the epilogue warps (from warp 2 on) read a finished accumulator (one accumulator row a thread, 16 tokens a load), turn
 // the block through shared memory, apply the bias and the activation or gate, and store 8 or 16 outputs of a token at a time. Tensor
-// memory holds two accumulators or more, so that the next tile's MMAs run under a tile's epilogue. The kernel is persistent: as many
-// clusters as fit the GPU walk over the tiles.
+// memory holds two or four accumulators, so that the next tile's MMAs run under a tile's epilogue (one with two CTAs an SM, and one pair
+// of them in the WIDE form, see below). The kernel is persistent: as many clusters as fit the GPU walk over the tiles.
 //
 // The gated product's tiles of 256 outputs (256 gate and 256 up rows, whose two accumulators fill tensor memory: its MMAs wait for the
 // epilogue, and the last round of clusters is emptier) are kept where they load less for as many rounds (`wide_pays`). A tile of 128
@@ -641,7 +641,7 @@ extern "C" int tl_tc_pair_resident(int gated, int per_sm) {
 // tile_group = nullptr. gated (an activation code TL_ACT_*, or 0): W holds 2 N rows per group (gate then up) and
 // C = act(gate) * up (`bias`, ungrouped: 2 N numbers in the same order); a negated code: N rows and C = act(X W^T). row_weight,
 // weight_index (grouped and gated, or null): see `pair_weight`. out_dtype: TL_BF16 or TL_FP32. Grouped: the tile map's tiles hold at most tl_tc_pair_token_tile()
-// rows (plan_rows: the height the map was built with). per_sm: 1 or 2 CTAs an SM (see Smem). splits > 1 (plain, ungrouped,
+// rows (plan_rows: the height the map was built with). per_sm: 1, or 2 for the form of products bound by their weights (see Smem). splits > 1 (plain, ungrouped,
 // 32-bit output): the reduction is cut into `splits` runs of k-blocks, each a work item of its own, and C receives the
 // runs' partial results one behind the other, [splits, M, ldc], for the caller to add in order (a product with fewer
 // tiles than the GPU has pairs of SMs: a pair streams a tile's operands at the rate of its two SMs whatever else is idle).

@@ -1,7 +1,8 @@
 // What the kernels that move tiles with TMA share: mbarrier and bulk-tensor-copy wrappers for the device, and the host's
-// cache of tensor maps. A tensor map here always describes a 2D bfloat16 tensor [rows, cols] whose boxes are 64 columns
-// (128 bytes, one swizzle atom) wide and land in shared memory with the 128-byte swizzle: 16-byte piece c of row r of a
-// box lies at r * 128 + ((c ^ (r & 7)) << 4) from a base that is 1024-byte aligned.
+// cache of tensor maps. A tensor map here describes a 2D bfloat16 tensor [rows, cols] (`tensor_map`), or the gate and up rows of
+// gated weights as a 5D one (`gate_up_map`). Boxes are 64 columns (128 bytes, one swizzle atom) wide and land in shared memory
+// with the 128-byte swizzle: 16-byte piece c of row r of a box lies at r * 128 + ((c ^ (r & 7)) << 4) from a base that is
+// 1024-byte aligned.
 #pragma once
 #include <cuda.h>
 

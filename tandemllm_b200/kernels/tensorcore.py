@@ -467,7 +467,7 @@ class TensorCore:
         swap = avg <= 48
         bn = 16 if avg <= 12 else 32 if avg <= 24 else 64 if swap else 256
         if not swap and PROMPT_PRODUCT == "pair":
-            # few rows an expert: the products are bound by the experts' weights, and run two CTAs an SM on tiles of 128
+            # few rows an expert: the products are bound by the experts' weights and take the form for that, on tiles of 128 rows
             return swap, bn, lib().tl_tc_pair_token_tile(2 if avg <= PAIR_HALF_ROWS else 1)
         return swap, bn, lib().tl_tc_token_tile(int(swap), bn)
 

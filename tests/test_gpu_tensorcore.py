@@ -910,8 +910,9 @@ def test_prompt_products_through_either_kernel(which, monkeypatch):
 @pytest.mark.parametrize("gated", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(300, 520, 192), (129, 264, 72), (1000, 1792, 256)])
 def test_pair_product_with_two_ctas_an_sm(M, N, K, gated):
-    """The form with half the shared and tensor memory a CTA (the gated product on tiles of 128 token rows), which a
-    routing plan of tiles up to 128 rows selects: the same results as the plain rule, run twice the same bits."""
+    """The form for products bound by their weights (plain: half the shared and tensor memory a CTA, two an SM; gated: tiles of
+    128 token rows behind a deeper ring), which a routing plan of tiles up to 128 rows selects: the same results as the plain
+    rule, run twice the same bits."""
     impl, rt = tc()
     x, w = rnd(M, K, seed=81), rnd((2 if gated else 1) * N, K, seed=82, scale=0.1)
     outs = []
