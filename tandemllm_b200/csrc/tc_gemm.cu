@@ -115,9 +115,11 @@ __device__ __forceinline__ float plain_result(float v, int act) { return act < 0
 // DEEP: the swapped plain product where its CTAs are at most one an SM and have more k-blocks than the three stages that let three
 // CTAs share an SM: as many as fit (64 rows against 14336 x 2048, 112 CTAs 21.0 -> 18.7 us; 37 rows against 6144 x 2048, 48 CTAs
 // 16.7 -> 14.6 us).
-// FOUR: the swapped plain product of up to 16 rows with more CTAs than three an SM hold: three stages each, so that four share an SM
-// with as many bytes on their way (65536 outputs of 2048 are 512 CTAs: 444 and a second round of 68 at three an SM; a step of 8 rows at
-// 8192 tokens 890 -> 868 us with it, of 64 rows, whose experts' down products are as many CTAs, 1374 -> 1346).
+// FOUR: the swapped plain product of up to 16 rows whose CTAs take a round less at four an SM than at three: three stages each, so that four
+// share an SM with as many bytes on their way (65536 outputs of 2048 are 512 CTAs: 444 and a second round of 68 at three an SM; a step of
+// 8 rows at 8192 tokens 890 -> 868 us with it, of 64 rows, whose experts' down products are as many CTAs, 1374 -> 1346). With as many rounds
+// either way the shorter ring loses (8 rows, outputs of 2048: 57344, 448 CTAs, 62 -> 55 us; 76032, 594 CTAs, 68 and 74; 151936 111 and 115).
+// A grouped product's grid is an upper bound (the tiles of empty experts leave at once), so there the line is three an SM.
 constexpr int USUAL = 0, DEEP = 1, FOUR = 2;
 template <int BN, bool SWAP, bool SWIGLU, int FORM = USUAL>
 struct Smem {
@@ -691,8 +693,11 @@ static int launch_one(const CUtensorMap& tmW, const CUtensorMap& tmX, const TcPa
   if constexpr (SWAP && !SWIGLU && BN <= 128) {
     if (!p.tile_group && (long long)grid.x * grid.y * grid.z <= sm_count() && p.k_blocks_per_split > Smem<BN, SWAP, SWIGLU>::STAGES)
       return launch_form<BN, SWAP, SWIGLU, TOut, DEEP>(tmW, tmX, p, grid, stream);
-    if constexpr (BN == 16)
-      if ((long long)grid.x * grid.y * grid.z > 3 * sm_count()) return launch_form<BN, SWAP, SWIGLU, TOut, FOUR>(tmW, tmX, p, grid, stream);
+    if constexpr (BN == 16) {
+      const long long ctas = (long long)grid.x * grid.y * grid.z, three = 3 * sm_count(), four = 4 * sm_count();
+      if (p.tile_group ? ctas > three : (ctas + four - 1) / four < (ctas + three - 1) / three)
+        return launch_form<BN, SWAP, SWIGLU, TOut, FOUR>(tmW, tmX, p, grid, stream);
+    }
   }
   return launch_form<BN, SWAP, SWIGLU, TOut, USUAL>(tmW, tmX, p, grid, stream);
 }
