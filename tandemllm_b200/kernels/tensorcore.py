@@ -659,7 +659,7 @@ def _attention_flex(self, part, q, cache, table, step, gate, ld_gate: int, out_s
 def _split_tiles(self, step, big_rows: int, small_rows: int):
     """(tiles of requests that bring more than `small_rows` rows, cut into `big_rows` rows; one tile for each of the other
     requests; the most rows of those), tiles int32 [n, 3] = (request, first row, rows) on the device, or None; the other requests'
-    longest context is at ("small_context", small_rows). Kept on the step."""
+    contexts are at ("small_contexts", small_rows). Kept on the step."""
     key = ("split_tiles", big_rows, small_rows)
     if key not in step.host:
         starts = step.host["row_start"]
@@ -671,7 +671,7 @@ def _split_tiles(self, step, big_rows: int, small_rows: int):
             else:
                 big += [(b, r0, min(big_rows, starts[b + 1] - r0)) for r0 in range(starts[b], starts[b + 1], big_rows)]
         at = step.host.get("start_pos")
-        step.host["small_context", small_rows] = max((at[b] + n for b, _, n in small), default=0) if at else step.max_context
+        step.host["small_contexts", small_rows] = [at[b] + n if at else step.max_context for b, _, n in small]
         both = torch.tensor(big + small, dtype=torch.int32).reshape(-1, 3).to(self.device, non_blocking=True)
         step.host[key] = (both[:len(big)] if big else None, both[len(big):] if small else None,
                           max((t[2] for t in small), default=0))
@@ -711,10 +711,9 @@ def _prompt_attention(self, q, cache, table, step, scale, window, out, runtime) 
         elif span_keys:
             ops.attention_join(scratch, step.positions, window, out, spans, span_keys)
     if n_small:
-        # A row a request, and contexts of any length: without spans the longest context is one CTA's chain (23 rows at 201 to 4100
-        # keys, 184 CTAs: 57 us a layer; a step of 512 rows beside them 2360 -> 2271 us with the gated products, two layers of eight).
+        # A row a request, and contexts of any length: without spans the longest context is one CTA's chain.
         # The scratch has a tile's places, wherever the rows lie: behind one portion or on both sides of it.
-        spans, span_keys = self._row_spans(n_small * Hk, step.host["small_context", 16 // G])
+        spans, span_keys = self._row_spans(step.host["small_contexts", 16 // G], Hk, int(window or 0))
         places = n_small * small_max
         scratch = runtime.scratch("attention_rows", ops.attention_scratch_floats(places, Hq, D, spans)) if span_keys else None
         _check(lib().tl_paged_attention_mma_tiles(*head, small.data_ptr(), n_small, small_max, *place, ops.ptr(scratch), places, Hq, Hk, D,
@@ -724,13 +723,25 @@ def _prompt_attention(self, q, cache, table, step, scale, window, out, runtime) 
     return True
 
 
-def _row_spans(self, ctas: int, longest: int) -> tuple[int, int]:
-    """(spans, keys a span) of the keys of `ctas` small tiles whose longest context is `longest`: spans of 256 keys, doubled while the
-    longest contexts alone would still be four CTAs an SM; (1, 0) where the tiles fill the GPU or the contexts are short."""
-    if longest <= 512 or ctas >= 8 * self.sm_count:
+def _row_spans(self, contexts: list[int], kv_heads: int, window: int = 0) -> tuple[int, int]:
+    """(spans, keys a span) of the keys of small tiles with these contexts: spans of 256 keys, doubled while the longest contexts alone
+    would still be four CTAs an SM; (1, 0) where the tiles are as fast whole.
+
+    In keys of one CTA's chain (13 us a thousand): whole, the step takes the longest chain, or what all keys take (two CTAs' worth an
+    SM), and most of a chain more where the CTAs need a second round; in spans it takes two fifths of the longest, its share of all
+    keys, and the join with its launches. Beside a portion of 100 rows, 32 heads over 8, whole and in spans, us: 2 rows of 600 keys 38
+    and 36, 8 of 600 38 and 40, 23 of 1500 52 and 58, of 3000 71 and 72, 60 of 600 54 and 62, of 3000 130 and 114; unequal ones, 22 rows
+    of 201 to 4100 beside a portion of 512, 105 and 87, 30 of 250 to 2500 beside one of 300, 71 and 67, 30 of 100 to 1000 50 and 58."""
+    ctas, longest, sms = len(contexts) * kv_heads, max(contexts), self.sm_count
+    if longest <= 512 or ctas >= 8 * sms:
+        return 1, 0
+    seen = [min(c, window) for c in contexts] if window else contexts
+    far, keys = max(seen), sum(seen) * kv_heads / sms
+    whole = max(far, keys / 2) + (0.8 * far if ctas > 3 * sms else 0)
+    if whole <= 0.38 * far + keys / 2.65 + 300 + 10 * len(contexts):
         return 1, 0
     span = 256
-    while span < 2048 and ctas * -(-longest // (2 * span)) >= 4 * self.sm_count:
+    while span < 2048 and ctas * -(-longest // (2 * span)) >= 4 * sms:
         span *= 2
     spans = -(-longest // span)
     return (spans, span) if spans > 1 else (1, 0)

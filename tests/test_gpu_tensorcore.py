@@ -452,7 +452,7 @@ def test_decode_rows_beside_a_portion_cut_their_keys_into_spans_of_their_own(Hq,
         assert rel(out[starts[b]:starts[b] + n], want) < 2e-2, f"sequence {b}"
 
 
-@pytest.mark.parametrize("Hq,Hk,window", [(32, 8, None), (4, 4, 700), (8, 2, None)])
+@pytest.mark.parametrize("Hq,Hk,window", [(32, 8, None), (4, 4, 1500), (8, 2, None)])
 def test_decode_rows_on_both_sides_of_a_portion_cut_their_keys_as_on_one_side(Hq, Hk, window):
     """Decode rows first, a portion of 500 rows, then the last rows of another prompt: the same spans and the same bits as with the
     portion in front of all of them, and scratch for the tiles' rows, not for the rows that lie between them."""

@@ -1,8 +1,10 @@
-"""Which form a product takes, by sizes alone."""
+"""Which form a product or an attention takes, by sizes alone."""
+
+import types
 
 import pytest
 
-from tandemllm_b200.kernels import ops
+from tandemllm_b200.kernels import ops, tensorcore
 
 
 @pytest.mark.parametrize("M,N,K,run", [
@@ -16,3 +18,13 @@ from tandemllm_b200.kernels import ops
 def test_32_bit_products_in_runs_of_k(M, N, K, run, monkeypatch):
     monkeypatch.setattr(ops, "sm_count", lambda: 148)
     assert ops.simt_runs(M, N, K) == run
+
+
+@pytest.mark.parametrize("contexts,window,spans", [
+    ([512], 0, (1, 0)), ([600] * 2, 0, (3, 256)), ([600] * 8, 0, (1, 0)), ([1030] * 8, 0, (5, 256)), ([1500] * 23, 0, (1, 0)),
+    ([100 + 31 * i for i in range(30)], 0, (1, 0)), ([250 + 77 * i for i in range(30)], 0, (3, 1024)),
+    ([600] * 60, 0, (1, 0)), ([3000] * 60, 0, (2, 2048)), ([8192, 8000, 7000, 900], 0, (32, 256)),
+    ([201 + 185 * i for i in range(22)], 0, (4, 1024)), ([4000] * 4, 512, (1, 0)), ([4000] * 4, 2000, (16, 256)),
+    ([9000] * 148, 0, (1, 0))])                                                 # (the tiles alone fill the GPU)
+def test_decode_rows_beside_a_portion_in_spans_of_keys(contexts, window, spans):
+    assert tensorcore._row_spans(types.SimpleNamespace(sm_count=148), contexts, 8, window) == spans
