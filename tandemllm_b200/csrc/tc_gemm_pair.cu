@@ -77,7 +77,8 @@ inline int& skip_kb_for_test() {
 // FORM, gated products: EIGHTS brings gate and up rows as 2D boxes of eight, for weights that `gate_up_map` does not describe (as a
 // branch of the usual form's producer it cost a prompt of 2048 rows 3286 -> 3416 us). WIDE takes tiles of 256 outputs: a CTA brings 128
 // gate rows and the 128 up rows of the same outputs, whose two accumulators fill tensor memory, so the MMAs wait for the epilogue; a
-// stage has 48 KB for what two stages of the usual form need 64 for. Where that pays: `wide_pays`.
+// stage has 48 KB for what two stages of the usual form need 64 for (PER_SM 2: tiles of up to 128 token rows, two such CTAs an SM with two
+// stages of 40 KB and half the tensor memory each). Where that pays: `wide_pays`, `wide_pays_grouped`.
 enum Form { USUAL, EIGHTS, WIDE };
 template <bool GATED, int PER_SM, int FORM = USUAL>
 struct Smem {
@@ -85,16 +86,16 @@ struct Smem {
   static constexpr int W_TILES = FORM == WIDE ? 2 : 1;             // boxes of weight rows a stage, each with an accumulator
   static constexpr bool IN_TURN = GATED && FORM != WIDE;           // a box holds 8 gate rows and their 8 up rows in turn
   static constexpr int OUTS = IN_TURN ? ROWS / 2 : ROWS;           // outputs a CTA
-  static constexpr int CTAS = GATED ? 1 : PER_SM;                  // CTAs an SM
+  static constexpr int CTAS = GATED && FORM != WIDE ? 1 : PER_SM;  // CTAs an SM
   static constexpr int TMEM_COLS = CTAS == 2 ? 256 : 512;
   static constexpr int ACC_BUFS = TMEM_COLS / (W_TILES * TOKENS);  // accumulators (sets of them) in tensor memory
   // Epilogue warps: one a quarter of the accumulator's lanes, or two that take every other block of 16 tokens
-  static constexpr int EPI_WARPS = GATED && PER_SM == 1 ? 8 : 4;
+  static constexpr int EPI_WARPS = GATED && (PER_SM == 1 || FORM == WIDE) ? 8 : 4;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int A_BYTES = ROWS * TILE_K * 2;                // one box of weights
   static constexpr int B_BYTES = (TOKENS / 2) * TILE_K * 2;        // this CTA's half of the token rows, at most
   static constexpr int STAGE_BYTES = W_TILES * A_BYTES + B_BYTES;
-  static constexpr int STAGES = PER_SM == 2 ? (GATED ? 9 : 3) : (FORM == WIDE ? 4 : 6);
+  static constexpr int STAGES = FORM == WIDE ? 4 / PER_SM : PER_SM == 2 ? (GATED ? 9 : 3) : 6;
   static constexpr int TURN_BYTES = EPI_WARPS * 16 * 32 * 4;       // the epilogue warps' blocks
   static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */ + TURN_BYTES;
   static_assert(CTAS * TOTAL <= 227 * 1024, "the CTAs of an SM share its shared memory");
@@ -479,6 +480,16 @@ __global__ void __launch_bounds__(Smem<GATED, PER_SM, FORM>::THREADS, Smem<GATED
           ld16(taddr + S::TOKENS + c0, u);
 #pragma unroll
           for (int j = 0; j < 16; ++j) u[j] += b_up;
+          if (p.row_weight) {
+            const int block = c0 / STEP;
+            const float four = (block >> 1) == 0 ? rw[0] : ((block >> 1) == 1 ? rw[1] : ((block >> 1) == 2 ? rw[2] : rw[3]));
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float mine = __shfl_sync(0xffffffffu, four, 16 * (block & 1) + j);
+              v[j] *= mine;
+              u[j] *= mine;
+            }
+          }
           gate_all<CLAMPED, 16>(v, u, p);
         }
         __syncwarp();
@@ -622,6 +633,21 @@ static bool wide_pays(int M, int N, int K) {
   return usual >= 2 * wide && (wide == 1 || K >= 4096 || (K >= 2048 && 4LL * N * K <= 120 << 20));
 }
 
+// The same for the experts' products, whose tiles only the device knows (at most max_tiles): the longer the reduction, the more the bytes
+// count and the less the epilogue. One CTA an SM: always from a K of 5120 on; from 4096 on with many rounds and no half tile of outputs.
+// Usual and wide, us: 16 experts of 8192 x 5120, 256 rows each 707 and 659; 160 of 1536 x 5120, 307 each 1991 and 1711; 256 of 2048 x 7168, 128
+// each 3271 and 2546; 8 of 14336 x 4096, 512 each 952 and 864; 16 of 4096 x 4096, 512 each 484 and 450, but 175 each 212 and 220; 60 of 1408 x
+// 4096, 273 each 434 and 463; 32 of 1792 x 2048, 256 each 138 and 143. Few rows an expert (`per_sm` 2): from 5120 on, and from 4096 on with few
+// rounds, where two CTAs an SM end more evenly. 50 rows each: 16 of 4096 x 4096 271 and 216, 128 of 768 x 4096 343 and 293, 64 of 2048 x 6144
+// 612 and 541; 8 of 14336 x 4096 337 and 350, 128 of 1536 x 4096 523 and 535.
+static bool wide_pays_grouped(int max_tiles, int N, int K, int per_sm) {
+  const long long work = (long long)max_tiles * ceil_div(N, 2 * ROWS), pairs = sm_count() / 2;
+  if (K < 4096) return false;
+  if (per_sm == 2) return K >= 5120 || work < 4 * 2 * pairs;
+  const int rest = N % (2 * ROWS);
+  return K >= 5120 || (work >= 8 * pairs && (rest == 0 || rest > ROWS));
+}
+
 }  // namespace pair
 }  // namespace tl
 
@@ -676,7 +702,7 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
   // One box brings a tile's gate and up rows where the outputs are whole blocks of eight and the tensor whole groups; else eight rows a
   // box, sixteen boxes a stage: box rows past the outputs belong to others and their products are not stored.
   const long long per_group = tile_group ? rows_per_group : w_rows;
-  const bool wide = gated && !tile_group && per_sm == 1 && pair::wide_pays(M, N, K);
+  const bool wide = gated && (tile_group ? pair::wide_pays_grouped(max_tiles, N, K, per_sm) : per_sm == 1 && pair::wide_pays(M, N, K));
   const bool by_eights = gated && !wide && !(N % 8 == 0 && per_group >= 2 * (long long)N && w_rows % per_group == 0);
   if (gated && !wide && !by_eights) {
     if (int e = gate_up_map(W, w_rows, per_group, N, K, ldw, pair::ROWS, &tmW)) return e;
@@ -707,9 +733,11 @@ static int pair_product(const void* X, long long ldx, long long x_rows, const vo
                        : pair::launch<true, 1, float, false, pair::EIGHTS>(tmW, tmX, p, work, stream);
   }
   if (wide) {
-    if (out_dtype == TL_FP32) return pair::launch<true, 1, float, false, pair::WIDE>(tmW, tmX, p, work, stream);
-    return gated == TL_ACT_CLAMPED_SWISH ? pair::launch<true, 1, bf16, true, pair::WIDE>(tmW, tmX, p, work, stream)
-                                         : pair::launch<true, 1, bf16, false, pair::WIDE>(tmW, tmX, p, work, stream);
+#define TL_WIDE(T_, C_) \
+  (per_sm == 2 ? pair::launch<true, 2, T_, C_, pair::WIDE>(tmW, tmX, p, work, stream) : pair::launch<true, 1, T_, C_, pair::WIDE>(tmW, tmX, p, work, stream))
+    if (out_dtype == TL_FP32) return TL_WIDE(float, false);
+    return gated == TL_ACT_CLAMPED_SWISH ? TL_WIDE(bf16, true) : TL_WIDE(bf16, false);
+#undef TL_WIDE
   }
   if (gated == TL_ACT_CLAMPED_SWISH && out_dtype == TL_BF16)
     return per_sm == 2 ? pair::launch<true, 2, bf16, true>(tmW, tmX, p, work, stream)

@@ -748,6 +748,45 @@ def test_pair_product_with_the_gated_epilogue(M, H, I, act):
     assert rel(out, plain_activation(act, g) * u) < 1e-2
 
 
+@pytest.mark.parametrize("weighed", [False, True])
+@pytest.mark.parametrize("act", ["silu", "clamped_swish"])
+@pytest.mark.parametrize("tile", [256, 128])
+@pytest.mark.parametrize("R,E,I,H", [(600, 3, 200, 5120), (300, 5, 67, 5128), (150, 5, 256, 4096), (9000, 8, 2048, 4096)])
+def test_gated_pair_product_of_long_reductions_over_a_routing_plan(R, E, I, H, tile, act, weighed):
+    """The forms with gate and up accumulators side by side (a K of 5120 and more; of 4096 by rounds, both sides): the same bits as with
+    one expert's rows alone as a dense product against 128 outputs of it, which never takes them."""
+    from tandemllm_b200.kernels import ops
+    impl, rt = tc()
+    code = ops.activation_code(act)
+    ids = (torch.arange(R, dtype=torch.int32) ** 2 % E).view(R, 1).to(DEV)
+    plan = ops.MoePlan(R, E, tile, torch.device(DEV)).build(ids)
+    order = plan.sorted_pairs[:R].long()
+    g = torch.Generator(device=DEV).manual_seed(I + H)
+    x = torch.randn(R, H, device=DEV, generator=g).to(torch.bfloat16)[order]
+    w = (torch.randn(E, 2 * I, H, device=DEV, generator=g) * 0.02).to(torch.bfloat16)
+    wts = 2.0 ** torch.randint(-1, 2, (R, 1), device=DEV, generator=g).float()
+    out = torch.full((R, I), float("nan"), dtype=torch.bfloat16, device=DEV)
+    impl.gemm_pair(x, w.view(-1, H), None, out, rows_per_group=2 * I, plan=plan, gated=code, n_out=I, weights=wts if weighed else None)
+    torch.cuda.synchronize()
+    assert int(rt.status) == 0 and bool(torch.isfinite(out).all())
+    expert, n = ids.flatten()[order].long(), min(I, 128)
+    # (a weight that is a power of two may stand in front of the products: the same sums, scaled)
+    rows = x * wts[order].to(torch.bfloat16) if weighed else x
+    for e in range(E):
+        mine = rows[expert == e].contiguous()
+        if not mine.shape[0]:
+            continue
+        for at in {0, I - n}:
+            alone = torch.empty(mine.shape[0], n, dtype=torch.bfloat16, device=DEV)
+            impl.gemm_pair(mine, torch.cat([w[e, at:at + n], w[e, I + at:I + at + n]]), None, alone, gated=code, n_out=n)
+            assert torch.equal(alone, out[expert == e][:, at:at + n]), (e, at)
+    full = x[:40].double() @ w[expert[0]].double().T if not weighed else None
+    if full is not None and act == "silu":
+        same = expert[:40] == expert[0]
+        want = torch.nn.functional.silu(full[:, :I]) * full[:, I:]
+        assert float((out[:40][same].double() - want[same]).abs().max() / want[same].abs().max()) < 1e-2
+
+
 @pytest.mark.parametrize("act,dtype", [("silu", "bfloat16"), ("relu2", "bfloat16"), ("silu", "float32"), ("clamped_swish", "bfloat16")])
 @pytest.mark.parametrize("M,H,I", [(40, 72, 9480), (300, 136, 4744), (300, 64, 9472), (257, 2048, 9472)])
 def test_gated_pair_product_in_tiles_of_128_and_of_256_outputs(M, H, I, act, dtype):
